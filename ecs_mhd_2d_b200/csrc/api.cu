@@ -93,6 +93,7 @@ int ecs_ctx_create(int n, int dtype, const ecs_params* params, int max_batch, ec
   c->n = n; c->dtype = dtype; c->max_batch = max_batch; c->g = make_geom(n);
   c->nu = params->nu; c->eta = params->eta; c->b0x = params->b0x; c->b0y = params->b0y;
   if (const char* v = getenv("ECS_PDL")) c->pdl = atoi(v) != 0 ? 1 : 0;
+  if (const char* v = getenv("ECS_GROUP_MINB")) c->group_minb = atoi(v);
   if (const char* v = getenv("ECS_TGROUPS")) c->tgroups = std::max(1, std::min(ecs_ctx::MAXG, atoi(v)));
   if (const char* v = getenv("ECS_ROWTAN_XT")) c->rowtan_xt = atoi(v) == 4 ? 4 : 8;
   if (const char* v = getenv("ECS_PDL_MINB")) c->pdl_minb = std::max(1, atoi(v));

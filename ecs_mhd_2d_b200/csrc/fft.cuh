@@ -1,14 +1,14 @@
-// Warp-level FFTs of length N in {64, 128, 256} (one transform per warp).
+// Transforms of length N in {64, 128, 256}, two layouts.
 //
-// Data distribution: lane l holds E = N/32 complex values v[j] at "positions"
-// e = l + 32*j.
+// FP32: one transform per warp.  Lane l holds E = N/32 complex values v[j] at
+// "positions" e = l + 32*j.
 //
 //  * fft_dif : natural-order input  -> permuted output (lane l, register j holds X[spec_pos<N>(l, j)])
 //  * fft_dit : permuted input       -> natural-order output
 //
 // Both are unnormalised.  FWD uses exp(-2 pi i k/N), INV uses exp(+2 pi i k/N).
 //
-// Algorithm.  One radix-E pass over the register digits (the length-E DFT over
+// One radix-E pass over the register digits (the length-E DFT over
 // j, then the twiddles W_N^{l k1}), after which every register digit is a
 // finished frequency digit and the remaining 32-point DFTs run over the lane
 // digits.  Those are five "half-swap" radix-2 stages: stage t (lane bit t, span
@@ -30,9 +30,28 @@
 //   s_tw[tw_off(N, r) + i] = tw[i r],  i < N / (2 r),  tw_off(N, r) = N - N / r,
 // so that the lanes of a stage read consecutive entries, followed by the
 // radix-E pass's table s_tw[N + (k1-1)*32 + l] = W_N^{l k1}, k1 = 1..E-1.
+//
+// FP64 at N = 64 and 128: G = 32 / L transforms per warp, each on a group of L lanes
+// with E = N / L values per lane, natural order in and out (x[l + L j] in register
+// j).  Register passes with one exchange between them: at N = 64 (L = 8, E = 8)
+// radix 8, twiddles, the transposition of the values through the group's N-entry
+// shared buffer, radix 8; at N = 128 radix 16 (4 x 4), twiddles, transposition,
+// radix 8, either on 8 lanes of 16 values (the radix 16 in registers) or on 16 lanes
+// of 8 values (its last butterflies across lanes l, l + 8 after a half swap); the two
+// do the same operations in the same order and agree bit for bit.  The half-swap form above spends
+// most of its issue slots on selects and shuffles (a 128-point transform: 245
+// instructions per warp, 100 of them FP64); this form has few of either, 8 to 16
+// shared-memory accesses per lane and transform, and 83 to 92 FP64 instructions, so
+// that it runs at the FP64 and shared-memory rate of the SM instead of its issue
+// rate.  Measured, cycles per transform and SM at 16 warps: N = 128 93 -> 49 (8 lanes),
+// N = 64 47 -> 25; one warp alone takes 913 cycles for four transforms of 128 (1088
+// for two before).  The buffer is swizzled (entry (k, l) at k L + (l ^ (k mod L))):
+// eight lanes' 16-byte accesses fall on different banks in both directions.
 #pragma once
 
 #include "common.cuh"
+
+#include <math.h>
 
 namespace ecs {
 
@@ -40,11 +59,6 @@ __host__ __device__ constexpr int tw_first(int N) { return (N / 32 - 1) * 32; }
 // Shared-memory twiddle entries and the offset of the stride-r sub-table.
 __host__ __device__ constexpr int tw_smem(int N) { return N + tw_first(N); }
 __host__ __device__ constexpr int tw_off(int N, int r) { return N - N / r; }
-// Shared-memory region of the transforms of a CTA of W warps (the tables: the
-// transforms need no per-warp buffers), which every kernel that calls a
-// transform reserves at its start.
-__host__ __device__ constexpr int fft_smem(int N, int /*warps*/) { return tw_smem(N); }
-
 template <typename R, bool INV>
 __device__ __forceinline__ cplx<R> twid(const cplx<R>* __restrict__ tw, int idx) {
   cplx<R> w = tw[idx];
@@ -271,12 +285,224 @@ __host__ __device__ inline void twiddle_image(const C* half, C* img) {
   }
 }
 
-// Copy of the twiddle image into shared memory (cp.async: global -> shared
-// without a register round trip); each thread waits for its own copies and the
-// caller's __syncthreads makes the table visible.
+// ---------------------------------------------------------------------------
+// Group transforms (FP64)
+// ---------------------------------------------------------------------------
+
+// a W with W = c - i s (forward) or its conjugate (inverse).
+template <typename R, bool INV>
+__device__ __forceinline__ cplx<R> mul_cs(cplx<R> a, R c, R s) { return cmul(a, mk<R>(c, INV ? s : -s)); }
+
+// N = 128 on 16 lanes: lane l holds x[l + 16 j'], that is x[a + 8 j] with a = l mod 8
+// and j = h + 2 j', h = l / 8, so that the butterflies (j, j + 4, j + 8, j + 12) of dft16's
+// first pass lie within a lane (j = h and h + 2), and so do the first sums of its second
+// pass (j = 0, 2 on lanes h = 0; 1, 3 on lanes h = 1); its last sums pair lanes l and l ^ 8,
+// which swap half their values for them.  The operations are dft16's, in its order.
+// Then the transposition hands lane k1 the eight values of its output digit.
+template <typename R, bool INV, bool ZMID>
+__device__ __forceinline__ void dft16_lanes(cplx<R> (&x)[8], int l) {
+  const R c1 = R(0.92387953251128675612818318939678829), s1 = R(0.38268343236508977172845998403039887);
+  const bool h = (l >> 3) & 1;
+  // x[0], x[2], x[4], x[6]: j = h + 0, 4, 8, 12;  x[1], x[3], x[5], x[7]: j = h + 2, 6, 10, 14.
+  // ZMID (inputs 48..79 of 128 are zero, j = 6..9): x[3] and x[4].
+  if constexpr (ZMID) {
+    {
+      const cplx<R> s13 = cadd(x[2], x[6]), d13 = mul_mi<R, INV>(csub(x[2], x[6])), a = x[0];
+      x[0] = cadd(a, s13); x[2] = cadd(a, d13); x[4] = csub(a, s13); x[6] = csub(a, d13);
+    }
+    {
+      const cplx<R> s02 = cadd(x[1], x[5]), d02 = csub(x[1], x[5]), b = x[7], ib = mul_mi<R, INV>(b);
+      x[1] = cadd(s02, b); x[3] = csub(d02, ib); x[5] = csub(s02, b); x[7] = cadd(d02, ib);
+    }
+  } else {
+    dft4<R, INV>(x[0], x[2], x[4], x[6]);
+    dft4<R, INV>(x[1], x[3], x[5], x[7]);
+  }
+  // x[2 k] = A_h[k], x[2 k + 1] = A_{h+2}[k]; times W_16^{j k}
+  if (h) {
+    x[2] = mul_cs<R, INV>(x[2], c1, s1);
+    x[4] = mul_w8<R, INV>(x[4]);
+    x[6] = mul_cs<R, INV>(x[6], s1, c1);
+    x[3] = mul_cs<R, INV>(x[3], s1, c1);
+    x[5] = mul_mi<R, INV>(mul_w8<R, INV>(x[5]));
+    x[7] = mul_cs<R, INV>(x[7], -c1, -s1);
+  } else {
+    x[3] = mul_w8<R, INV>(x[3]);
+    x[5] = mul_mi<R, INV>(x[5]);
+    x[7] = mul_mi<R, INV>(mul_w8<R, INV>(x[7]));
+  }
+  // s = x[2k] + x[2k+1], d = x[2k] - x[2k+1] (lanes h = 1: times W_4): s02, d02 / s13, d13 of output k
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const cplx<R> s = cadd(x[2 * k], x[2 * k + 1]), d = csub(x[2 * k], x[2 * k + 1]), e = mul_mi<R, INV>(d);
+    x[2 * k] = s;
+    x[2 * k + 1] = h ? e : d;
+  }
+  // lanes h = 0 take k = 0, 1 of both, lanes h = 1 k = 2, 3
+  cplx<R> y[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {   // i = 2 (k mod 2) + (s or d)
+    const cplx<R> keep = h ? x[4 + i] : x[i], send = h ? x[i] : x[4 + i];
+    const cplx<R> recv = shfl_xor_c<R>(send, 8);
+    y[i] = cadd(keep, recv);
+    const cplx<R> t = csub(keep, recv);                       // s02 - s13 on lanes h = 0, its negative on h = 1
+    y[4 + i] = h ? mk<R>(-t.x, -t.y) : t;
+  }
+  // X[k + 4 m]: m = 0: s02 + s13, 1: d02 + d13, 2: s02 - s13, 3: d02 - d13; k = 2 h + (i / 2)
+  // register order: x[m + 4 kk], kk = k - 2 h
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk) {
+    x[4 * kk] = y[2 * kk]; x[4 * kk + 1] = y[2 * kk + 1]; x[4 * kk + 2] = y[4 + 2 * kk]; x[4 * kk + 3] = y[4 + 2 * kk + 1];
+  }
+}
+
+template <typename R, bool INV, bool ZBOX>
+__device__ __forceinline__ void fft_group16(cplx<R> (&x)[8], const cplx<R>* tw, cplx<R>* xb, int l) {
+  dft16_lanes<R, INV, ZBOX>(x, l);
+  const int a = l & 7, h2 = (l >> 3) * 2;
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {   // output digit k1 = 2 h + kk + 4 m; k1 = 0 has no twiddle
+      const int k1 = h2 + kk + 4 * m;
+      if (kk == 0 && m == 0) {
+        const cplx<R> t = cmul(x[0], twid<R, INV>(tw, k1 * 8 + a));
+        if (h2) x[0] = t;
+      } else {
+        x[4 * kk + m] = cmul(x[4 * kk + m], twid<R, INV>(tw, k1 * 8 + a));
+      }
+    }
+  __syncwarp();   // the group's reads of the previous exchange are done
+#pragma unroll
+  for (int kk = 0; kk < 2; ++kk)
+#pragma unroll
+    for (int m = 0; m < 4; ++m) {
+      const int k1 = h2 + kk + 4 * m;
+      xb[k1 * 8 + (a ^ (k1 & 7))] = x[4 * kk + m];
+    }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = xb[l * 8 + (i ^ (l & 7))];
+  dft_reg<R, INV, 8>(x);
+}
+
+// ---------------------------------------------------------------------------
+// The layout a kernel works in: L lanes and E values per transform, G transforms per
+// warp, TW table entries in shared memory, XB exchange entries per transform, the
+// position pos(l, j) of a spectrum along the transformed direction, and none(j):
+// element j of every lane lies outside the box.
+//
+//   warp layout   a warp per transform, exchanges by shuffles, and the two transforms
+//                 of a pass in lockstep: the shorter chain of dependent operations.
+//   group layout  (FP64 at N = 128) two transforms of 16 lanes per warp with 8 values
+//                 per lane and one exchange through shared memory: 30% fewer
+//                 instructions per transform, but half as many warps for the same
+//                 columns.  The column passes of batched tangents use it.
+// ---------------------------------------------------------------------------
+template <typename R_, int N_, bool GROUP_ = false> struct Xf {
+  static_assert(!GROUP_ || (sizeof(R_) == 8 && N_ == 128), "group layout: FP64, N = 128");
+  using R = R_;
+  static constexpr int N = N_;
+  static constexpr bool GROUP = GROUP_;
+  static constexpr int L = GROUP ? 16 : 32, E = N / L, G = 32 / L;
+  static constexpr int TW = GROUP ? N : tw_smem(N);
+  static constexpr int XB = GROUP ? N : 0;
+  static constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+  // A column pass brings the operands of its algebra through shared memory (see Operands).
+  static constexpr bool STAGED = !GROUP && N <= 128;
+  __device__ static __forceinline__ int pos(int l, int j) {
+    if constexpr (GROUP) return l + L * j;
+    else return spec_pos<N>(l, j);
+  }
+  __host__ __device__ static constexpr bool none(int j) { return GROUP && L * j > KMAX && L * j + L - 1 < N - KMAX; }
+  // Shared entries of the tables and of the exchange buffers of W warps.
+  __host__ __device__ static constexpr int smem(int W) { return TW + W * G * XB; }
+
+  const cplx<R>* tw;   // tables (shared memory)
+  cplx<R>* xb;         // the lane's exchange buffer
+  int l;               // lane within the transform
+
+  // `s` is the start of the shared region (tables, then the buffers); `warp` the
+  // warp's index among those that transform.
+  __device__ __forceinline__ Xf(cplx<R>* s, int warp) {
+    const int lane = threadIdx.x & 31;
+    tw = s; l = lane & (L - 1);
+    xb = s + TW + (warp * G + lane / L) * XB;
+  }
+  // kx and box slot (-1 outside the box) of the lane's element j.
+  __device__ __forceinline__ R kx(int j) const {
+    if constexpr (GROUP) return (R)l + R(j < E / 2 ? L * j : L * j - N);
+    else return (R)pos_to_k(spec_pos<N>(l, j), N);
+  }
+  __device__ __forceinline__ int slot(int j) const {
+    if constexpr (GROUP) {
+      const int p = l + L * j;
+      if (j < E / 2) return p <= KMAX ? p : -1;
+      return p >= N - KMAX ? p - N + M : -1;
+    } else {
+      return pos_to_slot(spec_pos<N>(l, j), N, KMAX, M);
+    }
+  }
+  // Natural order -> spectral positions (column forward, row inverse) ...
+  template <bool INV, bool ZBOX = false> __device__ __forceinline__ void to_spec(cplx<R> (&v)[E]) const {
+    if constexpr (GROUP) fft_group16<R, INV, ZBOX>(v, tw, xb, l);
+    else fft_dif<R, N, INV>(v, tw, l);
+  }
+  // ... and back.  ZBOX: the input vanishes outside the box.
+  template <bool INV, bool ZBOX = false> __device__ __forceinline__ void from_spec(cplx<R> (&v)[E]) const {
+    if constexpr (GROUP) fft_group16<R, INV, ZBOX>(v, tw, xb, l);
+    else fft_dit<R, N, INV>(v, tw, l);
+  }
+  // Two transforms in lockstep (warp layout).
+  template <bool INV> __device__ __forceinline__ void to_spec2(cplx<R> (&a)[E], cplx<R> (&b)[E]) const {
+    fft_dif2<R, N, INV>(a, b, tw, l);
+  }
+  template <bool INV> __device__ __forceinline__ void from_spec2(cplx<R> (&a)[E], cplx<R> (&b)[E]) const {
+    fft_dit2<R, N, INV>(a, b, tw, l);
+  }
+};
+
+// Device table of (R, N): the shared entries of the warp layout, the uncurling
+// multipliers (ky/k^2, -kx/k^2) / n^2 of every box mode [K][M] (mhd_jax.py:83-90; zero
+// at (0,0); n^2 is a power of two, so the scale is exact), and the shared entries of the
+// group layout where there is one.  The column passes divided for the multipliers at
+// every mode, two FP64 divisions or about 40 instructions per mode and pass against one
+// 16-byte load.  Built on the host when a context is created.
+template <typename R, int N> struct XfTable {
+  static constexpr bool GROUPS = sizeof(R) == 8 && N == 128;
+  static constexpr int mu = tw_smem(N), group = mu + Xf<R, N>::K * Xf<R, N>::M, size = group + (GROUPS ? N : 0);
+};
 template <typename R, int N>
-__device__ __forceinline__ void load_twiddles(cplx<R>* s_tw, const cplx<R>* __restrict__ g_img) {
-  for (int i = threadIdx.x; i < tw_smem(N); i += blockDim.x) cp_async_c<R>(s_tw + i, g_img + i);
+inline void xf_table(cplx<R>* img) {
+  using T = XfTable<R, N>;
+  using X = Xf<R, N>;
+  const long double twopi = 6.283185307179586476925286766559005768L;
+  auto w = [&](int k) {
+    const long double a = twopi * (long double)(k % N) / (long double)N;
+    return mk<R>((R)cosl(a), (R)(-sinl(a)));
+  };
+  cplx<R> half[N / 2];
+  for (int k = 0; k < N / 2; ++k) half[k] = w(k);
+  twiddle_image<cplx<R>, N>(half, img);
+  const R inv_n2 = R(1) / (R(N) * R(N));
+  for (int ky = 0; ky < X::K; ++ky)
+    for (int s = 0; s < X::M; ++s) {
+      const R rkx = (R)slot_to_kx(s, X::KMAX, X::M), rky = (R)ky, ksq = rkx * rkx + rky * rky;
+      img[T::mu + ky * X::M + s] = ksq == R(0) ? mk<R>(R(0), R(0)) : mk<R>(rky / ksq * inv_n2, (-rkx) / ksq * inv_n2);
+    }
+  if (T::GROUPS)   // W_N^{l k} at k 8 + l, l < 8
+    for (int k = 0; k < N / 8; ++k)
+      for (int l = 0; l < 8; ++l) img[T::group + k * 8 + l] = w(k * l);
+}
+
+// Copy of the layout's tables into shared memory (cp.async: global -> shared without a
+// register round trip); each thread waits for its own copies and the caller's
+// __syncthreads makes them visible.
+template <class X>
+__device__ __forceinline__ void load_tables(cplx<typename X::R>* s, const cplx<typename X::R>* __restrict__ g) {
+  using R = typename X::R;
+  if (X::GROUP) g += XfTable<R, X::N>::group;
+  for (int i = threadIdx.x; i < X::TW; i += blockDim.x) cp_async_c<R>(s + i, g + i);
   asm volatile("cp.async.wait_all;\n" ::: "memory");
 }
 

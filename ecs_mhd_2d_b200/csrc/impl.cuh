@@ -31,16 +31,39 @@
 namespace ecs {
 
 constexpr int XT = 8;
-constexpr int COLWARPS = 4;
 
-// Row kernels with NG (or 3 adjoint) input and NH (or NHA adjoint) output tiles: 7 tiles of K x (X+1).
-template <typename R, int N, int X = XT> size_t smem_row_rhs() { return (fft_smem(N, X) + 7 * Geomc<N>::K * (X + 1)) * sizeof(cplx<R>); }
-// Small batches use 2-row tiles: 4x more CTAs for the same rows.
+// Small batches use 2-row tiles: more CTAs for the same rows.
 constexpr int XTS = 2;
 template <int N> bool small_rows(int B) { return (long)B * (N / XT) < 2L * 148; }
-template <typename R, int N> size_t smem_row_tan2() { return (fft_smem(N, XT) + 11 * Geomc<N>::K * (XT + 1)) * sizeof(cplx<R>); }
-template <typename R, int N> size_t smem_row_phys() { return (fft_smem(N, XT) + NG * Geomc<N>::K * (XT + 1)) * sizeof(cplx<R>); }
-template <typename R, int N, int X = XT> size_t smem_row_2f() { return (fft_smem(N, X) + 2 * Geomc<N>::K * (X + 1)) * sizeof(cplx<R>); }
+
+// Shape of a row or column launch in layout F.
+struct Shape { dim3 grid, block; size_t smem; };
+// A row pass over B states with X-row tiles of `fields` fields in shared memory (an output
+// tile takes the place of its input's).
+template <class F, int X = XT> Shape row_shape(int B, int fields) {
+  return {dim3(B * (F::N / X)), dim3(X * F::L), (F::smem(X / F::G) + (size_t)fields * F::K * (X + 1)) * sizeof(cplx<typename F::R>)};
+}
+// A column pass over B states.
+template <class F> Shape col_shape(int B) {
+  return {dim3((B * col_units<F>() + COLWARPS - 1) / COLWARPS), dim3(COLWARPS * 32), 0};
+}
+inline int box_grid(int cols) { return (cols + COLWARPS - 1) / COLWARPS; }
+
+// Calls go(layout, its GROUP flag as a constant) for a tangent column pass of batch B:
+// the group layout (FP64 at n = 128) from 16 tangents on.  It needs 30% fewer
+// instructions per transform and holds half of a column's operands at a time in registers
+// instead of all in shared memory, but puts half as many warps on the same columns.
+// Measured per launch at batch 64, warp -> group: stage A 18.5 -> 15.1 us, C 32.3 -> 22.9,
+// D 22.5 -> 19.7, E and A 24.2 -> 20.9, B 17.3 -> 17.8; JVPs of T = 0.3, per-pass
+// launches: batch 4 4.1 -> 3.8 ms, 16 4.5 -> 4.0, 32 5.3 -> 4.5, 48 7.2 -> 6.7 (batch 1
+// 2.37 -> 2.48).  Below 16 the cluster-resident sweep runs (chain_batch), in the warp
+// layout; its results are those of the warp layout's passes bit for bit.
+template <typename R, int N, typename F> void with_layout(const ecs_ctx* c, int B, F&& go) {
+  if constexpr (sizeof(R) == 8 && N == 128) {
+    if (B >= c->group_minb) { go((Xf<R, N, true>*)nullptr, std::true_type{}); return; }
+  }
+  go((Xf<R, N>*)nullptr, std::false_type{});
+}
 
 // Launch a stepping kernel of batch B; with c->pdl set, with programmatic
 // stream serialization (the kernel waits on its predecessor itself, see
@@ -61,6 +84,11 @@ inline void launch_step(ecs_ctx* c, int B, void (*k)(P...), dim3 grid, dim3 bloc
   cfg.attrs = at; cfg.numAttrs = (c->pdl && B >= c->pdl_minb && !plain) ? 1 : 0;
   ++c->launches;
   cudaLaunchKernelEx(&cfg, k, args...);
+}
+
+template <typename... P, typename... A>
+inline void launch_step(ecs_ctx* c, int B, void (*k)(P...), const Shape& sh, cudaStream_t s, A... args) {
+  launch_step(c, B, k, sh.grid, sh.block, sh.smem, s, args...);
 }
 
 // launch_step for a kernel launched as clusters of `cl` CTAs along x.
@@ -100,15 +128,15 @@ int configure_chain() {
     st |= (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (chain_cl<N, W>() > 8) st |= (int)cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   };
-  attrs(k_tan_chain<R, N, W, false, false>, chain_smem<R, N, W, false, false>());
-  attrs(k_tan_chain<R, N, W, true, false>, chain_smem<R, N, W, true, false>());
+  attrs(k_tan_chain<R, N, W, false, false>, TanChainSmem<R, N, W, false, false>::bytes);
+  attrs(k_tan_chain<R, N, W, true, false>, TanChainSmem<R, N, W, true, false>::bytes);
   if constexpr (W == 8) {   // tangent slots in shared memory: the 8-warp shape only (smem)
-    attrs(k_tan_chain<R, N, W, false, true>, chain_smem<R, N, W, false, true>());
-    attrs(k_tan_chain<R, N, W, true, true>, chain_smem<R, N, W, true, true>());
+    attrs(k_tan_chain<R, N, W, false, true>, TanChainSmem<R, N, W, false, true>::bytes);
+    attrs(k_tan_chain<R, N, W, true, true>, TanChainSmem<R, N, W, true, true>::bytes);
   }
-  attrs(k_rk43_chain<R, N, W>, rk43_chain_smem<R, N, W>());
-  attrs(k_rk4_chain<R, N, W, false>, rk4_chain_smem<R, N, W, false>());
-  attrs(k_rk4_chain<R, N, W, true>, rk4_chain_smem<R, N, W, true>());
+  attrs(k_rk43_chain<R, N, W>, Rk43ChainSmem<R, N, W>::bytes);
+  attrs(k_rk4_chain<R, N, W, false>, Rk4ChainSmem<R, N, W, false>::bytes);
+  attrs(k_rk4_chain<R, N, W, true>, Rk4ChainSmem<R, N, W, true>::bytes);
   return st;
 }
 
@@ -118,7 +146,7 @@ template <typename R, int N, int W>
 int chain_clusters() {
   constexpr bool DSH = W == 8;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(chain_cl<N, W>()); cfg.blockDim = dim3(W * 32); cfg.dynamicSmemBytes = chain_smem<R, N, W, true, DSH>();
+  cfg.gridDim = dim3(chain_cl<N, W>()); cfg.blockDim = dim3(W * 32); cfg.dynamicSmemBytes = TanChainSmem<R, N, W, true, DSH>::bytes;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
   at[0].val.clusterDim.x = (unsigned)chain_cl<N, W>(); at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
@@ -134,20 +162,18 @@ int chain_clusters() {
 template <typename R, int N>
 int configure_kernels(ecs_ctx* c) {
   int st = ECS_OK;
-  st |= (int)cudaFuncSetAttribute(k_row_rhs<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_to_box<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_2f<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_from_box<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_2f<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_err<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_2f<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_phys<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_phys<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_tan<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_adj<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_tan2<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_tan2<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_adj2<R, N, XT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N>());
-  st |= (int)cudaFuncSetAttribute(k_row_rhs<R, N, XTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N, XTS>());
-  st |= (int)cudaFuncSetAttribute(k_row_err<R, N, XTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_2f<R, N, XTS>());
-  st |= (int)cudaFuncSetAttribute(k_row_tan<R, N, XTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N, XTS>());
-  st |= (int)cudaFuncSetAttribute(k_row_tan<R, N, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N, 4>());
-  st |= (int)cudaFuncSetAttribute(k_row_adj<R, N, XTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_row_rhs<R, N, XTS>());
+  auto smem = [&](auto* k, size_t bytes) {
+    st |= (int)cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  };
+  using X = Xf<R, N>;
+  auto rows = [&](auto* k, int fields) { smem(k, row_shape<X>(1, fields).smem); };
+  auto rows_s = [&](auto* k, int fields) { smem(k, row_shape<X, XTS>(1, fields).smem); };
+  rows(k_row_to_box<R, N, XT>, 2); rows(k_row_from_box<R, N, XT>, 2); rows(k_row_err<R, N, XT>, 2);
+  rows(k_row_phys<R, N, XT>, NG); rows(k_row_rhs<R, N, XT>, NG); rows(k_row_tan<R, N, XT>, NG);
+  rows(k_row_adj<R, N, XT>, NHA); rows(k_row_tan2<R, N, XT>, 2 * NG); rows(k_row_adj2<R, N, XT>, NHA);
+  rows_s(k_row_rhs<R, N, XTS>, NG); rows_s(k_row_err<R, N, XTS>, 2); rows_s(k_row_tan<R, N, XTS>, NG);
+  rows_s(k_row_adj<R, N, XTS>, NHA);
+  smem(k_row_tan<R, N, 4>, row_shape<X, 4>(1, NG).smem);
   if constexpr (N <= 128) {
     st |= configure_chain<R, N, 8>();
     st |= configure_chain<R, N, 16>();
@@ -167,7 +193,7 @@ int configure_kernels(ecs_ctx* c) {
 template <typename R, int N>
 void launch_row_to_box(ecs_ctx* c, const R* fields, cplx<R>* H, int B, cudaStream_t s) {
   RowFwdParams<R> p; p.fields = fields; p.H = H; p.tw = (const cplx<R>*)c->tw; p.B = B;
-  ++c->launches; k_row_to_box<R, N, XT><<<B * (N / XT), XT * 32, smem_row_2f<R, N>(), s>>>(p);
+  ++c->launches; { const Shape sh = row_shape<Xf<R, N>>(B, 2); k_row_to_box<R, N, XT><<<sh.grid, sh.block, sh.smem, s>>>(p); }
 }
 
 template <typename R, int N>
@@ -175,7 +201,7 @@ void launch_col_to_box(ecs_ctx* c, const cplx<R>* H, cplx<R>* V, int B, int nf, 
   ColBoxParams<R> p; p.H = H; p.V = V; p.tw = (const cplx<R>*)c->tw; p.B = B; p.nf = nf;
   p.vstride = vstride > 0 ? vstride : (long)nf * Geomc<N>::K * Geomc<N>::M;
   const int cols = B * nf * Geomc<N>::K;
-  ++c->launches; k_col_to_box<R, N><<<(cols + COLWARPS - 1) / COLWARPS, COLWARPS * 32, 0, s>>>(p);
+  ++c->launches; k_col_to_box<R, N><<<box_grid(cols), COLWARPS * 32, 0, s>>>(p);
 }
 
 template <typename R, int N>
@@ -185,7 +211,7 @@ void launch_col_from_box(ecs_ctx* c, const cplx<R>* V, cplx<R>* G2, int B, const
   p.sy = (ny * 2 * M_PI) / 8;   // symmetry.py:11 s = (n*2*pi)/8
   p.odd = (ny % 2 + 2) % 2 == 1; p.rot = rot; p.use_sym = use_sym; p.mult_ikx = mult_ikx; p.B = B;
   const int cols = B * 2 * Geomc<N>::K;
-  ++c->launches; k_col_from_box<R, N><<<(cols + COLWARPS - 1) / COLWARPS, COLWARPS * 32, 0, s>>>(p);
+  ++c->launches; k_col_from_box<R, N><<<box_grid(cols), COLWARPS * 32, 0, s>>>(p);
 }
 
 template <typename R, int N>
@@ -193,7 +219,7 @@ void launch_row_from_box(ecs_ctx* c, const cplx<R>* G2, R* out, const R* base, d
                          cudaStream_t s) {
   RowFromBoxParams<R> p; p.G = G2; p.out = out; p.base = base; p.rowsq = rowsq; p.tw = (const cplx<R>*)c->tw;
   p.B = B; p.mode = mode;
-  ++c->launches; k_row_from_box<R, N, XT><<<B * (N / XT), XT * 32, smem_row_2f<R, N>(), s>>>(p);
+  ++c->launches; { const Shape sh = row_shape<Xf<R, N>>(B, 2); k_row_from_box<R, N, XT><<<sh.grid, sh.block, sh.smem, s>>>(p); }
 }
 
 template <typename R, int N>
@@ -205,15 +231,14 @@ void launch_col_rk4(ecs_ctx* c, int B, int stage, int produce, int diss, cudaStr
   p.fhat = (const cplx<R>*)c->fhat; p.tw = (const cplx<R>*)c->tw; p.nu = (R)c->nu; p.eta = (R)c->eta;
   p.B = B; p.stage = stage; p.produce = produce; p.diss = diss; p.rec = rec; p.rec_bstride = rec_bstride;
   p.use_done = use_done;
-  const int cols = B * Geomc<N>::K * 2;   // one warp per (batch, ky, channel)
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
+  const Shape sh = col_shape<Xf<R, N>>(B);
   switch (stage) {
-    case COL_START: launch_step(c, B, k_col_rk4<R, N, COL_START>, g, bl, 0, s, p); break;
-    case COL_RK4_S1: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S1>, g, bl, 0, s, p); break;
-    case COL_RK4_S2: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S2>, g, bl, 0, s, p); break;
-    case COL_RK4_S3: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S3>, g, bl, 0, s, p); break;
-    case COL_RK4_S4: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S4>, g, bl, 0, s, p); break;
-    default: launch_step(c, B, k_col_rk4<R, N, COL_PLAIN>, g, bl, 0, s, p); break;
+    case COL_START: launch_step(c, B, k_col_rk4<R, N, COL_START>, sh, s, p); break;
+    case COL_RK4_S1: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S1>, sh, s, p); break;
+    case COL_RK4_S2: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S2>, sh, s, p); break;
+    case COL_RK4_S3: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S3>, sh, s, p); break;
+    case COL_RK4_S4: launch_step(c, B, k_col_rk4<R, N, COL_RK4_S4>, sh, s, p); break;
+    default: launch_step(c, B, k_col_rk4<R, N, COL_PLAIN>, sh, s, p); break;
   }
 }
 
@@ -223,8 +248,8 @@ void launch_row_rhs(ecs_ctx* c, int B, cudaStream_t s, const StepCtl* ctl = null
   RowParams<R> p{}; p.G = (const cplx<R>*)c->G; p.H = (cplx<R>*)c->H; p.tw = (const cplx<R>*)c->tw; p.ctl = ctl;
   p.phys = phys; p.phys_bstride = phys_bstride;
   p.b0x = (R)c->b0x; p.b0y = (R)c->b0y; p.B = B;
-  if (small_rows<N>(B)) launch_step(c, B, k_row_rhs<R, N, XTS>, dim3(B * (N / XTS)), dim3(XTS * 32), smem_row_rhs<R, N, XTS>(), s, p);
-  else launch_step(c, B, k_row_rhs<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_rhs<R, N>(), s, p);
+  if (small_rows<N>(B)) { launch_step(c, B, k_row_rhs<R, N, XTS>, row_shape<Xf<R, N>, XTS>(B, NG), s, p); return; }
+  launch_step(c, B, k_row_rhs<R, N, XT>, row_shape<Xf<R, N>>(B, NG), s, p);
 }
 
 template <typename R, int N>
@@ -233,16 +258,15 @@ void launch_col_rk43(ecs_ctx* c, int B, int stage, cudaStream_t s, cplx<R>* rec 
   p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.S = (cplx<R>*)c->S43; p.ctl = c->ctl;
   p.fhat = (const cplx<R>*)c->fhat; p.tw = (const cplx<R>*)c->tw; p.rec = rec; p.cap = cap;
   p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.stage = stage;
-  const int cols = B * Geomc<N>::K * 2;   // one warp per (batch, ky, channel)
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
+  const Shape sh = col_shape<Xf<R, N>>(B);
   switch (stage) {
-    case R43_START: launch_step(c, B, k_col_rk43<R, N, R43_START>, g, bl, 0, s, p); break;
-    case R43_INIT: launch_step(c, B, k_col_rk43<R, N, R43_INIT>, g, bl, 0, s, p); break;
-    case R43_A: launch_step(c, B, k_col_rk43<R, N, R43_A>, g, bl, 0, s, p); break;
-    case R43_B: launch_step(c, B, k_col_rk43<R, N, R43_B>, g, bl, 0, s, p); break;
-    case R43_C: launch_step(c, B, k_col_rk43<R, N, R43_C>, g, bl, 0, s, p); break;
-    case R43_D: launch_step(c, B, k_col_rk43<R, N, R43_D>, g, bl, 0, s, p); break;
-    default: launch_step(c, B, k_col_rk43<R, N, R43_E>, g, bl, 0, s, p); break;
+    case R43_START: launch_step(c, B, k_col_rk43<R, N, R43_START>, sh, s, p); break;
+    case R43_INIT: launch_step(c, B, k_col_rk43<R, N, R43_INIT>, sh, s, p); break;
+    case R43_A: launch_step(c, B, k_col_rk43<R, N, R43_A>, sh, s, p); break;
+    case R43_B: launch_step(c, B, k_col_rk43<R, N, R43_B>, sh, s, p); break;
+    case R43_C: launch_step(c, B, k_col_rk43<R, N, R43_C>, sh, s, p); break;
+    case R43_D: launch_step(c, B, k_col_rk43<R, N, R43_D>, sh, s, p); break;
+    default: launch_step(c, B, k_col_rk43<R, N, R43_E>, sh, s, p); break;
   }
 }
 
@@ -251,8 +275,8 @@ void launch_row_err(ecs_ctx* c, int B, double atol, cudaStream_t s, double* rec_
                     int cap = 0) {
   RowErrParams<R> p; p.G = (const cplx<R>*)c->G; p.ctl = c->ctl; p.tw = (const cplx<R>*)c->tw; p.atol = atol;
   p.rec_h = rec_h; p.rec_acc = rec_acc; p.cap = cap; p.B = B;
-  if (small_rows<N>(B)) launch_step(c, B, k_row_err<R, N, XTS>, dim3(B * (N / XTS)), dim3(XTS * 32), smem_row_2f<R, N, XTS>(), s, p);
-  else launch_step(c, B, k_row_err<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_2f<R, N>(), s, p);
+  if (small_rows<N>(B)) { launch_step(c, B, k_row_err<R, N, XTS>, row_shape<Xf<R, N>, XTS>(B, 2), s, p); return; }
+  launch_step(c, B, k_row_err<R, N, XT>, row_shape<Xf<R, N>>(B, 2), s, p);
 }
 
 template <typename R, int N>
@@ -260,11 +284,11 @@ void launch_regen(ecs_ctx* c, const cplx<R>* rec, const long* items, int nitems,
                   bool mean = true) {
   ColRegenParams<R> p; p.rec = rec; p.items = items; p.G = (cplx<R>*)c->Greg; p.tw = (const cplx<R>*)c->tw;
   p.nitems = nitems;
-  const int cols = nitems * Geomc<N>::K * 2;
-  ++c->launches; k_col_regen<R, N><<<(cols + COLWARPS - 1) / COLWARPS, COLWARPS * 32, 0, s>>>(p);
+  const Shape sc = col_shape<Xf<R, N>>(nitems), sr = row_shape<Xf<R, N>>(nitems, NG);
+  ++c->launches; k_col_regen<R, N><<<sc.grid, sc.block, 0, s>>>(p);
   RowPhysParams<R> q; q.G = (const cplx<R>*)c->Greg; q.phys = phys ? phys : (R*)c->Phys; q.tw = (const cplx<R>*)c->tw;
   q.b0x = mean ? (R)c->b0x : R(0); q.b0y = mean ? (R)c->b0y : R(0); q.nitems = nitems;   // no mean field in derivatives
-  ++c->launches; k_row_phys<R, N, XT><<<nitems * (N / XT), XT * 32, smem_row_phys<R, N>(), s>>>(q);
+  ++c->launches; k_row_phys<R, N, XT><<<sr.grid, sr.block, sr.smem, s>>>(q);
 }
 
 template <typename R, int N>
@@ -272,10 +296,21 @@ void launch_row_tan(ecs_ctx* c, int B, const R* phys, cudaStream_t s, long phys_
                     const StepCtl* ctl = nullptr) {
   RowTanParams<R> p{}; p.ctl = ctl; p.G = (const cplx<R>*)c->G; p.H = (cplx<R>*)c->H; p.phys = phys; p.tw = (const cplx<R>*)c->tw;
   p.B = B; p.phys_bstride = phys_bstride;
-  if (small_rows<N>(B)) launch_step(c, B, k_row_tan<R, N, XTS>, dim3(B * (N / XTS)), dim3(XTS * 32), smem_row_rhs<R, N, XTS>(), s, p);
-  else if (N == 128 && c->rowtan_xt == 4)   // 4-row tiles measured faster at n = 128 only
-    launch_step(c, B, k_row_tan<R, N, 4>, dim3(B * (N / 4)), dim3(4 * 32), smem_row_rhs<R, N, 4>(), s, p);
-  else launch_step(c, B, k_row_tan<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_rhs<R, N>(), s, p);
+  if (small_rows<N>(B)) { launch_step(c, B, k_row_tan<R, N, XTS>, row_shape<Xf<R, N>, XTS>(B, NG), s, p); return; }
+  if (N == 128 && c->rowtan_xt == 4)   // 4-row tiles measured faster at n = 128 only
+    launch_step(c, B, k_row_tan<R, N, 4>, row_shape<Xf<R, N>, 4>(B, NG), s, p);
+  else launch_step(c, B, k_row_tan<R, N, XT>, row_shape<Xf<R, N>>(B, NG), s, p);
+}
+
+// Calls go(stage as a constant).
+template <typename F> void col_tan_stage(int stage, F&& go) {
+#define ECS_ST(x) case x: go(std::integral_constant<int, x>{}); break
+  switch (stage) {
+    ECS_ST(TS_START); ECS_ST(T4_S1); ECS_ST(T4_S2); ECS_ST(T4_S3); ECS_ST(T4_S4); ECS_ST(T43_START); ECS_ST(T43_INIT);
+    ECS_ST(T43_A); ECS_ST(T43_B); ECS_ST(T43_C); ECS_ST(T43_D); ECS_ST(T43_EA);
+    default: go(std::integral_constant<int, T43_E>{}); break;
+  }
+#undef ECS_ST
 }
 
 template <typename R, int N>
@@ -287,23 +322,10 @@ void launch_col_tan(ecs_ctx* c, int B, int stage, int produce, const cplx<R>* re
   p.rec2 = rec2; p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.D = (cplx<R>*)c->D; p.nslot = nslot;
   p.rec = rec; p.dT = dT; p.t = t; p.h = h; p.dscale = dscale; p.tw = (const cplx<R>*)c->tw;
   p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.stage = stage; p.produce = produce;
-  const int cols = B * Geomc<N>::K * 2;   // one warp per (batch, ky, channel)
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
-  switch (stage) {
-    case TS_START: launch_step(c, B, k_col_tan<R, N, TS_START>, g, bl, 0, s, p); break;
-    case T4_S1: launch_step(c, B, k_col_tan<R, N, T4_S1>, g, bl, 0, s, p); break;
-    case T4_S2: launch_step(c, B, k_col_tan<R, N, T4_S2>, g, bl, 0, s, p); break;
-    case T4_S3: launch_step(c, B, k_col_tan<R, N, T4_S3>, g, bl, 0, s, p); break;
-    case T4_S4: launch_step(c, B, k_col_tan<R, N, T4_S4>, g, bl, 0, s, p); break;
-    case T43_START: launch_step(c, B, k_col_tan<R, N, T43_START>, g, bl, 0, s, p); break;
-    case T43_INIT: launch_step(c, B, k_col_tan<R, N, T43_INIT>, g, bl, 0, s, p); break;
-    case T43_A: launch_step(c, B, k_col_tan<R, N, T43_A>, g, bl, 0, s, p); break;
-    case T43_B: launch_step(c, B, k_col_tan<R, N, T43_B>, g, bl, 0, s, p); break;
-    case T43_C: launch_step(c, B, k_col_tan<R, N, T43_C>, g, bl, 0, s, p); break;
-    case T43_D: launch_step(c, B, k_col_tan<R, N, T43_D>, g, bl, 0, s, p); break;
-    case T43_EA: launch_step(c, B, k_col_tan<R, N, T43_EA>, g, bl, 0, s, p); break;
-    default: launch_step(c, B, k_col_tan<R, N, T43_E>, g, bl, 0, s, p); break;
-  }
+  with_layout<R, N>(c, B, [&](auto* x, auto grp) {
+    const Shape sh = col_shape<std::remove_pointer_t<decltype(x)>>(B);
+    col_tan_stage(stage, [&](auto st) { launch_step(c, B, k_col_tan<R, N, decltype(st)::value, decltype(grp)::value>, sh, s, p); });
+  });
 }
 
 template <typename R, int N>
@@ -312,8 +334,8 @@ void launch_row_adj(ecs_ctx* c, int B, const R* phys, cudaStream_t s, long phys_
   RowAdjParams<R> p{}; p.G = (const cplx<R>*)c->G; p.H = (cplx<R>*)c->H; p.phys = phys; p.tw = (const cplx<R>*)c->tw;
   p.phys_bstride = phys_bstride; p.ctl = ctl;
   p.B = B;
-  if (small_rows<N>(B)) launch_step(c, B, k_row_adj<R, N, XTS>, dim3(B * (N / XTS)), dim3(XTS * 32), smem_row_rhs<R, N, XTS>(), s, p);
-  else launch_step(c, B, k_row_adj<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_rhs<R, N>(), s, p);
+  if (small_rows<N>(B)) launch_step(c, B, k_row_adj<R, N, XTS>, row_shape<Xf<R, N>, XTS>(B, NHA), s, p);
+  else launch_step(c, B, k_row_adj<R, N, XT>, row_shape<Xf<R, N>>(B, NHA), s, p);
 }
 
 template <typename R, int N>
@@ -322,30 +344,28 @@ void launch_col_adj(ecs_ctx* c, int B, int stage, const cplx<R>* rec, const cplx
   ColAdjParams<R> p{}; p.ctl = ctl; p.rec_bstride = rec_bstride; p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.J = (cplx<R>*)c->D; p.nslot = nslot;
   p.rec = rec; p.rec_prev = rec_prev; p.hacc = c->hacc; p.t = t; p.h = h; p.tw = (const cplx<R>*)c->tw;
   p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.stage = stage;
-  const int cols = B * Geomc<N>::K * 2;   // one warp per (batch, ky, channel)
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
+  const Shape sh = col_shape<Xf<R, N>>(B);
   switch (stage) {
-    case AJ_PRE: launch_step(c, B, k_col_adj<R, N, AJ_PRE>, g, bl, 0, s, p); break;
-    case AJ_S4: launch_step(c, B, k_col_adj<R, N, AJ_S4>, g, bl, 0, s, p); break;
-    case AJ_S3: launch_step(c, B, k_col_adj<R, N, AJ_S3>, g, bl, 0, s, p); break;
-    case AJ_S2: launch_step(c, B, k_col_adj<R, N, AJ_S2>, g, bl, 0, s, p); break;
-    case AJ_S1: launch_step(c, B, k_col_adj<R, N, AJ_S1>, g, bl, 0, s, p); break;
-    case AJ43_INIT: launch_step(c, B, k_col_adj<R, N, AJ43_INIT>, g, bl, 0, s, p); break;
-    case AJ43_PRE: launch_step(c, B, k_col_adj<R, N, AJ43_PRE>, g, bl, 0, s, p); break;
-    case AJ43_S5: launch_step(c, B, k_col_adj<R, N, AJ43_S5>, g, bl, 0, s, p); break;
-    case AJ43_S4: launch_step(c, B, k_col_adj<R, N, AJ43_S4>, g, bl, 0, s, p); break;
-    case AJ43_S3: launch_step(c, B, k_col_adj<R, N, AJ43_S3>, g, bl, 0, s, p); break;
-    case AJ43_S2: launch_step(c, B, k_col_adj<R, N, AJ43_S2>, g, bl, 0, s, p); break;
-    default: launch_step(c, B, k_col_adj<R, N, AJ43_IPRE>, g, bl, 0, s, p); break;
+    case AJ_PRE: launch_step(c, B, k_col_adj<R, N, AJ_PRE>, sh, s, p); break;
+    case AJ_S4: launch_step(c, B, k_col_adj<R, N, AJ_S4>, sh, s, p); break;
+    case AJ_S3: launch_step(c, B, k_col_adj<R, N, AJ_S3>, sh, s, p); break;
+    case AJ_S2: launch_step(c, B, k_col_adj<R, N, AJ_S2>, sh, s, p); break;
+    case AJ_S1: launch_step(c, B, k_col_adj<R, N, AJ_S1>, sh, s, p); break;
+    case AJ43_INIT: launch_step(c, B, k_col_adj<R, N, AJ43_INIT>, sh, s, p); break;
+    case AJ43_PRE: launch_step(c, B, k_col_adj<R, N, AJ43_PRE>, sh, s, p); break;
+    case AJ43_S5: launch_step(c, B, k_col_adj<R, N, AJ43_S5>, sh, s, p); break;
+    case AJ43_S4: launch_step(c, B, k_col_adj<R, N, AJ43_S4>, sh, s, p); break;
+    case AJ43_S3: launch_step(c, B, k_col_adj<R, N, AJ43_S3>, sh, s, p); break;
+    case AJ43_S2: launch_step(c, B, k_col_adj<R, N, AJ43_S2>, sh, s, p); break;
+    default: launch_step(c, B, k_col_adj<R, N, AJ43_IPRE>, sh, s, p); break;
   }
 }
 
 template <typename R, int N, int SCHEME, int... ST>
 void launch_col_fx_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColFxParams<R>& p,
                       std::integer_sequence<int, ST...>) {
-  const int cols = B * Geomc<N>::K * 2;   // one warp per (batch, ky, channel)
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
-  ((stage == ST ? launch_step(c, B, k_col_fx<R, N, SCHEME, ST>, g, bl, 0, s, p) : void()), ...);
+  const Shape sh = col_shape<Xf<R, N>>(B);
+  ((stage == ST ? launch_step(c, B, k_col_fx<R, N, SCHEME, ST>, sh, s, p) : void()), ...);
 }
 
 template <typename R, int N>
@@ -365,15 +385,14 @@ void launch_row_tan2(ecs_ctx* c, int B, const cplx<R>* Ga, const cplx<R>* Gb, co
                      cudaStream_t s) {
   RowTan2Params<R> p; p.Ga = Ga; p.Gb = Gb; p.H = (cplx<R>*)c->H; p.phys_a = phys_a; p.phys_b = phys_b;
   p.tw = (const cplx<R>*)c->tw; p.B = B;
-  launch_step(c, B, k_row_tan2<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_tan2<R, N>(), s, p);
+  launch_step(c, B, k_row_tan2<R, N, XT>, row_shape<Xf<R, N>>(B, 2 * NG), s, p);
 }
 
 template <typename R, int N, int... ST>
 void launch_col_tdj_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColTdjParams<R>& p,
                        std::integer_sequence<int, ST...>) {
-  const int cols = B * Geomc<N>::K * 2;
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
-  ((stage == ST ? launch_step(c, B, k_col_tdj<R, N, ST>, g, bl, 0, s, p) : void()), ...);
+  const Shape sh = col_shape<Xf<R, N>>(B);
+  ((stage == ST ? launch_step(c, B, k_col_tdj<R, N, ST>, sh, s, p) : void()), ...);
 }
 
 template <typename R, int N>
@@ -388,9 +407,8 @@ void launch_col_tdj(ecs_ctx* c, int B, int stage, int produce, const cplx<R>* re
 template <typename R, int N, int SCHEME, int... ST>
 void launch_col_fxt_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColFxtParams<R>& p,
                        std::integer_sequence<int, ST...>) {
-  const int cols = B * Geomc<N>::K * 2;
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
-  ((stage == ST ? launch_step(c, B, k_col_fxt<R, N, SCHEME, ST>, g, bl, 0, s, p) : void()), ...);
+  const Shape sh = col_shape<Xf<R, N>>(B);
+  ((stage == ST ? launch_step(c, B, k_col_fxt<R, N, SCHEME, ST>, sh, s, p) : void()), ...);
 }
 
 // Tangent column pass of the RK4 / Lawson-RK6 linearisation (kernels_fxl.cuh).
@@ -407,9 +425,8 @@ void launch_col_fxt(ecs_ctx* c, int B, int scheme, int stage, int produce, const
 template <typename R, int N, int SCHEME, int... ST>
 void launch_col_fxa_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColFxaParams<R>& p,
                        std::integer_sequence<int, ST...>) {
-  const int cols = B * Geomc<N>::K * 2;
-  const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
-  ((stage == ST ? launch_step(c, B, k_col_fxa<R, N, SCHEME, ST>, g, bl, 0, s, p) : void()), ...);
+  const Shape sh = col_shape<Xf<R, N>>(B);
+  ((stage == ST ? launch_step(c, B, k_col_fxa<R, N, SCHEME, ST>, sh, s, p) : void()), ...);
 }
 
 // Adjoint column pass of the RK4 / Lawson-RK6 linearisation; stage S + 1 seeds a step.
@@ -515,7 +532,7 @@ struct Impl {
         constexpr int W = decltype(w)::value;
         constexpr bool DSM = decltype(dsm)::value;
         launch_cluster(c, B, chain_cl<N, W>(), k_rk4_chain<R, N, W, DSM>, dim3(B * chain_cl<N, W>()), dim3(W * 32),
-                       rk4_chain_smem<R, N, W, DSM>(), s, P);
+                       Rk4ChainSmem<R, N, W, DSM>::bytes, s, P);
       };
       chain_dispatch(c, B, true, go);
       return cuda_err(c, cudaGetLastError(), "rk4 chain");
@@ -707,10 +724,10 @@ struct Impl {
         P.atol = cfg->atol; P.rec_h = rec_h; P.rec_acc = rec_acc; P.amax = amax;
         if (c->chain_w == 8 || (c->chain_w == 0 && B <= c->chain_res8))
           launch_cluster(c, B, chain_cl<N, 8>(), k_rk43_chain<R, N, 8>, dim3(B * chain_cl<N, 8>()), dim3(8 * 32),
-                         rk43_chain_smem<R, N, 8>(), s, P);
+                         Rk43ChainSmem<R, N, 8>::bytes, s, P);
         else
           launch_cluster(c, B, chain_cl<N, 16>(), k_rk43_chain<R, N, 16>, dim3(B * chain_cl<N, 16>()), dim3(16 * 32),
-                         rk43_chain_smem<R, N, 16>(), s, P);
+                         Rk43ChainSmem<R, N, 16>::bytes, s, P);
         const long nbox = (long)B * 2 * K * M;
         ++c->launches; k_rk43_resolve<R><<<grid1d(nbox), 256, 0, s>>>((cplx<R>*)c->S43, c->ctl, (cplx<R>*)c->F, N, B);
         return cuda_err(c, cudaGetLastError(), "rk43 chain");
@@ -1456,10 +1473,10 @@ struct Impl {
           constexpr bool DSM = decltype(dsm)::value;
           if (W == 8 && dsh)
             launch_cluster(c, B, chain_cl<N, W>(), k_tan_chain<R, N, W, DSM, W == 8>, dim3(B * chain_cl<N, W>()),
-                           dim3(W * 32), chain_smem<R, N, W, DSM, W == 8>(), s, P);
+                           dim3(W * 32), TanChainSmem<R, N, W, DSM, W == 8>::bytes, s, P);
           else
             launch_cluster(c, B, chain_cl<N, W>(), k_tan_chain<R, N, W, DSM, false>, dim3(B * chain_cl<N, W>()),
-                           dim3(W * 32), chain_smem<R, N, W, DSM, false>(), s, P);
+                           dim3(W * 32), TanChainSmem<R, N, W, DSM, false>::bytes, s, P);
         };
         chain_dispatch(c, B, false, go);
         start = end;
@@ -1867,20 +1884,19 @@ struct Impl {
       ColTdaParams<R> p; p.Ha = (const cplx<R>*)c->H; p.Hb = (const cplx<R>*)c->Gx; p.G = (cplx<R>*)c->G;
       p.J = (cplx<R>*)c->D; p.nslot = nslot; p.rec = ra; p.hacc = c->hacc; p.h = h; p.tw = (const cplx<R>*)c->tw;
       p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B;
-      const int cols = B * K * 2;
-      const dim3 g((cols + COLWARPS - 1) / COLWARPS), bl(COLWARPS * 32);
+      const Shape sh = col_shape<Xf<R, N>>(B);
       switch (stage) {
-        case TA_SEED: launch_step(c, B, k_col_tda<R, N, TA_SEED>, g, bl, 0, s, p); break;
-        case TA_B: launch_step(c, B, k_col_tda<R, N, TA_B>, g, bl, 0, s, p); break;
-        case TA_C: launch_step(c, B, k_col_tda<R, N, TA_C>, g, bl, 0, s, p); break;
-        case TA_D: launch_step(c, B, k_col_tda<R, N, TA_D>, g, bl, 0, s, p); break;
-        default: launch_step(c, B, k_col_tda<R, N, TA_E>, g, bl, 0, s, p); break;
+        case TA_SEED: launch_step(c, B, k_col_tda<R, N, TA_SEED>, sh, s, p); break;
+        case TA_B: launch_step(c, B, k_col_tda<R, N, TA_B>, sh, s, p); break;
+        case TA_C: launch_step(c, B, k_col_tda<R, N, TA_C>, sh, s, p); break;
+        case TA_D: launch_step(c, B, k_col_tda<R, N, TA_D>, sh, s, p); break;
+        default: launch_step(c, B, k_col_tda<R, N, TA_E>, sh, s, p); break;
       }
     };
     auto row2 = [&](const R* pa, const R* pb) {
       RowAdj2Params<R> p; p.G = (const cplx<R>*)c->G; p.Ha = (cplx<R>*)c->H; p.Hb = (cplx<R>*)c->Gx;
       p.phys_a = pa; p.phys_b = pb; p.tw = (const cplx<R>*)c->tw; p.B = B;
-      launch_step(c, B, k_row_adj2<R, N, XT>, dim3(B * (N / XT)), dim3(XT * 32), smem_row_rhs<R, N>(), s, p);
+      launch_step(c, B, k_row_adj2<R, N, XT>, row_shape<Xf<R, N>>(B, NHA), s, p);
     };
     const long nch = (steps + CS - 1) / CS;
     for (long ch = nch - 1; ch >= 0; --ch) {
@@ -2523,23 +2539,16 @@ int ctx_init(ecs_ctx* c, const ecs_params* prm) {
   c->ctl = (StepCtl*)dev_alloc(c, (size_t)B * sizeof(StepCtl), &st);
   c->rowsq = (double*)dev_alloc(c, (size_t)B * N * sizeof(double), &st);
   c->Tbuf = (double*)dev_alloc(c, (size_t)B * sizeof(double), &st);
-  c->tw = dev_alloc(c, (size_t)tw_smem(N) * cb, &st);   // the shared-memory twiddle image
+  c->tw = dev_alloc(c, (size_t)XfTable<R, N>::size * cb, &st);
   c->fhat = dev_alloc(c, (size_t)Geomc<N>::K * Geomc<N>::M * cb, &st);
   if (st) return st;
   if (cudaMallocHost((void**)&c->hcount, sizeof(int)) != cudaSuccess) return set_err(c, ECS_ERR_OOM, "pinned alloc");
   if (cudaStreamCreateWithFlags(&c->cap_stream, cudaStreamNonBlocking) != cudaSuccess)
     return set_err(c, ECS_ERR_CUDA, "capture stream");
-  // twiddles exp(-2 pi i k/N), k < N/2, from long double
-  std::vector<cplx<R>> tw(N / 2);
-  const long double twopi = 6.283185307179586476925286766559005768L;
-  for (int k = 0; k < N / 2; ++k) {
-    long double a = twopi * (long double)k / (long double)N;
-    tw[k] = mk<R>((R)cosl(a), (R)(-sinl(a)));
-  }
-  std::vector<cplx<R>> img(tw_smem(N));
-  twiddle_image<cplx<R>, N>(tw.data(), img.data());
+  std::vector<cplx<R>> img(XfTable<R, N>::size);
+  xf_table<R, N>(img.data());
   cudaError_t e = cudaMemcpy(c->tw, img.data(), img.size() * cb, cudaMemcpyHostToDevice);
-  if (e != cudaSuccess) return cuda_err(c, e, "twiddle upload");
+  if (e != cudaSuccess) return cuda_err(c, e, "table upload");
   // forcing on the grid x_i = i/n * 2 * pi (mhd_jax.py:47), channel omega only
   std::vector<R> fr((size_t)2 * N * N, R(0));
   const double pi_lit = 3.14159265358979323846;

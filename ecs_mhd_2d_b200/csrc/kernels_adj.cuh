@@ -38,50 +38,53 @@ struct RowAdjParams {
   int B;
 };
 
+// Product adjoints of one point: (P1bar, P2bar) and P3bar -> (ubar, vbar) and (Bxbar, Bybar).
+template <typename R>
+__device__ __forceinline__ void row_adj_product(cplx<R> p12, R p3, cplx<R> uv, cplx<R> bb, cplx<R>& a, cplx<R>& q) {
+  const R p1 = p12.x, p2 = p12.y, u = uv.x, v = uv.y, bx = bb.x, by = bb.y;
+  a = mk<R>(R(2) * u * p1 - v * p2 + by * p3, -R(2) * v * p1 - u * p2 - bx * p3);
+  q = mk<R>(-R(2) * bx * p1 + by * p2 - v * p3, R(2) * by * p1 + bx * p2 + u * p3);
+}
+
+// s_G holds the three product rows and then the four adjoint rows (each group
+// reads and writes its own column of the tile).
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32) k_row_adj(RowAdjParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, L = X::L, K = X::K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_tw + fft_smem(N, XT);
-  cplx<R>* s_H = s_G + 3 * K * (XT + 1);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_G = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = x0 + w;
+  const int w = threadIdx.x / L;
+  const X xf(s_x, threadIdx.x >> 5);
   pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   pdl_wait();
   if (p.ctl && p.ctl[b].done) return;   // the whole CTA belongs to batch element b
-  const R* ph = phys_row<R, N>(p.phys + (size_t)b * p.phys_bstride, x);
-  R pu[E], pv[E], pbx[E], pby[E];
+  constexpr bool EARLY = E <= 4;        // see row_tan_body
+  const cplx<R>* ph = phys_row<R, N>(p.phys + (size_t)b * p.phys_bstride, x0 + w) + xf.l;
+  cplx<R> puv[E], pbb[E];
+  auto load_phys = [&]() {
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int e = lane + 32 * j;
-    pu[j] = ph[e]; pv[j] = ph[N + e]; pbx[j] = ph[2 * N + e]; pby[j] = ph[3 * N + e];
-  }
+    for (int j = 0; j < E; ++j) { puv[j] = ph[L * j]; pbb[j] = ph[N + L * j]; }
+  };
+  if constexpr (EARLY) load_phys();
   load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, 3 * K, x0);
   __syncthreads();
-  cplx<R> P12[E], P3[E];   // (P1bar, P2bar) and (P3bar, 0) in position order
+  cplx<R> P12[E], P3[E];   // (P1bar, P2bar) and (P3bar, 0)
+  row_inverse<XT, true>(s_G, w, xf, P12, P3);
+  if constexpr (!EARLY) load_phys();
 #pragma unroll
   for (int j = 0; j < E; ++j) {
-    P12[j] = packed_pair<R, N, XT>(s_G, s_G + K * (XT + 1), lane + 32 * j, w);
-    P3[j] = packed_one<R, N, XT>(s_G + 2 * K * (XT + 1), lane + 32 * j, w);
+    cplx<R> a, q;
+    row_adj_product<R>(P12[j], P3[j].x, puv[j], pbb[j], a, q);
+    P12[j] = a; P3[j] = q;
   }
-  fft_dif2<R, N, true>(P12, P3, s_tw, lane);
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const R p1 = P12[j].x, p2 = P12[j].y, p3 = P3[j].x;
-    const R u = pu[j], v = pv[j], bx = pbx[j], by = pby[j];
-    P12[j] = mk<R>(R(2) * u * p1 - v * p2 + by * p3, -R(2) * v * p1 - u * p2 - bx * p3);     // (ubar, vbar)
-    P3[j] = mk<R>(-R(2) * bx * p1 + by * p2 - v * p3, R(2) * by * p1 + bx * p2 + u * p3);    // (Bxbar, Bybar)
-  }
-  fft_dit2<R, N, false>(P12, P3, s_tw, lane);
-  split_store<R, N, XT>(P12, s_H, s_H + K * (XT + 1), w, lane);
-  split_store<R, N, XT>(P3, s_H + 2 * K * (XT + 1), s_H + 3 * K * (XT + 1), w, lane);
+  row_forward<XT, true>(P12, P3, s_G, w, xf);
   __syncthreads();
-  store_tile<R, N, XT>(p.H + (size_t)b * NHA * K * N, s_H, NHA * K, x0);
+  store_tile<R, N, XT>(p.H + (size_t)b * NHA * K * N, s_G, NHA * K, x0);
 }
 
 // ---------------------------------------------------------------------------
@@ -121,202 +124,227 @@ struct ColAdjParams {
 
 __device__ __forceinline__ double rdot2(double ax, double ay, double bx, double by) { return ax * bx + ay * by; }
 
+// Slots (bits of AdjSlot4 / AdjSlot43) that the algebra of a stage reads; they are
+// loaded together before the stage's stores.
+__host__ __device__ constexpr unsigned adj_jmask(int stage) {
+  return stage == AJ_PRE || stage == AJ_S1 ? (1u << J_OB)
+       : stage == AJ_S4 ? (1u << J_F2) | (1u << J_A1) | (1u << J_K2) | (1u << J_B3)
+       : stage == AJ_S3 ? (1u << J_F2) | (1u << J_K2)
+       : stage == AJ_S2 ? (1u << J_F2) | (1u << J_A1)
+       : stage == AJ43_PRE || stage == AJ43_IPRE ? (1u << JJ_K1)
+       : stage == AJ43_S5 || stage == AJ43_INIT ? (1u << JJ_X0)
+       : stage == AJ43_S4 ? (1u << JJ_X2) | (1u << JJ_K3P) | (1u << JJ_K2P) | (1u << JJ_K1PP)
+       : stage == AJ43_S3 ? (1u << JJ_XB) | (1u << JJ_K2)
+       : stage == AJ43_S2 ? (1u << JJ_XB) | (1u << JJ_K1P) : 0u;
+}
+
+// (c_ky/n^2) sum_m (-i mu_m) rfft2 of the adjoint rows of channel c in H: the box
+// cotangent N'(P)^T lambda at the lane's algebra elements.
+template <class X, class Mu>
+__device__ __forceinline__ void col_adj_xb(const cplx<typename X::R>* H, int b, int c, int ky, const X& xf,
+                                           const Mu& mu, cplx<typename X::R> (&xb)[X::E]) {
+  using R = typename X::R;
+  constexpr int E = X::E, L = X::L, K = X::K, N = X::N;
+  const cplx<R>* h0 = H + ((size_t)(b * NHA + 2 * c) * K + ky) * N;
+  const cplx<R>* h1 = h0 + (size_t)K * N;
+  const R cky = ky == 0 ? R(1) : R(2);
+  cplx<R> v1[E];
+#pragma unroll
+  for (int j = 0; j < E; ++j) { xb[j] = h0[xf.l + L * j]; v1[j] = h1[xf.l + L * j]; }
+  xf.template to_spec2<false>(xb, v1);
+  mu.wait();
+#pragma unroll
+  for (int j = 0; j < E; ++j) {
+    const int s = xf.slot(j);
+    if (s < 0) { xb[j] = mk<R>(0, 0); continue; }
+    const cplx<R> m = mu(s);
+    xb[j] = cscale(cadd(cimul(xb[j], -m.x), cimul(v1[j], -m.y)), cky);
+  }
+}
+
+// Inverse column transforms of lambda/c_ky times the product multipliers: the
+// product cotangents P1bar, P2bar (channel w) or P3bar (channel j) in G,
+// unscaled: Re sum mult_f lam e^{ik.x} (the row pass doubles ky > 0).
+template <class X>
+__device__ __forceinline__ void col_adj_emit(const cplx<typename X::R> (&lam)[X::E], cplx<typename X::R>* G, int b, int c,
+                                             int ky, bool act, const X& xf) {
+  using R = typename X::R;
+  constexpr int E = X::E;
+  auto mult = [&](cplx<R> (&z)[E], int f) {
+#pragma unroll
+    for (int j = 0; j < E; ++j)
+      z[j] = X::none(j) ? mk<R>(0, 0) : cscale_rn(lam[j], prod_mult<R>(f, xf.kx(j), (R)ky));
+  };
+  cplx<R> z[E];
+  if (c == 0) {
+    cplx<R> z1[E];
+    mult(z, 0); mult(z1, 1);
+    xf.template from_spec2<true>(z, z1);
+    col_put(z, G, NG, b, 0, ky, act, xf);
+    col_put(z1, G, NG, b, 1, ky, act, xf);
+  } else {
+    mult(z, 2);
+    xf.template from_spec<true>(z);
+    col_put(z, G, NG, b, 2, ky, act, xf);
+  }
+}
+
+// Sum over the lanes of a column's group, added to hacc by its first lane.
+template <class X>
+__device__ __forceinline__ void col_hacc(double* hacc, const ColId<X>& id, bool act, const X& xf, double part) {
+#pragma unroll
+  for (int o = X::L / 2; o >= 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+  if (act && xf.l == 0) hacc[((size_t)id.b * X::K + id.ky) * 2 + id.ch] += part;
+}
+
 template <typename R, int N, int STAGE>
-__global__ void __launch_bounds__(128) k_col_adj(ColAdjParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_adj(ColAdjParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int ch = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;   // one warp per (b, ky, channel)
+  ECS_COL_PROLOGUE(popc_c(adj_jmask(STAGE)), 1);   // the multipliers
+  const int ch = id.ch, b = id.b, ky = id.ky;
   if (p.ctl && p.ctl[b].done) return;
-  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec + (size_t)b * p.rec_bstride;
-  const cplx<R>* Qp = p.rec_prev ? p.rec_prev + (size_t)b * p.rec_bstride : nullptr;
+  const size_t row = ((size_t)ch * K + ky) * M;
+  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + (size_t)b * p.rec_bstride + row;
+  const cplx<R>* Qp = p.rec_prev ? p.rec_prev + (size_t)b * p.rec_bstride + row : nullptr;
   const R h = p.ctl ? (R)p.ctl[b].h : (R)p.h, t = (R)p.t;
   constexpr bool rk43 = STAGE >= AJ43_INIT;
   constexpr bool has_rhs = !(STAGE == AJ_PRE || STAGE == AJ43_PRE || STAGE == AJ43_IPRE);
   const R cky = ky == 0 ? R(1) : R(2);
-  const R inv_n2 = R(1) / (R(N) * R(N));
   const R coeff = ch == 0 ? p.nu : p.eta;
-
-  // Xbar_c = (c_ky/n^2) sum_m (-i mu_m) rfft2(fbar_{m,c}), m over the two uncurled fields of channel c
+  double hpart = 0.0, hdiv = 0.0;   // hdiv: the terms over h (RK4) or t (RK4(3))
+  constexpr unsigned JM = adj_jmask(STAGE);
+  Operands<X, JM> op(rows);
+  op.begin(J, VEC);
+  const TableRow<X, has_rhs && rows_fit(popc_c(JM), 1)> mu(rows + popc_c(JM) * M, mu_row<X>(p.tw, ky));
   cplx<R> xb[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) xb[j] = mk<R>(0, 0);
-  if (has_rhs) {
-    const cplx<R>* h0 = p.H + ((size_t)(b * NHA + 2 * ch) * K + ky) * N;
-    const cplx<R>* h1 = h0 + (size_t)K * N;
-    cplx<R> v1[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) { xb[j] = h0[lane + 32 * j]; v1[j] = h1[lane + 32 * j]; }
-    fft_dif2<R, N, false>(xb, v1, s_tw, lane);
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-      xb[j] = cadd(cimul(xb[j], -spectral_mu<R>(2, kx, ky)), cimul(v1[j], -spectral_mu<R>(3, kx, ky)));
-    }
-#pragma unroll
-    for (int j = 0; j < E; ++j) xb[j] = cscale(xb[j], cky * inv_n2);
-  }
-
-  double hpart = 0.0;
-  bool feed = true;
+  if (has_rhs) col_adj_xb(p.H, b, ch, ky, xf, mu, xb);
+  op.load(J, VEC, true, xf);
   cplx<R> lam[E];   // next adjoint-RHS input lambda / c_ky (multipliers applied per product below)
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    lam[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const bool in_mask = !(kx == 0 && ky == 0);
-    const size_t o = ((size_t)ch * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    const cplx<R> Xb = xb[j];
-    cplx<R> kb = mk<R>(0, 0);   // cotangent fed to the next adjoint RHS (before the h or t factor)
-    auto ip = [&](cplx<R> a, cplx<R> bb) { return rdot2(a.x, a.y, bb.x, bb.y); };
-    if (!rk43) {
-      const R e = in_mask ? exp(h / R(2) * L) : R(0);
-      const R dedh = e * L / R(2);
-      switch (STAGE) {
-        case AJ_PRE: {
-          const cplx<R> ob = J[J_OB * VEC + o];
-          J[J_F2 * VEC + o] = ob; J[J_A1 * VEC + o] = cdiv_k<6>(ob);
-          J[J_K2 * VEC + o] = cdiv_k<3>(ob); J[J_B3 * VEC + o] = cdiv_k<3>(ob);
-          kb = cdiv_k<6>(ob);                                   // k4bar
-          hpart += ip(kb, Q[Q_K4 * VEC + o]) / (double)h;
-        } break;
-        case AJ_S4: {
-          const cplx<R> f2b = cadd(J[J_F2 * VEC + o], Xb), b3b = cadd(J[J_B3 * VEC + o], Xb);
-          const cplx<R> b2b = J[J_K2 * VEC + o], b1b = J[J_A1 * VEC + o];
-          const cplx<R> f = Q[Q_F * VEC + o], k1 = Q[Q_K1 * VEC + o];
-          const double eb = ip(b3b, Q[Q_K3 * VEC + o]) + ip(b2b, Q[Q_K2 * VEC + o]) + ip(b1b, cscale(k1, e)) +
-                            ip(f2b, cscale(f, e));
-          hpart += eb * (double)dedh;
-          kb = cscale(b3b, e);                                     // k3bar
-          hpart += ip(kb, Q[Q_K3 * VEC + o]) / (double)h;
-          J[J_F2 * VEC + o] = cscale(f2b, e);                      // f1bar
-          J[J_A1 * VEC + o] = cscale(b1b, e);                      // a1bar
-          J[J_K2 * VEC + o] = cscale(b2b, e);                      // k2bar
-        } break;
-        case AJ_S3: {
-          J[J_F2 * VEC + o] = cadd(J[J_F2 * VEC + o], Xb);
-          kb = cadd(J[J_K2 * VEC + o], cscale(Xb, R(0.5)));        // k2bar final
-          hpart += ip(kb, Q[Q_K2 * VEC + o]) / (double)h;
-        } break;
-        case AJ_S2: {
-          const cplx<R> f1b = cadd(J[J_F2 * VEC + o], Xb);
-          const cplx<R> a1b = cadd(J[J_A1 * VEC + o], cscale(Xb, R(0.5)));
-          const double eb = ip(a1b, Q[Q_K1 * VEC + o]) + ip(f1b, Q[Q_F * VEC + o]);
-          hpart += eb * (double)dedh;
-          kb = cscale(a1b, e);                                     // k1bar
-          hpart += ip(kb, Q[Q_K1 * VEC + o]) / (double)h;
-          J[J_OB * VEC + o] = cscale(f1b, e);                      // fbar (without the RHS1 term)
-        } break;
-        default: {   // AJ_S1: fbar += X1bar; then seed the previous step (if any)
-          const cplx<R> fb = cadd(J[J_OB * VEC + o], Xb);
-          J[J_OB * VEC + o] = fb;
-          if (Qp) {
-            J[J_F2 * VEC + o] = fb; J[J_A1 * VEC + o] = cdiv_k<6>(fb);
-            J[J_K2 * VEC + o] = cdiv_k<3>(fb); J[J_B3 * VEC + o] = cdiv_k<3>(fb);
-            kb = cdiv_k<6>(fb);
-            hpart += ip(kb, Qp[Q_K4 * VEC + o]) / (double)h;
-          } else {
-            feed = false;
-          }
-        } break;
+  for (int i = 0; i < E; ++i) {
+      lam[i] = mk<R>(0, 0);
+      const int slot = xf.slot(i);
+      if (slot < 0) continue;
+      const R kx = xf.kx(i);
+      const bool in_mask = !(slot == 0 && ky == 0);
+      const R L = diss_L<R>(kx, (R)ky, coeff);
+      const cplx<R> Xb = has_rhs ? xb[i] : mk<R>(0, 0);
+      cplx<R> kb = mk<R>(0, 0);   // cotangent fed to the next adjoint RHS (before the h or t factor)
+      auto JV = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
+      auto JW = [&](int q, cplx<R> v) { J[q * VEC + slot] = v; };
+      auto QV = [&](int q) -> cplx<R> { return __ldg(Q + q * VEC + slot); };
+      auto ip = [&](cplx<R> a, cplx<R> bb) { return rdot2(a.x, a.y, bb.x, bb.y); };
+      if (!rk43) {
+        const R e = in_mask ? exp(h / R(2) * L) : R(0);
+        const R dedh = e * L / R(2);
+        switch (STAGE) {
+          case AJ_PRE: {
+            const cplx<R> ob = JV(J_OB);
+            JW(J_F2, ob); JW(J_A1, cdiv_k<6>(ob));
+            JW(J_K2, cdiv_k<3>(ob)); JW(J_B3, cdiv_k<3>(ob));
+            kb = cdiv_k<6>(ob);                                   // k4bar
+            hdiv += ip(kb, QV(Q_K4));
+          } break;
+          case AJ_S4: {
+            const cplx<R> f2b = cadd(JV(J_F2), Xb), b3b = cadd(JV(J_B3), Xb);
+            const cplx<R> b2b = JV(J_K2), b1b = JV(J_A1);
+            const cplx<R> f = QV(Q_F), k1 = QV(Q_K1);
+            const double eb = ip(b3b, QV(Q_K3)) + ip(b2b, QV(Q_K2)) + ip(b1b, cscale(k1, e)) +
+                              ip(f2b, cscale(f, e));
+            hpart += eb * (double)dedh;
+            kb = cscale(b3b, e);                                     // k3bar
+            hdiv += ip(kb, QV(Q_K3));
+            JW(J_F2, cscale(f2b, e));                      // f1bar
+            JW(J_A1, cscale(b1b, e));                      // a1bar
+            JW(J_K2, cscale(b2b, e));                      // k2bar
+          } break;
+          case AJ_S3: {
+            JW(J_F2, cadd(JV(J_F2), Xb));
+            kb = cadd(JV(J_K2), cscale(Xb, R(0.5)));        // k2bar final
+            hdiv += ip(kb, QV(Q_K2));
+          } break;
+          case AJ_S2: {
+            const cplx<R> f1b = cadd(JV(J_F2), Xb);
+            const cplx<R> a1b = cadd(JV(J_A1), cscale(Xb, R(0.5)));
+            const double eb = ip(a1b, QV(Q_K1)) + ip(f1b, QV(Q_F));
+            hpart += eb * (double)dedh;
+            kb = cscale(a1b, e);                                     // k1bar
+            hdiv += ip(kb, QV(Q_K1));
+            JW(J_OB, cscale(f1b, e));                      // fbar (without the RHS1 term)
+          } break;
+          default: {   // AJ_S1: fbar += X1bar; then seed the previous step (if any)
+            const cplx<R> fb = cadd(JV(J_OB), Xb);
+            JW(J_OB, fb);
+            if (Qp) {
+              JW(J_F2, fb); JW(J_A1, cdiv_k<6>(fb));
+              JW(J_K2, cdiv_k<3>(fb)); JW(J_B3, cdiv_k<3>(fb));
+              kb = cdiv_k<6>(fb);
+              hdiv += ip(kb, __ldg(Qp + Q_K4 * VEC + slot));
+            }
+          } break;
+        }
+        kb = cscale(kb, h);
+      } else {
+        const cplx<R> eg = QV(RR_E);   // (e, e L h/2) of the attempt, e = exp(t L h/2)
+        const R e = eg.x;
+        const R dedt = eg.y;
+        switch (STAGE) {
+          case AJ43_PRE:      // from (xbar_f, k5bar) in (X0, K1) slots: RHS5 input = k5bar
+          case AJ43_IPRE: {   // initial k1 = t v(x0): input = k1bar
+            kb = JV(JJ_K1);
+            hdiv += ip(kb, QV(STAGE == AJ43_PRE ? RR_K5 : RR_K1));
+          } break;
+          case AJ43_S5: {     // xbar_f += Xbar5; distribute to x2, k1'', k2', k3', k4
+            const cplx<R> xfb = cadd(JV(JJ_X0), Xb);
+            JW(JJ_X2, xfb);
+            JW(JJ_K1PP, cdiv_k<6>(cscale(xfb, h)));
+            JW(JJ_K2P, cdiv_k<3>(cscale(xfb, h)));
+            JW(JJ_K3P, cdiv_k<3>(cscale(xfb, h)));
+            kb = cdiv_k<6>(cscale(xfb, h));                       // k4bar
+            hdiv += ip(kb, QV(RR_K4));
+          } break;
+          case AJ43_S4: {     // Y4 = x2 + h k3'
+            const cplx<R> x2b = cadd(JV(JJ_X2), Xb);
+            const cplx<R> k3pb = cadd(JV(JJ_K3P), cscale(Xb, h));
+            const cplx<R> k2pb = JV(JJ_K2P), k1ppb = JV(JJ_K1PP);
+            const cplx<R> x0 = QV(RR_X0), k1 = QV(RR_K1);
+            const double eb = ip(k3pb, QV(RR_K3)) + ip(k2pb, QV(RR_K2)) +
+                              ip(k1ppb, cscale(k1, e)) + ip(x2b, cscale(x0, e));
+            hpart += eb * (double)dedt;
+            kb = cscale(k3pb, e);                                    // k3bar
+            hdiv += ip(kb, QV(RR_K3));
+            JW(JJ_K2, cscale(k2pb, e));                    // k2bar (partial)
+            JW(JJ_K1P, cscale(k1ppb, e));                  // k1'bar (partial)
+            JW(JJ_XB, cscale(x2b, e));                     // xbar (partial)
+          } break;
+          case AJ43_S3: {     // Y3 = x + h k2/2
+            JW(JJ_XB, cadd(JV(JJ_XB), Xb));
+            kb = cadd(JV(JJ_K2), cscale(cscale(Xb, h), R(0.5)));   // k2bar final
+            hdiv += ip(kb, QV(RR_K2));
+          } break;
+          case AJ43_S2: {     // Y2 = x + h k1'/2; then x0bar, k1bar of this attempt
+            const cplx<R> xbb = cadd(JV(JJ_XB), Xb);
+            const cplx<R> k1pb = cadd(JV(JJ_K1P), cscale(cscale(Xb, h), R(0.5)));
+            const double eb = ip(k1pb, QV(RR_K1)) + ip(xbb, QV(RR_X0));
+            hpart += eb * (double)dedt;
+            JW(JJ_X0, cscale(xbb, e));
+            JW(JJ_K1, cscale(k1pb, e));
+          } break;
+          default: {          // AJ43_INIT: initial k1 = t v(x0): x0bar += Xbar
+            JW(JJ_X0, cadd(JV(JJ_X0), Xb));
+          } break;
+        }
+        kb = cscale(kb, t);
       }
-      kb = cscale(kb, h);
-    } else {
-      const cplx<R> eg = Q[RR_E * VEC + o];   // (e, e L h/2) of the attempt, e = exp(t L h/2)
-      const R e = eg.x;
-      const R dedt = eg.y;
-      switch (STAGE) {
-        case AJ43_PRE:      // from (xbar_f, k5bar) in (X0, K1) slots: RHS5 input = k5bar
-        case AJ43_IPRE: {   // initial k1 = t v(x0): input = k1bar
-          kb = J[JJ_K1 * VEC + o];
-          hpart += ip(kb, Q[(STAGE == AJ43_PRE ? RR_K5 : RR_K1) * VEC + o]) / (double)t;
-        } break;
-        case AJ43_S5: {     // xbar_f += Xbar5; distribute to x2, k1'', k2', k3', k4
-          const cplx<R> xfb = cadd(J[JJ_X0 * VEC + o], Xb);
-          J[JJ_X2 * VEC + o] = xfb;
-          J[JJ_K1PP * VEC + o] = cdiv_k<6>(cscale(xfb, h));
-          J[JJ_K2P * VEC + o] = cdiv_k<3>(cscale(xfb, h));
-          J[JJ_K3P * VEC + o] = cdiv_k<3>(cscale(xfb, h));
-          kb = cdiv_k<6>(cscale(xfb, h));                       // k4bar
-          hpart += ip(kb, Q[RR_K4 * VEC + o]) / (double)t;
-        } break;
-        case AJ43_S4: {     // Y4 = x2 + h k3'
-          const cplx<R> x2b = cadd(J[JJ_X2 * VEC + o], Xb);
-          const cplx<R> k3pb = cadd(J[JJ_K3P * VEC + o], cscale(Xb, h));
-          const cplx<R> k2pb = J[JJ_K2P * VEC + o], k1ppb = J[JJ_K1PP * VEC + o];
-          const cplx<R> x0 = Q[RR_X0 * VEC + o], k1 = Q[RR_K1 * VEC + o];
-          const double eb = ip(k3pb, Q[RR_K3 * VEC + o]) + ip(k2pb, Q[RR_K2 * VEC + o]) +
-                            ip(k1ppb, cscale(k1, e)) + ip(x2b, cscale(x0, e));
-          hpart += eb * (double)dedt;
-          kb = cscale(k3pb, e);                                    // k3bar
-          hpart += ip(kb, Q[RR_K3 * VEC + o]) / (double)t;
-          J[JJ_K2 * VEC + o] = cscale(k2pb, e);                    // k2bar (partial)
-          J[JJ_K1P * VEC + o] = cscale(k1ppb, e);                  // k1'bar (partial)
-          J[JJ_XB * VEC + o] = cscale(x2b, e);                     // xbar (partial)
-        } break;
-        case AJ43_S3: {     // Y3 = x + h k2/2
-          J[JJ_XB * VEC + o] = cadd(J[JJ_XB * VEC + o], Xb);
-          kb = cadd(J[JJ_K2 * VEC + o], cscale(cscale(Xb, h), R(0.5)));   // k2bar final
-          hpart += ip(kb, Q[RR_K2 * VEC + o]) / (double)t;
-        } break;
-        case AJ43_S2: {     // Y2 = x + h k1'/2; then x0bar, k1bar of this attempt
-          const cplx<R> xbb = cadd(J[JJ_XB * VEC + o], Xb);
-          const cplx<R> k1pb = cadd(J[JJ_K1P * VEC + o], cscale(cscale(Xb, h), R(0.5)));
-          const double eb = ip(k1pb, Q[RR_K1 * VEC + o]) + ip(xbb, Q[RR_X0 * VEC + o]);
-          hpart += eb * (double)dedt;
-          J[JJ_X0 * VEC + o] = cscale(xbb, e);
-          J[JJ_K1 * VEC + o] = cscale(k1pb, e);
-          feed = false;
-        } break;
-        default: {          // AJ43_INIT: initial k1 = t v(x0): x0bar += Xbar
-          J[JJ_X0 * VEC + o] = cadd(J[JJ_X0 * VEC + o], Xb);
-          feed = false;
-        } break;
-      }
-      kb = cscale(kb, t);
-    }
-    // lambda = kb; the product multipliers vanish at (0,0), which the mask removes
-    lam[j] = cdiv_r(kb, cky);
+      // lambda = kb; the product multipliers vanish at (0,0), which the mask removes
+      lam[i] = cscale(kb, ky == 0 ? R(1) : R(0.5));   // kb / c_ky, exactly
   }
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) hpart += __shfl_xor_sync(0xffffffffu, hpart, o);
-  if (lane == 0) p.hacc[((size_t)b * K + ky) * 2 + ch] += hpart;
-  if (!feed) return;
-  // unscaled inverses Re sum mult_f lam e^{ik.x} (the row pass doubles ky > 0):
-  // P1bar, P2bar from channel w, P3bar from channel j
-  if (ch == 0) {
-    cplx<R> z0[E], z1[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-      z0[j] = cscale(lam[j], prod_mult<R>(0, kx, ky));
-      z1[j] = cscale(lam[j], prod_mult<R>(1, kx, ky));
-    }
-    fft_dit2<R, N, true>(z0, z1, s_tw, lane);
-    cplx<R>* g0 = p.G + ((size_t)(b * NG + 0) * K + ky) * N;
-    cplx<R>* g1 = g0 + (size_t)K * N;
-#pragma unroll
-    for (int j = 0; j < E; ++j) { g0[lane + 32 * j] = z0[j]; g1[lane + 32 * j] = z1[j]; }
-  } else {
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-      lam[j] = cscale(lam[j], prod_mult<R>(2, kx, ky));
-    }
-    col_inverse1<R, N>(lam, p.G, NG, b, 2, ky, lane, s_tw, R(1));
-  }
+  col_hacc(p.hacc, id, true, xf, hpart + hdiv / (double)(rk43 ? t : h));
+  if (STAGE == AJ43_S2 || STAGE == AJ43_INIT || (STAGE == AJ_S1 && !Qp)) return;   // nothing follows
+  col_adj_emit(lam, p.G, b, ch, ky, true, xf);
 }
 
 // Rejected Lawson-RK4(3) attempt in reverse: k1_next = e (e k1) ((e, e L h/2) from the attempt's record).

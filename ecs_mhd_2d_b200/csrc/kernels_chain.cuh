@@ -9,17 +9,17 @@
 // One thread-block cluster of CL = N / W CTAs of W warps serves one tangent
 // (W = 16: 8 CTAs at n = 128, a portable cluster; W = 8: 16 CTAs, half the
 // warps per SM and no register cap below 255):
-//   * a column pass gives each warp fixed columns (ky, channel) of the box --
+//   * a column pass gives each warp a fixed column (ky, channel) of the box --
 //     column c of tangent b on warp c / CL of CTA c % CL -- and runs the same
-//     per-column body as k_col_tan (col_tan_body), so the arithmetic and the
-//     rounding are those of the launch-per-pass sweep;
+//     transforms and the same algebra per mode as k_col_tan (tan_algebra), so the
+//     arithmetic and the rounding are those of the launch-per-pass sweep;
 //   * a row pass gives CTA r the W physical rows W r .. W r + W - 1, one warp
 //     per row, and runs k_row_tan's body (row_tan_body) with W-row tiles;
 //   * a rejected attempt updates the tangent's carried k1 column by column on
-//     the same warps as the column passes (tan_reject_at).
+//     the same warps as the column passes (tan_reject_k1).
 // Consecutive passes of the same kind (column stages and rejects) touch only
 // the warp's own box rows, so they follow each other without a barrier (a
-// __syncwarp orders the lanes' writes before the next pass's staged reads).
+// __syncwarp orders the lanes' writes before the next pass's reads).
 // Between a column pass and a row pass the cluster synchronises with the
 // hardware cluster barrier (arrive.release / wait.acquire), whose
 // release/acquire makes one pass's writes visible to the next pass's readers on
@@ -27,19 +27,29 @@
 // that are co-scheduled by construction (a cluster), so no wait in this kernel
 // spins on memory.
 //
+// What bounds a chain is the length of one warp's path through a pass, and on that
+// path the instruction fetch: a pass is a straight line that every warp runs once, so
+// code that does not stay in the instruction caches comes from L2.  A column pass
+// therefore has ONE copy of its transforms for all stages, and only the algebra of the
+// stage is selected at run time; the operands of the algebra are in shared memory, or
+// on their way there before the forward transform starts.  Measured (one copy of the
+// column body per stage and operands staged per pass -> this): 256 Lawson-RK4 steps of one
+// state at n = 128 7.88 -> 6.84 ms, 1024 steps of 8 states at n = 64 16.1 -> 14.7 ms, an
+// adaptive solve of T = 0.5 at n = 128 5.1 -> 4.3 ms.
+//
 // The intermediate arrays between the passes travel one of two ways (template
 // flag DSM):
 //   * DSM = false: through global memory (G, H; L2-resident at these sizes);
 //   * DSM = true: through distributed shared memory -- a column pass writes its
 //     inverse transforms straight into the G tiles of the CTAs that own those
-//     physical rows (col_uv_to_tiles), and a row pass sends its H tile to the
+//     physical rows (col_to_tiles), and a row pass sends its H tile to the
 //     shared rows of the warps that transform those columns (scatter_h_tile),
 //     so neither array leaves the cluster.  The first pass of a launch reads and
 //     the last one writes global G / H, which carries the state from one launch
 //     to the next (a launch ends before a row pass, at a regeneration chunk).
 // With DSH (8-warp CTAs only, for shared-memory room) each column warp keeps its
-// column's tangent slots ([S_NSLOT][M]) in shared memory for the whole launch:
-// loaded at the start, written back to global D at the end.
+// column's state slots in shared memory for the whole launch: loaded at the start,
+// written back at the end.
 //
 // The same layout runs the primal: k_rk4_chain (fixed-step Lawson-RK4 steps)
 // and k_rk43_chain (adaptive attempts with the error norm and the accept/reject
@@ -67,32 +77,29 @@ template <int N, int W> __host__ __device__ constexpr int chain_cl() { return N 
 template <int N, int W> __host__ __device__ constexpr int chain_colwarps() {
   return (2 * ((N - 1) / 3 + 1) + chain_cl<N, W>() - 1) / chain_cl<N, W>();
 }
-// Operand rows staged per column warp: the largest col_tan_nop over the adaptive
-// stages (8), or, with the tangent slots in shared memory (DSH), the largest
-// number of record rows a stage reads (5, stage C).
-constexpr int CH_NOP = 8, CH_NOP_DSH = 5;
-// Shared-memory regions of a chain kernel (offsets in complex entries), with
-// `stage` complex entries of column staging per column warp: twiddles; with
-// DSM the G tile and the column warps' H rows; the column staging overlaid
-// with the row tiles; with DSH the column warps' tangent slots [S_NSLOT][M].
-template <int N, int W, bool DSM, bool DSH = false> struct ChainSmem {
-  static constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  static constexpr int CW = chain_colwarps<N, W>();
-  static constexpr int tw = 0;
-  static constexpr int gt = fft_smem(N, W);                        // G tile (DSM)
-  static constexpr int hc = gt + (DSM ? NG * K * (W + 1) : 0);     // column warps' H rows (DSM)
-  static constexpr int work = hc + (DSM ? CW * 2 * N : 0);         // staging / row tiles
-  static constexpr int row = (DSM ? NH : NG + NH) * K * (W + 1);
-  static constexpr int ds_at(int stage) { return work + (CW * stage > row ? CW * stage : row); }
-  static constexpr int end_at(int stage) { return ds_at(stage) + (DSH ? CW * S_NSLOT * M : 0); }
+// Shared-memory regions of a chain kernel (offsets in complex entries): tables; with DSM
+// the G tile and the column warps' H rows; a work area that the row tile (without DSM)
+// and the column warps' staged operand rows (STG rows of M each) take in turn; SLOTS
+// resident rows of M per column warp.
+template <typename R, int N, int W, bool DSM, int STG, int SLOTS> struct ChainSmem {
+  using X = Xf<R, N>;
+  static constexpr int K = X::K, M = X::M, CW = chain_colwarps<N, W>();
+  static constexpr int gt = X::smem(W);
+  static constexpr int hc = gt + (DSM ? NG * K * (W + 1) : 0);
+  static constexpr int work = hc + (DSM ? CW * 2 * N : 0);
+  static constexpr int row = DSM ? 0 : NG * K * (W + 1);
+  static constexpr int ds = work + (CW * STG * M > row ? CW * STG * M : row);
+  static constexpr size_t bytes = (size_t)(ds + CW * SLOTS * M) * sizeof(cplx<R>);
 };
-template <typename R, int N, int W, bool DSM, bool DSH = false>
-__host__ __device__ constexpr size_t chain_smem_for(int stage) {
-  return (size_t)ChainSmem<N, W, DSM, DSH>::end_at(stage) * sizeof(cplx<R>);
-}
-template <typename R, int N, int W, bool DSM, bool DSH = false> __host__ __device__ constexpr size_t chain_smem() {
-  return chain_smem_for<R, N, W, DSM, DSH>((DSH ? CH_NOP_DSH : CH_NOP) * (2 * ((N - 1) / 3) + 1));
-}
+// Staged rows: of the tangent sweep the record rows a stage reads (5, stage C) and,
+// unless the slots are resident, its slots (8 together); of an attempt of the primal
+// its slots (4), unless resident.  Lawson-RK4 steps keep F, A1, K2 and the real e.
+// Resident beside them: the column's multipliers, and of the primal its forcing.
+template <typename R, int N, int W, bool DSM, bool DSH>
+using TanChainSmem = ChainSmem<R, N, W, DSM, DSH ? 5 : 8, (DSH ? S_NSLOT : 0) + 1>;
+template <typename R, int N, int W, bool DSM> using Rk4ChainSmem = ChainSmem<R, N, W, DSM, 0, 6>;
+template <typename R, int N, int W>
+using Rk43ChainSmem = ChainSmem<R, N, W, false, W == 8 ? 0 : 4, (W == 8 ? S_NSLOT : 0) + 2>;
 
 template <typename R>
 struct ChainParams {
@@ -109,84 +116,144 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;\n" ::: "memory");
 }
 
-template <typename R, int N, int W, bool DSM, bool DSH>
-__device__ __forceinline__ void chain_col(const ChainParams<R>& P, const ChainOp& op, int b, int rank, int w,
-                                          int lane, const cplx<R>* s_tw, cplx<R>* my_op, const cplx<R>* hrows,
-                                          cplx<R>* gtile, cplx<R>* dsh) {
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+// The column that the calling warp owns in its state's column passes, or -1: warp w of
+// CTA `rank` owns column w CL + rank (channel its lowest bit).
+template <int N, int W> __device__ __forceinline__ int chain_column(int rank) {
+  const int w = (int)(threadIdx.x >> 5), c = w * chain_cl<N, W>() + rank;
+  return w < chain_colwarps<N, W>() && c < 2 * ((N - 1) / 3 + 1) ? c : -1;
+}
+
+// Rows `mask` of a column (row q at from + q pitch, M entries) on their way to
+// consecutive shared rows at `to`; returns the place after them.
+template <typename R, int M>
+__device__ __forceinline__ cplx<R>* stage_rows(cplx<R>* to, const cplx<R>* from, size_t pitch, unsigned mask) {
+  for (; mask; mask &= mask - 1) {
+    const cplx<R>* q = from + (__ffs((int)mask) - 1) * pitch;
+    for (int s = threadIdx.x & 31; s < M; s += 32) cp_async_c<R>(to + s, q + s);
+    to += M;
+  }
+  return to;
+}
+// A resident row of a column's table, as TableRow reads one.
+template <typename R> struct SharedRow {
+  const cplx<R>* s;
+  __device__ __forceinline__ cplx<R> operator()(int slot) const { return s[slot]; }
+};
+__device__ __forceinline__ void staged_wait() {
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+  __syncwarp();
+}
+
+// The derivative of a column from its product rows: the warp's shared rows `hrows`, or
+// (null) global H; one copy of the transforms.
+template <class X>
+__device__ __forceinline__ void chain_rhs(const cplx<typename X::R>* H, const ColId<X>& id, const X& xf,
+                                          const cplx<typename X::R>* hrows, cplx<typename X::R> (&r)[X::E]) {
+  const cplx<typename X::R>* h0 =
+      hrows ? hrows : H + ((size_t)(id.b * NH + (id.ch == 0 ? 0 : 2)) * X::K + id.ky) * X::N;
+  col_rhs_rows(h0, h0 + (hrows ? (size_t)X::N : (size_t)X::K * X::N), id.ch, id.ky, xf, r);
+}
+
+// The stage's algebra on the lane's modes; ops(std::integral_constant of the stage).
+template <int STAGE, bool DSH, class X>
+__device__ __forceinline__ void chain_tan_algebra(const TanCol<typename X::R>& c, typename X::R coeff, const ColId<X>& id,
+                                                  const X& xf, const cplx<typename X::R>* rows, cplx<typename X::R>* D,
+                                                  size_t DS, const cplx<typename X::R> (&r)[X::E],
+                                                  cplx<typename X::R> (&x)[X::E]) {
+  using R = typename X::R;
+  constexpr int M = X::M;
+  constexpr unsigned DM = tan_dmask(STAGE), QM = tan_qmask(STAGE), QM2 = tan_qmask2(STAGE);
+  constexpr int NQ = popc_c(QM), NQ2 = popc_c(QM2);
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    x[i] = tan_algebra<STAGE>(c, diss_L<R>(xf.kx(i), (R)id.ky, coeff), !(slot == 0 && id.ky == 0),
+                              tan_has_rhs(STAGE) ? r[i] : mk<R>(0, 0), slot,
+                              [&](int q) { return rows[bit_rank(QM, q) * M + slot]; },
+                              [&](int q) { return rows[(NQ + bit_rank(QM2, q)) * M + slot]; },
+                              [&](int d) { return DSH ? D[d * M + slot] : rows[(NQ + NQ2 + bit_rank(DM, d)) * M + slot]; },
+                              [&](int d, cplx<R> v) { D[d * DS + slot] = v; });
+  }
+}
+
+template <int W, bool DSM, bool DSH, class X>
+__device__ __forceinline__ void chain_col(const ChainParams<typename X::R>& P, const ChainOp& op, TanCol<typename X::R> c,
+                                          const ColId<X>& id, const X& xf, const cplx<typename X::R>* hrows,
+                                          cplx<typename X::R>* gtile, cplx<typename X::R>* dsh, cplx<typename X::R>* rows,
+                                          const SharedRow<typename X::R>& mu) {
+  using R = typename X::R;
+  constexpr int K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  constexpr int CL = chain_cl<N, W>();
-  const int c = w * CL + rank;   // this warp's column of the tangent
-  if (w >= chain_colwarps<N, W>() || c >= 2 * K) return;
-  const int colid = b * 2 * K + c;
-  ColTanParams<R> p = P.col;
-  p.rec = P.rec + (size_t)op.rec * VEC;
-  p.rec2 = P.rec + (size_t)op.rec2 * VEC;
-  p.h = op.h;
-  p.stage = op.stage;
-  p.produce = op.produce;
+  const ColTanParams<R>& p = P.col;
+  c.h = (R)op.h;   // (the adaptive stages use dpar / t, not dpar / h)
+  const size_t at = ((size_t)id.ch * K + id.ky) * M;
+  cplx<R>* D = DSH ? dsh : p.D + (size_t)id.b * p.nslot * VEC + at;
+  constexpr size_t DS = DSH ? (size_t)M : VEC;
+  const cplx<R>* rec = P.rec + (size_t)op.rec * VEC;
   if (op.kind == CH_REJECT) {
-    const int ch = c & 1, ky = c >> 1;
-    cplx<R>* Db = p.D + (size_t)b * p.nslot * VEC;
-    const R dpar = (R)(p.dT[b] * p.dscale);
-    for (int s = lane; s < M; s += 32) {
-      const size_t o = ((size_t)ch * K + ky) * M + s;
-      if constexpr (DSH) dsh[S_K1 * M + s] = tan_reject_k1<R>(p.rec, VEC, o, dpar, dsh[S_K1 * M + s]);
-      else tan_reject_at<R>(Db, p.rec, VEC, o, dpar);
-    }
+    for (int s = xf.l; s < M; s += 32) D[S_K1 * DS + s] = tan_reject_k1<R>(rec, VEC, at + s, c.dpar, D[S_K1 * DS + s]);
     return;
   }
+  cplx<R>* to = stage_rows<R, M>(rows, rec + at, VEC, tan_qmask(op.stage));
+  to = stage_rows<R, M>(to, P.rec + (size_t)op.rec2 * VEC + at, VEC, tan_qmask2(op.stage));
+  if constexpr (!DSH) stage_rows<R, M>(to, D, VEC, tan_dmask(op.stage));
+  cplx<R> r[X::E], x[X::E];
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) r[i] = x[i] = mk<R>(0, 0);
+  if (tan_has_rhs(op.stage)) chain_rhs(p.H, id, xf, hrows, r);
+  staged_wait();
+  const R coeff = id.ch == 0 ? p.nu : p.eta;
   switch (op.stage) {
-    case T43_START: col_tan_body<R, N, T43_START, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_INIT: col_tan_body<R, N, T43_INIT, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_A: col_tan_body<R, N, T43_A, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_B: col_tan_body<R, N, T43_B, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_C: col_tan_body<R, N, T43_C, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_D: col_tan_body<R, N, T43_D, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    case T43_EA: col_tan_body<R, N, T43_EA, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
-    default: col_tan_body<R, N, T43_E, DSM ? W : 0, DSH>(p, colid, lane, s_tw, my_op, hrows, gtile, dsh); break;
+    case T43_START: chain_tan_algebra<T43_START, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_INIT: chain_tan_algebra<T43_INIT, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_A: chain_tan_algebra<T43_A, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_B: chain_tan_algebra<T43_B, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_C: chain_tan_algebra<T43_C, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_D: chain_tan_algebra<T43_D, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    case T43_EA: chain_tan_algebra<T43_EA, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
+    default: chain_tan_algebra<T43_E, DSH>(c, coeff, id, xf, rows, D, DS, r, x); break;
   }
+  if (op.produce && tan_has_input(op.stage))
+    col_inverse_uv<DSM ? W : 0>(x, p.G, id.b, id.ch, id.ky, true, xf, mu, gtile);
 }
 
 // Grid: B clusters of CL CTAs (cluster b = tangent b; the cluster shape is a
 // launch attribute), W * 32 threads each.
 template <typename R, int N, int W, bool DSM, bool DSH>
 __global__ void __launch_bounds__(W * 32, 1) k_tan_chain(ChainParams<R> P) {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
+  using X = Xf<R, N>;
+  constexpr int K = X::K, M = X::M, CL = chain_cl<N, W>();
   constexpr size_t VEC = (size_t)2 * K * M;
-  constexpr int CL = chain_cl<N, W>();
-  constexpr int NOPW = DSH ? CH_NOP_DSH : CH_NOP;
-  static_assert(N <= 128, "staged column operands need n <= 128");
-  static_assert(col_tan_nop<N, T43_C>() <= CH_NOP && col_tan_nop<N, T43_EA>() <= CH_NOP &&
-                col_tan_nop<N, T43_A>() <= CH_NOP && col_tan_nop<N, T43_D>() <= CH_NOP, "staging rows");
-  static_assert(popc_c(tan_qmask(T43_C)) <= CH_NOP_DSH && popc_c(tan_qmask(T43_EA)) + popc_c(tan_qmask2(T43_EA)) <= CH_NOP_DSH,
-                "record rows staged with the slots in shared memory");
-  using SM = ChainSmem<N, W, DSM, DSH>;
+  using SM = TanChainSmem<R, N, W, DSM, DSH>;
+  static_assert(DSH || popc_c(tan_qmask(T43_C)) + popc_c(tan_dmask(T43_C)) <= 8, "staged rows");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_tw = s_base + SM::tw;
   cplx<R>* s_gt = s_base + SM::gt;
-  cplx<R>* s_hc = s_base + SM::hc;
-  cplx<R>* s_work = s_base + SM::work;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const X xf(s_base, threadIdx.x >> 5);
   const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
-  const int wc = w < chain_colwarps<N, W>() ? w : 0;
-  const int cown = w * CL + rank;   // this warp's column (tangent slots in shared memory)
-  const bool owns = w < chain_colwarps<N, W>() && cown < 2 * K;
-  cplx<R>* dsh = s_base + SM::ds_at(NOPW * M) + (size_t)wc * S_NSLOT * M;
-  cplx<R>* dglob = P.col.D + (size_t)b * P.col.nslot * VEC + ((size_t)(cown & 1) * K + (cown >> 1)) * M;
-  load_twiddles<R, N>(s_tw, P.col.tw);
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  cplx<R>* my_h = s_base + SM::hc + (size_t)wc * 2 * N;
+  cplx<R>* my_rows = s_base + SM::work + (size_t)wc * (DSH ? 5 : 8) * M;
+  cplx<R>* my_mu = s_base + SM::ds + (size_t)wc * ((DSH ? S_NSLOT : 0) + 1) * M;
+  cplx<R>* dsh = my_mu + M;
+  cplx<R>* dglob = P.col.D + (size_t)b * P.col.nslot * VEC + ((size_t)id.ch * K + id.ky) * M;
+  load_tables<X>(s_base, P.col.tw);
   pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
-  if constexpr (DSH) {
-    if (owns)
+  if (cw >= 0) {
+    for (int e = xf.l; e < M; e += 32) my_mu[e] = mu_row<X>(P.col.tw, id.ky)[e];
+    if constexpr (DSH)
       for (int d = 0; d < S_NSLOT; ++d)
-        for (int e = lane; e < M; e += 32) dsh[d * M + e] = dglob[d * VEC + e];
+        for (int e = xf.l; e < M; e += 32) dsh[d * M + e] = dglob[d * VEC + e];
   }
+  const TanCol<R> tc(P.col, b, 0);
   __syncthreads();
-  cplx<R>* my_op = s_work + (size_t)wc * NOPW * M;
   int prev = -1;   // kind class of the previous pass: 0 column-like, 1 row
+  ChainOp next = P.ops[P.op0];
   for (int i = P.op0; i < P.op1; ++i) {
-    const ChainOp op = P.ops[i];
+    const ChainOp op = next;
+    if (i + 1 < P.op1) next = P.ops[i + 1];   // on its way during this pass
     const int cls = op.kind == CH_ROW ? 1 : 0;
     if (prev >= 0 && (cls != prev || cls == 1)) cluster_barrier();
     else if (prev >= 0) __syncwarp();
@@ -195,21 +262,18 @@ __global__ void __launch_bounds__(W * 32, 1) k_tan_chain(ChainParams<R> P) {
     if (cls) {
       RowTanParams<R> rp = P.row;
       rp.phys = P.phys + (size_t)(op.item - P.item0) * N * NPH * N;
-      if constexpr (DSM)
-        row_tan_body<R, N, W, true>(rp, b, rank * W, s_tw, s_gt, s_work, first, last ? nullptr : s_hc);
-      else
-        row_tan_body<R, N, W>(rp, b, rank * W, s_tw, s_work, s_work + NG * K * (W + 1));
-    } else {
-      chain_col<R, N, W, DSM, DSH>(P, op, b, rank, w, lane, s_tw, my_op,
-                                   (DSM && !first) ? s_hc + (size_t)wc * 2 * N : nullptr,
-                                   (DSM && !last) ? s_gt : nullptr, dsh);
+      cplx<R>* tile = DSM ? s_gt : s_base + SM::work;
+      row_tan_body<W, DSM>(rp, b, rank * W, xf, tile, tile, first, last ? nullptr : s_base + SM::hc);
+    } else if (cw >= 0) {
+      chain_col<W, DSM, DSH>(P, op, tc, id, xf, (DSM && !first) ? my_h : nullptr, (DSM && !last) ? s_gt : nullptr, dsh, my_rows,
+                             SharedRow<R>{my_mu});
     }
   }
   if constexpr (DSH) {   // the slots back to global memory for the next launch and the JVP output
     __syncwarp();
-    if (owns)
+    if (cw >= 0)
       for (int d = 0; d < S_NSLOT; ++d)
-        for (int e = lane; e < M; e += 32) dglob[d * VEC + e] = dsh[d * M + e];
+        for (int e = xf.l; e < M; e += 32) dglob[d * VEC + e] = dsh[d * M + e];
   }
   if constexpr (DSM) cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
 }
@@ -218,9 +282,10 @@ __global__ void __launch_bounds__(W * 32, 1) k_tan_chain(ChainParams<R> P) {
 // Lawson-RK4 steps of the primal (timestepping.lawson_rk4,
 // jax_scripts/lib/timestepping.py:69-80) in one launch: cluster b advances
 // state b through `steps` steps, each stage a row pass (k_row_rhs's body,
-// W-row tiles) and a column pass (k_col_rk4's body), with the same layout and
-// barriers as k_tan_chain.  The stage input of the first stage is in G (from a
-// COL_START column pass before the launch).
+// W-row tiles) and a column pass (k_col_rk4's transforms and algebra), with the same
+// layout and barriers as k_tan_chain.  The stage input of the first stage is in G (from
+// a COL_START column pass before the launch).  Each column warp keeps its column's
+// state, A1, K2, e, forcing and multipliers in shared memory; the state goes back to global F at the end.
 // ---------------------------------------------------------------------------
 template <typename R>
 struct Rk4ChainParams {
@@ -230,56 +295,79 @@ struct Rk4ChainParams {
   int last_produce;   // inverse transforms after the last stage (the next stage input)
 };
 
-// per column warp: 3 complex rows (F, A1, K2) and one real row (e), in complex units
-template <typename R, int N, int W, bool DSM> __host__ __device__ constexpr size_t rk4_chain_smem() {
-  return chain_smem_for<R, N, W, DSM>(4 * (2 * ((N - 1) / 3) + 1));
+template <int STAGE, class X>
+__device__ __forceinline__ void chain_rk4_algebra(const ColParams<typename X::R>& p, const ColId<X>& id, const X& xf,
+                                                  const Rk4Rows<typename X::R>& w, typename X::R h,
+                                                  const SharedRow<typename X::R>& forcing,
+                                                  const cplx<typename X::R> (&r)[X::E], cplx<typename X::R> (&x)[X::E]) {
+  using C = cplx<typename X::R>;
+  // loaded together: a load of a row cannot move over a store to another
+  C f[X::E], a1[X::E], k2[X::E];
+  typename X::R e[X::E];
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    f[i] = w.F[slot];
+    if (STAGE == COL_RK4_S3) { a1[i] = w.A1[slot]; k2[i] = w.K2[slot]; }
+    if (rk4_reads_e(STAGE)) e[i] = w.e[slot];
+  }
+  col_rk4_algebra<STAGE>(p, id, xf, w, h, [&](int q, int i, int) { return q == 0 ? f[i] : q == 1 ? a1[i] : k2[i]; },
+                         [&](int i, int) { return e[i]; }, forcing, r, x);
 }
 
 template <typename R, int N, int W, bool DSM>
 __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  constexpr int CL = chain_cl<N, W>();
-  static_assert(N <= 128, "staged column operands need n <= 128");
-  using SM = ChainSmem<N, W, DSM>;
+  using X = Xf<R, N>;
+  constexpr int M = X::M, CL = chain_cl<N, W>();
+  using SM = Rk4ChainSmem<R, N, W, DSM>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_tw = s_base + SM::tw;
   cplx<R>* s_gt = s_base + SM::gt;
   cplx<R>* s_hc = s_base + SM::hc;
-  cplx<R>* s_work = s_base + SM::work;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const X xf(s_base, threadIdx.x >> 5);
   const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
-  const int cidx = w * CL + rank;   // this warp's column of the state
-  const bool has_col = w < chain_colwarps<N, W>() && cidx < 2 * K;
-  const int colid = b * 2 * K + cidx;
-  cplx<R>* my_c = s_work + (size_t)(has_col ? w : 0) * 4 * M;
-  R* my_e = reinterpret_cast<R*>(my_c + 3 * M);
-  const cplx<R>* my_h = DSM ? s_hc + (size_t)(has_col ? w : 0) * 2 * N : nullptr;
-  load_twiddles<R, N>(s_tw, P.col.tw);
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  const size_t at = ((size_t)(b * 2 + id.ch) * X::K + id.ky) * M;
+  cplx<R>* my_s = s_base + SM::ds + (size_t)wc * 6 * M;
+  R* my_e = reinterpret_cast<R*>(my_s + 3 * M);
+  const SharedRow<R> forcing{my_s + 4 * M}, mu{my_s + 5 * M};
+  const Rk4Rows<R> w{my_s, my_s + M, my_s + 2 * M, my_e};
+  const cplx<R>* my_h = DSM ? s_hc + (size_t)wc * 2 * N : nullptr;
+  load_tables<X>(s_base, P.col.tw);
   pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) {
+      my_s[s] = P.col.F[at + s]; my_e[s] = P.col.Etab[at + s];
+      my_s[4 * M + s] = P.col.fhat[id.ky * M + s]; my_s[5 * M + s] = mu_row<X>(P.col.tw, id.ky)[s];
+    }
+  const R h = (R)P.col.ctl[b].h;
   __syncthreads();
   for (long step = 0; step < P.steps; ++step) {
+#pragma unroll 1
     for (int st = COL_RK4_S1; st <= COL_RK4_S4; ++st) {
       if (step > 0 || st > COL_RK4_S1) cluster_barrier();   // column pass -> row pass
       const bool first = step == 0 && st == COL_RK4_S1, last = step == P.steps - 1 && st == COL_RK4_S4;
-      if constexpr (DSM)
-        row_rhs_body<R, N, W, true>(P.row, b, rank * W, s_tw, s_gt, s_work, first, s_hc);
-      else
-        row_rhs_body<R, N, W>(P.row, b, rank * W, s_tw, s_work, s_work + NG * K * (W + 1));
+      cplx<R>* tile = DSM ? s_gt : s_base + SM::work;
+      row_rhs_body<W, DSM>(P.row, b, rank * W, xf, tile, tile, first, s_hc);
       cluster_barrier();                                     // row pass -> column pass
-      if (!has_col) continue;
-      ColParams<R> p = P.col;
-      p.stage = st;
-      p.produce = last ? P.last_produce : 1;
-      cplx<R>* gt = (DSM && !last) ? s_gt : nullptr;
+      if (cw < 0) continue;
+      cplx<R> r[X::E], x[X::E];
+      chain_rhs(P.col.H, id, xf, my_h, r);
       switch (st) {
-        case COL_RK4_S1: col_rk4_body<R, N, COL_RK4_S1, DSM ? W : 0>(p, colid, lane, s_tw, my_c, my_e, my_h, gt); break;
-        case COL_RK4_S2: col_rk4_body<R, N, COL_RK4_S2, DSM ? W : 0>(p, colid, lane, s_tw, my_c, my_e, my_h, gt); break;
-        case COL_RK4_S3: col_rk4_body<R, N, COL_RK4_S3, DSM ? W : 0>(p, colid, lane, s_tw, my_c, my_e, my_h, gt); break;
-        default: col_rk4_body<R, N, COL_RK4_S4, DSM ? W : 0>(p, colid, lane, s_tw, my_c, my_e, my_h, gt); break;
+        case COL_RK4_S1: chain_rk4_algebra<COL_RK4_S1>(P.col, id, xf, w, h, forcing, r, x); break;
+        case COL_RK4_S2: chain_rk4_algebra<COL_RK4_S2>(P.col, id, xf, w, h, forcing, r, x); break;
+        case COL_RK4_S3: chain_rk4_algebra<COL_RK4_S3>(P.col, id, xf, w, h, forcing, r, x); break;
+        default: chain_rk4_algebra<COL_RK4_S4>(P.col, id, xf, w, h, forcing, r, x); break;
       }
+      if (!last || P.last_produce)
+        col_inverse_uv<DSM ? W : 0>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, (DSM && !last) ? s_gt : nullptr);
     }
   }
+  __syncwarp();
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) P.col.F[at + s] = my_s[s];
   if constexpr (DSM) cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
 }
 
@@ -287,8 +375,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
 // Adaptive Lawson-RK4(3) attempts of the primal (timestepping.lawson_rk43,
 // jax_scripts/lib/timestepping.py:151-335) in one launch: cluster b runs state
 // b's attempts until it completes or `amax` attempts were made -- the column
-// stages A..E (k_col_rk43's body), the four RHS row passes (k_row_rhs's body)
-// and the error norm (k_row_err's body); each CTA's maximum goes to the
+// stages A..E (k_col_rk43's transforms and algebra), the four RHS row passes
+// (k_row_rhs's body) and the error norm (k_row_err's body); each CTA's maximum goes to the
 // cluster through distributed shared memory, CTA 0 makes the accept/reject
 // decision and the step-size update on the control block (rk43_control, as
 // the last block of k_row_err does), and every CTA reads it after the next
@@ -304,56 +392,95 @@ struct Rk43ChainParams {
   int* rec_acc;    // optional [B][cap] accept flags
   long amax;       // attempts at most
 };
-constexpr int CH_NOP43 = 5;   // rows staged per column warp by an attempt stage (slots + forcing)
 
-template <typename R, int N, int W> __host__ __device__ constexpr size_t rk43_chain_smem() {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  constexpr size_t col = (size_t)chain_colwarps<N, W>() * CH_NOP43 * M;
-  constexpr size_t row = (size_t)(NG + NH) * K * (W + 1);
-  return (fft_smem(N, W) + (col > row ? col : row)) * sizeof(cplx<R>);
+template <int STAGE, bool DSH, class X>
+__device__ __forceinline__ void chain_rk43_algebra(const Col43Params<typename X::R>& p, const R43Col<typename X::R>& c,
+                                                   const ColId<X>& id, const X& xf, const cplx<typename X::R>* rows,
+                                                   cplx<typename X::R>* S, size_t SS, const SharedRow<typename X::R>& forcing,
+                                                   const cplx<typename X::R> (&r)[X::E], cplx<typename X::R> (&x)[X::E]) {
+  using R = typename X::R;
+  constexpr size_t VEC = (size_t)2 * X::K * X::M;
+  constexpr int M = X::M;
+  constexpr unsigned SMASK = r43_smask(STAGE);
+  const R coeff = id.ch == 0 ? p.nu : p.eta;
+  const int ix = DSH ? (c.pend ? S_XF : S_X0) : 0, ik = DSH ? (c.pend ? S_K5 : S_K1) : 1;   // stage A
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    const cplx<R> v = STAGE == R43_A ? mk<R>(0, 0) : with_forcing<R>(r[i], forcing, id.ch, id.ky, slot);
+    cplx<R> xs = mk<R>(0, 0), ks = xs;
+    if constexpr (STAGE == R43_A) { xs = (DSH ? S : rows)[ix * M + slot]; ks = (DSH ? S : rows)[ik * M + slot]; }
+    x[i] = r43_algebra<STAGE>(c, diss_L<R>(xf.kx(i), (R)id.ky, coeff), v, xs, ks, VEC, slot,
+                              [&](int q) { return DSH ? S[q * M + slot] : rows[bit_rank(SMASK, q) * M + slot]; },
+                              [&](int q, cplx<R> a) { S[q * SS + slot] = a; });
+  }
 }
 
 template <typename R, int N, int W>
 __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  constexpr int CL = chain_cl<N, W>();
-  static_assert(N <= 128, "staged column operands need n <= 128");
-  static_assert(col_rk43_nop<N, R43_C>() <= CH_NOP43 && col_rk43_nop<N, R43_D>() <= CH_NOP43 &&
-                col_rk43_nop<N, R43_B>() <= CH_NOP43 && col_rk43_nop<N, R43_E>() <= CH_NOP43, "staging rows");
+  using X = Xf<R, N>;
+  constexpr int M = X::M, CL = chain_cl<N, W>();
+  constexpr size_t VEC = (size_t)2 * X::K * M;
+  constexpr bool DSH = W == 8;   // slots in shared memory
+  constexpr size_t SS = DSH ? (size_t)M : VEC;
+  using SM = Rk43ChainSmem<R, N, W>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_work = s_tw + fft_smem(N, W);
+  cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_work = s_base + SM::work;
   __shared__ double s_max[W];
   __shared__ double s_part;   // this CTA's error maximum, read by CTA 0 of the cluster
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const X xf(s_base, threadIdx.x >> 5);
   const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
-  const int cidx = w * CL + rank;   // this warp's column of the state
-  const bool has_col = w < chain_colwarps<N, W>() && cidx < 2 * K;
-  const int colid = b * 2 * K + cidx;
-  cplx<R>* my_op = s_work + (size_t)(has_col ? w : 0) * CH_NOP43 * M;
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  cplx<R>* sglob = P.col.S + (size_t)b * S_NSLOT * VEC + ((size_t)id.ch * X::K + id.ky) * M;
+  cplx<R>* my_s = s_base + SM::ds + (size_t)wc * ((DSH ? S_NSLOT : 0) + 2) * M;
+  const SharedRow<R> forcing{my_s}, mu{my_s + M};
+  cplx<R>* S = DSH ? my_s + 2 * M : sglob;
+  cplx<R>* rows = s_work + (size_t)wc * (DSH ? 0 : 4) * M;
   StepCtl* ctl = P.col.ctl + b;
-  load_twiddles<R, N>(s_tw, P.col.tw);
+  load_tables<X>(s_base, P.col.tw);
   pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (cw >= 0) {
+    for (int e = xf.l; e < M; e += 32) {
+      my_s[e] = P.col.fhat[id.ky * M + e];
+      my_s[M + e] = mu_row<X>(P.col.tw, id.ky)[e];
+    }
+    if constexpr (DSH)
+      for (int d = 0; d < S_NSLOT; ++d)
+        for (int e = xf.l; e < M; e += 32) S[d * M + e] = sglob[d * VEC + e];
+  }
   __syncthreads();
   for (long a = 0; a < P.amax; ++a) {
     if (*(volatile int*)&ctl->done) break;   // written by CTA 0 before the last cluster barrier
-    if (has_col) col_rk43_body<R, N, R43_A>(P.col, colid, lane, s_tw, my_op);
-    cluster_barrier();
+    const R43Col<R> c(P.col, b, id.ch, id.ky, VEC, X::K, M);
 #pragma unroll 1
-    for (int st = R43_B; st <= R43_E; ++st) {
-      row_rhs_body<R, N, W>(P.row, b, rank * W, s_tw, s_work, s_work + NG * K * (W + 1));
-      cluster_barrier();
-      if (has_col) {
+    for (int st = R43_A; st <= R43_E; ++st) {
+      if (st != R43_A) {
+        row_rhs_body<W>(P.row, b, rank * W, xf, s_work, s_work);
+        cluster_barrier();
+      }
+      if (cw >= 0) {
+        if constexpr (!DSH) stage_rows<R, M>(rows, sglob, VEC, st == R43_A ? r43_amask(c.pend) : r43_smask(st));
+        cplx<R> r[X::E], x[X::E];
+#pragma unroll
+        for (int i = 0; i < X::E; ++i) r[i] = x[i] = mk<R>(0, 0);
+        if (st != R43_A) chain_rhs(P.col.H, id, xf, (const cplx<R>*)nullptr, r);
+        if constexpr (!DSH) staged_wait();
         switch (st) {
-          case R43_B: col_rk43_body<R, N, R43_B>(P.col, colid, lane, s_tw, my_op); break;
-          case R43_C: col_rk43_body<R, N, R43_C>(P.col, colid, lane, s_tw, my_op); break;
-          case R43_D: col_rk43_body<R, N, R43_D>(P.col, colid, lane, s_tw, my_op); break;
-          default: col_rk43_body<R, N, R43_E>(P.col, colid, lane, s_tw, my_op); break;
+          case R43_A: chain_rk43_algebra<R43_A, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
+          case R43_B: chain_rk43_algebra<R43_B, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
+          case R43_C: chain_rk43_algebra<R43_C, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
+          case R43_D: chain_rk43_algebra<R43_D, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
+          default: chain_rk43_algebra<R43_E, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
         }
+        if (st == R43_E) col_inverse1(x, P.col.G, NG, b, id.ch, id.ky, true, xf, R(1) / (R(N) * R(N)));
+        else col_inverse_uv(x, P.col.G, b, id.ch, id.ky, true, xf, mu);
       }
       cluster_barrier();
     }
-    const double bm = row_err_max<R, N, W>(P.col.G, b, rank * W, s_tw, s_work, s_max);
+    const double bm = row_err_max<W>(P.col.G, b, rank * W, xf, s_work, s_max);
     if (threadIdx.x == 0) s_part = bm;
     cluster_barrier();
     if (rank == 0 && threadIdx.x == 0) {
@@ -368,6 +495,12 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
                    P.rec_acc && at < cap ? P.rec_acc + (size_t)b * cap : nullptr);
     }
     cluster_barrier();
+  }
+  if constexpr (DSH) {
+    __syncwarp();
+    if (cw >= 0)
+      for (int d = 0; d < S_NSLOT; ++d)
+        for (int e = xf.l; e < M; e += 32) sglob[d * VEC + e] = S[d * M + e];
   }
 }
 

@@ -14,6 +14,7 @@
 
 #include "kernels.cuh"
 #include "kernels_rk43.cuh"
+#include "kernels_adj.cuh"
 
 namespace ecs {
 
@@ -45,41 +46,59 @@ template <int SCHEME, int STAGE> struct FxTraits {
   static constexpr int last = SCHEME == FX_RK4 ? 4 : SCHEME == FX_RK6 ? 8 : 4;
 };
 
+// Slots that a stage reads before it writes any (bits of FxSlot); they are loaded
+// together before the stage's stores.
+__host__ __device__ constexpr unsigned fx_smask(int scheme, int stage) {
+  const unsigned F = 1u << X_F;
+  if (stage == 0) return F;
+  if (scheme == FX_RK4)
+    return F | (stage == 2 || stage == 4 ? 1u << X_K1 : 0u) | (stage >= 3 ? 1u << (X_K1 + 1) : 0u) |
+           (stage == 4 ? 1u << (X_K1 + 2) : 0u);
+  if (scheme == FX_RK6) return stage == 8 ? F | (1u << X_K1) | (1u << (X_K1 + 2)) | (1u << (X_K1 + 3)) |
+                                                (1u << (X_K1 + 5)) | (1u << (X_K1 + 6))
+                                          : F | (((1u << (stage - 1)) - 1u) << X_K1);
+  return stage == 1 ? F : stage == 2 ? F | (1u << X_K1) : stage == 3 ? 1u << X_FT
+       : F | (1u << X_K1) | (1u << X_A1) | (1u << X_K2T);
+}
+
 template <typename R, int N, int SCHEME, int STAGE>
-__global__ void __launch_bounds__(128) k_col_fx(ColFxParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fx(ColFxParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
   using Tr = FxTraits<SCHEME, STAGE>;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int c = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;   // one warp per (b, ky, channel)
+  ECS_COL_PROLOGUE(popc_c(fx_smask(SCHEME, STAGE)), 2);   // the forcing, the multipliers
+  const int c = id.ch, b = id.b, ky = id.ky;
   const R h = (R)p.ctl[b].h;
   const R coeff = c == 0 ? p.nu : p.eta;
-  cplx<R>* S = p.S + (size_t)b * S_NSLOT * VEC;
-  const R* Et = p.Etab + (size_t)b * VEC;
+  const size_t row = ((size_t)c * K + ky) * M;
+  cplx<R>* S = p.S + (size_t)b * S_NSLOT * VEC + row;
+  const R* Et = p.Etab + (size_t)b * VEC + row;
+  cplx<R>* rec = p.rec ? p.rec + row : nullptr;
+  constexpr unsigned SM = fx_smask(SCHEME, STAGE);
+  Operands<X, SM> op(rows);
+  op.begin(S, VEC);
+  constexpr int n = popc_c(SM);
+  const TableRow<X, Tr::rhs == 1 && rows_fit(n, 2)> forcing(rows + n * M, p.fhat + ky * M);
+  const TableRow<X, rows_fit(n, 2)> mu(rows + (n + 1) * M, mu_row<X>(p.tw, ky));
   cplx<R> r[E];
-  if (Tr::rhs) col_load_rhs<R, N>(p.H, b, c, ky, lane, s_tw, r);
+  if (Tr::rhs) col_load_rhs(p.H, b, c, ky, xf, r);
+  op.load(S, VEC, true, xf);
   cplx<R> x[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    x[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
+  for (int i = 0; i < E; ++i) {
+    x[i] = mk<R>(0, 0);
+    const int slot = xf.slot(i);
     if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const size_t o = ((size_t)c * K + ky) * M + slot;
-    auto Q = [&](int q) -> cplx<R>& { return S[q * VEC + o]; };
-    const R L = diss_L<R>(kx, ky, coeff);   // masked: zero at (0,0)
+    const R kx = xf.kx(i);
+    auto Q = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
+    auto W = [&](int q, cplx<R> a) { S[q * VEC + slot] = a; };
+    auto put = [&](int q, cplx<R> a) { if (rec) rec[q * VEC + slot] = a; };
+    const R L = diss_L<R>(kx, (R)ky, coeff);   // zero at (0,0)
     cplx<R> v = mk<R>(0, 0);
     if (Tr::rhs) {
-      v = r[j];
-      if (Tr::rhs == 1 && c == 0 && !(kx == 0 && ky == 0)) v = cadd(v, p.fhat[ky * M + slot]);
+      v = r[i];
+      if (Tr::rhs == 1 && c == 0 && !(slot == 0 && ky == 0)) v = cadd(v, forcing(slot));
     }
     cplx<R> xin = mk<R>(0, 0);
     if (STAGE == 0) {
@@ -92,115 +111,118 @@ __global__ void __launch_bounds__(128) k_col_fx(ColFxParams<R> p) {
       if (STAGE == 3) xs = cadd(f, cdiv_k<2>(Q(X_K1 + 1)));
       if (STAGE == 4) xs = cadd(f, Q(X_K1 + 2));
       const cplx<R> k = cscale(cadd(v, cscale(xs, L)), h);            // timestepping.py:40-43
-      if (p.rec) {   // record: f0, k_s, x_{s+1}
-        if (STAGE == 1) p.rec[o] = f;
-        p.rec[STAGE * VEC + o] = k;
-      }
+      // record: f0, k_s, x_{s+1}
+      if (STAGE == 1) put(0, f);
+      put(STAGE, k);
       if (STAGE < 4) {
-        Q(X_K1 + STAGE - 1) = k;
+        W(X_K1 + STAGE - 1, k);
         xin = STAGE < 3 ? cadd(f, cdiv_k<2>(k)) : cadd(f, k);
-        if (p.rec) p.rec[(4 + STAGE) * VEC + o] = xin;
+        put(4 + STAGE, xin);
       } else {
         const cplx<R> fn = cadd(cadd(cadd(cadd(f, cdiv_k<6>(Q(X_K1))), cdiv_k<3>(Q(X_K1 + 1))),
                                      cdiv_k<3>(Q(X_K1 + 2))), cdiv_k<6>(k));   // :44
-        Q(X_F) = fn;
+        W(X_F, fn);
         xin = fn;
       }
     } else if (SCHEME == FX_RK6) {
-      const R e = Et[o];
+      const R e = __ldg(Et + slot);
       const cplx<R> k = cscale(v, h);
-      auto K_ = [&](int s) -> cplx<R>& { return Q(X_K1 + s - 1); };
-      auto scale_all = [&](int upto) {   // f, k1..k_upto *= e
-        Q(X_F) = cscale(Q(X_F), e);
-        for (int s = 1; s <= upto; ++s) K_(s) = cscale(K_(s), e);
-      };
-      if (p.rec) {   // record: f0, k_s (before any factor)
-        if (STAGE == 1) p.rec[o] = Q(X_F);
-        p.rec[STAGE * VEC + o] = k;
+      // record: f0, k_s (before any factor)
+      if (STAGE == 1) put(0, Q(X_F));
+      put(STAGE, k);
+      // f, k1..k_{STAGE-1} and the new k, times e after stages 1, 3..7 and stored
+      constexpr bool SC = STAGE != 2 && STAGE != 8;
+      cplx<R> f = Q(X_F), K_[9];
+#pragma unroll
+      for (int q = 1; q < 9; ++q) K_[q] = mk<R>(0, 0);
+#pragma unroll
+      for (int q = 1; q < STAGE; ++q)
+        if ((SM >> (X_K1 + q - 1)) & 1u) K_[q] = Q(X_K1 + q - 1);
+      K_[STAGE] = k;
+      if (SC) {
+        f = cscale_rn(f, e);
+        W(X_F, f);
+#pragma unroll
+        for (int q = 1; q <= STAGE; ++q) { K_[q] = cscale_rn(K_[q], e); W(X_K1 + q - 1, K_[q]); }
+      } else if (STAGE == 2) {
+        W(X_K1 + 1, k);
       }
       switch (STAGE) {
         case 1:   // :110-112
-          K_(1) = k; scale_all(1);
-          xin = cadd(Q(X_F), cdiv_k<6>(K_(1)));
+          xin = cadd(f, cdiv_k<6>(K_[1]));
           break;
         case 2:   // :113
-          K_(2) = k;
-          xin = cadd(cadd(Q(X_F), cdiv_k<12>(K_(1))), cdiv_k<12>(K_(2)));
+          xin = cadd(cadd(f, cdiv_k<12>(K_[1])), cdiv_k<12>(K_[2]));
           break;
         case 3:   // :114-115
-          K_(3) = k; scale_all(3);
-          xin = cadd(csub(Q(X_F), cdiv_k<33>(cscale(K_(2), R(4)))), cdiv_k<11>(cscale(K_(3), R(5))));
+          xin = cadd(csub(f, cdiv_k<33>(cscale(K_[2], R(4)))), cdiv_k<11>(cscale(K_[3], R(5))));
           break;
         case 4:   // :116-117
-          K_(4) = k; scale_all(4);
-          xin = cadd(csub(csub(Q(X_F), cdiv_k<4>(K_(1))), cdiv_k<44>(cscale(K_(2), R(29)))),
-                     cdiv_k<22>(cscale(K_(3), R(31))));
+          xin = cadd(csub(csub(f, cdiv_k<4>(K_[1])), cdiv_k<44>(cscale(K_[2], R(29)))),
+                     cdiv_k<22>(cscale(K_[3], R(31))));
           break;
         case 5:   // :118-119
-          K_(5) = k; scale_all(5);
-          xin = cadd(cadd(csub(cadd(cadd(Q(X_F), cdiv_k<11>(cscale(K_(1), R(3)))), cdiv_k<33>(cscale(K_(2), R(8)))),
-                               cdiv_k<11>(cscale(K_(3), R(4)))), cdiv_k<11>(K_(4))),
-                     cdiv_k<33>(cscale(K_(5), R(14))));
+          xin = cadd(cadd(csub(cadd(cadd(f, cdiv_k<11>(cscale(K_[1], R(3)))), cdiv_k<33>(cscale(K_[2], R(8)))),
+                               cdiv_k<11>(cscale(K_[3], R(4)))), cdiv_k<11>(K_[4])),
+                     cdiv_k<33>(cscale(K_[5], R(14))));
           break;
         case 6:   // :120-121
-          K_(6) = k; scale_all(6);
-          xin = cadd(csub(cadd(cadd(csub(csub(Q(X_F), cdiv_k<48>(cscale(K_(1), R(17)))), cdiv_k<12>(cscale(K_(2), R(5)))),
-                                    K_(3)), K_(4)), cdiv_k<12>(cscale(K_(5), R(13)))),
-                     cdiv_k<16>(cscale(K_(6), R(11))));
+          xin = cadd(csub(cadd(cadd(csub(csub(f, cdiv_k<48>(cscale(K_[1], R(17)))), cdiv_k<12>(cscale(K_[2], R(5)))),
+                                    K_[3]), K_[4]), cdiv_k<12>(cscale(K_[5], R(13)))),
+                     cdiv_k<16>(cscale(K_[6], R(11))));
           break;
         case 7:   // :122-123
-          K_(7) = k; scale_all(7);
-          xin = cadd(csub(cadd(csub(csub(cadd(cadd(Q(X_F), cdiv_k<39>(cscale(K_(1), R(20)))),
-                                                  cdiv_k<39>(cscale(K_(2), R(12)))),
-                                             cdiv_k<39>(cscale(K_(3), R(31)))), cdiv_k<39>(K_(4))),
-                                   cdiv_k<39>(cscale(K_(5), R(34)))), cdiv_k<39>(cscale(K_(6), R(11)))),
-                     cdiv_k<39>(cscale(K_(7), R(16))));
+          xin = cadd(csub(cadd(csub(csub(cadd(cadd(f, cdiv_k<39>(cscale(K_[1], R(20)))),
+                                                  cdiv_k<39>(cscale(K_[2], R(12)))),
+                                             cdiv_k<39>(cscale(K_[3], R(31)))), cdiv_k<39>(K_[4])),
+                                   cdiv_k<39>(cscale(K_[5], R(34)))), cdiv_k<39>(cscale(K_[6], R(11)))),
+                     cdiv_k<39>(cscale(K_[7], R(16))));
           break;
         default: {   // 8: :124
           const R c1 = R(13) / R(200), c3 = R(4) / R(25), c4 = R(11) / R(40);
-          const cplx<R> fn = cadd(cadd(cadd(Q(X_F), cscale(cadd(K_(1), k), c1)), cscale(cadd(K_(3), K_(7)), c3)),
-                                  cscale(cadd(K_(4), K_(6)), c4));
-          Q(X_F) = fn;
+          const cplx<R> fn = cadd(cadd(cadd(f, cscale(cadd(K_[1], k), c1)), cscale(cadd(K_[3], K_[7]), c3)),
+                                  cscale(cadd(K_[4], K_[6]), c4));
+          W(X_F, fn);
           xin = fn;
         } break;
       }
-      if (p.rec && STAGE < 8) p.rec[(8 + STAGE) * VEC + o] = xin;   // the stage input x_{s+1}
+      if (STAGE < 8) put(8 + STAGE, xin);   // the stage input x_{s+1}
     } else {   // FX_TD4, timestepping.py:137-144; v_fn and its derivative include dissipation
       switch (STAGE) {
         case 1: {   // k1 = h v(f); next: the transforms of k1 (tangent input of jac(f, k1))
           const cplx<R> k1 = cscale(cadd(v, cscale(Q(X_F), L)), h);
-          Q(X_K1) = k1;
-          if (p.rec) { p.rec[TR_F * VEC + o] = Q(X_F); p.rec[TR_K1 * VEC + o] = k1; }
+          W(X_K1, k1);
+          put(TR_F, Q(X_F)); put(TR_K1, k1);
           xin = k1;
         } break;
         case 2: {   // a1 = h jac(f, k1); f_temp = f + k1/2 + a1/8
           const cplx<R> k1 = Q(X_K1);
           const cplx<R> a1 = cscale(cadd(v, cscale(k1, L)), h);
-          Q(X_A1) = a1;
+          W(X_A1, a1);
           const cplx<R> ft = cadd(cadd(Q(X_F), cdiv_k<2>(k1)), cdiv_k<8>(a1));
-          Q(X_FT) = ft;
-          if (p.rec) { p.rec[TR_A1 * VEC + o] = a1; p.rec[TR_FT * VEC + o] = ft; }
+          W(X_FT, ft);
+          put(TR_A1, a1); put(TR_FT, ft);
           xin = ft;
         } break;
         case 3: {   // k2 = h v(f_temp)
           const cplx<R> k2 = cscale(cadd(v, cscale(Q(X_FT), L)), h);
-          Q(X_K2T) = k2;
-          if (p.rec) p.rec[TR_K2 * VEC + o] = k2;
+          W(X_K2T, k2);
+          put(TR_K2, k2);
           xin = k2;
         } break;
         default: {  // a2 = h jac(f_temp, k2); f = f + k1 + a1/6 + a2/3
           const cplx<R> a2 = cscale(cadd(v, cscale(Q(X_K2T), L)), h);
-          if (p.rec) p.rec[TR_A2 * VEC + o] = a2;
+          put(TR_A2, a2);
           const cplx<R> fn = cadd(cadd(cadd(Q(X_F), Q(X_K1)), cdiv_k<6>(Q(X_A1))), cdiv_k<3>(a2));
-          Q(X_F) = fn;
+          W(X_F, fn);
           xin = fn;
         } break;
       }
     }
-    x[j] = xin;
+    x[i] = xin;
   }
   if (!p.produce) return;
-  col_inverse_uv<R, N>(x, p.G, b, c, ky, lane, s_tw);
+  col_inverse_uv(x, p.G, b, c, ky, id.act, xf, mu);
 }
 
 // ---------------------------------------------------------------------------
@@ -235,21 +257,22 @@ __device__ __forceinline__ void acc_tan_products(R u, R v, R bx, R by, R du, R d
   p3 += (u * dby + by * du) - (v * dbx + bx * dv);             // dP3
 }
 
+// The tile of Ga holds the H tile at the end (each group reads and writes its own
+// column of the tiles).
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32) k_row_tan2(RowTan2Params<R> p) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan2(RowTan2Params<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, L = X::L, K = X::K, F = K * (XT + 1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_Ga = s_tw + fft_smem(N, XT);
-  cplx<R>* s_Gb = s_Ga + NG * K * (XT + 1);
-  cplx<R>* s_H = s_Gb + NG * K * (XT + 1);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_Ga = s_x + X::smem(XT / X::G);
+  cplx<R>* s_Gb = s_Ga + NG * F;
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = x0 + w;
+  const int w = threadIdx.x / L;
+  const X xf(s_x, threadIdx.x >> 5);
   pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   pdl_wait();
   load_tile<R, N, XT>(s_Ga, p.Ga + (size_t)b * NG * K * N, NG * K, x0);
   load_tile<R, N, XT>(s_Gb, p.Gb + (size_t)b * NG * K * N, NG * K, x0);
@@ -260,31 +283,21 @@ __global__ void __launch_bounds__(XT * 32) k_row_tan2(RowTan2Params<R> p) {
   for (int j = 0; j < E; ++j) { W[j] = mk<R>(0, 0); p3[j] = R(0); }
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {   // pass 0: Gb about phys_a; pass 1: Ga about phys_b
-    const cplx<R>* sg = pass == 0 ? s_Gb : s_Ga;
-    const R* ph = phys_row<R, N>(pass == 0 ? p.phys_a : p.phys_b, x);
+    const cplx<R>* ph = phys_row<R, N>(pass == 0 ? p.phys_a : p.phys_b, x0 + w) + xf.l;
     cplx<R> duv[E], dbb[E];
+    row_inverse<XT>(pass == 0 ? s_Gb : s_Ga, w, xf, duv, dbb);
 #pragma unroll
     for (int j = 0; j < E; ++j) {
-      const int q = lane + 32 * j;
-      duv[j] = packed_pair<R, N, XT>(sg + 0 * K * (XT + 1), sg + 1 * K * (XT + 1), q, w);
-      dbb[j] = packed_pair<R, N, XT>(sg + 2 * K * (XT + 1), sg + 3 * K * (XT + 1), q, w);
-    }
-    fft_dif2<R, N, true>(duv, dbb, s_tw, lane);
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = lane + 32 * j;
-      acc_tan_products<R>(ph[e], ph[N + e], ph[2 * N + e], ph[3 * N + e], duv[j].x, duv[j].y, dbb[j].x, dbb[j].y,
-                          W[j], p3[j]);
+      const cplx<R> uv = ph[L * j], bb = ph[N + L * j];
+      acc_tan_products<R>(uv.x, uv.y, bb.x, bb.y, duv[j].x, duv[j].y, dbb[j].x, dbb[j].y, W[j], p3[j]);
     }
   }
   cplx<R> Z[E];
 #pragma unroll
   for (int j = 0; j < E; ++j) Z[j] = mk<R>(p3[j], R(0));
-  fft_dit2<R, N, false>(W, Z, s_tw, lane);
-  split_store<R, N, XT>(W, s_H, s_H + K * (XT + 1), w, lane);
-  store_one<R, N, XT>(Z, s_H + 2 * K * (XT + 1), w, lane);
+  row_forward<XT>(W, Z, s_Ga, w, xf);
   __syncthreads();
-  store_tile<R, N, XT>(p.H + (size_t)b * NH * K * N, s_H, NH * K, x0);
+  store_tile<R, N, XT>(p.H + (size_t)b * NH * K * N, s_Ga, NH * K, x0);
 }
 
 enum TdTanSlot { DT_F = 0, DT_K1, DT_A1, DT_FT, DT_K2, DT_NSLOT };
@@ -304,64 +317,70 @@ struct ColTdjParams {
   int B, produce;
 };
 
+__host__ __device__ constexpr unsigned tdj_dmask(int stage) {   // slots read (bits of TdTanSlot)
+  return stage <= 1 ? 1u << DT_F : stage == 2 ? (1u << DT_F) | (1u << DT_K1) : stage == 3 ? 1u << DT_FT
+       : (1u << DT_F) | (1u << DT_K1) | (1u << DT_A1) | (1u << DT_K2);
+}
+
 template <typename R, int N, int STAGE>
-__global__ void __launch_bounds__(128) k_col_tdj(ColTdjParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_tdj(ColTdjParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int c = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;
-  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec;
+  ECS_COL_PROLOGUE(popc_c(tdj_dmask(STAGE)), 2);   // the record row, the multipliers
+  const int c = id.ch, b = id.b, ky = id.ky;
+  const size_t row = ((size_t)c * K + ky) * M;
+  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + row;
   const R h = (R)p.h;
   const R dpar = (R)(p.dT[b] * p.dscale);   // dh
+  const R dpar_h = dpar / h;
   const R coeff = c == 0 ? p.nu : p.eta;
+  constexpr unsigned DM = tdj_dmask(STAGE);
+  Operands<X, DM> op(rows);
+  op.begin(D, VEC);
+  constexpr int QV = STAGE == 1 ? (int)TR_K1 : STAGE == 2 ? (int)TR_A1 : STAGE == 3 ? (int)TR_K2 : (int)TR_A2;
+  const TableRow<X, STAGE != 0> rq(rows + popc_c(DM) * M, Q + QV * VEC);
+  const TableRow<X, true> mu(rows + (popc_c(DM) + 1) * M, mu_row<X>(p.tw, ky));
   cplx<R> r[E];
-  if (STAGE != 0) col_load_rhs<R, N>(p.H, b, c, ky, lane, s_tw, r);
+  if (STAGE != 0) col_load_rhs(p.H, b, c, ky, xf, r);
+  op.load(D, VEC, true, xf);
   cplx<R> x[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    x[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const size_t o = ((size_t)c * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    auto Dq = [&](int q) -> cplx<R>& { return D[q * VEC + o]; };
-    // d(h X) = (dh/h) (h X) + h dX, with the recorded h X and dX = r + L dx (no forcing)
-    auto dk = [&](int q, cplx<R> dxin) { return cadd(cscale(Q[q * VEC + o], dpar / h), cscale(cadd(r[j], cscale(dxin, L)), h)); };
-    cplx<R> xin = mk<R>(0, 0);
-    switch (STAGE) {
-      case 0: xin = Dq(DT_F); break;
-      case 1: { const cplx<R> dk1 = dk(TR_K1, Dq(DT_F)); Dq(DT_K1) = dk1; xin = dk1; } break;
-      case 2: {
-        const cplx<R> dk1 = Dq(DT_K1);
-        const cplx<R> da1 = dk(TR_A1, dk1);
-        Dq(DT_A1) = da1;
-        const cplx<R> dft = cadd(cadd(Dq(DT_F), cdiv_k<2>(dk1)), cdiv_k<8>(da1));
-        Dq(DT_FT) = dft;
-        xin = dft;
-      } break;
-      case 3: { const cplx<R> dk2 = dk(TR_K2, Dq(DT_FT)); Dq(DT_K2) = dk2; xin = dk2; } break;
-      default: {
-        const cplx<R> da2 = dk(TR_A2, Dq(DT_K2));
-        const cplx<R> dfn = cadd(cadd(cadd(Dq(DT_F), Dq(DT_K1)), cdiv_k<6>(Dq(DT_A1))), cdiv_k<3>(da2));
-        Dq(DT_F) = dfn;
-        xin = dfn;
-      } break;
-    }
-    x[j] = xin;
+  for (int i = 0; i < E; ++i) {
+      x[i] = mk<R>(0, 0);
+      const int slot = xf.slot(i);
+      if (slot < 0) continue;
+      const R L = diss_L<R>(xf.kx(i), (R)ky, coeff);
+      auto DV = [&](int d) -> cplx<R> { return op.get(d, i, slot); };
+      auto DW = [&](int d, cplx<R> v) { D[d * VEC + slot] = v; };
+      // d(h X) = (dh/h) (h X) + h dX, with the recorded h X and dX = r + L dx (no forcing)
+      auto dk = [&](cplx<R> dxin) { return cadd(cscale(rq(slot), dpar_h), cscale(cadd(r[i], cscale(dxin, L)), h)); };
+      cplx<R> xin = mk<R>(0, 0);
+      switch (STAGE) {
+        case 0: xin = DV(DT_F); break;
+        case 1: { const cplx<R> dk1 = dk(DV(DT_F)); DW(DT_K1, dk1); xin = dk1; } break;
+        case 2: {
+          const cplx<R> dk1 = DV(DT_K1);
+          const cplx<R> da1 = dk(dk1);
+          DW(DT_A1, da1);
+          const cplx<R> dft = cadd(cadd(DV(DT_F), cdiv_k<2>(dk1)), cdiv_k<8>(da1));
+          DW(DT_FT, dft);
+          xin = dft;
+        } break;
+        case 3: { const cplx<R> dk2 = dk(DV(DT_FT)); DW(DT_K2, dk2); xin = dk2; } break;
+        default: {
+          const cplx<R> da2 = dk(DV(DT_K2));
+          const cplx<R> dfn = cadd(cadd(cadd(DV(DT_F), DV(DT_K1)), cdiv_k<6>(DV(DT_A1))), cdiv_k<3>(da2));
+          DW(DT_F, dfn);
+          xin = dfn;
+        } break;
+      }
+      x[i] = xin;
   }
   if (!p.produce) return;
   // dk1, dk2 go to Gb (paired with the point f / f_temp); df, dft, df' to Ga
-  col_inverse_uv<R, N>(x, (STAGE == 1 || STAGE == 3) ? p.Gb : p.Ga, b, c, ky, lane, s_tw);
+  col_inverse_uv(x, (STAGE == 1 || STAGE == 3) ? p.Gb : p.Ga, b, c, ky, id.act, xf, mu);
 }
 
 // ---------------------------------------------------------------------------
@@ -387,46 +406,32 @@ struct RowAdj2Params {
 };
 
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32) k_row_adj2(RowAdj2Params<R> p) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj2(RowAdj2Params<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, L = X::L, K = X::K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_tw + fft_smem(N, XT);
-  cplx<R>* s_H = s_G + 3 * K * (XT + 1);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_G = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = x0 + w;
+  const int w = threadIdx.x / L;
+  const X xf(s_x, threadIdx.x >> 5);
   pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   pdl_wait();
   load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, 3 * K, x0);
   __syncthreads();
   cplx<R> P12[E], P3[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    P12[j] = packed_pair<R, N, XT>(s_G, s_G + K * (XT + 1), lane + 32 * j, w);
-    P3[j] = packed_one<R, N, XT>(s_G + 2 * K * (XT + 1), lane + 32 * j, w);
-  }
-  fft_dif2<R, N, true>(P12, P3, s_tw, lane);
+  row_inverse<XT, true>(s_G, w, xf, P12, P3);
 #pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
-    const R* ph = phys_row<R, N>(pass == 0 ? p.phys_a : p.phys_b, x);
+    const cplx<R>* ph = phys_row<R, N>(pass == 0 ? p.phys_a : p.phys_b, x0 + w) + xf.l;
     cplx<R> A[E], Bv[E];
 #pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = lane + 32 * j;
-      const R p1 = P12[j].x, p2 = P12[j].y, p3 = P3[j].x;
-      const R u = ph[e], v = ph[N + e], bx = ph[2 * N + e], by = ph[3 * N + e];
-      A[j] = mk<R>(R(2) * u * p1 - v * p2 + by * p3, -R(2) * v * p1 - u * p2 - bx * p3);     // (ubar, vbar)
-      Bv[j] = mk<R>(-R(2) * bx * p1 + by * p2 - v * p3, R(2) * by * p1 + bx * p2 + u * p3);  // (Bxbar, Bybar)
-    }
-    fft_dit2<R, N, false>(A, Bv, s_tw, lane);
-    split_store<R, N, XT>(A, s_H, s_H + K * (XT + 1), w, lane);
-    split_store<R, N, XT>(Bv, s_H + 2 * K * (XT + 1), s_H + 3 * K * (XT + 1), w, lane);
+    for (int j = 0; j < E; ++j) row_adj_product<R>(P12[j], P3[j].x, ph[L * j], ph[N + L * j], A[j], Bv[j]);
+    row_forward<XT, true>(A, Bv, s_G, w, xf);
     __syncthreads();
-    store_tile<R, N, XT>((pass == 0 ? p.Ha : p.Hb) + (size_t)b * NHA * K * N, s_H, NHA * K, x0);
+    store_tile<R, N, XT>((pass == 0 ? p.Ha : p.Hb) + (size_t)b * NHA * K * N, s_G, NHA * K, x0);
     __syncthreads();
   }
 }
@@ -449,133 +454,89 @@ struct ColTdaParams {
   int B;
 };
 
-// (c_ky/n^2) sum_m (-i mu_m) rfft2 of the adjoint rows of channel c in H: the box cotangent N'(P)^T lambda.
-template <typename R, int N>
-__device__ __forceinline__ void col_adj_xb(const cplx<R>* __restrict__ H, int b, int c, int ky, int lane,
-                                           const cplx<R>* s_tw, cplx<R> (&xb)[N / 32]) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
-  const cplx<R>* h0 = H + ((size_t)(b * NHA + 2 * c) * K + ky) * N;
-  const cplx<R>* h1 = h0 + (size_t)K * N;
-  cplx<R> v1[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) { xb[j] = h0[lane + 32 * j]; v1[j] = h1[lane + 32 * j]; }
-  fft_dif2<R, N, false>(xb, v1, s_tw, lane);
-  const R cky = ky == 0 ? R(1) : R(2);
-  const R inv_n2 = R(1) / (R(N) * R(N));
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-    xb[j] = cscale(cadd(cimul(xb[j], -spectral_mu<R>(2, kx, ky)), cimul(v1[j], -spectral_mu<R>(3, kx, ky))), cky * inv_n2);
-  }
-}
-
-// Inverse column transforms of lambda/c_ky times the product multipliers: the
-// product cotangents P1bar, P2bar (channel w) or P3bar (channel j) in G.
-template <typename R, int N>
-__device__ __forceinline__ void col_adj_emit(cplx<R> (&lam)[N / 32], cplx<R>* __restrict__ G, int b, int c, int ky,
-                                             int lane, const cplx<R>* s_tw) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
-  if (c == 0) {
-    cplx<R> z0[E], z1[E];
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-      z0[j] = cscale(lam[j], prod_mult<R>(0, kx, ky));
-      z1[j] = cscale(lam[j], prod_mult<R>(1, kx, ky));
-    }
-    fft_dit2<R, N, true>(z0, z1, s_tw, lane);
-    cplx<R>* g0 = G + ((size_t)(b * NG + 0) * K + ky) * N;
-    cplx<R>* g1 = g0 + (size_t)K * N;
-#pragma unroll
-    for (int j = 0; j < E; ++j) { g0[lane + 32 * j] = z0[j]; g1[lane + 32 * j] = z1[j]; }
-  } else {
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int kx = pos_to_k(spec_pos<N>(lane, j), N);
-      lam[j] = cscale(lam[j], prod_mult<R>(2, kx, ky));
-    }
-    col_inverse1<R, N>(lam, G, NG, b, 2, ky, lane, s_tw, R(1));
-  }
+__host__ __device__ constexpr unsigned tda_jmask(int stage) {   // slots read (bits of TdAdjSlot)
+  return stage == TA_SEED ? 1u << JT_F
+       : stage == TA_B ? 1u << JT_A2
+       : stage == TA_C ? (1u << JT_F) | (1u << JT_K1) | (1u << JT_A1) | (1u << JT_FT) | (1u << JT_K2)
+       : stage == TA_D ? (1u << JT_F) | (1u << JT_K1) | (1u << JT_A1) : (1u << JT_F) | (1u << JT_K1);
 }
 
 template <typename R, int N, int STAGE>
-__global__ void __launch_bounds__(128) k_col_tda(ColTdaParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_tda(ColTdaParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int c = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;
-  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec;
+  ECS_COL_PROLOGUE(popc_c(tda_jmask(STAGE)), 2);   // the record row, the multipliers
+  const int c = id.ch, b = id.b, ky = id.ky;
+  const size_t row = ((size_t)c * K + ky) * M;
+  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + row;
   const R h = (R)p.h;
   const R coeff = c == 0 ? p.nu : p.eta;
-  const R cky = ky == 0 ? R(1) : R(2);
+  constexpr unsigned JM = tda_jmask(STAGE);
+  Operands<X, JM> op(rows);
+  op.begin(J, VEC);
+  constexpr int QV = STAGE == TA_SEED ? (int)TR_A2 : STAGE == TA_B ? (int)TR_K2 : STAGE == TA_C ? (int)TR_A1 : (int)TR_K1;
+  const TableRow<X, STAGE != TA_E> rq(rows + popc_c(JM) * M, Q + QV * VEC);
+  const TableRow<X, STAGE != TA_SEED> mu(rows + (popc_c(JM) + 1) * M, mu_row<X>(p.tw, ky));
   cplx<R> xa[E], xbb[E];
-  if (STAGE != TA_SEED) col_adj_xb<R, N>(p.Ha, b, c, ky, lane, s_tw, xa);
-  if (STAGE == TA_B || STAGE == TA_D) col_adj_xb<R, N>(p.Hb, b, c, ky, lane, s_tw, xbb);
-  double hpart = 0.0;
+  if (STAGE != TA_SEED) col_adj_xb(p.Ha, b, c, ky, xf, mu, xa);
+  if (STAGE == TA_B || STAGE == TA_D) col_adj_xb(p.Hb, b, c, ky, xf, mu, xbb);
+  op.load(J, VEC, true, xf);
+  double hdiv = 0.0;   // the terms over h
   cplx<R> lam[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    lam[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const size_t o = ((size_t)c * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    auto Jq = [&](int q) -> cplx<R>& { return J[q * VEC + o]; };
-    auto ip = [&](cplx<R> a, cplx<R> bb) { return (double)a.x * (double)bb.x + (double)a.y * (double)bb.y; };
-    cplx<R> kb = mk<R>(0, 0);   // cotangent whose h-multiple feeds the next adjoint pass
-    switch (STAGE) {
-      case TA_SEED: {
-        const cplx<R> fb = Jq(JT_F);
-        const cplx<R> a2b = cdiv_k<3>(fb);
-        Jq(JT_A2) = a2b; Jq(JT_K1) = fb; Jq(JT_A1) = cdiv_k<6>(fb);
-        hpart += ip(a2b, Q[TR_A2 * VEC + o]) / (double)h;
-        kb = a2b;
-      } break;
-      case TA_B: {
-        const cplx<R> k2b = cadd(xa[j], cscale(Jq(JT_A2), h * L));
-        Jq(JT_K2) = k2b; Jq(JT_FT) = xbb[j];
-        hpart += ip(k2b, Q[TR_K2 * VEC + o]) / (double)h;
-        kb = k2b;
-      } break;
-      case TA_C: {
-        const cplx<R> ftb = cadd(cadd(Jq(JT_FT), xa[j]), cscale(Jq(JT_K2), h * L));
-        Jq(JT_F) = cadd(Jq(JT_F), ftb);
-        Jq(JT_K1) = cadd(Jq(JT_K1), cdiv_k<2>(ftb));
-        const cplx<R> a1b = cadd(Jq(JT_A1), cdiv_k<8>(ftb));
-        Jq(JT_A1) = a1b;
-        hpart += ip(a1b, Q[TR_A1 * VEC + o]) / (double)h;
-        kb = a1b;
-      } break;
-      case TA_D: {
-        const cplx<R> k1b = cadd(cadd(Jq(JT_K1), xa[j]), cscale(Jq(JT_A1), h * L));
-        Jq(JT_K1) = k1b;
-        Jq(JT_F) = cadd(Jq(JT_F), xbb[j]);
-        hpart += ip(k1b, Q[TR_K1 * VEC + o]) / (double)h;
-        kb = k1b;
-      } break;
-      default: {   // TA_E: the cotangent of the step's start state
-        Jq(JT_F) = cadd(cadd(Jq(JT_F), xa[j]), cscale(Jq(JT_K1), h * L));
-      } break;
-    }
-    lam[j] = cdiv_r(cscale(kb, h), cky);
+  for (int i = 0; i < E; ++i) {
+      lam[i] = mk<R>(0, 0);
+      const int slot = xf.slot(i);
+      if (slot < 0) continue;
+      const R L = diss_L<R>(xf.kx(i), (R)ky, coeff);
+      auto JV = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
+      auto JW = [&](int q, cplx<R> v) { J[q * VEC + slot] = v; };
+      auto ip = [&](cplx<R> a) {
+        const cplx<R> v = rq(slot);
+        return (double)a.x * (double)v.x + (double)a.y * (double)v.y;
+      };
+      cplx<R> kb = mk<R>(0, 0);   // cotangent whose h-multiple feeds the next adjoint pass
+      switch (STAGE) {
+        case TA_SEED: {
+          const cplx<R> fb = JV(JT_F);
+          const cplx<R> a2b = cdiv_k<3>(fb);
+          JW(JT_A2, a2b); JW(JT_K1, fb); JW(JT_A1, cdiv_k<6>(fb));
+          hdiv += ip(a2b);
+          kb = a2b;
+        } break;
+        case TA_B: {
+          const cplx<R> k2b = cadd(xa[i], cscale(JV(JT_A2), h * L));
+          JW(JT_K2, k2b); JW(JT_FT, xbb[i]);
+          hdiv += ip(k2b);
+          kb = k2b;
+        } break;
+        case TA_C: {
+          const cplx<R> ftb = cadd(cadd(JV(JT_FT), xa[i]), cscale(JV(JT_K2), h * L));
+          JW(JT_F, cadd(JV(JT_F), ftb));
+          JW(JT_K1, cadd(JV(JT_K1), cdiv_k<2>(ftb)));
+          const cplx<R> a1b = cadd(JV(JT_A1), cdiv_k<8>(ftb));
+          JW(JT_A1, a1b);
+          hdiv += ip(a1b);
+          kb = a1b;
+        } break;
+        case TA_D: {
+          const cplx<R> k1b = cadd(cadd(JV(JT_K1), xa[i]), cscale(JV(JT_A1), h * L));
+          JW(JT_K1, k1b);
+          JW(JT_F, cadd(JV(JT_F), xbb[i]));
+          hdiv += ip(k1b);
+          kb = k1b;
+        } break;
+        default: {   // TA_E: the cotangent of the step's start state
+          JW(JT_F, cadd(cadd(JV(JT_F), xa[i]), cscale(JV(JT_K1), h * L)));
+        } break;
+      }
+      lam[i] = cscale(cscale(kb, h), ky == 0 ? R(1) : R(0.5));   // h kb / c_ky
   }
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) hpart += __shfl_xor_sync(0xffffffffu, hpart, off);
-  if (lane == 0) p.hacc[((size_t)b * K + ky) * 2 + c] += hpart;
+  col_hacc(p.hacc, id, id.act, xf, hdiv / (double)h);
   if (STAGE == TA_E) return;
-  col_adj_emit<R, N>(lam, p.G, b, c, ky, lane, s_tw);
+  col_adj_emit(lam, p.G, b, c, ky, id.act, xf);
 }
 
 // Box entries back into the full half spectrum, leaving every other entry as it is
@@ -635,7 +596,7 @@ __global__ void k_fx_setup(const double* T, int nc, int ms, int div, StepCtl* ct
     if (i % per == 0) { ctl[b].t = tseg; ctl[b].h = (double)h; }
     const int slot = i % g.M; const long r = i / g.M; const int ky = r % g.K; const int c = (r / g.K) & 1;
     const int kx = slot_to_kx(slot, g.kmax, g.M);
-    const R L = diss_L<R>(kx, ky, (R)(c == 0 ? nu : eta));
+    const R L = diss_L<R>((R)kx, (R)ky, (R)(c == 0 ? nu : eta));
     const bool msk = !(kx == 0 && ky == 0);
     Etab[i] = msk ? exp(h / R(div) * L) : R(0);
   }

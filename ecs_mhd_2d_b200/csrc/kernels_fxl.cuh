@@ -101,68 +101,78 @@ struct ColFxtParams {
   int B, produce;
 };
 
+// Slots that stage s reads before its stores: df0, the stage input (with the
+// dissipation in v), and the dk_j of the next stage input's weights.
+__host__ __device__ constexpr unsigned fxt_dmask(int scheme, int s) {
+  unsigned m = 1u << FT_F;
+  if (s == 0) return m;
+  if (fxl_diss_in_v(scheme) && s > 1) m |= 1u << FT_X;
+  for (int j = 1; j < s; ++j)
+    if (fxl_a(scheme, s + 1, j) != 0.0) m |= 1u << (FT_K1 + j - 1);
+  return m;
+}
+
 template <typename R, int N, int SCHEME, int STAGE>
-__global__ void __launch_bounds__(128) k_col_fxt(ColFxtParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fxt(ColFxtParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
   constexpr int S = fxl_stages(SCHEME);
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int c = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;
-  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec;
+  ECS_COL_PROLOGUE(popc_c(fxt_dmask(SCHEME, STAGE)), 1);   // the multipliers
+  const int c = id.ch, b = id.b, ky = id.ky;
+  const size_t row = ((size_t)c * K + ky) * M;
+  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + row;
   const R h = (R)p.h;
   const R dh = (R)(p.dT[b] * p.dscale);
+  const R dh_h = dh / h;
   const R coeff = c == 0 ? p.nu : p.eta;
+  constexpr unsigned DM = fxt_dmask(SCHEME, STAGE);
+  Operands<X, DM> op(rows);
+  op.begin(D, VEC);
+  const TableRow<X, rows_fit(popc_c(DM), 1)> mu(rows + popc_c(DM) * M, mu_row<X>(p.tw, ky));
   cplx<R> r[E];
-  if (STAGE > 0) col_load_rhs<R, N>(p.H, b, c, ky, lane, s_tw, r);
+  if (STAGE > 0) col_load_rhs(p.H, b, c, ky, xf, r);
+  op.load(D, VEC, true, xf);
   cplx<R> x[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    x[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const size_t o = ((size_t)c * K + ky) * M + slot;
-    auto Dq = [&](int q) -> cplx<R>& { return D[q * VEC + o]; };
-    auto Qv = [&](int q) -> cplx<R> { return Q[q * VEC + o]; };
-    if (STAGE == 0) {
-      x[j] = Dq(FT_F);
-      continue;
-    }
-    const R L = diss_L<R>(kx, ky, coeff);   // masked: zero at (0,0)
-    const bool msk = !(kx == 0 && ky == 0);
-    // the integrating factor of the linearisation's step (as k_fx_setup forms it)
-    const R e = SCHEME == FX_RK6 ? (msk ? exp(h / R(6) * L) : R(0)) : R(1);
-    const R cf = R(fxl_tau(SCHEME)) * L * dh;   // d(e^m) = m cf e^m
-    cplx<R> rv = r[j];                          // N'(x_s) dx_s (no forcing)
-    if (fxl_diss_in_v(SCHEME)) rv = cadd(rv, cscale(STAGE == 1 ? Dq(FT_F) : Dq(FT_X), L));
-    const cplx<R> dk = cadd(cscale(Qv(fxr_k(STAGE)), dh / h), cscale(rv, h));
-    Dq(FT_K1 + STAGE - 1) = dk;
-    constexpr int sn = STAGE + 1;               // S + 1: the step's result
-    constexpr int pn = fxl_p(SCHEME, sn);
-    cplx<R> acc = cscale(cadd(Dq(FT_F), cscale(Qv(fxr_f()), R(pn) * cf)), fxl_pow(e, pn));
+  for (int i = 0; i < E; ++i) {
+      x[i] = mk<R>(0, 0);
+      const int slot = xf.slot(i);
+      if (slot < 0) continue;
+      auto DV = [&](int d) -> cplx<R> { return op.get(d, i, slot); };
+      auto DW = [&](int d, cplx<R> v) { D[d * VEC + slot] = v; };
+      auto Qv = [&](int q) -> cplx<R> { return __ldg(Q + q * VEC + slot); };
+      if (STAGE == 0) {
+        x[i] = DV(FT_F);
+        continue;
+      }
+      const R L = diss_L<R>(xf.kx(i), (R)ky, coeff);   // zero at (0,0)
+      const bool msk = !(slot == 0 && ky == 0);
+      // the integrating factor of the linearisation's step (as k_fx_setup forms it)
+      const R e = SCHEME == FX_RK6 ? (msk ? exp(h / R(6) * L) : R(0)) : R(1);
+      const R cf = R(fxl_tau(SCHEME)) * L * dh;   // d(e^m) = m cf e^m
+      cplx<R> rv = r[i];                          // N'(x_s) dx_s (no forcing)
+      if constexpr (fxl_diss_in_v(SCHEME)) rv = cadd(rv, cscale(STAGE == 1 ? DV(FT_F) : DV(FT_X), L));
+      const cplx<R> dk = cadd(cscale(Qv(fxr_k(STAGE)), dh_h), cscale(rv, h));
+      DW(FT_K1 + STAGE - 1, dk);
+      constexpr int sn = STAGE + 1;               // S + 1: the step's result
+      constexpr int pn = fxl_p(SCHEME, sn);
+      cplx<R> acc = cscale(cadd(DV(FT_F), cscale(Qv(fxr_f()), R(pn) * cf)), fxl_pow(e, pn));
 #pragma unroll
-    for (int jj = 1; jj <= STAGE; ++jj) {
-      const double a = fxl_a(SCHEME, sn, jj);
-      if (a == 0.0) continue;
-      const int m = pn - fxl_p(SCHEME, jj);
-      const cplx<R> dkj = jj == STAGE ? dk : Dq(FT_K1 + jj - 1);
-      acc = cadd(acc, cscale(cadd(dkj, cscale(Qv(fxr_k(jj)), R(m) * cf)), R(a) * fxl_pow(e, m)));
-    }
-    if (STAGE < S) Dq(FT_X) = acc;
-    else Dq(FT_F) = acc;
-    x[j] = acc;
+      for (int q = 1; q <= STAGE; ++q) {
+        const double a = fxl_a(SCHEME, sn, q);
+        if (a == 0.0) continue;
+        const int m = pn - fxl_p(SCHEME, q);
+        const cplx<R> dkj = q == STAGE ? dk : DV(FT_K1 + q - 1);
+        acc = cadd(acc, cscale(cadd(dkj, cscale(Qv(fxr_k(q)), R(m) * cf)), R(a) * fxl_pow(e, m)));
+      }
+      if (STAGE < S) DW(FT_X, acc);
+      else DW(FT_F, acc);
+      x[i] = acc;
   }
   if (!p.produce) return;
-  col_inverse_uv<R, N>(x, p.G, b, c, ky, lane, s_tw);
+  col_inverse_uv(x, p.G, b, c, ky, id.act, xf, mu);
 }
 
 // ---------------------------------------------------------------------------
@@ -191,88 +201,99 @@ struct ColFxaParams {
   int B;
 };
 
+// Slots that a stage reads before its stores: f0bar, kbar_s and the kbar_j that
+// xbar_s is distributed to (and kbar_{s-1}, the next emission).
+__host__ __device__ constexpr unsigned fxa_jmask(int scheme, int s) {
+  unsigned m = 1u << FA_F;
+  if (s > fxl_stages(scheme)) return m;
+  m |= 1u << (FA_K1 + s - 1);
+  for (int j = 1; j < s; ++j)
+    if (fxl_a(scheme, s, j) != 0.0 || j == s - 1) m |= 1u << (FA_K1 + j - 1);
+  return m;
+}
+
 template <typename R, int N, int SCHEME, int STAGE>
-__global__ void __launch_bounds__(128) k_col_fxa(ColFxaParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fxa(ColFxaParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
   constexpr int S = fxl_stages(SCHEME);
   constexpr bool SEED = STAGE == S + 1;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  const int c = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;
-  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec;
+  ECS_COL_PROLOGUE(popc_c(fxa_jmask(SCHEME, STAGE)), 1);   // the multipliers
+  const int c = id.ch, b = id.b, ky = id.ky;
+  const size_t row = ((size_t)c * K + ky) * M;
+  cplx<R>* J = p.J + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + row;
   const R h = (R)p.h;
   const R coeff = c == 0 ? p.nu : p.eta;
-  const R cky = ky == 0 ? R(1) : R(2);
+  constexpr unsigned JM = fxa_jmask(SCHEME, STAGE);
+  Operands<X, JM> op(rows);
+  op.begin(J, VEC);
+  const TableRow<X, !SEED && rows_fit(popc_c(JM), 1)> mu(rows + popc_c(JM) * M, mu_row<X>(p.tw, ky));
   cplx<R> xa[E];
-  if (!SEED) col_adj_xb<R, N>(p.H, b, c, ky, lane, s_tw, xa);
-  double hpart = 0.0;
+  if (!SEED) col_adj_xb(p.H, b, c, ky, xf, mu, xa);
+  op.load(J, VEC, true, xf);
+  double hpart = 0.0, hdiv = 0.0;   // hdiv: the terms over h
   cplx<R> lam[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    lam[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const size_t o = ((size_t)c * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    const bool msk = !(kx == 0 && ky == 0);
-    const R e = SCHEME == FX_RK6 ? (msk ? exp(h / R(6) * L) : R(0)) : R(1);
-    const R tl = R(fxl_tau(SCHEME)) * L;        // d(e^m)/dh = m tl e^m
-    auto Jq = [&](int q) -> cplx<R>& { return J[q * VEC + o]; };
-    auto Qv = [&](int q) -> cplx<R> { return Q[q * VEC + o]; };
-    auto ip = [&](cplx<R> a, cplx<R> bb) { return (double)a.x * (double)bb.x + (double)a.y * (double)bb.y; };
-    cplx<R> kb = mk<R>(0, 0);   // the kbar whose h-multiple feeds the next adjoint row pass
-    if (SEED) {
-      constexpr int P = fxl_p(SCHEME, S + 1);
-      const cplx<R> fb = Jq(FA_F);
-      const R eP = fxl_pow(e, P);
-      Jq(FA_F) = cscale(fb, eP);
-      if (P > 0) hpart += ip(fb, cscale(Qv(fxr_f()), R(P) * tl * eP));
+  for (int i = 0; i < E; ++i) {
+      lam[i] = mk<R>(0, 0);
+      const int slot = xf.slot(i);
+      if (slot < 0) continue;
+      const R L = diss_L<R>(xf.kx(i), (R)ky, coeff);
+      const bool msk = !(slot == 0 && ky == 0);
+      const R e = SCHEME == FX_RK6 ? (msk ? exp(h / R(6) * L) : R(0)) : R(1);
+      const R tl = R(fxl_tau(SCHEME)) * L;        // d(e^m)/dh = m tl e^m
+      auto JV = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
+      auto JW = [&](int q, cplx<R> v) { J[q * VEC + slot] = v; };
+      auto Qv = [&](int q) -> cplx<R> { return __ldg(Q + q * VEC + slot); };
+      auto ip = [&](cplx<R> a, cplx<R> bb) { return (double)a.x * (double)bb.x + (double)a.y * (double)bb.y; };
+      cplx<R> kb = mk<R>(0, 0);   // the kbar whose h-multiple feeds the next adjoint row pass
+      if constexpr (SEED) {
+        constexpr int P = fxl_p(SCHEME, S + 1);
+        const cplx<R> fb = JV(FA_F);
+        const R eP = fxl_pow(e, P);
+        JW(FA_F, cscale(fb, eP));
+        if (P > 0) hpart += ip(fb, cscale(Qv(fxr_f()), R(P) * tl * eP));
 #pragma unroll
-      for (int jj = 1; jj <= S; ++jj) {
-        const double bw = fxl_a(SCHEME, S + 1, jj);
-        const int m = P - fxl_p(SCHEME, jj);
-        const R em = fxl_pow(e, m);
-        Jq(FA_K1 + jj - 1) = cscale(fb, R(bw) * em);
-        if (bw != 0.0 && m > 0) hpart += ip(fb, cscale(Qv(fxr_k(jj)), R(bw) * R(m) * tl * em));
-      }
-      kb = Jq(FA_K1 + S - 1);
-    } else {
-      constexpr int ps = fxl_p(SCHEME, STAGE);
-      const cplx<R> ks = Jq(FA_K1 + STAGE - 1);   // kbar_s, complete
-      hpart += ip(ks, Qv(fxr_k(STAGE))) / (double)h;
-      cplx<R> xb = xa[j];
-      if (fxl_diss_in_v(SCHEME)) xb = cadd(xb, cscale(ks, h * L));
-      const R eps = fxl_pow(e, ps);
-      Jq(FA_F) = cadd(Jq(FA_F), cscale(xb, eps));
-      if (ps > 0) hpart += ip(xb, cscale(Qv(fxr_f()), R(ps) * tl * eps));
+        for (int q = 1; q <= S; ++q) {
+          const double bw = fxl_a(SCHEME, S + 1, q);
+          const int m = P - fxl_p(SCHEME, q);
+          const R em = fxl_pow(e, m);
+          const cplx<R> kq = cscale(fb, R(bw) * em);
+          JW(FA_K1 + q - 1, kq);
+          if (bw != 0.0 && m > 0) hpart += ip(fb, cscale(Qv(fxr_k(q)), R(bw) * R(m) * tl * em));
+          if (q == S) kb = kq;
+        }
+      } else {
+        constexpr int ps = fxl_p(SCHEME, STAGE);
+        const cplx<R> ks = JV(FA_K1 + STAGE - 1);   // kbar_s, complete
+        hdiv += ip(ks, Qv(fxr_k(STAGE)));
+        cplx<R> xb = xa[i];
+        if (fxl_diss_in_v(SCHEME)) xb = cadd(xb, cscale(ks, h * L));
+        const R eps = fxl_pow(e, ps);
+        JW(FA_F, cadd(JV(FA_F), cscale(xb, eps)));
+        if (ps > 0) hpart += ip(xb, cscale(Qv(fxr_f()), R(ps) * tl * eps));
 #pragma unroll
-      for (int jj = 1; jj < STAGE; ++jj) {
-        const double a = fxl_a(SCHEME, STAGE, jj);
-        if (a == 0.0) continue;
-        const int m = ps - fxl_p(SCHEME, jj);
-        const R em = fxl_pow(e, m);
-        Jq(FA_K1 + jj - 1) = cadd(Jq(FA_K1 + jj - 1), cscale(xb, R(a) * em));
-        if (m > 0) hpart += ip(xb, cscale(Qv(fxr_k(jj)), R(a) * R(m) * tl * em));
+        for (int q = 1; q < STAGE; ++q) {
+          const double a = fxl_a(SCHEME, STAGE, q);
+          if (a == 0.0 && q < STAGE - 1) continue;
+          cplx<R> kq = JV(FA_K1 + q - 1);
+          if (a != 0.0) {
+            const int m = ps - fxl_p(SCHEME, q);
+            const R em = fxl_pow(e, m);
+            kq = cadd(kq, cscale(xb, R(a) * em));
+            JW(FA_K1 + q - 1, kq);
+            if (m > 0) hpart += ip(xb, cscale(Qv(fxr_k(q)), R(a) * R(m) * tl * em));
+          }
+          if (q == STAGE - 1) kb = kq;
+        }
       }
-      if (STAGE > 1) kb = Jq(FA_K1 + STAGE - 2);
-    }
-    lam[j] = cdiv_r(cscale(kb, h), cky);
+      lam[i] = cscale(cscale(kb, h), ky == 0 ? R(1) : R(0.5));   // h kb / c_ky
   }
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) hpart += __shfl_xor_sync(0xffffffffu, hpart, off);
-  if (lane == 0) p.hacc[((size_t)b * K + ky) * 2 + c] += hpart;
+  col_hacc(p.hacc, id, id.act, xf, hpart + hdiv / (double)h);
   if (STAGE == 1) return;
-  col_adj_emit<R, N>(lam, p.G, b, c, ky, lane, s_tw);
+  col_adj_emit(lam, p.G, b, c, ky, id.act, xf);
 }
 
 }  // namespace ecs

@@ -47,158 +47,147 @@ struct Col43Params {
   int B, stage;
 };
 
-// Slots (bits of Rk43Slot) that the algebra of an attempt stage reads after its
-// forward transform; they are staged per column into shared memory.
+// Slots (bits of Rk43Slot) that the algebra of an attempt stage reads; they are
+// loaded together before the stage's stores.
 __host__ __device__ constexpr unsigned r43_smask(int stage) {
-  return stage == R43_B ? (1u << S_XE)
+  return stage == R43_START ? (1u << S_X0)
+       : stage == R43_B ? (1u << S_XE)
        : stage == R43_C ? (1u << S_XE) | (1u << S_K1E) | (1u << S_K2) | (1u << S_E)
        : stage == R43_D ? (1u << S_K1) | (1u << S_K2) | (1u << S_K3) | (1u << S_X2)
        : stage == R43_E ? (1u << S_K4) : 0u;
 }
-__host__ __device__ constexpr int popc_r43(unsigned m) { return m ? (int)(m & 1u) + popc_r43(m >> 1) : 0; }
-
-// Slot rows staged per warp by an attempt stage (+ the forcing row), n <= 128.
-template <int N, int STAGE> __host__ __device__ constexpr int col_rk43_nop() {
-  return (N <= 128 && popc_r43(r43_smask(STAGE)) > 0) ? popc_r43(r43_smask(STAGE)) + 1 : 0;
+// What an attempt stage needs beside its operands: the candidate's step and the column's
+// record rows of the attempt (or null).
+template <typename R>
+struct R43Col {
+  R t, h;
+  int pend;
+  cplx<R>* rec;
+  __device__ __forceinline__ R43Col(const Col43Params<R>& p, int b, int ch, int ky, size_t VEC, int K, int M) {
+    const StepCtl& c = p.ctl[b];
+    t = (R)c.t; h = (R)c.h; pend = c.pending_accept;
+    rec = p.rec ? p.rec + ((size_t)b * p.cap + (c.attempts < p.cap ? c.attempts : p.cap - 1)) * RR_NREC * VEC +
+                      ((size_t)ch * K + ky) * M
+                : nullptr;
+  }
+};
+// Slots that stage A reads: the carried state and k1.
+__host__ __device__ constexpr unsigned r43_amask(int pend) {
+  return pend ? (1u << S_XF) | (1u << S_K5) : (1u << S_X0) | (1u << S_K1);
 }
 
-// One warp's column `colid` of an attempt stage; `my_op` is the warp's staging
-// buffer (col_rk43_nop rows of M entries).
-template <typename R, int N, int STAGE>
-__device__ __forceinline__ void col_rk43_body(const Col43Params<R>& p, int colid, int lane, const cplx<R>* s_tw,
-                                              cplx<R>* my_op) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__host__ __device__ constexpr unsigned r43_omask(int stage) { return stage == R43_A ? r43_amask(0) : r43_smask(stage); }
+
+// The algebra of an attempt stage at one mode: the stage input from the derivative v.
+// SV(q) reads and SW(q, a) writes slot q (stage A reads its two operands as xs and ks).
+template <int STAGE, typename R, class SVf, class SWf>
+__device__ __forceinline__ cplx<R> r43_algebra(const R43Col<R>& c, R L, cplx<R> v, cplx<R> xs, cplx<R> ks, size_t VEC,
+                                               int slot, SVf&& SV, SWf&& SW) {
+  const R t = c.t, h = c.h;
+  auto put = [&](int q, cplx<R> a) { if (c.rec) c.rec[q * VEC + slot] = a; };
+  const cplx<R> kv = cscale_rn(v, t);              // mod_vel_fn = t * vel_fn (timestepping.py:243)
+  cplx<R> xin = mk<R>(0, 0);
+  switch (STAGE) {
+    case R43_START: xin = SV(S_X0); break;
+    case R43_INIT: SW(S_K1, kv); break;
+    case R43_A: {                                  // :266-270
+      if (c.pend) { SW(S_X0, xs); SW(S_K1, ks); }
+      put(RR_X0, xs); put(RR_K1, ks);
+      const R e = exp((t * L) * h / R(2));         // e = exp(mod_L * h/2), not masked (:263)
+      const cplx<R> eg = mk<R>(e, e * (L * h * R(0.5)));
+      SW(S_E, eg);
+      put(RR_E, eg);
+      const cplx<R> xe = cscale_rn(xs, e), k1e = cscale_rn(ks, e);
+      SW(S_XE, xe); SW(S_K1E, k1e);
+      xin = cadd(xe, cscale(cscale_rn(k1e, h), R(0.5)));
+      put(RR_Y2, xin);
+    } break;
+    case R43_B: {                                  // :270-271
+      SW(S_K2, kv);
+      put(RR_K2, kv);
+      xin = cadd(SV(S_XE), cscale(cscale_rn(kv, h), R(0.5)));
+      put(RR_Y3, xin);
+    } break;
+    case R43_C: {                                  // :271-280
+      put(RR_K3, kv);
+      const R e = SV(S_E).x;
+      const cplx<R> x2 = cscale_rn(SV(S_XE), e);
+      const cplx<R> k1ee = cscale_rn(SV(S_K1E), e);
+      const cplx<R> k2e = cscale_rn(SV(S_K2), e);
+      const cplx<R> k3e = cscale_rn(kv, e);
+      SW(S_X2, x2); SW(S_K1, k1ee);                // k1 carried on rejection is e^2 k1 (:297)
+      SW(S_K2, k2e); SW(S_K3, k3e);
+      xin = cadd_scaled_rn(x2, k3e, h);
+      put(RR_Y4, xin);
+    } break;
+    case R43_D: {                                  // :280-281
+      SW(S_K4, kv);
+      put(RR_K4, kv);
+      const cplx<R> acc = cadd(cadd(cadd(cdiv_k<6>(SV(S_K1)), cdiv_k<3>(SV(S_K2))), cdiv_k<3>(SV(S_K3))), cdiv_k<6>(kv));
+      xin = cadd_scaled_rn(SV(S_X2), acc, h);
+      SW(S_XF, xin);
+      put(RR_XF, xin);
+    } break;
+    default: {                                     // R43_E: :282, :288
+      SW(S_K5, kv);
+      put(RR_K5, kv);
+      xin = cdiv_k<6>(cscale_rn(csub(kv, SV(S_K4)), h));
+    } break;
+  }
+  return xin;
+}
+
+// The derivative of channel ch at mode (slot, ky): r plus the forcing.
+template <typename R, class Forcing>
+__device__ __forceinline__ cplx<R> with_forcing(cplx<R> r, const Forcing& forcing, int ch, int ky, int slot) {
+  return ch == 0 && !(slot == 0 && ky == 0) ? cadd(r, forcing(slot)) : r;   // r is zero at (0,0)
+}
+
+// An attempt stage of one column; `rows`: shared room for its operands.
+template <int STAGE, class X>
+__device__ __forceinline__ void col_rk43_body(const Col43Params<typename X::R>& p, const ColId<X>& id, const X& xf,
+                                              cplx<typename X::R>* rows) {
+  using R = typename X::R;
+  constexpr int N = X::N, E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  const int ch = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;   // one warp per (b, ky, channel)
-  const StepCtl& c = p.ctl[b];
-  if (c.done) return;
-  const R t = (R)c.t, h = (R)c.h;
-  const int pend = c.pending_accept;
-  cplx<R>* S = p.S + (size_t)b * S_NSLOT * VEC;
-  cplx<R>* rec = p.rec ? p.rec + ((size_t)b * p.cap + (c.attempts < p.cap ? c.attempts : p.cap - 1)) * RR_NREC * VEC
-                       : nullptr;
-  const bool has_rhs = STAGE != R43_A && STAGE != R43_START;
-  // The slot rows (and, for the vorticity, the forcing row) that the algebra
-  // reads after the forward transform, copied into the warp's shared buffer
-  // with cp.async before it, so that their latency overlaps it (n <= 128).
-  constexpr unsigned SM = N <= 128 ? r43_smask(STAGE) : 0u;
-  constexpr int NS = popc_r43(SM), NOP = NS > 0 ? NS + 1 : 0;   // + the forcing row
-  if constexpr (NOP > 0) {
-    const size_t row = ((size_t)ch * K + ky) * M;
-    int v = 0;
-#pragma unroll
-    for (int bit = 0; bit < 16; ++bit) {
-      if ((SM >> bit) & 1u) {
-        for (int s2 = lane; s2 < M; s2 += 32) cp_async_v(my_op + v * M + s2, S + bit * VEC + row + s2);
-        ++v;
-      }
-    }
-    if (ch == 0)
-      for (int s2 = lane; s2 < M; s2 += 32) cp_async_v(my_op + NS * M + s2, p.fhat + ky * M + s2);
-  }
-  cplx<R> r[E];
-  if (has_rhs) col_load_rhs<R, N>(p.H, b, ch, ky, lane, s_tw, r);
-  if constexpr (NOP > 0) {
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncwarp();
-  }
-  // staged (or, without staging, global) slot values at a slot
-  auto SV = [&](int q, size_t o, int slot) -> cplx<R> {
-    if constexpr (NOP > 0) return my_op[popc_r43(SM & ((1u << q) - 1u)) * M + slot];
-    else return S[q * VEC + o];
-  };
+  const int ch = id.ch, b = id.b, ky = id.ky;
+  if (p.ctl[b].done) return;
+  const R43Col<R> c(p, b, ch, ky, VEC, K, M);
+  cplx<R>* S = p.S + (size_t)b * S_NSLOT * VEC + ((size_t)ch * K + ky) * M;
+  constexpr bool has_rhs = STAGE != R43_A && STAGE != R43_START;
+  constexpr int n = popc_c(r43_omask(STAGE));
+  Operands<X, r43_omask(STAGE)> op(rows);
+  const TableRow<X, has_rhs> forcing(rows + n * M, p.fhat + ky * M);
+  const TableRow<X, STAGE != R43_INIT && STAGE != R43_E> mu(rows + (n + 1) * M, mu_row<X>(p.tw, ky));
+  // stage A: the carried state and k1, which an accepted attempt left in S_XF and S_K5
+  const size_t at_x = STAGE == R43_A && c.pend ? (S_XF - S_X0) * VEC : 0, at_k = STAGE == R43_A && c.pend ? (S_K5 - S_K1) * VEC : 0;
+  auto from = [&](int q) { return S + q * VEC + (q == S_X0 ? at_x : at_k); };
+  if constexpr (STAGE == R43_A) op.begin(from); else op.begin(S, VEC);
+  cplx<R> r[E], x[E];
+  if (has_rhs) col_load_rhs(p.H, b, ch, ky, xf, r);
+  if constexpr (STAGE == R43_A) op.load(from, true, xf); else op.load(S, VEC, true, xf);
   const R coeff = ch == 0 ? p.nu : p.eta;
-  cplx<R> x[E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    x[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
+  for (int i = 0; i < E; ++i) {
+    x[i] = mk<R>(0, 0);
+    const int slot = xf.slot(i);
     if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    cplx<R> v = mk<R>(0, 0);
-    if (has_rhs) {
-      v = r[j];                                                        // zero at (0,0)
-      if (ch == 0 && !(kx == 0 && ky == 0)) {
-        if constexpr (NOP > 0) v = cadd(v, my_op[NS * M + slot]);
-        else v = cadd(v, p.fhat[ky * M + slot]);
-      }
-    }
-    const size_t o = ((size_t)ch * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    const cplx<R> kv = cscale_rn(v, t);              // mod_vel_fn = t * vel_fn (timestepping.py:243)
-    cplx<R> xin = mk<R>(0, 0);
-    switch (STAGE) {
-      case R43_START: xin = S[S_X0 * VEC + o]; break;
-      case R43_INIT: S[S_K1 * VEC + o] = kv; break;
-      case R43_A: {                                  // :266-270
-        const cplx<R> xs = pend ? S[S_XF * VEC + o] : S[S_X0 * VEC + o];
-        const cplx<R> ks = pend ? S[S_K5 * VEC + o] : S[S_K1 * VEC + o];
-        if (pend) { S[S_X0 * VEC + o] = xs; S[S_K1 * VEC + o] = ks; }
-        if (rec) { rec[RR_X0 * VEC + o] = xs; rec[RR_K1 * VEC + o] = ks; }
-        const R e = exp((t * L) * h / R(2));         // e = exp(mod_L * h/2), not masked (:263)
-        const cplx<R> eg = mk<R>(e, e * (L * h * R(0.5)));
-        S[S_E * VEC + o] = eg;
-        if (rec) rec[RR_E * VEC + o] = eg;
-        const cplx<R> xe = cscale_rn(xs, e), k1e = cscale_rn(ks, e);
-        S[S_XE * VEC + o] = xe; S[S_K1E * VEC + o] = k1e;
-        xin = cadd(xe, cscale(cscale_rn(k1e, h), R(0.5)));
-        if (rec) rec[RR_Y2 * VEC + o] = xin;
-      } break;
-      case R43_B: {                                  // :270-271
-        S[S_K2 * VEC + o] = kv;
-        if (rec) rec[RR_K2 * VEC + o] = kv;
-        xin = cadd(SV(S_XE, o, slot), cscale(cscale_rn(kv, h), R(0.5)));
-        if (rec) rec[RR_Y3 * VEC + o] = xin;
-      } break;
-      case R43_C: {                                  // :271-280
-        if (rec) rec[RR_K3 * VEC + o] = kv;
-        const R e = SV(S_E, o, slot).x;
-        const cplx<R> x2 = cscale_rn(SV(S_XE, o, slot), e);
-        const cplx<R> k1ee = cscale_rn(SV(S_K1E, o, slot), e);
-        const cplx<R> k2e = cscale_rn(SV(S_K2, o, slot), e);
-        const cplx<R> k3e = cscale_rn(kv, e);
-        S[S_X2 * VEC + o] = x2; S[S_K1 * VEC + o] = k1ee;   // k1 carried on rejection is e^2 k1 (:297)
-        S[S_K2 * VEC + o] = k2e; S[S_K3 * VEC + o] = k3e;
-        xin = cadd_scaled_rn(x2, k3e, h);
-        if (rec) rec[RR_Y4 * VEC + o] = xin;
-      } break;
-      case R43_D: {                                  // :280-281
-        S[S_K4 * VEC + o] = kv;
-        if (rec) rec[RR_K4 * VEC + o] = kv;
-        const cplx<R> acc = cadd(cadd(cadd(cdiv_k<6>(SV(S_K1, o, slot)), cdiv_k<3>(SV(S_K2, o, slot))),
-                                      cdiv_k<3>(SV(S_K3, o, slot))), cdiv_k<6>(kv));
-        xin = cadd_scaled_rn(SV(S_X2, o, slot), acc, h);
-        S[S_XF * VEC + o] = xin;
-        if (rec) rec[RR_XF * VEC + o] = xin;
-      } break;
-      default: {                                     // R43_E: :282, :288
-        S[S_K5 * VEC + o] = kv;
-        if (rec) rec[RR_K5 * VEC + o] = kv;
-        xin = cdiv_k<6>(cscale_rn(csub(kv, SV(S_K4, o, slot)), h));
-      } break;
-    }
-    x[j] = xin;
+    const cplx<R> v = has_rhs ? with_forcing<R>(r[i], forcing, ch, ky, slot) : mk<R>(0, 0);
+    x[i] = r43_algebra<STAGE>(c, diss_L<R>(xf.kx(i), (R)ky, coeff), v, STAGE == R43_A ? op.get(S_X0, i, slot) : mk<R>(0, 0),
+                              STAGE == R43_A ? op.get(S_K1, i, slot) : mk<R>(0, 0), VEC, slot,
+                              [&](int q) { return op.get(q, i, slot); },
+                              [&](int q, cplx<R> a) { S[q * VEC + slot] = a; });
   }
   if (STAGE == R43_INIT) return;
-  if (STAGE == R43_E) col_inverse1<R, N>(x, p.G, NG, b, ch, ky, lane, s_tw, R(1) / (R(N) * R(N)));
-  else col_inverse_uv<R, N>(x, p.G, b, ch, ky, lane, s_tw);
+  if (STAGE == R43_E) col_inverse1(x, p.G, NG, b, ch, ky, true, xf, R(1) / (R(N) * R(N)));
+  else col_inverse_uv(x, p.G, b, ch, ky, true, xf, mu);
 }
 
 template <typename R, int N, int STAGE>
-__global__ void __launch_bounds__(128) k_col_rk43(Col43Params<R> p) {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  constexpr int NOP = col_rk43_nop<N, STAGE>();
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  __shared__ __align__(16) cplx<R> s_op[(NOP > 0 ? NOP : 1) * 4 * M];   // 4 warps per CTA
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  col_rk43_body<R, N, STAGE>(p, colid, lane, s_tw, s_op + (threadIdx.x >> 5) * NOP * M);
+__global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_rk43(Col43Params<R> p) {
+  using X = Xf<R, N>;
+  ECS_COL_PROLOGUE(popc_c(r43_omask(STAGE)), 2);   // the forcing, the multipliers
+  col_rk43_body<STAGE>(p, id, xf, rows);
 }
 
 // Error norm max|irfft2(d)| of the two channels (timestepping.py:288-291) with
@@ -234,22 +223,21 @@ __device__ __forceinline__ void rk43_control(StepCtl& c, double atol, double err
 }
 
 // max |irfft2(d)| over rows x0 .. x0 + XT - 1 of state b (the inverse column
-// transforms of d in G fields 0 and 1), one warp per row; valid in thread 0.
-template <typename R, int N, int XT>
-__device__ __forceinline__ double row_err_max(const cplx<R>* G, int b, int x0, const cplx<R>* s_tw, cplx<R>* s_G,
-                                              double* s_max) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
-  load_tile<R, N, XT>(s_G, G + (size_t)b * NG * K * N, 2 * K, x0);
+// transforms of d in G fields 0 and 1), one group per row; s_max holds one value
+// per warp; valid in every thread.
+template <int XT, class X>
+__device__ __forceinline__ double row_err_max(const cplx<typename X::R>* G, int b, int x0, const X& xf,
+                                              cplx<typename X::R>* s_G, double* s_max) {
+  using R = typename X::R;
+  constexpr int N = X::N;
+  load_tile<R, N, XT>(s_G, G + (size_t)b * NG * X::K * N, 2 * X::K, x0);
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  cplx<R> z[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) z[j] = packed_pair<R, N, XT>(s_G, s_G + K * (XT + 1), lane + 32 * j, w);
-  fft_dif<R, N, true>(z, s_tw, lane);
+  cplx<R> z[X::E];
+  load_pair<XT>(s_G, s_G + X::K * (XT + 1), threadIdx.x / X::L, xf, z);
+  xf.template to_spec<true, true>(z);
   double m = 0.0;
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
+  for (int j = 0; j < X::E; ++j) {
     const double a = fabs((double)z[j].x), bb = fabs((double)z[j].y);
     m = (a > m || isnan(a)) ? a : m;
     m = (bb > m || isnan(bb)) ? bb : m;
@@ -259,28 +247,29 @@ __device__ __forceinline__ double row_err_max(const cplx<R>* G, int b, int x0, c
     const double q = __shfl_xor_sync(0xffffffffu, m, o);
     m = (q > m || isnan(q)) ? q : m;
   }
-  if (lane == 0) s_max[w] = m;
+  if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = m;
   __syncthreads();
   double bm = s_max[0];
-  for (int i = 1; i < XT; ++i) bm = (s_max[i] > bm || isnan(s_max[i])) ? s_max[i] : bm;
+  for (int i = 1; i < XT / X::G; ++i) bm = (s_max[i] > bm || isnan(s_max[i])) ? s_max[i] : bm;
   return bm;
 }
 
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32) k_row_err(RowErrParams<R> p) {
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_err(RowErrParams<R> p) {
+  using X = Xf<R, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_tw + fft_smem(N, XT);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_G = s_x + X::smem(XT / X::G);
   __shared__ double s_max[XT];
   __shared__ int s_last;
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
   pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   pdl_wait();
   StepCtl& c = p.ctl[b];
   if (c.done) return;
-  const double bm = row_err_max<R, N, XT>(p.G, b, x0, s_tw, s_G, s_max);
+  const double bm = row_err_max<XT>(p.G, b, x0, X(s_x, threadIdx.x >> 5), s_G, s_max);
   if (threadIdx.x == 0) {
     // non-negative doubles (and NaN with the sign bit clear) order like their bit patterns
     atomicMax(&c.err_bits, (unsigned long long)__double_as_longlong(fabs(bm)));

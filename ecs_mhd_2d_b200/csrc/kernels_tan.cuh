@@ -32,28 +32,29 @@ struct ColRegenParams {
 };
 
 template <typename R, int N>
-__global__ void __launch_bounds__(128) k_col_regen(ColRegenParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
+__global__ void __launch_bounds__(COLWARPS * 32) k_col_regen(ColRegenParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  load_twiddles<R, N>(s_tw, p.tw);
+  __shared__ __align__(16) cplx<R> s_x[X::smem(COLWARPS)];
+  load_tables<X>(s_x, p.tw);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int col = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (col >= p.nitems * K * 2) return;
-  const int ch = col & 1, ik = col >> 1, it = ik / K, ky = ik - it * K;   // one warp per (item, ky, channel)
-  const cplx<R>* y = p.rec + (size_t)p.items[it] * VEC + (size_t)(ch * K + ky) * M;
-  cplx<R> x[E];
+  const X xf(s_x, threadIdx.x >> 5);
+  const ColId<X> id(p.nitems);   // the items in the place of batch elements
+  if (id.none) return;
+  const cplx<R>* y = p.rec + (size_t)p.items[id.b] * VEC + (size_t)(id.ch * K + id.ky) * M;
+  cplx<R> x[X::E];
 #pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    x[j] = slot >= 0 ? y[slot] : mk<R>(0, 0);
+  for (int i = 0; i < X::E; ++i) {
+    x[i] = mk<R>(0, 0);
+    if (X::none(i)) continue;
+    const int slot = xf.slot(i);
+    if (slot >= 0) x[i] = y[slot];
   }
-  col_inverse_uv<R, N>(x, p.G, it, ch, ky, lane, s_tw);
+  col_inverse_uv(x, p.G, id.b, id.ch, id.ky, id.act, xf, TableRow<X, false>(nullptr, mu_row<X>(p.tw, id.ky)));
 }
 
-// Physical fields of each item: Phys[it][x][NPH][pos] (B_x, B_y include b0).
+// Physical fields of each item: Phys[it][x][2][N] (see phys_row; B_x, B_y include b0).
 template <typename R>
 struct RowPhysParams {
   const cplx<R>* G;   // [nitems][NG][K][N]
@@ -64,32 +65,26 @@ struct RowPhysParams {
 };
 
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32) k_row_phys(RowPhysParams<R> p) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_phys(RowPhysParams<R> p) {
+  using X = Xf<R, N>;
+  constexpr int E = X::E, L = X::L, K = X::K;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_tw + fft_smem(N, XT);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_G = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int it = blockIdx.x / tiles, x0 = (blockIdx.x - it * tiles) * XT;
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   load_tile<R, N, XT>(s_G, p.G + (size_t)it * NG * K * N, NG * K, x0);
   __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = x0 + w;
-  R* ph = p.phys + (((size_t)it * N + x) * NPH) * N;
+  const X xf(s_x, threadIdx.x >> 5);
+  const int w = threadIdx.x / L;
+  cplx<R>* ph = const_cast<cplx<R>*>(phys_row<R, N>(p.phys + (size_t)it * N * NPH * N, x0 + w)) + xf.l;
   cplx<R> uv[E], bb[E];
+  row_inverse<XT>(s_G, w, xf, uv, bb);
 #pragma unroll
   for (int j = 0; j < E; ++j) {
-    uv[j] = packed_pair<R, N, XT>(s_G, s_G + K * (XT + 1), lane + 32 * j, w);
-    bb[j] = packed_pair<R, N, XT>(s_G + 2 * K * (XT + 1), s_G + 3 * K * (XT + 1), lane + 32 * j, w);
-  }
-  fft_dif2<R, N, true>(uv, bb, s_tw, lane);
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int e = lane + 32 * j;
-    ph[e] = uv[j].x; ph[N + e] = uv[j].y;
-    ph[2 * N + e] = bb[j].x + p.b0x; ph[3 * N + e] = bb[j].y + p.b0y;   // B carries the mean field (mhd_jax.py:145-149)
+    ph[L * j] = uv[j];
+    ph[N + L * j] = mk<R>(bb[j].x + p.b0x, bb[j].y + p.b0y);   // B carries the mean field (mhd_jax.py:145-149)
   }
 }
 
@@ -107,81 +102,72 @@ struct RowTanParams {
   int B;
 };
 
-// The linearised products of one row in physical space (dP1, dP2 in duv, dP3 in dbb).
-template <typename R, int E>
-__device__ __forceinline__ void row_tan_products(cplx<R> (&duv)[E], cplx<R> (&dbb)[E], const R (&pu)[E],
-                                                 const R (&pv)[E], const R (&pbx)[E], const R (&pby)[E]) {
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const R du = duv[j].x, dv = duv[j].y, dbx = dbb[j].x, dby = dbb[j].y;
-    const R u = pu[j], v = pv[j], bx = pbx[j], by = pby[j];
-    duv[j] = mk<R>(R(2) * (fpm(u, du, v, dv) - fpm(bx, dbx, by, dby)),     // dP1
-                   fpp(bx, dby, by, dbx) - fpp(u, dv, v, du));              // dP2
-    dbb[j] = mk<R>(fpp(u, dby, by, du) - fpp(v, dbx, bx, dv), R(0));        // dP3
-  }
+// The linearised products of one row in physical space: (dP1, dP2) and dP3.
+template <typename R>
+__device__ __forceinline__ cplx<R> tan_p12(cplx<R> d, cplx<R> db, cplx<R> uv, cplx<R> bb) {
+  return mk<R>(R(2) * (fpm(uv.x, d.x, uv.y, d.y) - fpm(bb.x, db.x, bb.y, db.y)),
+               fpp(bb.x, db.y, bb.y, db.x) - fpp(uv.x, d.y, uv.y, d.x));
+}
+template <typename R>
+__device__ __forceinline__ R tan_p3(cplx<R> d, cplx<R> db, cplx<R> uv, cplx<R> bb) {
+  return fpp(uv.x, db.y, bb.y, d.x) - fpp(uv.y, db.x, bb.x, d.y);
 }
 
-// Rows x0 .. x0 + XT - 1 of tangent b, one warp per row (the CTA's XT warps);
-// s_G and s_H are the tile buffers (NG and NH rows of K x (XT + 1)).
+// Rows x0 .. x0 + XT - 1 of tangent b, one group per row; s_G and s_H are the tile
+// buffers (NG and NH rows of K x (XT + 1), the same memory allowed: see row_rhs_body).
 // CX (cluster-resident passes): s_G already holds the tile (written
-// by the column pass) unless load_g, and the H tile goes to the column warps'
+// by the column pass) unless load_g, and the H tile goes to the column groups'
 // rows at `hcols` (scatter_h_tile) unless that is null (global H).
-template <typename R, int N, int XT, bool CX = false>
-__device__ __forceinline__ void row_tan_body(const RowTanParams<R>& p, int b, int x0, const cplx<R>* s_tw,
-                                             cplx<R>* s_G, cplx<R>* s_H, bool load_g = true,
-                                             cplx<R>* hcols = nullptr) {
-  constexpr int E = N / 32;
-  constexpr int K = (N - 1) / 3 + 1;
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x = x0 + w;
-  // primal u, v, B_x, B_y of this row, loaded first so that the loads overlap
-  // the tile load and the inverse transforms (n <= 128); at n = 256 they would
-  // hold 4 E = 32 registers across the transform, so they are loaded after it
-  const R* ph = phys_row<R, N>(p.phys + (size_t)b * p.phys_bstride, x);
-  R pu[E], pv[E], pbx[E], pby[E];
+template <int XT, bool CX = false, class X>
+__device__ __forceinline__ void row_tan_body(const RowTanParams<typename X::R>& p, int b, int x0, const X& xf,
+                                             cplx<typename X::R>* s_G, cplx<typename X::R>* s_H, bool load_g = true,
+                                             cplx<typename X::R>* hcols = nullptr) {
+  using R = typename X::R;
+  constexpr int E = X::E, L = X::L, K = X::K, N = X::N;
+  const int w = threadIdx.x / L;
+  // primal (u, v), (B_x, B_y) of this row, loaded first so that the loads overlap
+  // the tile load and the inverse transforms where a lane holds four values or fewer;
+  // else they would hold 4 E registers across the transform, and are loaded after it
+  constexpr bool EARLY = E <= 4;
+  const cplx<R>* ph = phys_row<R, N>(p.phys + (size_t)b * p.phys_bstride, x0 + w) + xf.l;
+  cplx<R> puv[E], pbb[E];
   auto load_phys = [&]() {
 #pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = lane + 32 * j;
-      pu[j] = ph[e]; pv[j] = ph[N + e]; pbx[j] = ph[2 * N + e]; pby[j] = ph[3 * N + e];
-    }
+    for (int j = 0; j < E; ++j) { puv[j] = ph[L * j]; pbb[j] = ph[N + L * j]; }
   };
-  if constexpr (N <= 128) load_phys();
+  if constexpr (EARLY) load_phys();
   if (!CX || load_g) load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, NG * K, x0);
   __syncthreads();
   cplx<R> duv[E], dbb[E];
+  row_inverse<XT>(s_G, w, xf, duv, dbb);
+  if constexpr (!EARLY) load_phys();
 #pragma unroll
   for (int j = 0; j < E; ++j) {
-    const int q = lane + 32 * j;
-    duv[j] = packed_pair<R, N, XT>(s_G + 0 * K * (XT + 1), s_G + 1 * K * (XT + 1), q, w);
-    dbb[j] = packed_pair<R, N, XT>(s_G + 2 * K * (XT + 1), s_G + 3 * K * (XT + 1), q, w);
+    const cplx<R> d = duv[j], db = dbb[j];
+    duv[j] = tan_p12<R>(d, db, puv[j], pbb[j]);
+    dbb[j] = mk<R>(tan_p3<R>(d, db, puv[j], pbb[j]), R(0));
   }
-  fft_dif2<R, N, true>(duv, dbb, s_tw, lane);
-  if constexpr (N > 128) load_phys();
-  row_tan_products<R, E>(duv, dbb, pu, pv, pbx, pby);
-  fft_dit2<R, N, false>(duv, dbb, s_tw, lane);
-  split_store<R, N, XT>(duv, s_H, s_H + K * (XT + 1), w, lane);
-  store_one<R, N, XT>(dbb, s_H + 2 * K * (XT + 1), w, lane);
+  row_forward<XT>(duv, dbb, s_H, w, xf);
   __syncthreads();
   if constexpr (CX) {
-    if (hcols) { scatter_h_tile<R, N, XT>(s_H, hcols, x0); return; }
+    if (hcols) { scatter_h_tile<XT>(s_H, hcols, x0, xf); return; }
   }
   store_tile<R, N, XT>(p.H + (size_t)b * NH * K * N, s_H, NH * K, x0);
 }
 
 template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * 32, 2) k_row_tan(RowTanParams<R> p) {
-  constexpr int K = (N - 1) / 3 + 1;
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan(RowTanParams<R> p) {
+  using X = Xf<R, N>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_tw = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_tw + fft_smem(N, XT);
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_G = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
   pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
+  load_tables<X>(s_x, p.tw);
   pdl_wait();
   if (p.ctl && p.ctl[b].done) return;   // the whole CTA belongs to batch element b
-  row_tan_body<R, N, XT>(p, b, x0, s_tw, s_G, s_G + NG * K * (XT + 1));
+  row_tan_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_G, s_G);
 }
 
 // ---------------------------------------------------------------------------
@@ -222,252 +208,214 @@ struct ColTanParams {
   const cplx<R>* rec2;  // T43_EA: the next attempt's record (h is the next attempt's step)
 };
 
-// Record vectors (bits of Rk43Rec) and tangent slots (bits of Rk43Slot) that the
-// stage algebra of an adaptive stage reads; they are staged per column into
-// shared memory at the start (see k_col_tan).
+// Record vectors (bits of Rk4Rec / Rk43Rec; tan_qmask2: of the next attempt, from
+// rec2) and tangent slots (bits of TanSlot / Rk43Slot) that the algebra of a stage
+// reads; they are loaded together before the stage's stores.
 __host__ __device__ constexpr unsigned tan_qmask(int stage) {
-  return stage == T43_INIT ? (1u << RR_K1)
+  return stage == T4_S1 ? (1u << Q_F) | (1u << Q_K1)
+       : stage == T4_S2 ? (1u << Q_K2)
+       : stage == T4_S3 ? (1u << Q_F) | (1u << Q_K1) | (1u << Q_K2) | (1u << Q_K3)
+       : stage == T4_S4 ? (1u << Q_K4)
+       : stage == T43_INIT ? (1u << RR_K1)
        : stage == T43_A ? (1u << RR_X0) | (1u << RR_K1) | (1u << RR_E)
        : stage == T43_B ? (1u << RR_K2)
        : stage == T43_C ? (1u << RR_X0) | (1u << RR_K1) | (1u << RR_K2) | (1u << RR_K3) | (1u << RR_E)
        : stage == T43_D ? (1u << RR_K4)
        : stage == T43_E || stage == T43_EA ? (1u << RR_K5) : 0u;
 }
-// Record vectors of the next attempt read by T43_EA (from rec2).
 __host__ __device__ constexpr unsigned tan_qmask2(int stage) {
   return stage == T43_EA ? (1u << RR_X0) | (1u << RR_K1) | (1u << RR_E) : 0u;
 }
 __host__ __device__ constexpr unsigned tan_dmask(int stage) {
-  return stage == T43_START ? (1u << S_X0)
+  return stage == TS_START || stage == T4_S1 || stage == T4_S2 || stage == T4_S4 ? (1u << D_F)
+       : stage == T4_S3 ? (1u << D_F) | (1u << D_A1) | (1u << D_K2)
+       : stage == T43_START ? (1u << S_X0)
        : stage == T43_A ? (1u << S_X0) | (1u << S_K1)
        : stage == T43_B ? (1u << S_XE)
        : stage == T43_C ? (1u << S_XE) | (1u << S_K1E) | (1u << S_K2)
        : stage == T43_D ? (1u << S_K1) | (1u << S_K2) | (1u << S_K3) | (1u << S_X2)
        : stage == T43_E || stage == T43_EA ? (1u << S_XF) : 0u;
 }
-__host__ __device__ constexpr int popc_c(unsigned m) { return m ? (int)(m & 1u) + popc_c(m >> 1) : 0; }
 
-// Operand rows staged per warp by a tangent column stage (shared memory, M entries each).
-template <int N, int STAGE> __host__ __device__ constexpr int col_tan_nop() {
-  return N <= 128 ? popc_c(tan_qmask(STAGE)) + popc_c(tan_qmask2(STAGE)) + popc_c(tan_dmask(STAGE)) : 0;
+__host__ __device__ constexpr int tan_rows(int stage) {
+  return popc_c(tan_dmask(stage)) + popc_c(tan_qmask(stage)) + popc_c(tan_qmask2(stage));
 }
 
-// One warp's column `colid` of a tangent column stage; `my_op` is the warp's
-// staging buffer (col_tan_nop rows of M entries), `s_tw` the twiddle image.
-// CX > 0 (cluster-resident passes with CX-row tiles): the product rows come from
-// `hrows` (the warp's rows in shared memory, see scatter_h_tile) and the
-// inverse transforms go to the cluster's G tiles at `gtile` (col_uv_to_tiles);
-// a null pointer selects global H / G instead.
-// DSH (cluster-resident adaptive passes): the tangent slots of this column live
-// in shared memory at `dsh` ([S_NSLOT][M]) instead of global D.
-template <typename R, int N, int STAGE, int CX = 0, bool DSH = false>
-__device__ __forceinline__ void col_tan_body(const ColTanParams<R>& p, int colid, int lane, const cplx<R>* s_tw,
-                                             cplx<R>* my_op, const cplx<R>* hrows = nullptr,
-                                             cplx<R>* gtile = nullptr, cplx<R>* dsh = nullptr) {
-  constexpr int E = N / 32;
-  constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
-  constexpr size_t VEC = (size_t)2 * K * M;
-  const int ch = colid & 1, bk = colid >> 1, b = bk / K, ky = bk - b * K;   // one warp per (b, ky, channel)
-  if (p.ctl && p.ctl[b].done) return;
-  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC;
-  const cplx<R>* Q = p.rec + (size_t)b * p.rec_bstride;
+// What the algebra of a tangent stage needs beside its operands.
+template <typename R>
+struct TanCol {
+  R h, t, dpar, dpar_h, dpar_t;   // dpar: dh (Lawson-RK4) or dt (Lawson-RK4(3))
+  const R* etab;                  // the column's factors exp(h/2 L) mask, or null
+  __device__ __forceinline__ TanCol(const ColTanParams<R>& p, int b, size_t at) {
+    h = p.ctl ? (R)p.ctl[b].h : (R)p.h; t = (R)p.t;
+    dpar = (R)(p.dT[b] * (p.dscale_b ? p.dscale_b[b] : p.dscale));
+    dpar_h = dpar / h; dpar_t = dpar / t;
+    etab = p.etab ? p.etab + at : nullptr;
+  }
+};
+__host__ __device__ constexpr bool tan_has_rhs(int stage) { return !(stage == TS_START || stage == T43_A || stage == T43_START); }
+__host__ __device__ constexpr bool tan_has_input(int stage) { return !(stage == T43_INIT || stage == T43_E); }
+
+// The algebra of a tangent stage at one mode: the stage input from the derivative dv
+// (the tangent has no forcing).  QV(q), Q2V(q) read rows of the primal record (and of
+// the next attempt's), DV(d) reads and DW(d, v) writes tangent slot d.
+template <int STAGE, typename R, class QVf, class Q2Vf, class DVf, class DWf>
+__device__ __forceinline__ cplx<R> tan_algebra(const TanCol<R>& c, R L, bool in_mask, cplx<R> dv, int slot, QVf&& QV,
+                                               Q2Vf&& Q2V, DVf&& DV, DWf&& DW) {
+  const R h = c.h, t = c.t, dpar = c.dpar, dpar_h = c.dpar_h, dpar_t = c.dpar_t;
+  const R* etab = c.etab;
   constexpr bool rk43 = STAGE >= T43_INIT;
-  constexpr bool has_rhs = !(STAGE == TS_START || STAGE == T43_A || STAGE == T43_START);
-  const R h = p.ctl ? (R)p.ctl[b].h : (R)p.h, t = (R)p.t;
-  const R dpar = (R)(p.dT[b] * (p.dscale_b ? p.dscale_b[b] : p.dscale));   // dh (RK4) or dt (RK4(3))
-  // The record vectors and tangent slots the stage algebra reads, this column's
-  // rows of them (M entries each), copied into the warp's shared buffer with
-  // cp.async before the forward transform, so that their latency overlaps it
-  // without holding registers (adaptive stages, n <= 128: static shared memory).
-  constexpr unsigned QM = N <= 128 ? tan_qmask(STAGE) : 0u, DM = (N <= 128 && !DSH) ? tan_dmask(STAGE) : 0u;
-  constexpr unsigned QM2 = N <= 128 ? tan_qmask2(STAGE) : 0u;
-  constexpr int NQ = popc_c(QM), NQ2 = popc_c(QM2), NOP = NQ + NQ2 + popc_c(DM);
-  const cplx<R>* Q2 = p.rec2;
-  if constexpr (NOP > 0) {
-    const size_t row = ((size_t)ch * K + ky) * M;
-    int v = 0;
-#pragma unroll
-    for (int bit = 0; bit < 16; ++bit) {
-      if ((QM >> bit) & 1u) {
-        for (int s2 = lane; s2 < M; s2 += 32) cp_async_c<R>(my_op + v * M + s2, Q + bit * VEC + row + s2);
-        ++v;
-      }
+  cplx<R> xin = mk<R>(0, 0);
+  if (!rk43) {
+    // Lawson-RK4: e = exp(h/2 L) mask, de = e L dh/2; dk = dh v + h dv with v = k/h
+    const R ex = etab ? __ldg(etab + slot) : in_mask ? exp(h / R(2) * L) : R(0);
+    const R de = ex * L * (dpar / R(2));
+    auto dk_of = [&](int q) { return lin2_rn(QV(q), dpar_h, dv, h); };
+    switch (STAGE) {
+      case TS_START: xin = DV(D_F); break;
+      case T4_S1: {
+        const cplx<R> dk1 = dk_of(Q_K1);
+        const cplx<R> df1 = lin2_rn(QV(Q_F), de, DV(D_F), ex);
+        const cplx<R> da1 = lin2_rn(QV(Q_K1), de, dk1, ex);
+        DW(D_F, df1); DW(D_A1, da1);
+        xin = cadd(df1, cscale(da1, R(0.5)));
+      } break;
+      case T4_S2: {
+        const cplx<R> dk2 = dk_of(Q_K2);
+        DW(D_K2, dk2);
+        xin = cadd(DV(D_F), cscale(dk2, R(0.5)));
+      } break;
+      case T4_S3: {
+        const cplx<R> dk3 = dk_of(Q_K3);
+        const cplx<R> f1 = cscale_rn(QV(Q_F), ex), a1 = cscale_rn(QV(Q_K1), ex);
+        const cplx<R> df2 = lin2_rn(f1, de, DV(D_F), ex);
+        const cplx<R> db1 = lin2_rn(a1, de, DV(D_A1), ex);
+        const cplx<R> db2 = lin2_rn(QV(Q_K2), de, DV(D_K2), ex);
+        const cplx<R> db3 = lin2_rn(QV(Q_K3), de, dk3, ex);
+        xin = cadd(df2, db3);
+        DW(D_F, cadd(cadd(cadd(df2, cdiv_k<6>(db1)), cdiv_k<3>(db2)), cdiv_k<3>(db3)));
+      } break;
+      default: {   // T4_S4
+        const cplx<R> dk4 = dk_of(Q_K4);
+        xin = cadd(DV(D_F), cdiv_k<6>(dk4));
+        DW(D_F, xin);
+      } break;
     }
-#pragma unroll
-    for (int bit = 0; bit < 16; ++bit) {
-      if ((QM2 >> bit) & 1u) {
-        for (int s2 = lane; s2 < M; s2 += 32) cp_async_c<R>(my_op + v * M + s2, Q2 + bit * VEC + row + s2);
-        ++v;
-      }
-    }
-#pragma unroll
-    for (int bit = 0; bit < 16; ++bit) {
-      if ((DM >> bit) & 1u) {
-        for (int s2 = lane; s2 < M; s2 += 32) cp_async_c<R>(my_op + v * M + s2, D + bit * VEC + row + s2);
-        ++v;
-      }
-    }
-  }
-  cplx<R> r[E];
-  if (has_rhs) {
-    if (CX > 0 && hrows) col_rhs_rows<R, N>(hrows, hrows + N, ch, ky, lane, s_tw, r);
-    else col_load_rhs<R, N>(p.H, b, ch, ky, lane, s_tw, r);
-  }
-  if constexpr (NOP > 0) {
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncwarp();
-  }
-  const R coeff = ch == 0 ? p.nu : p.eta;
-  cplx<R> x[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    x[j] = mk<R>(0, 0);
-    const int slot = pos_to_slot(spec_pos<N>(lane, j), N, KMAX, M);
-    if (slot < 0) continue;
-    const int kx = slot_to_kx(slot, KMAX, M);
-    const bool in_mask = !(kx == 0 && ky == 0);
-    cplx<R> dv = mk<R>(0, 0);
-    if (has_rhs) dv = r[j];                              // the tangent has no forcing
-    const size_t o = ((size_t)ch * K + ky) * M + slot;
-    const R L = diss_L<R>(kx, ky, coeff);
-    cplx<R> xin = mk<R>(0, 0);
-    if (!rk43) {
-      // Lawson-RK4: e = exp(h/2 L) mask, de = e L dh/2; dk = dh v + h dv with v = k/h
-      const R e = p.etab ? p.etab[(size_t)b * VEC + o] : in_mask ? exp(h / R(2) * L) : R(0);
-      const R de = e * L * (dpar / R(2));
-      auto dk_of = [&](int q) { return lin2_rn(Q[q * VEC + o], dpar / h, dv, h); };
-      switch (STAGE) {
-        case TS_START: xin = D[D_F * VEC + o]; break;
-        case T4_S1: {
-          const cplx<R> dk1 = dk_of(Q_K1);
-          const cplx<R> df1 = lin2_rn(Q[Q_F * VEC + o], de, D[D_F * VEC + o], e);
-          const cplx<R> da1 = lin2_rn(Q[Q_K1 * VEC + o], de, dk1, e);
-          D[D_F * VEC + o] = df1; D[D_A1 * VEC + o] = da1;
-          xin = cadd(df1, cscale(da1, R(0.5)));
-        } break;
-        case T4_S2: {
-          const cplx<R> dk2 = dk_of(Q_K2);
-          D[D_K2 * VEC + o] = dk2;
-          xin = cadd(D[D_F * VEC + o], cscale(dk2, R(0.5)));
-        } break;
-        case T4_S3: {
-          const cplx<R> dk3 = dk_of(Q_K3);
-          const cplx<R> f1 = cscale_rn(Q[Q_F * VEC + o], e), a1 = cscale_rn(Q[Q_K1 * VEC + o], e);
-          const cplx<R> df2 = lin2_rn(f1, de, D[D_F * VEC + o], e);
-          const cplx<R> db1 = lin2_rn(a1, de, D[D_A1 * VEC + o], e);
-          const cplx<R> db2 = lin2_rn(Q[Q_K2 * VEC + o], de, D[D_K2 * VEC + o], e);
-          const cplx<R> db3 = lin2_rn(Q[Q_K3 * VEC + o], de, dk3, e);
-          xin = cadd(df2, db3);
-          D[D_F * VEC + o] = cadd(cadd(cadd(df2, cdiv_k<6>(db1)), cdiv_k<3>(db2)), cdiv_k<3>(db3));
-        } break;
-        default: {   // T4_S4
-          const cplx<R> dk4 = dk_of(Q_K4);
-          xin = cadd(D[D_F * VEC + o], cdiv_k<6>(dk4));
-          D[D_F * VEC + o] = xin;
-        } break;
-      }
-    } else {
-      // Lawson-RK4(3): e = exp(t L h/2), de = e L h/2 dt; dk = dt v + t dv with v = k/t
-      // staged operands (shared memory) or, without staging, global memory
-      auto QV = [&](int q) -> cplx<R> {
-        if constexpr (NOP > 0) return my_op[popc_c(QM & ((1u << q) - 1u)) * M + slot];
-        else return Q[q * VEC + o];
-      };
-      // (e, e L h/2) of this attempt from the primal record (stages A and C use them)
-      const cplx<R> eg = (STAGE == T43_A || STAGE == T43_C) ? QV(RR_E) : mk<R>(0, 0);
-      [[maybe_unused]] const R e = eg.x;
-      [[maybe_unused]] const R de = eg.y * dpar;
-      auto Q2V = [&](int q) -> cplx<R> {
-        if constexpr (NOP > 0) return my_op[(NQ + popc_c(QM2 & ((1u << q) - 1u))) * M + slot];
-        else return Q2[q * VEC + o];
-      };
-      auto DV = [&](int d) -> cplx<R> {
-        if constexpr (DSH) return dsh[d * M + slot];
-        else if constexpr (NOP > 0) return my_op[(NQ + NQ2 + popc_c(DM & ((1u << d) - 1u))) * M + slot];
-        else return D[d * VEC + o];
-      };
-      auto DW = [&](int d, cplx<R> v) {
-        if constexpr (DSH) dsh[d * M + slot] = v;
-        else D[d * VEC + o] = v;
-      };
-      auto dk_of = [&](int q) { return lin2_rn(QV(q), dpar / t, dv, t); };
-      // the A and E algebra, written with explicitly rounded operations: the
-      // merged pass T43_EA computes exactly what T43_E followed by T43_A does
-      auto stage_e = [&]() { return lin2_rn(QV(RR_K5), dpar / t, dv, t); };   // dk5
-      auto stage_a = [&](cplx<R> x0, cplx<R> k1, cplx<R> eg_, cplx<R> dx0, cplx<R> dk1, R h_) {
-        const R e_ = eg_.x, de_ = mul_rn(eg_.y, dpar);
-        const cplx<R> dxe = lin2_rn(x0, de_, dx0, e_), dk1e = lin2_rn(k1, de_, dk1, e_);
-        DW(S_XE, dxe); DW(S_K1E, dk1e);
-        cplx<R> half = cscale(dk1e, h_);
-        half.x = mul_rn(half.x, R(0.5)); half.y = mul_rn(half.y, R(0.5));
-        return mk<R>(add_rn(dxe.x, half.x), add_rn(dxe.y, half.y));
-      };
-      switch (STAGE) {
-        case T43_START: xin = DV(S_X0); break;
-        case T43_INIT: DW(S_K1, dk_of(RR_K1)); break;
-        case T43_A: xin = stage_a(QV(RR_X0), QV(RR_K1), eg, DV(S_X0), DV(S_K1), h); break;
-        case T43_B: {
-          const cplx<R> dk2 = dk_of(RR_K2);
-          DW(S_K2, dk2);
-          xin = cadd(DV(S_XE), cscale(cscale(dk2, h), R(0.5)));
-        } break;
-        case T43_C: {
-          const cplx<R> dk3 = dk_of(RR_K3);
-          const cplx<R> xe = cscale_rn(QV(RR_X0), e), k1e = cscale_rn(QV(RR_K1), e);
-          const cplx<R> dx2 = lin2_rn(xe, de, DV(S_XE), e);
-          const cplx<R> dk1ee = lin2_rn(k1e, de, DV(S_K1E), e);
-          const cplx<R> dk2e = lin2_rn(QV(RR_K2), de, DV(S_K2), e);
-          const cplx<R> dk3e = lin2_rn(QV(RR_K3), de, dk3, e);
-          DW(S_X2, dx2); DW(S_K1, dk1ee); DW(S_K2, dk2e); DW(S_K3, dk3e);
-          xin = cadd_scaled_rn(dx2, dk3e, h);
-        } break;
-        case T43_D: {
-          const cplx<R> dk4 = dk_of(RR_K4);
-          const cplx<R> acc = cadd(cadd(cadd(cdiv_k<6>(DV(S_K1)), cdiv_k<3>(DV(S_K2))),
-                                        cdiv_k<3>(DV(S_K3))), cdiv_k<6>(dk4));
-          xin = cadd_scaled_rn(DV(S_X2), acc, h);
-          DW(S_XF, xin);
-        } break;
-        case T43_E: {   // accepted attempt, promote (dxf, dk5) -> (dx0, dk1)
-          DW(S_K1, stage_e());
-          DW(S_X0, DV(S_XF));
-        } break;
-        default: {      // T43_EA: T43_E, then T43_A of the next attempt on the promoted values
-          const cplx<R> dk1 = stage_e(), dx0 = DV(S_XF);
-          DW(S_K1, dk1);
-          DW(S_X0, dx0);
-          xin = stage_a(Q2V(RR_X0), Q2V(RR_K1), Q2V(RR_E), dx0, dk1, h);
-        } break;
-      }
-    }
-    x[j] = xin;
-  }
-  if (!p.produce || STAGE == T43_INIT || STAGE == T43_E) return;
-  if constexpr (CX > 0) {
-    if (gtile) {
-      cplx<R> wu[E], wv[E];
-      col_uv_transform<R, N>(x, ky, lane, s_tw, wu, wv);
-      col_uv_to_tiles<R, N, CX>(wu, wv, gtile, ch, ky, lane);
-      return;
+  } else {
+    // Lawson-RK4(3): e = exp(t L h/2), de = e L h/2 dt; dk = dt v + t dv with v = k/t;
+    // (e, e L h/2) of this attempt from the primal record (stages A and C use them)
+    const cplx<R> eg = (STAGE == T43_A || STAGE == T43_C) ? QV(RR_E) : mk<R>(0, 0);
+    [[maybe_unused]] const R ex = eg.x;
+    [[maybe_unused]] const R de = eg.y * dpar;
+    auto dk_of = [&](int q) { return lin2_rn(QV(q), dpar_t, dv, t); };
+    // the A and E algebra, written with explicitly rounded operations: the
+    // merged pass T43_EA computes exactly what T43_E followed by T43_A does
+    auto stage_e = [&]() { return lin2_rn(QV(RR_K5), dpar_t, dv, t); };   // dk5
+    auto stage_a = [&](cplx<R> x0, cplx<R> k1, cplx<R> eg_, cplx<R> dx0, cplx<R> dk1, R h_) {
+      const R e_ = eg_.x, de_ = mul_rn(eg_.y, dpar);
+      const cplx<R> dxe = lin2_rn(x0, de_, dx0, e_), dk1e = lin2_rn(k1, de_, dk1, e_);
+      DW(S_XE, dxe); DW(S_K1E, dk1e);
+      cplx<R> half = cscale(dk1e, h_);
+      half.x = mul_rn(half.x, R(0.5)); half.y = mul_rn(half.y, R(0.5));
+      return mk<R>(add_rn(dxe.x, half.x), add_rn(dxe.y, half.y));
+    };
+    switch (STAGE) {
+      case T43_START: xin = DV(S_X0); break;
+      case T43_INIT: DW(S_K1, dk_of(RR_K1)); break;
+      case T43_A: xin = stage_a(QV(RR_X0), QV(RR_K1), eg, DV(S_X0), DV(S_K1), h); break;
+      case T43_B: {
+        const cplx<R> dk2 = dk_of(RR_K2);
+        DW(S_K2, dk2);
+        xin = cadd(DV(S_XE), cscale(cscale(dk2, h), R(0.5)));
+      } break;
+      case T43_C: {
+        const cplx<R> dk3 = dk_of(RR_K3);
+        const cplx<R> xe = cscale_rn(QV(RR_X0), ex), k1e = cscale_rn(QV(RR_K1), ex);
+        const cplx<R> dx2 = lin2_rn(xe, de, DV(S_XE), ex);
+        const cplx<R> dk1ee = lin2_rn(k1e, de, DV(S_K1E), ex);
+        const cplx<R> dk2e = lin2_rn(QV(RR_K2), de, DV(S_K2), ex);
+        const cplx<R> dk3e = lin2_rn(QV(RR_K3), de, dk3, ex);
+        DW(S_X2, dx2); DW(S_K1, dk1ee); DW(S_K2, dk2e); DW(S_K3, dk3e);
+        xin = cadd_scaled_rn(dx2, dk3e, h);
+      } break;
+      case T43_D: {
+        const cplx<R> dk4 = dk_of(RR_K4);
+        const cplx<R> acc = cadd(cadd(cadd(cdiv_k<6>(DV(S_K1)), cdiv_k<3>(DV(S_K2))),
+                                      cdiv_k<3>(DV(S_K3))), cdiv_k<6>(dk4));
+        xin = cadd_scaled_rn(DV(S_X2), acc, h);
+        DW(S_XF, xin);
+      } break;
+      case T43_E: {   // accepted attempt, promote (dxf, dk5) -> (dx0, dk1)
+        DW(S_K1, stage_e());
+        DW(S_X0, DV(S_XF));
+      } break;
+      default: {      // T43_EA: T43_E, then T43_A of the next attempt on the promoted values
+        const cplx<R> dk1 = stage_e(), dx0 = DV(S_XF);
+        DW(S_K1, dk1);
+        DW(S_X0, dx0);
+        xin = stage_a(Q2V(RR_X0), Q2V(RR_K1), Q2V(RR_E), dx0, dk1, h);
+      } break;
     }
   }
-  col_inverse_uv<R, N>(x, p.G, b, ch, ky, lane, s_tw);
+  return xin;
 }
 
-template <typename R, int N, int STAGE>
-__global__ void __launch_bounds__(128) k_col_tan(ColTanParams<R> p) {
-  constexpr int K = (N - 1) / 3 + 1, M = 2 * ((N - 1) / 3) + 1;
-  constexpr int NOP = col_tan_nop<N, STAGE>();
-  __shared__ __align__(16) cplx<R> s_tw[fft_smem(N, 4)];
-  __shared__ __align__(16) cplx<R> s_op[(NOP > 0 ? NOP : 1) * 4 * M];   // 4 warps per CTA
-  pdl_trigger();
-  load_twiddles<R, N>(s_tw, p.tw);
-  pdl_wait();
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const int colid = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (colid >= p.B * K * 2) return;
-  col_tan_body<R, N, STAGE>(p, colid, lane, s_tw, s_op + (threadIdx.x >> 5) * NOP * M);
+// A tangent column stage of one column; `rows`: shared room for its operands.
+template <int STAGE, class X>
+__device__ __forceinline__ void col_tan_body(const ColTanParams<typename X::R>& p, const ColId<X>& id, const X& xf,
+                                             cplx<typename X::R>* rows) {
+  using R = typename X::R;
+  constexpr int E = X::E, K = X::K, M = X::M;
+  constexpr size_t VEC = (size_t)2 * K * M;
+  const int ch = id.ch, b = id.b, ky = id.ky;
+  const bool act = id.act && !(p.ctl && p.ctl[b].done);
+  if (!__any_sync(0xffffffffu, act)) return;
+  const size_t row = ((size_t)ch * K + ky) * M;
+  cplx<R>* D = p.D + (size_t)b * p.nslot * VEC + row;
+  const cplx<R>* Q = p.rec + (size_t)b * p.rec_bstride + row;
+  const cplx<R>* Q2 = p.rec2 + row;
+  const TanCol<R> c(p, b, (size_t)b * VEC + row);
+  constexpr unsigned DM = tan_dmask(STAGE), QM = tan_qmask(STAGE), QM2 = tan_qmask2(STAGE);
+  // Group layout: the operands of half of the lane's elements at a time; up to two slots
+  // whole and before the transform (more would not fit into the registers beside it).
+  constexpr int EH = X::STAGED ? E : (E + 1) / 2;
+  constexpr bool EARLY = X::GROUP && popc_c(DM) <= 2;
+  Operands<X, DM, EARLY ? E : EH> d(rows);
+  Operands<X, QM, EH> q(rows + popc_c(DM) * M);
+  Operands<X, QM2, EH> q2(rows + (popc_c(DM) + popc_c(QM)) * M);
+  d.begin(D, VEC); q.begin(Q, VEC); q2.begin(Q2, VEC);
+  constexpr int n = tan_rows(STAGE);
+  const TableRow<X, rows_fit(n, 1)> mu(rows + n * M, mu_row<X>(p.tw, ky));
+  if constexpr (EARLY) d.load(D, VEC, act, xf);
+  cplx<R> r[E], x[E];
+  if (tan_has_rhs(STAGE)) col_load_rhs(p.H, b, ch, ky, xf, r);
+  const R coeff = ch == 0 ? p.nu : p.eta;
+#pragma unroll
+  for (int i0 = 0; i0 < E; i0 += EH) {
+    if constexpr (!EARLY) d.load(D, VEC, act, xf, i0);
+    q.load(Q, VEC, act, xf, i0);
+    q2.load(Q2, VEC, act, xf, i0);
+#pragma unroll
+    for (int i = i0; i < i0 + EH && i < E; ++i) {
+      x[i] = mk<R>(0, 0);
+      if (X::none(i)) continue;
+      const int slot = act ? xf.slot(i) : -1;
+      if (slot < 0) continue;
+      x[i] = tan_algebra<STAGE>(c, diss_L<R>(xf.kx(i), (R)ky, coeff), !(slot == 0 && ky == 0),
+                                tan_has_rhs(STAGE) ? r[i] : mk<R>(0, 0), slot,
+                                [&](int a) { return q.get(a, i, slot); }, [&](int a) { return q2.get(a, i, slot); },
+                                [&](int a) { return d.get(a, i, slot); },
+                                [&](int a, cplx<R> v) { D[a * VEC + slot] = v; });
+    }
+  }
+  if (p.produce && tan_has_input(STAGE)) col_inverse_uv(x, p.G, b, ch, ky, act, xf, mu);
+}
+
+template <typename R, int N, int STAGE, bool GRP = false>
+__global__ void __launch_bounds__(COLWARPS * 32, GRP ? 3 : 1) k_col_tan(ColTanParams<R> p) {
+  using X = Xf<R, N, GRP>;
+  ECS_COL_PROLOGUE(tan_rows(STAGE), 1);   // the multipliers
+  col_tan_body<STAGE>(p, id, xf, rows);
 }
 
 // Rejected Lawson-RK4(3) attempt: the carried k1 becomes e^2 k1 (timestepping.py:267,275,297);

@@ -42,9 +42,9 @@ constexpr size_t CB = sizeof(double2);
 constexpr size_t al(size_t x) { return (x + 255) / 256 * 256; }
 
 // Byte layout of the static scratch (sized for n = 128, batch = 4).
-constexpr size_t OFF_TW64 = 0;                                                   // twiddle image, n = 64
-constexpr size_t OFF_TW128 = al(OFF_TW64 + tw_smem(64) * CB);                    // twiddle image, n = 128
-constexpr size_t OFF_CTL = al(OFF_TW128 + tw_smem(128) * CB);                    // step controls (zeroed)
+constexpr size_t OFF_TW64 = 0;                                                   // tables, n = 64
+constexpr size_t OFF_TW128 = al(OFF_TW64 + XfTable<double, 64>::size * CB);    // tables, n = 128
+constexpr size_t OFF_CTL = al(OFF_TW128 + XfTable<double, 128>::size * CB);    // step controls (zeroed)
 constexpr size_t OFF_FIELDS = al(OFF_CTL + NA_MAX_BATCH * sizeof(StepCtl));      // [forcing; 0] real [2][n][n]
 constexpr size_t OFF_FBOX = al(OFF_FIELDS + 2 * NA_MAX_N * NA_MAX_N * sizeof(double));   // forcing box [2][K][M]
 constexpr size_t OFF_F = al(OFF_FBOX + 2 * NA_K * NA_M * CB);                    // input box [B][2][K][M]
@@ -63,21 +63,17 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[NA_BYTES];
 namespace {
 
 template <int N>
-int na_setup_twiddles(unsigned char* base, size_t off) {
-  std::vector<double2> tw(N / 2);
-  const long double twopi = 6.283185307179586476925286766559005768L;
-  for (int k = 0; k < N / 2; ++k) {
-    const long double a = twopi * (long double)k / (long double)N;
-    tw[k] = make_double2((double)cosl(a), (double)(-sinl(a)));
-  }
-  std::vector<double2> img(tw_smem(N));
-  twiddle_image<double2, N>(tw.data(), img.data());
+int na_setup_tables(unsigned char* base, size_t off) {
+  std::vector<double2> img(XfTable<double, N>::size);
+  xf_table<double, N>(img.data());
   return cudaMemcpy(base + off, img.data(), img.size() * CB, cudaMemcpyHostToDevice) == cudaSuccess ? ECS_OK
                                                                                                   : ECS_ERR_CUDA;
 }
 
-template <int N> size_t na_smem_rhs() { return (fft_smem(N, NA_XT) + (NG + NH) * ((N - 1) / 3 + 1) * (NA_XT + 1)) * CB; }
-template <int N> size_t na_smem_2f() { return (fft_smem(N, NA_XT) + 2 * ((N - 1) / 3 + 1) * (NA_XT + 1)) * CB; }
+template <int N> using NaXf = Xf<double, N>;
+constexpr int col_ctas(int warps) { return (warps + 3) / 4; }
+template <int N> size_t na_smem_rhs() { return (NaXf<N>::smem(NA_XT / NaXf<N>::G) + NG * NaXf<N>::K * (NA_XT + 1)) * CB; }
+template <int N> size_t na_smem_2f() { return (NaXf<N>::smem(NA_XT / NaXf<N>::G) + 2 * NaXf<N>::K * (NA_XT + 1)) * CB; }
 
 // One-time set-up on the current device (synchronous).  It holds the mutex that
 // context set-up and every graph capture of this library take, so its
@@ -92,7 +88,7 @@ int na_setup(unsigned char** out) {
     // need the device address, which only cudaGetSymbolAddress gives.
     if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || !p) return ECS_ERR_CUDA;
     unsigned char* base = static_cast<unsigned char*>(p);
-    if (na_setup_twiddles<64>(base, OFF_TW64) || na_setup_twiddles<128>(base, OFF_TW128)) return ECS_ERR_CUDA;
+    if (na_setup_tables<64>(base, OFF_TW64) || na_setup_tables<128>(base, OFF_TW128)) return ECS_ERR_CUDA;
     cudaError_t e = cudaFuncSetAttribute(k_row_rhs<double, 128, NA_XT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)na_smem_rhs<128>());
     if (e == cudaSuccess)
@@ -124,9 +120,9 @@ int na_state_vel(unsigned char* base, double nu, double eta, double b0x, double 
   if (e != cudaSuccess) return ECS_ERR_CUDA;
   // forcing spectrum on the box, mask[0,0] = False
   RowFwdParams<double> rf{}; rf.fields = fields; rf.H = H; rf.tw = tw; rf.B = 1;
-  k_row_to_box<double, N, NA_XT><<<N / NA_XT, NA_XT * 32, na_smem_2f<N>(), s>>>(rf);
+  k_row_to_box<double, N, NA_XT><<<N / NA_XT, NA_XT * NaXf<N>::L, na_smem_2f<N>(), s>>>(rf);
   ColBoxParams<double> cbp{}; cbp.H = H; cbp.V = fbox; cbp.tw = tw; cbp.vstride = 2L * K * M; cbp.B = 1; cbp.nf = 2;
-  k_col_to_box<double, N><<<(2 * K + 3) / 4, 128, 0, s>>>(cbp);
+  k_col_to_box<double, N><<<col_ctas((2 * K + NaXf<N>::G - 1) / NaXf<N>::G), 128, 0, s>>>(cbp);
   if (cudaMemsetAsync(fbox, 0, CB, s) != cudaSuccess) return ECS_ERR_CUDA;
   // state_vel: gather box, column inverse, row products, column forward, scatter
   const long nbox = (long)B * 2 * K * M;
@@ -135,14 +131,14 @@ int na_state_vel(unsigned char* base, double nu, double eta, double b0x, double 
   cp.H = H; cp.G = G; cp.F = F; cp.A1 = nullptr; cp.K2 = nullptr; cp.OUT = OUT; cp.Etab = nullptr; cp.ctl = ctl;
   cp.fhat = fbox; cp.tw = tw; cp.nu = nu; cp.eta = eta; cp.B = B; cp.stage = COL_START; cp.produce = 1;
   cp.diss = 0; cp.rec = nullptr; cp.rec_bstride = 0;
-  const int cols = B * K * 2;   // one warp per (batch, ky, channel)
-  k_col_rk4<double, N, COL_START><<<(cols + 3) / 4, 128, 0, s>>>(cp);
+  const int cols = col_ctas(col_units<NaXf<N>>() * B);
+  k_col_rk4<double, N, COL_START><<<cols, 128, 0, s>>>(cp);
   RowParams<double> rp{};
   rp.G = G; rp.H = H; rp.ctl = nullptr; rp.phys = nullptr; rp.phys_bstride = 0;
   rp.tw = tw; rp.b0x = b0x; rp.b0y = b0y; rp.B = B;
-  k_row_rhs<double, N, NA_XT><<<B * (N / NA_XT), NA_XT * 32, na_smem_rhs<N>(), s>>>(rp);
+  k_row_rhs<double, N, NA_XT><<<B * (N / NA_XT), NA_XT * NaXf<N>::L, na_smem_rhs<N>(), s>>>(rp);
   cp.stage = COL_PLAIN; cp.produce = 0; cp.diss = diss;
-  k_col_rk4<double, N, COL_PLAIN><<<(cols + 3) / 4, 128, 0, s>>>(cp);
+  k_col_rk4<double, N, COL_PLAIN><<<cols, 128, 0, s>>>(cp);
   const long nfull = (long)B * 2 * N * (N / 2 + 1);
   k_scatter_box<double><<<(int)((nfull + 255) / 256), 256, 0, s>>>(OUT, dfdt, N, B);
   return cudaGetLastError() == cudaSuccess ? ECS_OK : ECS_ERR_CUDA;
