@@ -46,13 +46,15 @@ struct ecs_ctx {
   // k_rk4_chain for Lawson-RK4 stepping) run batches up to the number of
   // 16-warp clusters the device holds at once; batches up to the number of
   // 8-warp clusters (16 CTAs each at n = 128) use those.  Measured at n = 128
-  // FP64 (matvecs/s, state-steps/s; launch per pass -> chain): batch 1 11.2 ->
-  // 12.5 and 23.4k -> 30.1k, batch 4 30.3 -> 50.5 and 67.5k -> 120k, batch 8
-  // 59.4 -> 68.7 and 111k -> 165k; at batch 16 the launch-per-pass path is ahead.
+  // FP64 (ms per JVP of T = 0.3, per 64 steps; launch per pass -> chain): batch 1
+  // 2.35 -> 2.00 and 2.12 -> 1.82, batch 8 3.89 -> 3.10 and 4.49 -> 2.87, batch 12
+  // 3.43 -> 3.11 and 4.71 -> 2.91; at batch 16 the launch-per-pass path is ahead
+  // (3.98 against 5.37, 3.91 against 5.11).  The adaptive solve has its own range
+  // (rk43_solve).
   int chain_res8 = 0, chain_res16 = 0;   // clusters of each shape the device holds at once (set at creation)
   int chain_w = 0;                  // warps per CTA forced for the chains (ECS_CHAIN_WARPS=8 or 16; 0: by batch as above)
   int chain_dsh = 1;                // the 8-warp tangent chain keeps each column's tangent slots in shared memory (ECS_CHAIN_DSLOTS=0: global)
-  int chain_dsm = -1;               // G / H exchange of the chains: 1 distributed shared memory, 0 global memory (ECS_CHAIN_DSMEM; -1: global for the tangent chain, shared for Lawson-RK4, as measured)
+  int chain_dsm = -1;               // G / H exchange: 1 distributed shared memory, 0 global memory of the tangent and Lawson-RK4 chains (ECS_CHAIN_DSMEM; -1: shared, 9% faster at n = 128: 2.20 -> 2.00 ms per batch-1 JVP of T = 0.3, 2.01 -> 1.82 ms per 64 steps)
   int chain_minb = 1, chain_maxb = -1;         // batch range of the tangent chain (ECS_CHAIN_MINB / ECS_CHAIN_MAXB; -1: chain_res16; 0: off)
   int rk4chain_minb = 1, rk4chain_maxb = -1;   // batch range of the Lawson-RK4 chain (ECS_RK4CHAIN_MINB / ECS_RK4CHAIN_MAXB)
   int rk43chain_minb = 1, rk43chain_maxb = -1; // batch range of the adaptive Lawson-RK4(3) solve's chain (ECS_RK43CHAIN_MINB / _MAXB)

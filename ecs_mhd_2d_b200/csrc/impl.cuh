@@ -710,7 +710,15 @@ struct Impl {
     launch_col_rk43<R, N>(c, B, R43_START, s);
     launch_row_rhs<R, N>(c, B, s, c->ctl);
     launch_col_rk43<R, N>(c, B, R43_INIT, s);
-    if (launch && chain_batch(c, B, c->rk43chain_minb, c->rk43chain_maxb)) {
+    // Candidates take different numbers of attempts, so a second round of clusters starts
+    // as the first ones finish: 8-warp clusters pay up to 1.75 times those that run at
+    // once, 16-warp ones up to twice.  Measured, 8 warps / 16 warps / launch per pass
+    // (ms, T = 0.2, atol 1e-8): n = 64, batch 1 1.03 / 1.49 / 1.73, 24 2.34 / 2.74 / 4.51,
+    // 32 3.16 / 2.76 / 4.96, 64 4.80 / 3.81 / 5.40; n = 128, batch 1 1.45 / 2.13 / 1.87,
+    // 12 4.13 / 5.12 / 7.43, 16 5.45 / 5.17 / 7.36, 24 7.30 / 6.10 / 7.77,
+    // 32 9.29 / 8.21 / 7.94.
+    const int res8 = c->chain_res8 + 3 * c->chain_res8 / 4, res16 = 2 * c->chain_res16;
+    if (launch && chain_batch(c, B, c->rk43chain_minb, c->rk43chain_maxb < 0 ? res16 : c->rk43chain_maxb)) {
       // the attempts as one cluster-resident launch, no host round trip (k_rk43_chain)
       if constexpr (N <= 128) {
         Rk43ChainParams<R> P{};
@@ -722,7 +730,7 @@ struct Impl {
         r.G = (const cplx<R>*)c->G; r.H = (cplx<R>*)c->H; r.tw = (const cplx<R>*)c->tw; r.ctl = c->ctl;
         r.b0x = (R)c->b0x; r.b0y = (R)c->b0y; r.B = B;
         P.atol = cfg->atol; P.rec_h = rec_h; P.rec_acc = rec_acc; P.amax = amax;
-        if (c->chain_w == 8 || (c->chain_w == 0 && B <= c->chain_res8))
+        if (c->chain_w == 8 || (c->chain_w == 0 && B <= res8))
           launch_cluster(c, B, chain_cl<N, 8>(), k_rk43_chain<R, N, 8>, dim3(B * chain_cl<N, 8>()), dim3(8 * 32),
                          Rk43ChainSmem<R, N, 8>::bytes, s, P);
         else
@@ -1478,7 +1486,7 @@ struct Impl {
             launch_cluster(c, B, chain_cl<N, W>(), k_tan_chain<R, N, W, DSM, false>, dim3(B * chain_cl<N, W>()),
                            dim3(W * 32), TanChainSmem<R, N, W, DSM, false>::bytes, s, P);
         };
-        chain_dispatch(c, B, false, go);
+        chain_dispatch(c, B, true, go);
         start = end;
       };
       for (size_t i = 0; i < ops.size(); ++i) {

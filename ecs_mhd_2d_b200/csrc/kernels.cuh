@@ -333,16 +333,17 @@ __device__ __forceinline__ void col_inverse_uv(const cplx<typename X::R> (&x)[X:
 }
 
 // One plain inverse transform along x of a box column, scaled, to field f of
-// G[b] (nf fields per batch element).
-template <class X>
+// G[b] (nf fields per batch element; or to the cluster's G tiles, see col_put).
+template <int CX = 0, class X>
 __device__ __forceinline__ void col_inverse1(const cplx<typename X::R> (&x)[X::E], cplx<typename X::R>* G, int nf, int b,
-                                             int f, int ky, bool act, const X& xf, typename X::R scale) {
+                                             int f, int ky, bool act, const X& xf, typename X::R scale,
+                                             cplx<typename X::R>* gtile = nullptr) {
   using R = typename X::R;
   cplx<R> w[X::E];
 #pragma unroll
   for (int j = 0; j < X::E; ++j) w[j] = X::none(j) ? mk<R>(0, 0) : cscale_rn(x[j], scale);
   xf.template from_spec<true, true>(w);
-  col_put(w, G, nf, b, f, ky, act, xf);
+  col_put<CX>(w, G, nf, b, f, ky, act, xf, gtile);
 }
 
 // ---------------------------------------------------------------------------

@@ -99,7 +99,7 @@ template <typename R, int N, int W, bool DSM, bool DSH>
 using TanChainSmem = ChainSmem<R, N, W, DSM, DSH ? 5 : 8, (DSH ? S_NSLOT : 0) + 1>;
 template <typename R, int N, int W, bool DSM> using Rk4ChainSmem = ChainSmem<R, N, W, DSM, 0, 6>;
 template <typename R, int N, int W>
-using Rk43ChainSmem = ChainSmem<R, N, W, false, W == 8 ? 0 : 4, (W == 8 ? S_NSLOT : 0) + 2>;
+using Rk43ChainSmem = ChainSmem<R, N, W, true, W == 8 ? 0 : 4, (W == 8 ? S_NSLOT : 0) + 2>;
 
 template <typename R>
 struct ChainParams {
@@ -376,12 +376,15 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
 // jax_scripts/lib/timestepping.py:151-335) in one launch: cluster b runs state
 // b's attempts until it completes or `amax` attempts were made -- the column
 // stages A..E (k_col_rk43's transforms and algebra), the four RHS row passes
-// (k_row_rhs's body) and the error norm (k_row_err's body); each CTA's maximum goes to the
-// cluster through distributed shared memory, CTA 0 makes the accept/reject
-// decision and the step-size update on the control block (rk43_control, as
-// the last block of k_row_err does), and every CTA reads it after the next
-// cluster barrier.  The G and H arrays go through global memory.  Set-up,
-// START and INIT passes run before the launch.
+// (k_row_rhs's body) and the error norm (k_row_err's body).  G and H never leave the
+// cluster (an attempt starts from the slots alone).  Each CTA sends its error maximum to
+// every CTA of the cluster, and after one cluster barrier every CTA makes the same
+// accept/reject decision and step-size update (rk43_control, as the last block of
+// k_row_err does) on its own copy of the control block, which CTA 0 writes back at the
+// end.  Set-up, START and INIT passes run before the launch.
+// Measured at n = 128 FP64, T = 0.2, atol 1e-8 (G and H through global memory, CTA 0
+// deciding behind a second barrier -> this): batch 1 1.55 -> 1.45 ms, batch 8 4.28 -> 3.99;
+// at n = 64 1.26 -> 1.03 and 2.08 -> 1.67.
 // ---------------------------------------------------------------------------
 template <typename R>
 struct Rk43ChainParams {
@@ -427,9 +430,11 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
   using SM = Rk43ChainSmem<R, N, W>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_work = s_base + SM::work;
+  cplx<R>* s_gt = s_base + SM::gt;
+  cplx<R>* s_hc = s_base + SM::hc;
   __shared__ double s_max[W];
-  __shared__ double s_part;   // this CTA's error maximum, read by CTA 0 of the cluster
+  __shared__ double s_errs[CL];   // the error maxima of the cluster's CTAs
+  __shared__ StepCtl s_ctl;       // state b's control block, the same in every CTA
   const X xf(s_base, threadIdx.x >> 5);
   const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
   const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
@@ -438,10 +443,11 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
   cplx<R>* my_s = s_base + SM::ds + (size_t)wc * ((DSH ? S_NSLOT : 0) + 2) * M;
   const SharedRow<R> forcing{my_s}, mu{my_s + M};
   cplx<R>* S = DSH ? my_s + 2 * M : sglob;
-  cplx<R>* rows = s_work + (size_t)wc * (DSH ? 0 : 4) * M;
-  StepCtl* ctl = P.col.ctl + b;
+  cplx<R>* rows = s_base + SM::work + (size_t)wc * (DSH ? 0 : 4) * M;
+  const cplx<R>* my_h = s_hc + (size_t)wc * 2 * N;
   load_tables<X>(s_base, P.col.tw);
   pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (threadIdx.x == 0) s_ctl = P.col.ctl[b];
   if (cw >= 0) {
     for (int e = xf.l; e < M; e += 32) {
       my_s[e] = P.col.fhat[id.ky * M + e];
@@ -451,14 +457,13 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
       for (int d = 0; d < S_NSLOT; ++d)
         for (int e = xf.l; e < M; e += 32) S[d * M + e] = sglob[d * VEC + e];
   }
-  __syncthreads();
-  for (long a = 0; a < P.amax; ++a) {
-    if (*(volatile int*)&ctl->done) break;   // written by CTA 0 before the last cluster barrier
-    const R43Col<R> c(P.col, b, id.ch, id.ky, VEC, X::K, M);
+  cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  for (long a = 0; a < P.amax && !s_ctl.done; ++a) {
+    const R43Col<R> c(P.col, s_ctl, b, id.ch, id.ky, VEC, X::K, M);
 #pragma unroll 1
     for (int st = R43_A; st <= R43_E; ++st) {
       if (st != R43_A) {
-        row_rhs_body<W>(P.row, b, rank * W, xf, s_work, s_work);
+        row_rhs_body<W, true>(P.row, b, rank * W, xf, s_gt, s_gt, false, s_hc);
         cluster_barrier();
       }
       if (cw >= 0) {
@@ -466,7 +471,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
         cplx<R> r[X::E], x[X::E];
 #pragma unroll
         for (int i = 0; i < X::E; ++i) r[i] = x[i] = mk<R>(0, 0);
-        if (st != R43_A) chain_rhs(P.col.H, id, xf, (const cplx<R>*)nullptr, r);
+        if (st != R43_A) chain_rhs(P.col.H, id, xf, my_h, r);
         if constexpr (!DSH) staged_wait();
         switch (st) {
           case R43_A: chain_rk43_algebra<R43_A, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
@@ -475,33 +480,32 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk43_chain(Rk43ChainParams<R> P) 
           case R43_D: chain_rk43_algebra<R43_D, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
           default: chain_rk43_algebra<R43_E, DSH>(P.col, c, id, xf, rows, S, SS, forcing, r, x); break;
         }
-        if (st == R43_E) col_inverse1(x, P.col.G, NG, b, id.ch, id.ky, true, xf, R(1) / (R(N) * R(N)));
-        else col_inverse_uv(x, P.col.G, b, id.ch, id.ky, true, xf, mu);
+        if (st == R43_E) col_inverse1<W>(x, P.col.G, NG, b, id.ch, id.ky, true, xf, R(1) / (R(N) * R(N)), s_gt);
+        else col_inverse_uv<W>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, s_gt);
       }
       cluster_barrier();
     }
-    const double bm = row_err_max<W>(P.col.G, b, rank * W, xf, s_work, s_max);
-    if (threadIdx.x == 0) s_part = bm;
+    const double bm = row_err_max<W>(P.col.G, b, rank * W, xf, s_gt, s_max, false);
+    if (threadIdx.x < CL)
+      *cooperative_groups::this_cluster().map_shared_rank(&s_errs[rank], (unsigned)threadIdx.x) = bm;
     cluster_barrier();
-    if (rank == 0 && threadIdx.x == 0) {
-      cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    if (threadIdx.x == 0) {
       double err = 0.0;
-      for (int r = 0; r < CL; ++r) {
-        const double q = *cl.map_shared_rank(&s_part, (unsigned)r);
-        err = (q > err || isnan(q)) ? q : err;
-      }
-      const int at = ctl->attempts, cap = P.col.cap;
-      rk43_control(*ctl, P.atol, err, P.rec_h && at < cap ? P.rec_h + (size_t)b * cap : nullptr,
-                   P.rec_acc && at < cap ? P.rec_acc + (size_t)b * cap : nullptr);
+      for (int r = 0; r < CL; ++r) err = (s_errs[r] > err || isnan(s_errs[r])) ? s_errs[r] : err;
+      const int at = s_ctl.attempts, cap = P.col.cap;
+      const bool rec = rank == 0 && at < cap;
+      rk43_control(s_ctl, P.atol, err, rec && P.rec_h ? P.rec_h + (size_t)b * cap : nullptr,
+                   rec && P.rec_acc ? P.rec_acc + (size_t)b * cap : nullptr);
     }
-    cluster_barrier();
+    __syncthreads();
   }
+  if (rank == 0 && threadIdx.x == 0) P.col.ctl[b] = s_ctl;
   if constexpr (DSH) {
     __syncwarp();
     if (cw >= 0)
       for (int d = 0; d < S_NSLOT; ++d)
         for (int e = xf.l; e < M; e += 32) sglob[d * VEC + e] = S[d * M + e];
   }
-}
+}   // (no CTA writes a peer's shared memory after the last cluster barrier)
 
 }  // namespace ecs

@@ -63,8 +63,7 @@ struct R43Col {
   R t, h;
   int pend;
   cplx<R>* rec;
-  __device__ __forceinline__ R43Col(const Col43Params<R>& p, int b, int ch, int ky, size_t VEC, int K, int M) {
-    const StepCtl& c = p.ctl[b];
+  __device__ __forceinline__ R43Col(const Col43Params<R>& p, const StepCtl& c, int b, int ch, int ky, size_t VEC, int K, int M) {
     t = (R)c.t; h = (R)c.h; pend = c.pending_accept;
     rec = p.rec ? p.rec + ((size_t)b * p.cap + (c.attempts < p.cap ? c.attempts : p.cap - 1)) * RR_NREC * VEC +
                       ((size_t)ch * K + ky) * M
@@ -152,7 +151,7 @@ __device__ __forceinline__ void col_rk43_body(const Col43Params<typename X::R>& 
   constexpr size_t VEC = (size_t)2 * K * M;
   const int ch = id.ch, b = id.b, ky = id.ky;
   if (p.ctl[b].done) return;
-  const R43Col<R> c(p, b, ch, ky, VEC, K, M);
+  const R43Col<R> c(p, p.ctl[b], b, ch, ky, VEC, K, M);
   cplx<R>* S = p.S + (size_t)b * S_NSLOT * VEC + ((size_t)ch * K + ky) * M;
   constexpr bool has_rhs = STAGE != R43_A && STAGE != R43_START;
   constexpr int n = popc_c(r43_omask(STAGE));
@@ -223,14 +222,14 @@ __device__ __forceinline__ void rk43_control(StepCtl& c, double atol, double err
 }
 
 // max |irfft2(d)| over rows x0 .. x0 + XT - 1 of state b (the inverse column
-// transforms of d in G fields 0 and 1), one group per row; s_max holds one value
-// per warp; valid in every thread.
+// transforms of d in G fields 0 and 1, or in the tile s_G already unless load_g), one
+// warp per row; s_max holds one value per warp; valid in every thread.
 template <int XT, class X>
 __device__ __forceinline__ double row_err_max(const cplx<typename X::R>* G, int b, int x0, const X& xf,
-                                              cplx<typename X::R>* s_G, double* s_max) {
+                                              cplx<typename X::R>* s_G, double* s_max, bool load_g = true) {
   using R = typename X::R;
   constexpr int N = X::N;
-  load_tile<R, N, XT>(s_G, G + (size_t)b * NG * X::K * N, 2 * X::K, x0);
+  if (load_g) load_tile<R, N, XT>(s_G, G + (size_t)b * NG * X::K * N, 2 * X::K, x0);
   __syncthreads();
   cplx<R> z[X::E];
   load_pair<XT>(s_G, s_G + X::K * (XT + 1), threadIdx.x / X::L, xf, z);
