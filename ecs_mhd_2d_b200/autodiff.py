@@ -154,8 +154,7 @@ def jvp_multi(primals, tangents, param_dicts, mode="Lawson_RK4", ctx=None):
     for (f, _, _, _) in ts:
         if f.shape[0] != 1:
             raise ValueError("jvp_multi: one tangent per candidate")
-    key = _ctx.physics_key(param_dicts[0])
-    if any(_ctx.physics_key(pd) != key for pd in param_dicts[1:]):
+    if not _ctx.same_physics(param_dicts):
         raise ValueError("jvp_multi: the candidates' param dicts differ in grid or physics")
     cfgs = (_lib.EcsShootCfg * B)()
     for b, pd in enumerate(param_dicts):
@@ -201,8 +200,7 @@ def loss_grad_multi(inputs, param_dicts, mode="Lawson_RK4", ctx=None):
     for (f, _, _, _) in xs:
         if f.shape != (1, 2, n, n) or f.dtype != dtype:
             raise ValueError("loss_grad_multi: every input is one state of the same grid and dtype")
-    key = _ctx.physics_key(param_dicts[0])
-    if any(_ctx.physics_key(pd) != key for pd in param_dicts[1:]):
+    if not _ctx.same_physics(param_dicts):
         raise ValueError("loss_grad_multi: the candidates' param dicts differ in grid or physics")
     cfgs = (_lib.EcsShootCfg * B)()
     for b, pd in enumerate(param_dicts):

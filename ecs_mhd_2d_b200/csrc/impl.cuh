@@ -222,14 +222,21 @@ void launch_row_from_box(ecs_ctx* c, const cplx<R>* G2, R* out, const R* base, d
   ++c->launches; { const Shape sh = row_shape<Xf<R, N>>(B, 2); k_row_from_box<R, N, XT><<<sh.grid, sh.block, sh.smem, s>>>(p); }
 }
 
-template <typename R, int N>
-void launch_col_rk4(ecs_ctx* c, int B, int stage, int produce, int diss, cudaStream_t s, cplx<R>* rec = nullptr,
-                    long rec_bstride = 0, int use_done = 0) {
+template <typename R>
+ColParams<R> col_params(ecs_ctx* c, int B) {
   ColParams<R> p{};
   p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.F = (cplx<R>*)c->F; p.A1 = (cplx<R>*)c->A1;
   p.K2 = (cplx<R>*)c->K2; p.OUT = (cplx<R>*)c->OUT; p.Etab = (const R*)c->Etab; p.ctl = c->ctl;
   p.fhat = (const cplx<R>*)c->fhat; p.tw = (const cplx<R>*)c->tw; p.nu = (R)c->nu; p.eta = (R)c->eta;
-  p.B = B; p.stage = stage; p.produce = produce; p.diss = diss; p.rec = rec; p.rec_bstride = rec_bstride;
+  p.B = B;
+  return p;
+}
+
+template <typename R, int N>
+void launch_col_rk4(ecs_ctx* c, int B, int stage, int produce, int diss, cudaStream_t s, cplx<R>* rec = nullptr,
+                    long rec_bstride = 0, int use_done = 0) {
+  ColParams<R> p = col_params<R>(c, B);
+  p.stage = stage; p.produce = produce; p.diss = diss; p.rec = rec; p.rec_bstride = rec_bstride;
   p.use_done = use_done;
   const Shape sh = col_shape<Xf<R, N>>(B);
   switch (stage) {
@@ -482,13 +489,12 @@ struct Impl {
   }
 
   static int state_vel(ecs_ctx* c, const cplx<R>* fhat, cplx<R>* dfdt, int B, int diss, cudaStream_t s) {
-    const long nbox = (long)B * 2 * K * M;
-    ++c->launches; k_gather_box<R><<<grid1d(nbox), 256, 0, s>>>(fhat, (cplx<R>*)c->F, N, B);
-    launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s);
+    ColParams<R> p = col_params<R>(c, B);
+    p.diss = diss;
+    launch_step(c, B, k_col_full_start<R, N>, col_shape<Xf<R, N>>(B), s, p, fhat);
     launch_row_rhs<R, N>(c, B, s);
-    launch_col_rk4<R, N>(c, B, COL_PLAIN, 0, diss, s);
-    const long nfull = (long)B * 2 * N * (N / 2 + 1);
-    ++c->launches; k_scatter_box<R><<<grid1d(nfull), 256, 0, s>>>((const cplx<R>*)c->OUT, dfdt, N, B);
+    const Shape vel{dim3((B * 2 * (N / 2 + 1) + COLWARPS - 1) / COLWARPS), dim3(COLWARPS * 32), 0};
+    launch_step(c, B, k_col_full_vel<R, N>, vel, s, p, fhat, dfdt);
     return cuda_err(c, cudaGetLastError(), "state_vel");
   }
 
@@ -519,11 +525,7 @@ struct Impl {
   static int rk4_chain(ecs_ctx* c, int B, long steps, cudaStream_t s) {
     if constexpr (N <= 128) {
       Rk4ChainParams<R> P{};
-      ColParams<R>& p = P.col;
-      p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.F = (cplx<R>*)c->F; p.A1 = (cplx<R>*)c->A1;
-      p.K2 = (cplx<R>*)c->K2; p.OUT = (cplx<R>*)c->OUT; p.Etab = (const R*)c->Etab; p.ctl = c->ctl;
-      p.fhat = (const cplx<R>*)c->fhat; p.tw = (const cplx<R>*)c->tw; p.nu = (R)c->nu; p.eta = (R)c->eta;
-      p.B = B;
+      P.col = col_params<R>(c, B);
       RowParams<R>& q = P.row;
       q.G = (const cplx<R>*)c->G; q.H = (cplx<R>*)c->H; q.tw = (const cplx<R>*)c->tw;
       q.b0x = (R)c->b0x; q.b0y = (R)c->b0y; q.B = B;
