@@ -121,6 +121,11 @@ struct PlainOrder {
   PlainOrder& operator=(const PlainOrder&) = delete;
 };
 
+// Lawson-RK6 keeps 11 rows per column: too many for a 16-warp CTA in FP64 at n = 128.
+template <typename R, int N, int W, int SCHEME> constexpr bool fx_chain_fits() {
+  return FxChainSmem<R, N, W, SCHEME>::bytes <= 227 * 1024;
+}
+
 template <typename R, int N, int W>
 int configure_chain() {
   int st = 0;
@@ -137,6 +142,9 @@ int configure_chain() {
   attrs(k_rk43_chain<R, N, W>, Rk43ChainSmem<R, N, W>::bytes);
   attrs(k_rk4_chain<R, N, W, false>, Rk4ChainSmem<R, N, W, false>::bytes);
   attrs(k_rk4_chain<R, N, W, true>, Rk4ChainSmem<R, N, W, true>::bytes);
+  if constexpr (fx_chain_fits<R, N, W, FX_RK4>()) attrs(k_fx_chain<R, N, W, FX_RK4>, FxChainSmem<R, N, W, FX_RK4>::bytes);
+  if constexpr (fx_chain_fits<R, N, W, FX_RK6>()) attrs(k_fx_chain<R, N, W, FX_RK6>, FxChainSmem<R, N, W, FX_RK6>::bytes);
+  if constexpr (fx_chain_fits<R, N, W, FX_TD4>()) attrs(k_fx_chain<R, N, W, FX_TD4>, FxChainSmem<R, N, W, FX_TD4>::bytes);
   return st;
 }
 
@@ -375,13 +383,18 @@ void launch_col_fx_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColFxP
   ((stage == ST ? launch_step(c, B, k_col_fx<R, N, SCHEME, ST>, sh, s, p) : void()), ...);
 }
 
-template <typename R, int N>
-void launch_col_fx(ecs_ctx* c, int B, int scheme, int stage, int produce, cudaStream_t s, cplx<R>* rec = nullptr) {
-  ColFxParams<R> p;
-  p.rec = rec;
+template <typename R>
+ColFxParams<R> col_fx_params(ecs_ctx* c, int B) {
+  ColFxParams<R> p{};
   p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.S = (cplx<R>*)c->S43; p.Etab = (const R*)c->Etab; p.ctl = c->ctl;
   p.fhat = (const cplx<R>*)c->fhat; p.tw = (const cplx<R>*)c->tw; p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B;
-  p.produce = produce;
+  return p;
+}
+
+template <typename R, int N>
+void launch_col_fx(ecs_ctx* c, int B, int scheme, int stage, int produce, cudaStream_t s, cplx<R>* rec = nullptr) {
+  ColFxParams<R> p = col_fx_params<R>(c, B);
+  p.rec = rec; p.produce = produce;
   if (scheme == FX_RK4) launch_col_fx_sw<R, N, FX_RK4>(c, B, stage, s, p, std::make_integer_sequence<int, 5>{});
   else if (scheme == FX_RK6) launch_col_fx_sw<R, N, FX_RK6>(c, B, stage, s, p, std::make_integer_sequence<int, 9>{});
   else launch_col_fx_sw<R, N, FX_TD4>(c, B, stage, s, p, std::make_integer_sequence<int, 5>{});
@@ -522,14 +535,20 @@ struct Impl {
 
   // Lawson-RK4 steps of the box states in c->F as one cluster-resident launch
   // (k_rk4_chain), after the COL_START pass; no inverse transforms after the last stage.
-  static int rk4_chain(ecs_ctx* c, int B, long steps, cudaStream_t s) {
+  // rec, phys: optional records of the steps (see Rk4ChainParams); use_done skips the
+  // candidates whose ctl.done is set.
+  static int rk4_chain(ecs_ctx* c, int B, long steps, cudaStream_t s, int last_produce = 0, cplx<R>* rec = nullptr,
+                       long rec_bstride = 0, R* phys = nullptr, int use_done = 0) {
     if constexpr (N <= 128) {
       Rk4ChainParams<R> P{};
       P.col = col_params<R>(c, B);
+      P.col.rec = rec; P.col.rec_bstride = rec_bstride; P.col.use_done = use_done;
+      P.rec_step = (long)Q_NREC * 2 * K * M;
+      P.row.phys = phys; P.row.phys_bstride = (long)N * NPH * N; P.phys_step = B * P.row.phys_bstride;
       RowParams<R>& q = P.row;
       q.G = (const cplx<R>*)c->G; q.H = (cplx<R>*)c->H; q.tw = (const cplx<R>*)c->tw;
       q.b0x = (R)c->b0x; q.b0y = (R)c->b0y; q.B = B;
-      P.steps = steps; P.last_produce = 0;
+      P.steps = steps; P.last_produce = last_produce;
       auto go = [&](auto w, auto dsm) {
         constexpr int W = decltype(w)::value;
         constexpr bool DSM = decltype(dsm)::value;
@@ -549,6 +568,10 @@ struct Impl {
   // in the Lawson-RK4 chain range (chain_batch) run as one cluster-resident launch.
   static int integrate_rk4(ecs_ctx* c, int B, long steps, cudaStream_t s) {
     if (steps <= 0) return ECS_OK;
+    if (chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb)) {
+      launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s);
+      return rk4_chain(c, B, steps, s);
+    }
     constexpr int GS = 16;
     auto one_step = [&](cudaStream_t st_, bool last) {
       for (int st = 1; st <= 4; ++st) {
@@ -575,7 +598,6 @@ struct Impl {
       gk.B = B;
     }
     launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s);
-    if (chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb)) return rk4_chain(c, B, steps, s);
     long it = 0;
     while (steps - it > GS) {   // the final step (no inverse transforms) is launched directly
       cudaError_t e = cudaGraphLaunch(gk.exec, s);
@@ -587,8 +609,51 @@ struct Impl {
     return cuda_err(c, cudaGetLastError(), "integrate_rk4");
   }
 
+  // Whether a batch of B runs the other fixed-step modes through k_fx_chain: the range of
+  // the Lawson-RK4 chain, or, where only 8-warp clusters have the room, two rounds of them
+  // (Lawson-RK6 in FP64 at n = 128, 32 steps, launch per pass / chain: batch 8 4.31 / 3.83 ms,
+  // 14 4.79 / 3.85, 16 5.32 / 5.68).
+  static bool fx_chain_batch(const ecs_ctx* c, int scheme, int B) {
+    if constexpr (N <= 128) {
+      if (scheme == FX_RK6 && !fx_chain_fits<R, N, 16, FX_RK6>())
+        return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? 2 * c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
+      return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
+    }
+    return false;
+  }
+  // `steps` steps of the states in slot X_F of S43 as one cluster-resident launch, after the
+  // stage-0 pass (TDRK4: phys, one record of physical fields per state).
+  static int fx_chain(ecs_ctx* c, int scheme, int B, long steps, cudaStream_t s, R* phys, cplx<R>* rec = nullptr,
+                      long rec_step = 0) {
+    if constexpr (N <= 128) {
+      FxChainParams<R> P{};
+      P.col = col_fx_params<R>(c, B);
+      P.col.rec = rec; P.rec_step = rec_step; P.steps = steps;
+      RowParams<R>& q = P.row;
+      q.G = (const cplx<R>*)c->G; q.H = (cplx<R>*)c->H; q.tw = (const cplx<R>*)c->tw;
+      q.phys = phys; q.phys_bstride = (long)N * NPH * N;
+      q.b0x = (R)c->b0x; q.b0y = (R)c->b0y; q.B = B;
+      auto go = [&](auto w, auto sch) {
+        constexpr int W = decltype(w)::value, S = decltype(sch)::value;
+        if constexpr (fx_chain_fits<R, N, W, S>())
+          launch_cluster(c, B, chain_cl<N, W>(), k_fx_chain<R, N, W, S>, dim3(B * chain_cl<N, W>()), dim3(W * 32),
+                         FxChainSmem<R, N, W, S>::bytes, s, P);
+      };
+      auto with_w = [&](auto sch) {
+        const bool w16 = fx_chain_fits<R, N, 16, decltype(sch)::value>();
+        const int w = c->chain_w && (c->chain_w == 8 || w16) ? c->chain_w : (B <= c->chain_res8 || !w16 ? 8 : 16);
+        if (w == 8) go(std::integral_constant<int, 8>{}, sch);
+        else go(std::integral_constant<int, 16>{}, sch);
+      };
+      if (scheme == FX_RK6) with_w(std::integral_constant<int, FX_RK6>{});
+      else if (scheme == FX_TD4) with_w(std::integral_constant<int, FX_TD4>{});
+      else with_w(std::integral_constant<int, FX_RK4>{});
+    }
+    return cuda_err(c, cudaGetLastError(), "fixed-step chain");
+  }
+
   // Fixed-step RK4 / Lawson-RK6 / TDRK4 over `steps` steps from slot X_F of S43
-  // (h and e from fx_setup); 16-step CUDA graphs per scheme.
+  // (h and e from fx_setup): one cluster-resident launch, or 16-step CUDA graphs per scheme.
   static int integrate_fx(ecs_ctx* c, int scheme, int B, long steps, cudaStream_t s) {
     PlainOrder plain_order(c);
     if (steps <= 0) return ECS_OK;
@@ -600,7 +665,11 @@ struct Impl {
       if (st) return st;
       phys = (R*)c->fxphys;
     }
-    const int nst = scheme == FX_RK6 ? 8 : 4;
+    if (fx_chain_batch(c, scheme, B)) {
+      launch_col_fx<R, N>(c, B, scheme, 0, 1, s);
+      return fx_chain(c, scheme, B, steps, s, phys);
+    }
+    const int nst = fx_stages(scheme);
     auto one_step = [&](cudaStream_t st_, bool last) {
       for (int q = 1; q <= nst; ++q) {
         const int produce = (q == nst && last) ? 0 : 1;
@@ -885,6 +954,10 @@ struct Impl {
   static void record_rk4_segment(ecs_ctx* c, cplx<R>* rec, long steps, cudaStream_t s) {
     const size_t VEC = 2UL * K * M;
     launch_col_rk4<R, N>(c, 1, COL_START, 1, 0, s);
+    if (chain_batch(c, 1, c->rk4chain_minb, c->rk4chain_maxb)) {
+      rk4_chain(c, 1, steps, s, 0, rec);
+      return;
+    }
     for (long it = 0; it < steps; ++it) {
       cplx<R>* rs = rec + (size_t)it * Q_NREC * VEC;
       for (int k = 1; k <= 4; ++k) {
@@ -986,7 +1059,12 @@ struct Impl {
     R* phys = (R*)c->fxphys;
     cplx<R>* rec = (cplx<R>*)L.rec;
     launch_col_fx<R, N>(c, 1, FX_TD4, 0, 1, s);
-    for (long it = 0; it < steps; ++it) {
+    const bool chain = fx_chain_batch(c, FX_TD4, 1);
+    if (chain) {
+      st = fx_chain(c, FX_TD4, 1, steps, s, phys, rec, (long)TR_NREC * VEC);
+      if (st) return st;
+    }
+    for (long it = 0; !chain && it < steps; ++it) {
       cplx<R>* rs = rec + (size_t)it * TR_NREC * VEC;
       for (int q = 1; q <= 4; ++q) {
         if (q == 2 || q == 4) launch_row_tan<R, N>(c, 1, phys, s, 0);
@@ -1091,7 +1169,12 @@ struct Impl {
                                                     c->nu, c->eta, 1);
     cplx<R>* rec = (cplx<R>*)L.rec;
     launch_col_fx<R, N>(c, 1, scheme, 0, 1, s);
-    for (long it = 0; it < steps; ++it) {
+    const bool chain = fx_chain_batch(c, scheme, 1);
+    if (chain) {
+      st = fx_chain(c, scheme, 1, steps, s, nullptr, rec, (long)NR * VEC);
+      if (st) return st;
+    }
+    for (long it = 0; !chain && it < steps; ++it) {
       cplx<R>* rs = rec + (size_t)it * NR * VEC;
       for (int q = 1; q <= S; ++q) {
         launch_row_rhs<R, N>(c, 1, s);
@@ -2413,10 +2496,19 @@ struct Impl {
     // forward solves with a checkpoint every SEG steps (the loss has no phase-condition part)
     cplx<R>* ckpt = (cplx<R>*)m.ckpt;
     launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s, nullptr, 0, 1);
+    // (the candidates' step counts are multiples of seg, so a chain of seg steps suits all)
+    const bool chain = chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
     for (long it = 0; it < smax; ++it) {
       if (it % seg == 0) {
         e = cudaMemcpyAsync(ckpt + (size_t)(it / seg) * B * VEC, F, B * vb, cudaMemcpyDeviceToDevice, s);
         if (e != cudaSuccess) return cuda_err(c, e, "loss_grad_multi checkpoint");
+      }
+      if (chain) {
+        st = rk4_chain(c, B, seg, s, 1, nullptr, 0, nullptr, 1);
+        if (st) return st;
+        ++c->launches; k_pool_count<<<(B + 127) / 128, 128, 0, s>>>(c->ctl, B, (int)seg);
+        it += seg - 1;
+        continue;
       }
       for (int q = 1; q <= 4; ++q) {
         launch_row_rhs<R, N>(c, B, s, c->ctl);
@@ -2459,7 +2551,11 @@ struct Impl {
       ++c->launches;
       k_grad_segment<R><<<grid1d((long)B * VEC), 256, 0, s>>>(F, ckpt, m.nseg, (int)r, c->ctl, (long)VEC, B);
       launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s, nullptr, 0, 1);
-      for (long it = 0; it < seg; ++it) {
+      if (chain) {
+        st = rk4_chain(c, B, seg, s, 0, grec, rstride, gphys, 1);
+        if (st) return st;
+      }
+      for (long it = 0; !chain && it < seg; ++it) {
         for (int q = 1; q <= 4; ++q) {
           launch_row_rhs<R, N>(c, B, s, c->ctl, gphys + (size_t)(it * 4 + q - 1) * B * pstride, pstride);
           launch_col_rk4<R, N>(c, B, q, (q == 4 && it == seg - 1) ? 0 : 1, 0, s, grec + (size_t)it * Q_NREC * VEC,

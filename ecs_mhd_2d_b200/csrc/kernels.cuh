@@ -1120,14 +1120,14 @@ static __global__ void k_pool_init(StepCtl* ctl, int first, int count, int steps
   c.attempts = 0; c.accepted = 0; c.rejected = 0; c.pending_accept = 0;
 }
 
-// Slot pool: count one finished step per active slot; a slot whose budget is
+// Slot pool: count `steps` finished steps per active slot; a slot whose budget is
 // spent is marked done and skipped by every later launch.
-static __global__ void k_pool_count(StepCtl* ctl, int B) {
+static __global__ void k_pool_count(StepCtl* ctl, int B, int steps = 1) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= B) return;
   StepCtl& c = ctl[b];
   if (c.done || c.steps_total <= 0) return;
-  c.steps_done += 1;
+  c.steps_done += steps;
   if (c.steps_done >= c.steps_total) c.done = 1;
 }
 

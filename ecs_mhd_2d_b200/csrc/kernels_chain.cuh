@@ -56,6 +56,9 @@
 // decision in the kernel), below.
 #pragma once
 
+#include <utility>
+
+#include "kernels_fx.cuh"
 #include "kernels_tan.cuh"
 
 namespace ecs {
@@ -293,6 +296,8 @@ struct Rk4ChainParams {
   RowParams<R> row;
   long steps;
   int last_produce;   // inverse transforms after the last stage (the next stage input)
+  long rec_step;      // col.rec: entries from a step's record to the next step's
+  long phys_step;     // row.phys: values from a stage's record to the next stage's
 };
 
 template <int STAGE, class X>
@@ -337,6 +342,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
   const cplx<R>* my_h = DSM ? s_hc + (size_t)wc * 2 * N : nullptr;
   load_tables<X>(s_base, P.col.tw);
   pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (P.col.use_done && P.col.ctl[b].done) return;   // the whole cluster
   if (cw >= 0)
     for (int s = xf.l; s < M; s += 32) {
       my_s[s] = P.col.F[at + s]; my_e[s] = P.col.Etab[at + s];
@@ -345,21 +351,25 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
   const R h = (R)P.col.ctl[b].h;
   __syncthreads();
   for (long step = 0; step < P.steps; ++step) {
+    ColParams<R> col = P.col;
+    if (col.rec) col.rec += step * P.rec_step;
 #pragma unroll 1
     for (int st = COL_RK4_S1; st <= COL_RK4_S4; ++st) {
       if (step > 0 || st > COL_RK4_S1) cluster_barrier();   // column pass -> row pass
       const bool first = step == 0 && st == COL_RK4_S1, last = step == P.steps - 1 && st == COL_RK4_S4;
       cplx<R>* tile = DSM ? s_gt : s_base + SM::work;
-      row_rhs_body<W, DSM>(P.row, b, rank * W, xf, tile, tile, first, s_hc);
+      RowParams<R> row = P.row;
+      if (row.phys) row.phys += (step * 4 + st - COL_RK4_S1) * P.phys_step;
+      row_rhs_body<W, DSM>(row, b, rank * W, xf, tile, tile, first, s_hc);
       cluster_barrier();                                     // row pass -> column pass
       if (cw < 0) continue;
       cplx<R> r[X::E], x[X::E];
       chain_rhs(P.col.H, id, xf, my_h, r);
       switch (st) {
-        case COL_RK4_S1: chain_rk4_algebra<COL_RK4_S1>(P.col, id, xf, w, h, forcing, r, x); break;
-        case COL_RK4_S2: chain_rk4_algebra<COL_RK4_S2>(P.col, id, xf, w, h, forcing, r, x); break;
-        case COL_RK4_S3: chain_rk4_algebra<COL_RK4_S3>(P.col, id, xf, w, h, forcing, r, x); break;
-        default: chain_rk4_algebra<COL_RK4_S4>(P.col, id, xf, w, h, forcing, r, x); break;
+        case COL_RK4_S1: chain_rk4_algebra<COL_RK4_S1>(col, id, xf, w, h, forcing, r, x); break;
+        case COL_RK4_S2: chain_rk4_algebra<COL_RK4_S2>(col, id, xf, w, h, forcing, r, x); break;
+        case COL_RK4_S3: chain_rk4_algebra<COL_RK4_S3>(col, id, xf, w, h, forcing, r, x); break;
+        default: chain_rk4_algebra<COL_RK4_S4>(col, id, xf, w, h, forcing, r, x); break;
       }
       if (!last || P.last_produce)
         col_inverse_uv<DSM ? W : 0>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, (DSM && !last) ? s_gt : nullptr);
@@ -369,6 +379,113 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
   if (cw >= 0)
     for (int s = xf.l; s < M; s += 32) P.col.F[at + s] = my_s[s];
   if constexpr (DSM) cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
+}
+
+// ---------------------------------------------------------------------------
+// Steps of the other fixed-step modes (RK4, Lawson-RK6, TDRK4; kernels_fx.cuh) in one
+// launch, with the layout of k_rk4_chain; the slots, e, forcing and multipliers of a
+// column stay in shared memory.  The passes are k_row_rhs's (k_row_tan's for TDRK4's
+// Jacobian-vector products, on the physical fields that the row's own warp left in
+// row.phys the pass before) and k_col_fx's.  The stage input of the first stage is in G.
+// Measured, 32 steps, launch per pass -> this: n = 128, batch 1 Lawson-RK6 2.75 -> 1.97 ms,
+// RK4 1.35 -> 0.93, TDRK4 1.36 -> 0.98; batch 12 5.27 -> 3.83, 2.38 -> 1.44, 2.22 -> 1.56;
+// n = 64, batch 8 2.41 -> 1.10, 1.09 -> 0.54, 1.09 -> 0.57.
+// ---------------------------------------------------------------------------
+template <typename R>
+struct FxChainParams {
+  ColFxParams<R> col;
+  RowParams<R> row;   // phys, phys_bstride: TDRK4
+  long steps;
+  int last_produce;
+  long rec_step;      // col.rec: entries from a step's record to the next step's
+};
+
+__host__ __device__ constexpr int fx_nslot(int scheme) { return scheme == FX_RK6 ? 8 : scheme == FX_TD4 ? 5 : 4; }
+template <typename R, int N, int W, int SCHEME> using FxChainSmem = ChainSmem<R, N, W, true, 0, fx_nslot(SCHEME) + 3>;
+
+template <int SCHEME, int STAGE, class X>
+__device__ __forceinline__ void chain_fx_algebra(typename X::R h, typename X::R coeff, const ColId<X>& id, const X& xf,
+                                                 cplx<typename X::R>* S, const typename X::R* e,
+                                                 const SharedRow<typename X::R>& forcing, cplx<typename X::R>* rec,
+                                                 const cplx<typename X::R> (&r)[X::E], cplx<typename X::R> (&x)[X::E]) {
+  using R = typename X::R;
+  constexpr int M = X::M;
+  constexpr size_t VEC = (size_t)2 * X::K * M;
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    x[i] = mk<R>(0, 0);
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    cplx<R> v = r[i];
+    if (fx_rhs(SCHEME, STAGE) == 1 && id.ch == 0 && !(slot == 0 && id.ky == 0)) v = cadd(v, forcing(slot));
+    x[i] = fx_algebra<SCHEME, STAGE, R>(h, diss_L<R>(xf.kx(i), (R)id.ky, coeff), v,
+                                        [&](int q) -> cplx<R> { return S[q * M + slot]; },
+                                        [&](int q, cplx<R> a) { S[q * M + slot] = a; }, [&]() { return e[slot]; },
+                                        [&](int q, cplx<R> a) { if (rec) rec[q * VEC + slot] = a; });
+  }
+}
+template <int SCHEME, class X, int... ST, typename... A>
+__device__ __forceinline__ void chain_fx_stage(int st, std::integer_sequence<int, ST...>, A&&... a) {
+  ((st == ST + 1 ? chain_fx_algebra<SCHEME, ST + 1, X>(a...) : (void)0), ...);
+}
+
+template <typename R, int N, int W, int SCHEME>
+__global__ void __launch_bounds__(W * 32, 1) k_fx_chain(FxChainParams<R> P) {
+  using X = Xf<R, N>;
+  constexpr int M = X::M, CL = chain_cl<N, W>(), NS = fx_nslot(SCHEME);
+  constexpr size_t VEC = (size_t)2 * X::K * M;
+  using SM = FxChainSmem<R, N, W, SCHEME>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_gt = s_base + SM::gt;
+  cplx<R>* s_hc = s_base + SM::hc;
+  const X xf(s_base, threadIdx.x >> 5);
+  const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  const size_t at = ((size_t)id.ch * X::K + id.ky) * M;
+  cplx<R>* F = P.col.S + (size_t)b * S_NSLOT * VEC + X_F * VEC + at;
+  cplx<R>* S = s_base + SM::ds + (size_t)wc * (NS + 3) * M;
+  R* e = reinterpret_cast<R*>(S + NS * M);
+  const SharedRow<R> forcing{S + (NS + 1) * M}, mu{S + (NS + 2) * M};
+  const cplx<R>* my_h = s_hc + (size_t)wc * 2 * N;
+  load_tables<X>(s_base, P.col.tw);
+  pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) {
+      S[X_F * M + s] = F[s];
+      if (SCHEME == FX_RK6) e[s] = P.col.Etab[(size_t)b * VEC + at + s];
+      S[(NS + 1) * M + s] = P.col.fhat[id.ky * M + s];
+      S[(NS + 2) * M + s] = mu_row<X>(P.col.tw, id.ky)[s];
+    }
+  const R h = (R)P.col.ctl[b].h, coeff = id.ch == 0 ? P.col.nu : P.col.eta;
+  cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  RowTanParams<R> tan{};
+  tan.G = P.row.G; tan.H = P.row.H; tan.phys = P.row.phys; tan.phys_bstride = P.row.phys_bstride; tan.tw = P.row.tw;
+  for (long step = 0; step < P.steps; ++step) {
+    cplx<R>* rec = P.col.rec ? P.col.rec + step * P.rec_step + at : nullptr;
+#pragma unroll 1
+    for (int st = 1; st <= fx_stages(SCHEME); ++st) {
+      if (step > 0 || st > 1) cluster_barrier();   // column pass -> row pass
+      const bool first = step == 0 && st == 1, last = step == P.steps - 1 && st == fx_stages(SCHEME);
+      if (SCHEME == FX_TD4 && fx_rhs(SCHEME, 2) == 2 && (st & 1) == 0)
+        row_tan_body<W, true>(tan, b, rank * W, xf, s_gt, s_gt, false, s_hc);
+      else
+        row_rhs_body<W, true>(P.row, b, rank * W, xf, s_gt, s_gt, first, s_hc);
+      cluster_barrier();                            // row pass -> column pass
+      if (cw < 0) continue;
+      cplx<R> r[X::E], x[X::E];
+      chain_rhs(P.col.H, id, xf, my_h, r);
+      chain_fx_stage<SCHEME, X>(st, std::make_integer_sequence<int, fx_stages(SCHEME)>{}, h, coeff, id, xf, S,
+                                (const R*)e, forcing, rec, r, x);
+      if (!last || P.last_produce)
+        col_inverse_uv<W>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, last ? nullptr : s_gt);
+    }
+  }
+  __syncwarp();
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) F[s] = S[X_F * M + s];
+  cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
 }
 
 // ---------------------------------------------------------------------------

@@ -40,11 +40,11 @@ struct ColFxParams {
                         // RK4 / Lawson-RK6 [f0, k_1..k_S, x_2..x_S] (see kernels_fxl.cuh)
 };
 
-template <int SCHEME, int STAGE> struct FxTraits {
-  // the right-hand side entering this stage: 0 none, 1 full (forcing), 2 Jacobian-vector product (no forcing)
-  static constexpr int rhs = STAGE == 0 ? 0 : (SCHEME == FX_TD4 && (STAGE == 2 || STAGE == 4)) ? 2 : 1;
-  static constexpr int last = SCHEME == FX_RK4 ? 4 : SCHEME == FX_RK6 ? 8 : 4;
-};
+// The right-hand side entering a stage: 0 none, 1 full (forcing), 2 Jacobian-vector product (no forcing).
+__host__ __device__ constexpr int fx_rhs(int scheme, int stage) {
+  return stage == 0 ? 0 : (scheme == FX_TD4 && (stage == 2 || stage == 4)) ? 2 : 1;
+}
+__host__ __device__ constexpr int fx_stages(int scheme) { return scheme == FX_RK6 ? 8 : 4; }
 
 // Slots that a stage reads before it writes any (bits of FxSlot); they are loaded
 // together before the stage's stores.
@@ -61,12 +61,140 @@ __host__ __device__ constexpr unsigned fx_smask(int scheme, int stage) {
        : F | (1u << X_K1) | (1u << X_A1) | (1u << X_K2T);
 }
 
+// The algebra of a stage at one mode: the stage input from the derivative v (forcing
+// included).  Q(q) reads and W(q, a) writes slot q, E() gives the factor e (Lawson-RK6)
+// and put(q, a) records.
+template <int SCHEME, int STAGE, typename R, class Qf, class Wf, class Ef, class Pf>
+__device__ __forceinline__ cplx<R> fx_algebra(R h, R L, cplx<R> v, Qf&& Q, Wf&& W, Ef&& E, Pf&& put) {
+  constexpr unsigned SM = fx_smask(SCHEME, STAGE);
+  cplx<R> xin = mk<R>(0, 0);
+  if (STAGE == 0) {
+    xin = Q(X_F);
+  } else if (SCHEME == FX_RK4) {
+    // v_fn includes dissipation L x at the stage input x (loss_functions.py:53, mhd_jax.py:171-173)
+    const cplx<R> f = Q(X_F);
+    cplx<R> xs = f;
+    if (STAGE == 2) xs = cadd(f, cdiv_k<2>(Q(X_K1)));
+    if (STAGE == 3) xs = cadd(f, cdiv_k<2>(Q(X_K1 + 1)));
+    if (STAGE == 4) xs = cadd(f, Q(X_K1 + 2));
+    const cplx<R> k = cscale(cadd(v, cscale(xs, L)), h);            // timestepping.py:40-43
+    // record: f0, k_s, x_{s+1}
+    if (STAGE == 1) put(0, f);
+    put(STAGE, k);
+    if (STAGE < 4) {
+      W(X_K1 + STAGE - 1, k);
+      xin = STAGE < 3 ? cadd(f, cdiv_k<2>(k)) : cadd(f, k);
+      put(4 + STAGE, xin);
+    } else {
+      const cplx<R> fn = cadd(cadd(cadd(cadd(f, cdiv_k<6>(Q(X_K1))), cdiv_k<3>(Q(X_K1 + 1))),
+                                   cdiv_k<3>(Q(X_K1 + 2))), cdiv_k<6>(k));   // :44
+      W(X_F, fn);
+      xin = fn;
+    }
+  } else if (SCHEME == FX_RK6) {
+    const R e = E();
+    const cplx<R> k = cscale(v, h);
+    // record: f0, k_s (before any factor)
+    if (STAGE == 1) put(0, Q(X_F));
+    put(STAGE, k);
+    // f, k1..k_{STAGE-1} and the new k, times e after stages 1, 3..7 and stored
+    constexpr bool SC = STAGE != 2 && STAGE != 8;
+    cplx<R> f = Q(X_F), K_[9];
+#pragma unroll
+    for (int q = 1; q < 9; ++q) K_[q] = mk<R>(0, 0);
+#pragma unroll
+    for (int q = 1; q < STAGE; ++q)
+      if ((SM >> (X_K1 + q - 1)) & 1u) K_[q] = Q(X_K1 + q - 1);
+    K_[STAGE] = k;
+    if (SC) {
+      f = cscale_rn(f, e);
+      W(X_F, f);
+#pragma unroll
+      for (int q = 1; q <= STAGE; ++q) { K_[q] = cscale_rn(K_[q], e); W(X_K1 + q - 1, K_[q]); }
+    } else if (STAGE == 2) {
+      W(X_K1 + 1, k);
+    }
+    switch (STAGE) {
+      case 1:   // :110-112
+        xin = cadd(f, cdiv_k<6>(K_[1]));
+        break;
+      case 2:   // :113
+        xin = cadd(cadd(f, cdiv_k<12>(K_[1])), cdiv_k<12>(K_[2]));
+        break;
+      case 3:   // :114-115
+        xin = cadd(csub(f, cdiv_k<33>(cscale(K_[2], R(4)))), cdiv_k<11>(cscale(K_[3], R(5))));
+        break;
+      case 4:   // :116-117
+        xin = cadd(csub(csub(f, cdiv_k<4>(K_[1])), cdiv_k<44>(cscale(K_[2], R(29)))),
+                   cdiv_k<22>(cscale(K_[3], R(31))));
+        break;
+      case 5:   // :118-119
+        xin = cadd(cadd(csub(cadd(cadd(f, cdiv_k<11>(cscale(K_[1], R(3)))), cdiv_k<33>(cscale(K_[2], R(8)))),
+                             cdiv_k<11>(cscale(K_[3], R(4)))), cdiv_k<11>(K_[4])),
+                   cdiv_k<33>(cscale(K_[5], R(14))));
+        break;
+      case 6:   // :120-121
+        xin = cadd(csub(cadd(cadd(csub(csub(f, cdiv_k<48>(cscale(K_[1], R(17)))), cdiv_k<12>(cscale(K_[2], R(5)))),
+                                  K_[3]), K_[4]), cdiv_k<12>(cscale(K_[5], R(13)))),
+                   cdiv_k<16>(cscale(K_[6], R(11))));
+        break;
+      case 7:   // :122-123
+        xin = cadd(csub(cadd(csub(csub(cadd(cadd(f, cdiv_k<39>(cscale(K_[1], R(20)))),
+                                                cdiv_k<39>(cscale(K_[2], R(12)))),
+                                           cdiv_k<39>(cscale(K_[3], R(31)))), cdiv_k<39>(K_[4])),
+                                 cdiv_k<39>(cscale(K_[5], R(34)))), cdiv_k<39>(cscale(K_[6], R(11)))),
+                   cdiv_k<39>(cscale(K_[7], R(16))));
+        break;
+      default: {   // 8: :124
+        const R c1 = R(13) / R(200), c3 = R(4) / R(25), c4 = R(11) / R(40);
+        const cplx<R> fn = cadd(cadd(cadd(f, cscale(cadd(K_[1], k), c1)), cscale(cadd(K_[3], K_[7]), c3)),
+                                cscale(cadd(K_[4], K_[6]), c4));
+        W(X_F, fn);
+        xin = fn;
+      } break;
+    }
+    if (STAGE < 8) put(8 + STAGE, xin);   // the stage input x_{s+1}
+  } else {   // FX_TD4, timestepping.py:137-144; v_fn and its derivative include dissipation
+    switch (STAGE) {
+      case 1: {   // k1 = h v(f); next: the transforms of k1 (tangent input of jac(f, k1))
+        const cplx<R> k1 = cscale(cadd(v, cscale(Q(X_F), L)), h);
+        W(X_K1, k1);
+        put(TR_F, Q(X_F)); put(TR_K1, k1);
+        xin = k1;
+      } break;
+      case 2: {   // a1 = h jac(f, k1); f_temp = f + k1/2 + a1/8
+        const cplx<R> k1 = Q(X_K1);
+        const cplx<R> a1 = cscale(cadd(v, cscale(k1, L)), h);
+        W(X_A1, a1);
+        const cplx<R> ft = cadd(cadd(Q(X_F), cdiv_k<2>(k1)), cdiv_k<8>(a1));
+        W(X_FT, ft);
+        put(TR_A1, a1); put(TR_FT, ft);
+        xin = ft;
+      } break;
+      case 3: {   // k2 = h v(f_temp)
+        const cplx<R> k2 = cscale(cadd(v, cscale(Q(X_FT), L)), h);
+        W(X_K2T, k2);
+        put(TR_K2, k2);
+        xin = k2;
+      } break;
+      default: {  // a2 = h jac(f_temp, k2); f = f + k1 + a1/6 + a2/3
+        const cplx<R> a2 = cscale(cadd(v, cscale(Q(X_K2T), L)), h);
+        put(TR_A2, a2);
+        const cplx<R> fn = cadd(cadd(cadd(Q(X_F), Q(X_K1)), cdiv_k<6>(Q(X_A1))), cdiv_k<3>(a2));
+        W(X_F, fn);
+        xin = fn;
+      } break;
+    }
+  }
+  return xin;
+}
+
 template <typename R, int N, int SCHEME, int STAGE>
 __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fx(ColFxParams<R> p) {
   using X = Xf<R, N>;
   constexpr int E = X::E, K = X::K, M = X::M;
   constexpr size_t VEC = (size_t)2 * K * M;
-  using Tr = FxTraits<SCHEME, STAGE>;
+  constexpr int rhs = fx_rhs(SCHEME, STAGE);
   ECS_COL_PROLOGUE(popc_c(fx_smask(SCHEME, STAGE)), 2);   // the forcing, the multipliers
   const int c = id.ch, b = id.b, ky = id.ky;
   const R h = (R)p.ctl[b].h;
@@ -79,10 +207,10 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fx(ColFxParams<R> p) {
   Operands<X, SM> op(rows);
   op.begin(S, VEC);
   constexpr int n = popc_c(SM);
-  const TableRow<X, Tr::rhs == 1 && rows_fit(n, 2)> forcing(rows + n * M, p.fhat + ky * M);
+  const TableRow<X, rhs == 1 && rows_fit(n, 2)> forcing(rows + n * M, p.fhat + ky * M);
   const TableRow<X, rows_fit(n, 2)> mu(rows + (n + 1) * M, mu_row<X>(p.tw, ky));
   cplx<R> r[E];
-  if (Tr::rhs) col_load_rhs(p.H, b, c, ky, xf, r);
+  if (rhs) col_load_rhs(p.H, b, c, ky, xf, r);
   op.load(S, VEC, true, xf);
   cplx<R> x[E];
 #pragma unroll
@@ -90,136 +218,15 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_fx(ColFxParams<R> p) {
     x[i] = mk<R>(0, 0);
     const int slot = xf.slot(i);
     if (slot < 0) continue;
-    const R kx = xf.kx(i);
-    auto Q = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
-    auto W = [&](int q, cplx<R> a) { S[q * VEC + slot] = a; };
-    auto put = [&](int q, cplx<R> a) { if (rec) rec[q * VEC + slot] = a; };
-    const R L = diss_L<R>(kx, (R)ky, coeff);   // zero at (0,0)
     cplx<R> v = mk<R>(0, 0);
-    if (Tr::rhs) {
+    if (rhs) {
       v = r[i];
-      if (Tr::rhs == 1 && c == 0 && !(slot == 0 && ky == 0)) v = cadd(v, forcing(slot));
+      if (rhs == 1 && c == 0 && !(slot == 0 && ky == 0)) v = cadd(v, forcing(slot));
     }
-    cplx<R> xin = mk<R>(0, 0);
-    if (STAGE == 0) {
-      xin = Q(X_F);
-    } else if (SCHEME == FX_RK4) {
-      // v_fn includes dissipation L x at the stage input x (loss_functions.py:53, mhd_jax.py:171-173)
-      const cplx<R> f = Q(X_F);
-      cplx<R> xs = f;
-      if (STAGE == 2) xs = cadd(f, cdiv_k<2>(Q(X_K1)));
-      if (STAGE == 3) xs = cadd(f, cdiv_k<2>(Q(X_K1 + 1)));
-      if (STAGE == 4) xs = cadd(f, Q(X_K1 + 2));
-      const cplx<R> k = cscale(cadd(v, cscale(xs, L)), h);            // timestepping.py:40-43
-      // record: f0, k_s, x_{s+1}
-      if (STAGE == 1) put(0, f);
-      put(STAGE, k);
-      if (STAGE < 4) {
-        W(X_K1 + STAGE - 1, k);
-        xin = STAGE < 3 ? cadd(f, cdiv_k<2>(k)) : cadd(f, k);
-        put(4 + STAGE, xin);
-      } else {
-        const cplx<R> fn = cadd(cadd(cadd(cadd(f, cdiv_k<6>(Q(X_K1))), cdiv_k<3>(Q(X_K1 + 1))),
-                                     cdiv_k<3>(Q(X_K1 + 2))), cdiv_k<6>(k));   // :44
-        W(X_F, fn);
-        xin = fn;
-      }
-    } else if (SCHEME == FX_RK6) {
-      const R e = __ldg(Et + slot);
-      const cplx<R> k = cscale(v, h);
-      // record: f0, k_s (before any factor)
-      if (STAGE == 1) put(0, Q(X_F));
-      put(STAGE, k);
-      // f, k1..k_{STAGE-1} and the new k, times e after stages 1, 3..7 and stored
-      constexpr bool SC = STAGE != 2 && STAGE != 8;
-      cplx<R> f = Q(X_F), K_[9];
-#pragma unroll
-      for (int q = 1; q < 9; ++q) K_[q] = mk<R>(0, 0);
-#pragma unroll
-      for (int q = 1; q < STAGE; ++q)
-        if ((SM >> (X_K1 + q - 1)) & 1u) K_[q] = Q(X_K1 + q - 1);
-      K_[STAGE] = k;
-      if (SC) {
-        f = cscale_rn(f, e);
-        W(X_F, f);
-#pragma unroll
-        for (int q = 1; q <= STAGE; ++q) { K_[q] = cscale_rn(K_[q], e); W(X_K1 + q - 1, K_[q]); }
-      } else if (STAGE == 2) {
-        W(X_K1 + 1, k);
-      }
-      switch (STAGE) {
-        case 1:   // :110-112
-          xin = cadd(f, cdiv_k<6>(K_[1]));
-          break;
-        case 2:   // :113
-          xin = cadd(cadd(f, cdiv_k<12>(K_[1])), cdiv_k<12>(K_[2]));
-          break;
-        case 3:   // :114-115
-          xin = cadd(csub(f, cdiv_k<33>(cscale(K_[2], R(4)))), cdiv_k<11>(cscale(K_[3], R(5))));
-          break;
-        case 4:   // :116-117
-          xin = cadd(csub(csub(f, cdiv_k<4>(K_[1])), cdiv_k<44>(cscale(K_[2], R(29)))),
-                     cdiv_k<22>(cscale(K_[3], R(31))));
-          break;
-        case 5:   // :118-119
-          xin = cadd(cadd(csub(cadd(cadd(f, cdiv_k<11>(cscale(K_[1], R(3)))), cdiv_k<33>(cscale(K_[2], R(8)))),
-                               cdiv_k<11>(cscale(K_[3], R(4)))), cdiv_k<11>(K_[4])),
-                     cdiv_k<33>(cscale(K_[5], R(14))));
-          break;
-        case 6:   // :120-121
-          xin = cadd(csub(cadd(cadd(csub(csub(f, cdiv_k<48>(cscale(K_[1], R(17)))), cdiv_k<12>(cscale(K_[2], R(5)))),
-                                    K_[3]), K_[4]), cdiv_k<12>(cscale(K_[5], R(13)))),
-                     cdiv_k<16>(cscale(K_[6], R(11))));
-          break;
-        case 7:   // :122-123
-          xin = cadd(csub(cadd(csub(csub(cadd(cadd(f, cdiv_k<39>(cscale(K_[1], R(20)))),
-                                                  cdiv_k<39>(cscale(K_[2], R(12)))),
-                                             cdiv_k<39>(cscale(K_[3], R(31)))), cdiv_k<39>(K_[4])),
-                                   cdiv_k<39>(cscale(K_[5], R(34)))), cdiv_k<39>(cscale(K_[6], R(11)))),
-                     cdiv_k<39>(cscale(K_[7], R(16))));
-          break;
-        default: {   // 8: :124
-          const R c1 = R(13) / R(200), c3 = R(4) / R(25), c4 = R(11) / R(40);
-          const cplx<R> fn = cadd(cadd(cadd(f, cscale(cadd(K_[1], k), c1)), cscale(cadd(K_[3], K_[7]), c3)),
-                                  cscale(cadd(K_[4], K_[6]), c4));
-          W(X_F, fn);
-          xin = fn;
-        } break;
-      }
-      if (STAGE < 8) put(8 + STAGE, xin);   // the stage input x_{s+1}
-    } else {   // FX_TD4, timestepping.py:137-144; v_fn and its derivative include dissipation
-      switch (STAGE) {
-        case 1: {   // k1 = h v(f); next: the transforms of k1 (tangent input of jac(f, k1))
-          const cplx<R> k1 = cscale(cadd(v, cscale(Q(X_F), L)), h);
-          W(X_K1, k1);
-          put(TR_F, Q(X_F)); put(TR_K1, k1);
-          xin = k1;
-        } break;
-        case 2: {   // a1 = h jac(f, k1); f_temp = f + k1/2 + a1/8
-          const cplx<R> k1 = Q(X_K1);
-          const cplx<R> a1 = cscale(cadd(v, cscale(k1, L)), h);
-          W(X_A1, a1);
-          const cplx<R> ft = cadd(cadd(Q(X_F), cdiv_k<2>(k1)), cdiv_k<8>(a1));
-          W(X_FT, ft);
-          put(TR_A1, a1); put(TR_FT, ft);
-          xin = ft;
-        } break;
-        case 3: {   // k2 = h v(f_temp)
-          const cplx<R> k2 = cscale(cadd(v, cscale(Q(X_FT), L)), h);
-          W(X_K2T, k2);
-          put(TR_K2, k2);
-          xin = k2;
-        } break;
-        default: {  // a2 = h jac(f_temp, k2); f = f + k1 + a1/6 + a2/3
-          const cplx<R> a2 = cscale(cadd(v, cscale(Q(X_K2T), L)), h);
-          put(TR_A2, a2);
-          const cplx<R> fn = cadd(cadd(cadd(Q(X_F), Q(X_K1)), cdiv_k<6>(Q(X_A1))), cdiv_k<3>(a2));
-          W(X_F, fn);
-          xin = fn;
-        } break;
-      }
-    }
-    x[i] = xin;
+    x[i] = fx_algebra<SCHEME, STAGE, R>(h, diss_L<R>(xf.kx(i), (R)ky, coeff), v,
+                                        [&](int q) -> cplx<R> { return op.get(q, i, slot); },
+                                        [&](int q, cplx<R> a) { S[q * VEC + slot] = a; }, [&]() { return __ldg(Et + slot); },
+                                        [&](int q, cplx<R> a) { if (rec) rec[q * VEC + slot] = a; });
   }
   if (!p.produce) return;
   col_inverse_uv(x, p.G, b, c, ky, id.act, xf, mu);
