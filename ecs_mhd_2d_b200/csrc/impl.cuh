@@ -126,6 +126,9 @@ template <typename R, int N, int W, int SCHEME> constexpr bool fx_chain_fits() {
   return FxChainSmem<R, N, W, SCHEME>::bytes <= 227 * 1024;
 }
 
+// The adjoint chain keeps and stages 11 rows per column, with the same limit.
+template <typename R, int N, int W> constexpr bool adj_chain_fits() { return AdjChainSmem<R, N, W>::bytes <= 227 * 1024; }
+
 template <typename R, int N, int W>
 int configure_chain() {
   int st = 0;
@@ -142,6 +145,7 @@ int configure_chain() {
   attrs(k_rk43_chain<R, N, W>, Rk43ChainSmem<R, N, W>::bytes);
   attrs(k_rk4_chain<R, N, W, false>, Rk4ChainSmem<R, N, W, false>::bytes);
   attrs(k_rk4_chain<R, N, W, true>, Rk4ChainSmem<R, N, W, true>::bytes);
+  if constexpr (adj_chain_fits<R, N, W>()) attrs(k_adj_chain<R, N, W>, AdjChainSmem<R, N, W>::bytes);
   if constexpr (fx_chain_fits<R, N, W, FX_RK4>()) attrs(k_fx_chain<R, N, W, FX_RK4>, FxChainSmem<R, N, W, FX_RK4>::bytes);
   if constexpr (fx_chain_fits<R, N, W, FX_RK6>()) attrs(k_fx_chain<R, N, W, FX_RK6>, FxChainSmem<R, N, W, FX_RK6>::bytes);
   if constexpr (fx_chain_fits<R, N, W, FX_TD4>()) attrs(k_fx_chain<R, N, W, FX_TD4>, FxChainSmem<R, N, W, FX_TD4>::bytes);
@@ -353,12 +357,21 @@ void launch_row_adj(ecs_ctx* c, int B, const R* phys, cudaStream_t s, long phys_
   else launch_step(c, B, k_row_adj<R, N, XT>, row_shape<Xf<R, N>>(B, NHA), s, p);
 }
 
+template <typename R>
+ColAdjParams<R> col_adj_params(ecs_ctx* c, int B, const cplx<R>* rec, const cplx<R>* rec_prev, double t, double h, int nslot,
+                               const StepCtl* ctl, long rec_bstride) {
+  ColAdjParams<R> p{};
+  p.ctl = ctl; p.rec_bstride = rec_bstride; p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.J = (cplx<R>*)c->D;
+  p.nslot = nslot; p.rec = rec; p.rec_prev = rec_prev; p.hacc = c->hacc; p.t = t; p.h = h; p.tw = (const cplx<R>*)c->tw;
+  p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B;
+  return p;
+}
+
 template <typename R, int N>
 void launch_col_adj(ecs_ctx* c, int B, int stage, const cplx<R>* rec, const cplx<R>* rec_prev, double t, double h,
                     int nslot, cudaStream_t s, const StepCtl* ctl = nullptr, long rec_bstride = 0) {
-  ColAdjParams<R> p{}; p.ctl = ctl; p.rec_bstride = rec_bstride; p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.J = (cplx<R>*)c->D; p.nslot = nslot;
-  p.rec = rec; p.rec_prev = rec_prev; p.hacc = c->hacc; p.t = t; p.h = h; p.tw = (const cplx<R>*)c->tw;
-  p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.stage = stage;
+  ColAdjParams<R> p = col_adj_params<R>(c, B, rec, rec_prev, t, h, nslot, ctl, rec_bstride);
+  p.stage = stage;
   const Shape sh = col_shape<Xf<R, N>>(B);
   switch (stage) {
     case AJ_PRE: launch_step(c, B, k_col_adj<R, N, AJ_PRE>, sh, s, p); break;
@@ -533,8 +546,16 @@ struct Impl {
     return B >= minb && B <= hi && (c->chain_res8 > 0 || c->chain_res16 > 0);
   }
 
+  // The batch range of the fixed-step chains: two rounds of 16-warp clusters pay in FP32 at
+  // n = 128 (32 steps, launch per pass / chain: Lawson-RK4 batch 16 1.91 / 1.64 ms, 24
+  // 2.02 / 1.66, Lawson-RK6 24 4.63 / 3.35), not in FP64 (Lawson-RK4 24 2.44 / 2.79).
+  static bool step_chain_batch(const ecs_ctx* c, int B) {
+    const int two = sizeof(R) == 4 && N == 128 ? 2 : 1;
+    return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb < 0 ? two * c->chain_res16 : c->rk4chain_maxb);
+  }
+
   // Lawson-RK4 steps of the box states in c->F as one cluster-resident launch
-  // (k_rk4_chain), after the COL_START pass; no inverse transforms after the last stage.
+  // (k_rk4_chain), after the COL_START pass.
   // rec, phys: optional records of the steps (see Rk4ChainParams); use_done skips the
   // candidates whose ctl.done is set.
   static int rk4_chain(ecs_ctx* c, int B, long steps, cudaStream_t s, int last_produce = 0, cplx<R>* rec = nullptr,
@@ -568,7 +589,7 @@ struct Impl {
   // in the Lawson-RK4 chain range (chain_batch) run as one cluster-resident launch.
   static int integrate_rk4(ecs_ctx* c, int B, long steps, cudaStream_t s) {
     if (steps <= 0) return ECS_OK;
-    if (chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb)) {
+    if (step_chain_batch(c, B)) {
       launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s);
       return rk4_chain(c, B, steps, s);
     }
@@ -609,6 +630,41 @@ struct Impl {
     return cuda_err(c, cudaGetLastError(), "integrate_rk4");
   }
 
+  // Whether B cotangents of Lawson-RK4 steps run through k_adj_chain: the range of the
+  // Lawson-RK4 chain, or, where only 8-warp clusters have the room, one round of them
+  // (FP64 at n = 128, 64 steps, launch per pass / chain: batch 7 4.23 / 2.29 ms, 8
+  // 4.05 / 4.24, 14 4.62 / 4.34).
+  static bool adj_chain_batch(const ecs_ctx* c, int B) {
+    if constexpr (N <= 128) {
+      if (!adj_chain_fits<R, N, 16>())
+        return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
+      return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
+    }
+    return false;
+  }
+  // Steps hi .. lo of the run recorded at rec (downwards) as one cluster-resident launch,
+  // after an AJ_PRE pass or the steps above; phys: physical fields from stage 1 of step lo on.
+  static int adj_chain(ecs_ctx* c, int B, long hi, long lo, const cplx<R>* rec, long rec_bstride, const R* phys,
+                       long phys_bstride, long phys_step, double h, int nslot, const StepCtl* ctl, cudaStream_t s) {
+    if constexpr (N <= 128) {
+      AdjChainParams<R> P{};
+      P.col = col_adj_params<R>(c, B, rec, nullptr, 0.0, h, nslot, ctl, rec_bstride);
+      RowAdjParams<R>& q = P.row;
+      q.G = (const cplx<R>*)c->G; q.H = (cplx<R>*)c->H; q.phys = phys; q.phys_bstride = phys_bstride;
+      q.tw = (const cplx<R>*)c->tw; q.B = B;
+      P.rec_step = (long)Q_NREC * 2 * K * M; P.phys_step = phys_step; P.hi = (int)hi; P.lo = (int)lo;
+      constexpr bool W16 = adj_chain_fits<R, N, 16>();
+      const int w = c->chain_w && (c->chain_w == 8 || W16) ? c->chain_w : (B <= c->chain_res8 || !W16 ? 8 : 16);
+      if (w == 8)
+        launch_cluster(c, B, chain_cl<N, 8>(), k_adj_chain<R, N, 8>, dim3(B * chain_cl<N, 8>()), dim3(8 * 32),
+                       AdjChainSmem<R, N, 8>::bytes, s, P);
+      else if constexpr (W16)
+        launch_cluster(c, B, chain_cl<N, 16>(), k_adj_chain<R, N, 16>, dim3(B * chain_cl<N, 16>()), dim3(16 * 32),
+                       AdjChainSmem<R, N, 16>::bytes, s, P);
+    }
+    return cuda_err(c, cudaGetLastError(), "adjoint chain");
+  }
+
   // Whether a batch of B runs the other fixed-step modes through k_fx_chain: the range of
   // the Lawson-RK4 chain, or, where only 8-warp clusters have the room, two rounds of them
   // (Lawson-RK6 in FP64 at n = 128, 32 steps, launch per pass / chain: batch 8 4.31 / 3.83 ms,
@@ -617,7 +673,7 @@ struct Impl {
     if constexpr (N <= 128) {
       if (scheme == FX_RK6 && !fx_chain_fits<R, N, 16, FX_RK6>())
         return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? 2 * c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
-      return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
+      return step_chain_batch(c, B);
     }
     return false;
   }
@@ -954,7 +1010,7 @@ struct Impl {
   static void record_rk4_segment(ecs_ctx* c, cplx<R>* rec, long steps, cudaStream_t s) {
     const size_t VEC = 2UL * K * M;
     launch_col_rk4<R, N>(c, 1, COL_START, 1, 0, s);
-    if (chain_batch(c, 1, c->rk4chain_minb, c->rk4chain_maxb)) {
+    if (step_chain_batch(c, 1)) {
       rk4_chain(c, 1, steps, s, 0, rec);
       return;
     }
@@ -2141,7 +2197,15 @@ struct Impl {
           };
           // seed the segment's last step from obar (J_OB)
           launch_col_adj<R, N>(c, B, AJ_PRE, rseg + (size_t)(cnt - 1) * Q_NREC * VEC, nullptr, 0.0, h, nslot, s);
-          for (long it = cnt - 1; it >= 0; --it) {
+          const bool chain = adj_chain_batch(c, B);
+          const long pst = (long)N * NPH * N, per = std::max<long>(1, ci / 4);   // steps whose fields are regenerated at once
+          for (long hi = cnt - 1; chain && hi >= 0; hi -= per) {
+            const long lo = std::max<long>(0, hi - per + 1);
+            launch_regen<R, N>(c, rseg, c->items + 4 * lo, (int)(4 * (hi - lo + 1)), s);
+            st = adj_chain(c, B, hi, lo, rseg, 0, (const R*)c->Phys, 0, pst, h, nslot, nullptr, s);
+            if (st) return st;
+          }
+          for (long it = cnt - 1; !chain && it >= 0; --it) {
             const cplx<R>* ra = rseg + (size_t)it * Q_NREC * VEC;
             const cplx<R>* rp = it > 0 ? rseg + (size_t)(it - 1) * Q_NREC * VEC : nullptr;
             for (int k = 4; k >= 1; --k) {
@@ -2497,7 +2561,7 @@ struct Impl {
     cplx<R>* ckpt = (cplx<R>*)m.ckpt;
     launch_col_rk4<R, N>(c, B, COL_START, 1, 0, s, nullptr, 0, 1);
     // (the candidates' step counts are multiples of seg, so a chain of seg steps suits all)
-    const bool chain = chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
+    const bool chain = step_chain_batch(c, B);
     for (long it = 0; it < smax; ++it) {
       if (it % seg == 0) {
         e = cudaMemcpyAsync(ckpt + (size_t)(it / seg) * B * VEC, F, B * vb, cudaMemcpyDeviceToDevice, s);
@@ -2564,7 +2628,12 @@ struct Impl {
       }
       launch_col_adj<R, N>(c, B, AJ_PRE, grec + (size_t)(seg - 1) * Q_NREC * VEC, nullptr, 0.0, 0.0, nslot, s,
                            c->ctl, rstride);
-      for (long it = seg - 1; it >= 0; --it) {
+      const bool achain = adj_chain_batch(c, B);
+      if (achain) {
+        st = adj_chain(c, B, seg - 1, 0, grec, rstride, gphys, pstride, (long)B * pstride, 0.0, nslot, c->ctl, s);
+        if (st) return st;
+      }
+      for (long it = seg - 1; !achain && it >= 0; --it) {
         const cplx<R>* ra = grec + (size_t)it * Q_NREC * VEC;
         const cplx<R>* rp = it > 0 ? grec + (size_t)(it - 1) * Q_NREC * VEC : nullptr;
         for (int k = 4; k >= 1; --k) {

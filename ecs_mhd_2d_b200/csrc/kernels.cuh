@@ -734,17 +734,18 @@ __device__ __forceinline__ void row_forward(cplx<typename X::R> (&a)[X::E], cplx
 // the state: place c / CL of CTA c % CL (CL = N / XT CTAs), group ky % G, with its two
 // rows of N at hcols + ((c / CL) G + ky % G) 2 N: P1, P2 (channel 0), or P3 in the
 // first (channel 1).
-template <int XT, class X>
+// ADJ: the 2 x 2 adjoint rows instead, (f, ky) to row f % 2 of channel f / 2.
+template <int XT, bool ADJ = false, class X>
 __device__ __forceinline__ void scatter_h_tile(const cplx<typename X::R>* s_H, cplx<typename X::R>* hcols, int x0,
                                                const X&) {
   constexpr int K = X::K, G = X::G, N = X::N, CL = X::N / XT;
   cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
-  for (int i = threadIdx.x; i < NH * K * XT; i += blockDim.x) {
+  for (int i = threadIdx.x; i < (ADJ ? NHA : NH) * K * XT; i += blockDim.x) {
     const int rr = i / XT, xt = i - rr * XT;
     const int f = rr / K, ky = rr - f * K;
-    const int c = 2 * (ky / G) + (f == 2 ? 1 : 0);
+    const int c = 2 * (ky / G) + (ADJ ? f >> 1 : f == 2 ? 1 : 0);
     cplx<typename X::R>* dst = cl.map_shared_rank(hcols, (unsigned)(c % CL));
-    dst[(((c / CL) * G + ky % G) * 2 + (f == 2 ? 0 : f)) * N + x0 + xt] = s_H[rr * (XT + 1) + xt];
+    dst[(((c / CL) * G + ky % G) * 2 + (ADJ ? f & 1 : f == 2 ? 0 : f)) * N + x0 + xt] = s_H[rr * (XT + 1) + xt];
   }
 }
 

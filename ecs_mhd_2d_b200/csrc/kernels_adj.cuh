@@ -46,23 +46,17 @@ __device__ __forceinline__ void row_adj_product(cplx<R> p12, R p3, cplx<R> uv, c
   q = mk<R>(-R(2) * bx * p1 + by * p2 - v * p3, R(2) * by * p1 + bx * p2 + u * p3);
 }
 
-// s_G holds the three product rows and then the four adjoint rows (each group
-// reads and writes its own column of the tile).
-template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p) {
-  using X = Xf<R, N>;
-  constexpr int E = X::E, L = X::L, K = X::K;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_G = s_x + X::smem(XT / X::G);
-  const int tiles = N / XT;
-  const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
+// Rows x0 .. x0 + XT - 1 of cotangent b; s_G holds the three product rows and then the
+// four adjoint rows (each warp reads and writes its own column of the tile).  CX
+// (cluster-resident passes): the tile is there already unless load_g, and the adjoint rows
+// go to the column warps' rows at `hcols` (scatter_h_tile) unless that is null.
+template <int XT, bool CX = false, class X>
+__device__ __forceinline__ void row_adj_body(const RowAdjParams<typename X::R>& p, int b, int x0, const X& xf,
+                                             cplx<typename X::R>* s_G, bool load_g = true,
+                                             cplx<typename X::R>* hcols = nullptr) {
+  using R = typename X::R;
+  constexpr int E = X::E, L = X::L, K = X::K, N = X::N;
   const int w = threadIdx.x / L;
-  const X xf(s_x, threadIdx.x >> 5);
-  pdl_trigger();
-  load_tables<X>(s_x, p.tw);
-  pdl_wait();
-  if (p.ctl && p.ctl[b].done) return;   // the whole CTA belongs to batch element b
   constexpr bool EARLY = E <= 4;        // see row_tan_body
   const cplx<R>* ph = phys_row<R, N>(p.phys + (size_t)b * p.phys_bstride, x0 + w) + xf.l;
   cplx<R> puv[E], pbb[E];
@@ -71,7 +65,7 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p)
     for (int j = 0; j < E; ++j) { puv[j] = ph[L * j]; pbb[j] = ph[N + L * j]; }
   };
   if constexpr (EARLY) load_phys();
-  load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, 3 * K, x0);
+  if (!CX || load_g) load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, 3 * K, x0);
   __syncthreads();
   cplx<R> P12[E], P3[E];   // (P1bar, P2bar) and (P3bar, 0)
   row_inverse<XT, true>(s_G, w, xf, P12, P3);
@@ -84,7 +78,24 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p)
   }
   row_forward<XT, true>(P12, P3, s_G, w, xf);
   __syncthreads();
+  if constexpr (CX) {
+    if (hcols) { scatter_h_tile<XT, true>(s_G, hcols, x0, xf); return; }
+  }
   store_tile<R, N, XT>(p.H + (size_t)b * NHA * K * N, s_G, NHA * K, x0);
+}
+
+template <typename R, int N, int XT>
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p) {
+  using X = Xf<R, N>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  const int tiles = N / XT;
+  const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
+  pdl_trigger();
+  load_tables<X>(s_x, p.tw);
+  pdl_wait();
+  if (p.ctl && p.ctl[b].done) return;   // the whole CTA belongs to batch element b
+  row_adj_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_x + X::smem(XT / X::G));
 }
 
 // ---------------------------------------------------------------------------
@@ -124,6 +135,12 @@ struct ColAdjParams {
 
 __device__ __forceinline__ double rdot2(double ax, double ay, double bx, double by) { return ax * bx + ay * by; }
 
+// Record rows (bits of Rk4Rec) that a Lawson-RK4 stage reads (AJ_S1: of the step before).
+__host__ __device__ constexpr unsigned adj4_qmask(int stage) {
+  return stage == AJ_S4 ? (1u << Q_F) | (1u << Q_K1) | (1u << Q_K2) | (1u << Q_K3)
+       : stage == AJ_S3 ? (1u << Q_K2)
+       : stage == AJ_S2 ? (1u << Q_F) | (1u << Q_K1) : (1u << Q_K4);
+}
 // Slots (bits of AdjSlot4 / AdjSlot43) that the algebra of a stage reads; they are
 // loaded together before the stage's stores.
 __host__ __device__ constexpr unsigned adj_jmask(int stage) {
@@ -141,12 +158,10 @@ __host__ __device__ constexpr unsigned adj_jmask(int stage) {
 // (c_ky/n^2) sum_m (-i mu_m) rfft2 of the adjoint rows of channel c in H: the box
 // cotangent N'(P)^T lambda at the lane's algebra elements.
 template <class X, class Mu>
-__device__ __forceinline__ void col_adj_xb(const cplx<typename X::R>* H, int b, int c, int ky, const X& xf,
+__device__ __forceinline__ void col_adj_rows(const cplx<typename X::R>* h0, const cplx<typename X::R>* h1, int ky, const X& xf,
                                            const Mu& mu, cplx<typename X::R> (&xb)[X::E]) {
   using R = typename X::R;
-  constexpr int E = X::E, L = X::L, K = X::K, N = X::N;
-  const cplx<R>* h0 = H + ((size_t)(b * NHA + 2 * c) * K + ky) * N;
-  const cplx<R>* h1 = h0 + (size_t)K * N;
+  constexpr int E = X::E, L = X::L;
   const R cky = ky == 0 ? R(1) : R(2);
   cplx<R> v1[E];
 #pragma unroll
@@ -161,13 +176,20 @@ __device__ __forceinline__ void col_adj_xb(const cplx<typename X::R>* H, int b, 
     xb[j] = cscale(cadd(cimul(xb[j], -m.x), cimul(v1[j], -m.y)), cky);
   }
 }
+template <class X, class Mu>
+__device__ __forceinline__ void col_adj_xb(const cplx<typename X::R>* H, int b, int c, int ky, const X& xf, const Mu& mu,
+                                           cplx<typename X::R> (&xb)[X::E]) {
+  const cplx<typename X::R>* h0 = H + ((size_t)(b * NHA + 2 * c) * X::K + ky) * X::N;
+  col_adj_rows(h0, h0 + (size_t)X::K * X::N, ky, xf, mu, xb);
+}
 
 // Inverse column transforms of lambda/c_ky times the product multipliers: the
 // product cotangents P1bar, P2bar (channel w) or P3bar (channel j) in G,
 // unscaled: Re sum mult_f lam e^{ik.x} (the row pass doubles ky > 0).
-template <class X>
+template <int CX = 0, class X>
 __device__ __forceinline__ void col_adj_emit(const cplx<typename X::R> (&lam)[X::E], cplx<typename X::R>* G, int b, int c,
-                                             int ky, bool act, const X& xf) {
+                                             int ky, bool act, const X& xf,
+                                             cplx<typename X::R>* gtile = nullptr) {
   using R = typename X::R;
   constexpr int E = X::E;
   auto mult = [&](cplx<R> (&z)[E], int f) {
@@ -180,12 +202,12 @@ __device__ __forceinline__ void col_adj_emit(const cplx<typename X::R> (&lam)[X:
     cplx<R> z1[E];
     mult(z, 0); mult(z1, 1);
     xf.template from_spec2<true>(z, z1);
-    col_put(z, G, NG, b, 0, ky, act, xf);
-    col_put(z1, G, NG, b, 1, ky, act, xf);
+    col_put<CX>(z, G, NG, b, 0, ky, act, xf, gtile);
+    col_put<CX>(z1, G, NG, b, 1, ky, act, xf, gtile);
   } else {
     mult(z, 2);
     xf.template from_spec<true>(z);
-    col_put(z, G, NG, b, 2, ky, act, xf);
+    col_put<CX>(z, G, NG, b, 2, ky, act, xf, gtile);
   }
 }
 
@@ -195,6 +217,122 @@ __device__ __forceinline__ void col_hacc(double* hacc, const ColId<X>& id, bool 
 #pragma unroll
   for (int o = X::L / 2; o >= 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
   if (act && xf.l == 0) hacc[((size_t)id.b * X::K + id.ky) * 2 + id.ch] += part;
+}
+
+// The algebra of an adjoint stage at one mode from the cotangent Xb of its adjoint
+// right-hand side: returns the cotangent fed to the next one (times h or t) and adds the
+// terms of the step-size accumulator to hpart, those over h (or t) to hdiv.  JV(q) reads
+// and JW(q, v) writes slot q, QV(q) reads the record, E() gives exp(h/2 L) mask
+// (Lawson-RK4); prev: a step precedes (AJ_S1), whose recorded k4 QP() gives.
+template <int STAGE, typename R, class JVf, class JWf, class QVf, class Ef, class QPf>
+__device__ __forceinline__ cplx<R> adj_algebra(R h, R t, R L, cplx<R> Xb, bool prev, double& hpart, double& hdiv, JVf&& JV,
+                                               JWf&& JW, QVf&& QV, Ef&& E, QPf&& QP) {
+  constexpr bool rk43 = STAGE >= AJ43_INIT;
+  auto ip = [&](cplx<R> a, cplx<R> bb) { return rdot2(a.x, a.y, bb.x, bb.y); };
+  cplx<R> kb = mk<R>(0, 0);
+  if (!rk43) {
+    const R e = E();
+    const R dedh = e * L / R(2);
+    switch (STAGE) {
+      case AJ_PRE: {
+        const cplx<R> ob = JV(J_OB);
+        JW(J_F2, ob); JW(J_A1, cdiv_k<6>(ob));
+        JW(J_K2, cdiv_k<3>(ob)); JW(J_B3, cdiv_k<3>(ob));
+        kb = cdiv_k<6>(ob);                                   // k4bar
+        hdiv += ip(kb, QV(Q_K4));
+      } break;
+      case AJ_S4: {
+        const cplx<R> f2b = cadd(JV(J_F2), Xb), b3b = cadd(JV(J_B3), Xb);
+        const cplx<R> b2b = JV(J_K2), b1b = JV(J_A1);
+        const cplx<R> f = QV(Q_F), k1 = QV(Q_K1);
+        const double eb = ip(b3b, QV(Q_K3)) + ip(b2b, QV(Q_K2)) + ip(b1b, cscale(k1, e)) +
+                          ip(f2b, cscale(f, e));
+        hpart += eb * (double)dedh;
+        kb = cscale(b3b, e);                                     // k3bar
+        hdiv += ip(kb, QV(Q_K3));
+        JW(J_F2, cscale(f2b, e));                      // f1bar
+        JW(J_A1, cscale(b1b, e));                      // a1bar
+        JW(J_K2, cscale(b2b, e));                      // k2bar
+      } break;
+      case AJ_S3: {
+        JW(J_F2, cadd(JV(J_F2), Xb));
+        kb = cadd(JV(J_K2), cscale(Xb, R(0.5)));        // k2bar final
+        hdiv += ip(kb, QV(Q_K2));
+      } break;
+      case AJ_S2: {
+        const cplx<R> f1b = cadd(JV(J_F2), Xb);
+        const cplx<R> a1b = cadd(JV(J_A1), cscale(Xb, R(0.5)));
+        const double eb = ip(a1b, QV(Q_K1)) + ip(f1b, QV(Q_F));
+        hpart += eb * (double)dedh;
+        kb = cscale(a1b, e);                                     // k1bar
+        hdiv += ip(kb, QV(Q_K1));
+        JW(J_OB, cscale(f1b, e));                      // fbar (without the RHS1 term)
+      } break;
+      default: {   // AJ_S1: fbar += X1bar; then seed the previous step (if any)
+        const cplx<R> fb = cadd(JV(J_OB), Xb);
+        JW(J_OB, fb);
+        if (prev) {
+          JW(J_F2, fb); JW(J_A1, cdiv_k<6>(fb));
+          JW(J_K2, cdiv_k<3>(fb)); JW(J_B3, cdiv_k<3>(fb));
+          kb = cdiv_k<6>(fb);
+          hdiv += ip(kb, QP());
+        }
+      } break;
+    }
+    kb = cscale(kb, h);
+  } else {
+    const cplx<R> eg = QV(RR_E);   // (e, e L h/2) of the attempt, e = exp(t L h/2)
+    const R e = eg.x;
+    const R dedt = eg.y;
+    switch (STAGE) {
+      case AJ43_PRE:      // from (xbar_f, k5bar) in (X0, K1) slots: RHS5 input = k5bar
+      case AJ43_IPRE: {   // initial k1 = t v(x0): input = k1bar
+        kb = JV(JJ_K1);
+        hdiv += ip(kb, QV(STAGE == AJ43_PRE ? RR_K5 : RR_K1));
+      } break;
+      case AJ43_S5: {     // xbar_f += Xbar5; distribute to x2, k1'', k2', k3', k4
+        const cplx<R> xfb = cadd(JV(JJ_X0), Xb);
+        JW(JJ_X2, xfb);
+        JW(JJ_K1PP, cdiv_k<6>(cscale(xfb, h)));
+        JW(JJ_K2P, cdiv_k<3>(cscale(xfb, h)));
+        JW(JJ_K3P, cdiv_k<3>(cscale(xfb, h)));
+        kb = cdiv_k<6>(cscale(xfb, h));                       // k4bar
+        hdiv += ip(kb, QV(RR_K4));
+      } break;
+      case AJ43_S4: {     // Y4 = x2 + h k3'
+        const cplx<R> x2b = cadd(JV(JJ_X2), Xb);
+        const cplx<R> k3pb = cadd(JV(JJ_K3P), cscale(Xb, h));
+        const cplx<R> k2pb = JV(JJ_K2P), k1ppb = JV(JJ_K1PP);
+        const cplx<R> x0 = QV(RR_X0), k1 = QV(RR_K1);
+        const double eb = ip(k3pb, QV(RR_K3)) + ip(k2pb, QV(RR_K2)) +
+                          ip(k1ppb, cscale(k1, e)) + ip(x2b, cscale(x0, e));
+        hpart += eb * (double)dedt;
+        kb = cscale(k3pb, e);                                    // k3bar
+        hdiv += ip(kb, QV(RR_K3));
+        JW(JJ_K2, cscale(k2pb, e));                    // k2bar (partial)
+        JW(JJ_K1P, cscale(k1ppb, e));                  // k1'bar (partial)
+        JW(JJ_XB, cscale(x2b, e));                     // xbar (partial)
+      } break;
+      case AJ43_S3: {     // Y3 = x + h k2/2
+        JW(JJ_XB, cadd(JV(JJ_XB), Xb));
+        kb = cadd(JV(JJ_K2), cscale(cscale(Xb, h), R(0.5)));   // k2bar final
+        hdiv += ip(kb, QV(RR_K2));
+      } break;
+      case AJ43_S2: {     // Y2 = x + h k1'/2; then x0bar, k1bar of this attempt
+        const cplx<R> xbb = cadd(JV(JJ_XB), Xb);
+        const cplx<R> k1pb = cadd(JV(JJ_K1P), cscale(cscale(Xb, h), R(0.5)));
+        const double eb = ip(k1pb, QV(RR_K1)) + ip(xbb, QV(RR_X0));
+        hpart += eb * (double)dedt;
+        JW(JJ_X0, cscale(xbb, e));
+        JW(JJ_K1, cscale(k1pb, e));
+      } break;
+      default: {          // AJ43_INIT: initial k1 = t v(x0): x0bar += Xbar
+        JW(JJ_X0, cadd(JV(JJ_X0), Xb));
+      } break;
+    }
+    kb = cscale(kb, t);
+  }
+  return kb;
 }
 
 template <typename R, int N, int STAGE>
@@ -212,7 +350,6 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_adj(ColAdjParams<R> p)
   const R h = p.ctl ? (R)p.ctl[b].h : (R)p.h, t = (R)p.t;
   constexpr bool rk43 = STAGE >= AJ43_INIT;
   constexpr bool has_rhs = !(STAGE == AJ_PRE || STAGE == AJ43_PRE || STAGE == AJ43_IPRE);
-  const R cky = ky == 0 ? R(1) : R(2);
   const R coeff = ch == 0 ? p.nu : p.eta;
   double hpart = 0.0, hdiv = 0.0;   // hdiv: the terms over h (RK4) or t (RK4(3))
   constexpr unsigned JM = adj_jmask(STAGE);
@@ -228,117 +365,12 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_adj(ColAdjParams<R> p)
       lam[i] = mk<R>(0, 0);
       const int slot = xf.slot(i);
       if (slot < 0) continue;
-      const R kx = xf.kx(i);
-      const bool in_mask = !(slot == 0 && ky == 0);
-      const R L = diss_L<R>(kx, (R)ky, coeff);
-      const cplx<R> Xb = has_rhs ? xb[i] : mk<R>(0, 0);
-      cplx<R> kb = mk<R>(0, 0);   // cotangent fed to the next adjoint RHS (before the h or t factor)
-      auto JV = [&](int q) -> cplx<R> { return op.get(q, i, slot); };
-      auto JW = [&](int q, cplx<R> v) { J[q * VEC + slot] = v; };
-      auto QV = [&](int q) -> cplx<R> { return __ldg(Q + q * VEC + slot); };
-      auto ip = [&](cplx<R> a, cplx<R> bb) { return rdot2(a.x, a.y, bb.x, bb.y); };
-      if (!rk43) {
-        const R e = in_mask ? exp(h / R(2) * L) : R(0);
-        const R dedh = e * L / R(2);
-        switch (STAGE) {
-          case AJ_PRE: {
-            const cplx<R> ob = JV(J_OB);
-            JW(J_F2, ob); JW(J_A1, cdiv_k<6>(ob));
-            JW(J_K2, cdiv_k<3>(ob)); JW(J_B3, cdiv_k<3>(ob));
-            kb = cdiv_k<6>(ob);                                   // k4bar
-            hdiv += ip(kb, QV(Q_K4));
-          } break;
-          case AJ_S4: {
-            const cplx<R> f2b = cadd(JV(J_F2), Xb), b3b = cadd(JV(J_B3), Xb);
-            const cplx<R> b2b = JV(J_K2), b1b = JV(J_A1);
-            const cplx<R> f = QV(Q_F), k1 = QV(Q_K1);
-            const double eb = ip(b3b, QV(Q_K3)) + ip(b2b, QV(Q_K2)) + ip(b1b, cscale(k1, e)) +
-                              ip(f2b, cscale(f, e));
-            hpart += eb * (double)dedh;
-            kb = cscale(b3b, e);                                     // k3bar
-            hdiv += ip(kb, QV(Q_K3));
-            JW(J_F2, cscale(f2b, e));                      // f1bar
-            JW(J_A1, cscale(b1b, e));                      // a1bar
-            JW(J_K2, cscale(b2b, e));                      // k2bar
-          } break;
-          case AJ_S3: {
-            JW(J_F2, cadd(JV(J_F2), Xb));
-            kb = cadd(JV(J_K2), cscale(Xb, R(0.5)));        // k2bar final
-            hdiv += ip(kb, QV(Q_K2));
-          } break;
-          case AJ_S2: {
-            const cplx<R> f1b = cadd(JV(J_F2), Xb);
-            const cplx<R> a1b = cadd(JV(J_A1), cscale(Xb, R(0.5)));
-            const double eb = ip(a1b, QV(Q_K1)) + ip(f1b, QV(Q_F));
-            hpart += eb * (double)dedh;
-            kb = cscale(a1b, e);                                     // k1bar
-            hdiv += ip(kb, QV(Q_K1));
-            JW(J_OB, cscale(f1b, e));                      // fbar (without the RHS1 term)
-          } break;
-          default: {   // AJ_S1: fbar += X1bar; then seed the previous step (if any)
-            const cplx<R> fb = cadd(JV(J_OB), Xb);
-            JW(J_OB, fb);
-            if (Qp) {
-              JW(J_F2, fb); JW(J_A1, cdiv_k<6>(fb));
-              JW(J_K2, cdiv_k<3>(fb)); JW(J_B3, cdiv_k<3>(fb));
-              kb = cdiv_k<6>(fb);
-              hdiv += ip(kb, __ldg(Qp + Q_K4 * VEC + slot));
-            }
-          } break;
-        }
-        kb = cscale(kb, h);
-      } else {
-        const cplx<R> eg = QV(RR_E);   // (e, e L h/2) of the attempt, e = exp(t L h/2)
-        const R e = eg.x;
-        const R dedt = eg.y;
-        switch (STAGE) {
-          case AJ43_PRE:      // from (xbar_f, k5bar) in (X0, K1) slots: RHS5 input = k5bar
-          case AJ43_IPRE: {   // initial k1 = t v(x0): input = k1bar
-            kb = JV(JJ_K1);
-            hdiv += ip(kb, QV(STAGE == AJ43_PRE ? RR_K5 : RR_K1));
-          } break;
-          case AJ43_S5: {     // xbar_f += Xbar5; distribute to x2, k1'', k2', k3', k4
-            const cplx<R> xfb = cadd(JV(JJ_X0), Xb);
-            JW(JJ_X2, xfb);
-            JW(JJ_K1PP, cdiv_k<6>(cscale(xfb, h)));
-            JW(JJ_K2P, cdiv_k<3>(cscale(xfb, h)));
-            JW(JJ_K3P, cdiv_k<3>(cscale(xfb, h)));
-            kb = cdiv_k<6>(cscale(xfb, h));                       // k4bar
-            hdiv += ip(kb, QV(RR_K4));
-          } break;
-          case AJ43_S4: {     // Y4 = x2 + h k3'
-            const cplx<R> x2b = cadd(JV(JJ_X2), Xb);
-            const cplx<R> k3pb = cadd(JV(JJ_K3P), cscale(Xb, h));
-            const cplx<R> k2pb = JV(JJ_K2P), k1ppb = JV(JJ_K1PP);
-            const cplx<R> x0 = QV(RR_X0), k1 = QV(RR_K1);
-            const double eb = ip(k3pb, QV(RR_K3)) + ip(k2pb, QV(RR_K2)) +
-                              ip(k1ppb, cscale(k1, e)) + ip(x2b, cscale(x0, e));
-            hpart += eb * (double)dedt;
-            kb = cscale(k3pb, e);                                    // k3bar
-            hdiv += ip(kb, QV(RR_K3));
-            JW(JJ_K2, cscale(k2pb, e));                    // k2bar (partial)
-            JW(JJ_K1P, cscale(k1ppb, e));                  // k1'bar (partial)
-            JW(JJ_XB, cscale(x2b, e));                     // xbar (partial)
-          } break;
-          case AJ43_S3: {     // Y3 = x + h k2/2
-            JW(JJ_XB, cadd(JV(JJ_XB), Xb));
-            kb = cadd(JV(JJ_K2), cscale(cscale(Xb, h), R(0.5)));   // k2bar final
-            hdiv += ip(kb, QV(RR_K2));
-          } break;
-          case AJ43_S2: {     // Y2 = x + h k1'/2; then x0bar, k1bar of this attempt
-            const cplx<R> xbb = cadd(JV(JJ_XB), Xb);
-            const cplx<R> k1pb = cadd(JV(JJ_K1P), cscale(cscale(Xb, h), R(0.5)));
-            const double eb = ip(k1pb, QV(RR_K1)) + ip(xbb, QV(RR_X0));
-            hpart += eb * (double)dedt;
-            JW(JJ_X0, cscale(xbb, e));
-            JW(JJ_K1, cscale(k1pb, e));
-          } break;
-          default: {          // AJ43_INIT: initial k1 = t v(x0): x0bar += Xbar
-            JW(JJ_X0, cadd(JV(JJ_X0), Xb));
-          } break;
-        }
-        kb = cscale(kb, t);
-      }
+      const cplx<R> kb = adj_algebra<STAGE, R>(
+          h, t, diss_L<R>(xf.kx(i), (R)ky, coeff), has_rhs ? xb[i] : mk<R>(0, 0), Qp != nullptr, hpart, hdiv,
+          [&](int q) -> cplx<R> { return op.get(q, i, slot); }, [&](int q, cplx<R> v) { J[q * VEC + slot] = v; },
+          [&](int q) -> cplx<R> { return __ldg(Q + q * VEC + slot); },
+          [&]() { return slot == 0 && ky == 0 ? R(0) : exp(h / R(2) * diss_L<R>(xf.kx(i), (R)ky, coeff)); },
+          [&]() -> cplx<R> { return __ldg(Qp + Q_K4 * VEC + slot); });
       // lambda = kb; the product multipliers vanish at (0,0), which the mask removes
       lam[i] = cscale(kb, ky == 0 ? R(1) : R(0.5));   // kb / c_ky, exactly
   }

@@ -140,6 +140,7 @@ __device__ __forceinline__ cplx<R>* stage_rows(cplx<R>* to, const cplx<R>* from,
 // A resident row of a column's table, as TableRow reads one.
 template <typename R> struct SharedRow {
   const cplx<R>* s;
+  __device__ __forceinline__ void wait() const {}
   __device__ __forceinline__ cplx<R> operator()(int slot) const { return s[slot]; }
 };
 __device__ __forceinline__ void staged_wait() {
@@ -485,6 +486,125 @@ __global__ void __launch_bounds__(W * 32, 1) k_fx_chain(FxChainParams<R> P) {
   __syncwarp();
   if (cw >= 0)
     for (int s = xf.l; s < M; s += 32) F[s] = S[X_F * M + s];
+  cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
+}
+
+// ---------------------------------------------------------------------------
+// The adjoint of a run of Lawson-RK4 steps (k_row_adj's and k_col_adj's passes, stages
+// AJ_S4 .. AJ_S1 of each step, last step first) in one launch, with the layout of
+// k_rk4_chain: cluster b runs cotangent b.  The slots, e and the multipliers of a column
+// stay in shared memory, its dL/dh accumulator in a register; the record rows of a stage
+// are on their way to shared memory before its transforms.  The first row pass reads
+// global G (an AJ_PRE pass, or the launch before), and the last column pass writes it if
+// a step precedes.
+// Measured, transpose products of 64 steps, launch per pass -> this: n = 64, batch 1
+// 1.81 -> 1.30 ms, batch 8 2.72 -> 1.30; n = 128, batch 1 2.94 -> 2.27, batch 7 4.23 -> 2.29.
+// ---------------------------------------------------------------------------
+template <typename R>
+struct AdjChainParams {
+  ColAdjParams<R> col;   // rec: of step 0 of the run; h (or ctl), J, nslot, hacc, ...
+  RowAdjParams<R> row;   // phys: of stage 1 of step `lo`
+  long rec_step;         // entries from a step's record to the next step's
+  long phys_step;        // values from a stage's physical fields to the next stage's
+  int hi, lo;            // steps hi .. lo, downwards
+};
+template <typename R, int N, int W> using AdjChainSmem = ChainSmem<R, N, W, true, 4, (int)J_NS4 + 2>;
+
+template <int STAGE, class X>
+__device__ __forceinline__ void chain_adj_algebra(typename X::R h, typename X::R coeff, const ColId<X>& id, const X& xf,
+                                                  bool prev, double& hpart, double& hdiv, cplx<typename X::R>* J,
+                                                  const typename X::R* e, const cplx<typename X::R>* rows,
+                                                  const cplx<typename X::R> (&xb)[X::E], cplx<typename X::R> (&lam)[X::E]) {
+  using R = typename X::R;
+  constexpr int M = X::M;
+  constexpr unsigned QM = adj4_qmask(STAGE);
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    lam[i] = mk<R>(0, 0);
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    const cplx<R> kb = adj_algebra<STAGE, R>(
+        h, R(0), diss_L<R>(xf.kx(i), (R)id.ky, coeff), xb[i], prev, hpart, hdiv,
+        [&](int q) -> cplx<R> { return J[q * M + slot]; }, [&](int q, cplx<R> v) { J[q * M + slot] = v; },
+        [&](int q) -> cplx<R> { return rows[bit_rank(QM, q) * M + slot]; }, [&]() { return e[slot]; },
+        [&]() -> cplx<R> { return rows[slot]; });
+    lam[i] = cscale(kb, id.ky == 0 ? R(1) : R(0.5));   // kb / c_ky, exactly
+  }
+}
+
+template <typename R, int N, int W>
+__global__ void __launch_bounds__(W * 32, 1) k_adj_chain(AdjChainParams<R> P) {
+  using X = Xf<R, N>;
+  constexpr int K = X::K, M = X::M, CL = chain_cl<N, W>(), NS = (int)J_NS4;
+  constexpr size_t VEC = (size_t)2 * K * M;
+  using SM = AdjChainSmem<R, N, W>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_gt = s_base + SM::gt;
+  cplx<R>* s_hc = s_base + SM::hc;
+  const X xf(s_base, threadIdx.x >> 5);
+  const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  const size_t at = ((size_t)id.ch * K + id.ky) * M;
+  cplx<R>* Jg = P.col.J + (size_t)b * P.col.nslot * VEC + at;
+  cplx<R>* rows = s_base + SM::work + (size_t)wc * 4 * M;
+  cplx<R>* J = s_base + SM::ds + (size_t)wc * (NS + 2) * M;
+  R* e = reinterpret_cast<R*>(J + NS * M);
+  const SharedRow<R> mu{J + (NS + 1) * M};
+  const cplx<R>* my_h = s_hc + (size_t)wc * 2 * N;
+  const cplx<R>* rec = P.col.rec + (size_t)b * P.col.rec_bstride + at;
+  double* hacc = P.col.hacc + ((size_t)b * K + id.ky) * 2 + id.ch;
+  load_tables<X>(s_base, P.col.tw);
+  pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (P.col.ctl && P.col.ctl[b].done) return;   // the whole cluster
+  const R h = P.col.ctl ? (R)P.col.ctl[b].h : (R)P.col.h, coeff = id.ch == 0 ? P.col.nu : P.col.eta;
+  double acc = 0.0;
+  if (cw >= 0) {
+    acc = *hacc;
+    for (int s = xf.l; s < M; s += 32) {
+      for (int q = 0; q < NS; ++q) J[q * M + s] = Jg[q * VEC + s];
+      e[s] = s == 0 && id.ky == 0 ? R(0) : exp(h / R(2) * diss_L<R>((R)slot_to_kx(s, X::KMAX, M), (R)id.ky, coeff));
+      J[(NS + 1) * M + s] = mu_row<X>(P.col.tw, id.ky)[s];
+    }
+  }
+  cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  for (int it = P.hi; it >= P.lo; --it) {
+    const cplx<R>* Q = rec + it * P.rec_step;
+#pragma unroll 1
+    for (int k = AJ_S4; k >= AJ_S1; --k) {
+      const bool first = it == P.hi && k == AJ_S4, last = it == P.lo && k == AJ_S1, prev = it > 0;
+      if (!first) cluster_barrier();   // column pass -> row pass
+      RowAdjParams<R> row = P.row;
+      row.phys += ((long)(it - P.lo) * 4 + k - AJ_S1) * P.phys_step;
+      row_adj_body<W, true>(row, b, rank * W, xf, s_gt, first, s_hc);
+      cluster_barrier();               // row pass -> column pass
+      if (cw < 0) continue;
+      if (k > AJ_S1) stage_rows<R, M>(rows, Q, VEC, adj4_qmask(k));
+      else if (prev) stage_rows<R, M>(rows, Q - P.rec_step, VEC, adj4_qmask(AJ_S1));
+      cplx<R> xb[X::E], lam[X::E];
+      col_adj_rows(my_h, my_h + N, id.ky, xf, mu, xb);
+      staged_wait();
+      double hpart = 0.0, hdiv = 0.0;
+      switch (k) {
+        case AJ_S4: chain_adj_algebra<AJ_S4>(h, coeff, id, xf, prev, hpart, hdiv, J, e, rows, xb, lam); break;
+        case AJ_S3: chain_adj_algebra<AJ_S3>(h, coeff, id, xf, prev, hpart, hdiv, J, e, rows, xb, lam); break;
+        case AJ_S2: chain_adj_algebra<AJ_S2>(h, coeff, id, xf, prev, hpart, hdiv, J, e, rows, xb, lam); break;
+        default: chain_adj_algebra<AJ_S1>(h, coeff, id, xf, prev, hpart, hdiv, J, e, rows, xb, lam); break;
+      }
+      double part = hpart + hdiv / (double)h;   // col_hacc
+#pragma unroll
+      for (int o = 16; o >= 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+      acc += part;
+      if (k > AJ_S1 || prev) col_adj_emit<W>(lam, P.col.G, b, id.ch, id.ky, true, xf, last ? nullptr : s_gt);
+    }
+  }
+  if (cw >= 0) {
+    __syncwarp();
+    for (int s = xf.l; s < M; s += 32)
+      for (int q = 0; q < NS; ++q) Jg[q * VEC + s] = J[q * M + s];
+    if (xf.l == 0) *hacc = acc;
+  }
   cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
 }
 

@@ -1,6 +1,6 @@
 """Cluster-resident steps of RK4, Lawson-RK6 and TDRK4 (k_fx_chain), and the recording
-Lawson-RK4 steps of linearisations and batched gradients (k_rk4_chain), equal the
-launches per pass bit for bit."""
+Lawson-RK4 steps of linearisations and batched gradients (k_rk4_chain) and their adjoint
+(k_adj_chain), equal the launches per pass bit for bit."""
 import numpy as np
 import pytest
 import torch
@@ -78,5 +78,25 @@ def test_batched_gradient(cuda, monkeypatch, n, B):
     def run():
         return [(torch.as_tensor(l).cpu(), {k: torch.as_tensor(q).cpu() for k, q in g.items()})
                 for l, g in E.loss_grad_multi(xs, pds)]
+
+    _equal(*_both(monkeypatch, run))
+
+
+# whole record, segments that do not divide the steps, chunks of two regenerated steps; one and several cotangents
+@pytest.mark.parametrize("n,B,ckpt,items", [(64, 1, 0, 0), (64, 3, 4, 8), (128, 1, 5, 0), (128, 10, 0, 8)])
+def test_transpose_product(cuda, monkeypatch, n, B, ckpt, items):
+    kw = dict(num_checkpoints=1, ministeps=11, shift_reflect_ny=1, rot=True)
+    pd = E.make_param_dict(n, 1 / 40, 1 / 40, forcing="kolmogorov+", **kw)
+    if ckpt:
+        pd["ckpt_every"] = ckpt
+    x = {"fields": torch.as_tensor(initial_condition(2, n), device="cuda"), "T": 0.05, "sx": 0.2}
+    ct = {"fields": torch.as_tensor(np.stack([initial_condition(40 + b, n) for b in range(B)]), device="cuda"),
+          "T": torch.linspace(0.4, -0.2, B, dtype=torch.float64), "sx": torch.linspace(-0.3, 0.1, B, dtype=torch.float64)}
+
+    def run():
+        if items:
+            monkeypatch.setenv("ECS_REGEN_ITEMS", str(items))
+        _, jacT = E.vjp(E.Objective(pd, "Lawson_RK4"), x)
+        return {k: torch.as_tensor(q).cpu() for k, q in jacT(ct)[0].items()}
 
     _equal(*_both(monkeypatch, run))
