@@ -129,6 +129,10 @@ template <typename R, int N, int W, int SCHEME> constexpr bool fx_chain_fits() {
 // The adjoint chain keeps and stages 11 rows per column, with the same limit.
 template <typename R, int N, int W> constexpr bool adj_chain_fits() { return AdjChainSmem<R, N, W>::bytes <= 227 * 1024; }
 
+template <typename R, int N, int W> constexpr bool td_chain_fits() {
+  return TdChainSmem<R, N, W>::bytes <= 227 * 1024;
+}
+
 template <typename R, int N, int W>
 int configure_chain() {
   int st = 0;
@@ -145,6 +149,7 @@ int configure_chain() {
   attrs(k_rk43_chain<R, N, W>, Rk43ChainSmem<R, N, W>::bytes);
   attrs(k_rk4_chain<R, N, W, false>, Rk4ChainSmem<R, N, W, false>::bytes);
   attrs(k_rk4_chain<R, N, W, true>, Rk4ChainSmem<R, N, W, true>::bytes);
+  if constexpr (td_chain_fits<R, N, W>()) attrs(k_tdj_chain<R, N, W>, TdChainSmem<R, N, W>::bytes);
   if constexpr (adj_chain_fits<R, N, W>()) attrs(k_adj_chain<R, N, W>, AdjChainSmem<R, N, W>::bytes);
   if constexpr (fx_chain_fits<R, N, W, FX_RK4>()) attrs(k_fx_chain<R, N, W, FX_RK4>, FxChainSmem<R, N, W, FX_RK4>::bytes);
   if constexpr (fx_chain_fits<R, N, W, FX_RK6>()) attrs(k_fx_chain<R, N, W, FX_RK6>, FxChainSmem<R, N, W, FX_RK6>::bytes);
@@ -428,12 +433,20 @@ void launch_col_tdj_sw(ecs_ctx* c, int B, int stage, cudaStream_t s, const ColTd
   ((stage == ST ? launch_step(c, B, k_col_tdj<R, N, ST>, sh, s, p) : void()), ...);
 }
 
+template <typename R>
+ColTdjParams<R> col_tdj_params(ecs_ctx* c, int B, int produce, const cplx<R>* rec, const double* dT, double h,
+                               double dscale, int nslot) {
+  ColTdjParams<R> p{};
+  p.H = (const cplx<R>*)c->H; p.Ga = (cplx<R>*)c->G; p.Gb = (cplx<R>*)c->Gx; p.D = (cplx<R>*)c->D;
+  p.nslot = nslot; p.rec = rec; p.dT = dT; p.h = h; p.dscale = dscale; p.tw = (const cplx<R>*)c->tw;
+  p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.produce = produce;
+  return p;
+}
+
 template <typename R, int N>
 void launch_col_tdj(ecs_ctx* c, int B, int stage, int produce, const cplx<R>* rec, const double* dT, double h,
                     double dscale, int nslot, cudaStream_t s) {
-  ColTdjParams<R> p; p.H = (const cplx<R>*)c->H; p.Ga = (cplx<R>*)c->G; p.Gb = (cplx<R>*)c->Gx; p.D = (cplx<R>*)c->D;
-  p.nslot = nslot; p.rec = rec; p.dT = dT; p.h = h; p.dscale = dscale; p.tw = (const cplx<R>*)c->tw;
-  p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.produce = produce;
+  const ColTdjParams<R> p = col_tdj_params<R>(c, B, produce, rec, dT, h, dscale, nslot);
   launch_col_tdj_sw<R, N>(c, B, stage, s, p, std::make_integer_sequence<int, 5>{});
 }
 
@@ -663,6 +676,27 @@ struct Impl {
                        AdjChainSmem<R, N, 16>::bytes, s, P);
     }
     return cuda_err(c, cudaGetLastError(), "adjoint chain");
+  }
+
+  // Whether B tangents of TDRK4 steps run through k_tdj_chain: the Lawson-RK4 chain's range,
+  // or two rounds of 8-warp clusters where only they have the room (FP64 at n = 128, 64 steps,
+  // launch per pass / chain: batch 8 4.51 / 4.31 ms, 14 4.79 / 4.29).  td_chain calls go(warps
+  // per CTA as a constant).
+  static bool td_chain_batch(const ecs_ctx* c, int B) {
+    if constexpr (N <= 128) {
+      if (!td_chain_fits<R, N, 16>())
+        return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? 2 * c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
+      return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb);
+    }
+    return false;
+  }
+  template <typename F> static void td_chain(const ecs_ctx* c, int B, F&& go) {
+    if constexpr (N <= 128) {
+      constexpr bool W16 = td_chain_fits<R, N, 16>();
+      const int w = c->chain_w && (c->chain_w == 8 || W16) ? c->chain_w : (B <= c->chain_res8 || !W16 ? 8 : 16);
+      if (w == 8) go(std::integral_constant<int, 8>{});
+      else if constexpr (W16) go(std::integral_constant<int, 16>{});
+    }
   }
 
   // Whether a batch of B runs the other fixed-step modes through k_fx_chain: the range of
@@ -1175,11 +1209,25 @@ struct Impl {
     const cplx<R>* Ga = (const cplx<R>*)c->G;
     const cplx<R>* Gb = (const cplx<R>*)c->Gx;
     launch_col_tdj<R, N>(c, B, 0, 1, rec, dT, L.h, dscale, nslot, s);
+    const bool chain = td_chain_batch(c, B);
     for (long a0 = 0; a0 < steps; a0 += CS) {
       const long cnt = std::min(CS, steps - a0);
       R* P = (R*)c->Phys;
       launch_regen<R, N>(c, rec, c->items + 4 * a0, (int)(2 * cnt), s, P, true);
       launch_regen<R, N>(c, rec, c->items + 4 * a0 + 2 * cnt, (int)(2 * cnt), s, P + 2 * cnt * pst, false);
+      if (chain) {
+        if constexpr (N <= 128) {
+          TdChainParams<R> Q{};
+          Q.col = col_tdj_params<R>(c, B, 1, rec + (size_t)a0 * TR_NREC * VEC, dT, L.h, dscale, nslot);
+          Q.phys = P; Q.cnt = (int)cnt; Q.produce = a0 + cnt < steps;
+          td_chain(c, B, [&](auto w) {
+            constexpr int W = decltype(w)::value;
+            launch_cluster(c, B, chain_cl<N, W>(), k_tdj_chain<R, N, W>, dim3(B * chain_cl<N, W>()), dim3(W * 32),
+                           TdChainSmem<R, N, W>::bytes, s, Q);
+          });
+        }
+        continue;
+      }
       for (long it = a0; it < a0 + cnt; ++it) {
         const cplx<R>* ra = rec + (size_t)it * TR_NREC * VEC;
         const R* pf = P + (size_t)(2 * (it - a0)) * pst;

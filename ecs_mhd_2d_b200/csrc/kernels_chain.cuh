@@ -609,6 +609,109 @@ __global__ void __launch_bounds__(W * 32, 1) k_adj_chain(AdjChainParams<R> P) {
 }
 
 // ---------------------------------------------------------------------------
+// Tangents of a run of TDRK4 steps (k_row_tan's, k_row_tan2's and k_col_tdj's passes) in one
+// launch, with the layout of k_rk4_chain.  The tiles of df and of dk1 / dk2 lie beside each
+// other; the H tile of a single row pass takes the second's place, that of a dual one the
+// first's.  The first row pass reads global Ga and the last column pass writes it.
+// Measured, tangents of 64 steps, launch per pass -> this: n = 64, batch 1 1.91 -> 1.33 ms,
+// batch 12 3.23 -> 1.32; n = 128, batch 1 3.13 -> 2.32, batch 7 4.68 -> 2.30.
+// ---------------------------------------------------------------------------
+template <typename R>
+struct TdChainParams {
+  ColTdjParams<R> col;   // rec: of step 0 of the run
+  const R* phys;         // [2 cnt][N][NPH][N] states f, f_temp of the run's steps, then k1, k2
+  int cnt, produce;
+};
+template <typename R, int N, int W> struct TdChainSmem {   // the second tile after the first's regions
+  using S = ChainSmem<R, N, W, true, 1, (int)DT_NSLOT + 1>;
+  static constexpr int gtb = (int)(S::bytes / sizeof(cplx<R>));
+  static constexpr size_t bytes = S::bytes + (size_t)NG * S::K * (W + 1) * sizeof(cplx<R>);
+};
+template <int STAGE, class X>
+__device__ __forceinline__ void chain_tdj_algebra(typename X::R h, typename X::R dpar_h, typename X::R coeff,
+                                                  const ColId<X>& id, const X& xf, cplx<typename X::R>* S,
+                                                  const cplx<typename X::R>* q, const cplx<typename X::R> (&r)[X::E],
+                                                  cplx<typename X::R> (&x)[X::E]) {
+  using R = typename X::R;
+#pragma unroll
+  for (int i = 0; i < X::E; ++i) {
+    x[i] = mk<R>(0, 0);
+    const int slot = xf.slot(i);
+    if (slot < 0) continue;
+    x[i] = tdj_algebra<STAGE, R>(h, dpar_h, diss_L<R>(xf.kx(i), (R)id.ky, coeff), r[i], q[slot],
+                                 [&](int d) -> cplx<R> { return S[d * X::M + slot]; },
+                                 [&](int d, cplx<R> v) { S[d * X::M + slot] = v; });
+  }
+}
+
+template <typename R, int N, int W>
+__global__ void __launch_bounds__(W * 32, 1) k_tdj_chain(TdChainParams<R> P) {
+  using X = Xf<R, N>;
+  constexpr int K = X::K, M = X::M, CL = chain_cl<N, W>(), NS = (int)DT_NSLOT;
+  constexpr size_t VEC = (size_t)2 * K * M, PST = (size_t)N * NPH * N;
+  using SM = typename TdChainSmem<R, N, W>::S;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<R>* s_base = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_ga = s_base + SM::gt;
+  cplx<R>* s_gb = s_base + TdChainSmem<R, N, W>::gtb;
+  cplx<R>* s_hc = s_base + SM::hc;
+  const X xf(s_base, threadIdx.x >> 5);
+  const int b = blockIdx.x / CL, rank = blockIdx.x - b * CL;
+  const int cw = chain_column<N, W>(rank), wc = cw < 0 ? 0 : (int)(threadIdx.x >> 5);
+  const ColId<X> id(cw < 0 ? 0 : cw, b, b + 1);
+  const size_t at = ((size_t)id.ch * K + id.ky) * M;
+  cplx<R>* D = P.col.D + (size_t)b * P.col.nslot * VEC + at;
+  cplx<R>* row = s_base + SM::work + (size_t)wc * M;
+  cplx<R>* S = s_base + SM::ds + (size_t)wc * (NS + 1) * M;
+  const SharedRow<R> mu{S + NS * M};
+  const cplx<R>* my_h = s_hc + (size_t)wc * 2 * N;
+  load_tables<X>(s_base, P.col.tw);
+  pdl_wait();   // launched with programmatic serialization: the predecessor's writes are visible past here
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) {
+      S[DT_F * M + s] = D[DT_F * VEC + s];
+      S[NS * M + s] = mu_row<X>(P.col.tw, id.ky)[s];
+    }
+  const R h = (R)P.col.h, dpar_h = (R)(P.col.dT[b] * P.col.dscale) / h, coeff = id.ch == 0 ? P.col.nu : P.col.eta;
+  cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  for (int it = 0; it < P.cnt; ++it) {
+#pragma unroll 1
+    for (int st = 1; st <= 4; ++st) {
+      if (it > 0 || st > 1) cluster_barrier();   // column pass -> row pass
+      const bool first = it == 0 && st == 1, last = it == P.cnt - 1 && st == 4;
+      const R* pa = P.phys + (size_t)(2 * it + (st > 2)) * PST;   // f, or f_temp
+      if (st & 1) {
+        RowTanParams<R> q{};
+        q.G = P.col.Ga; q.phys = pa;
+        row_tan_body<W, true>(q, b, rank * W, xf, s_ga, s_gb, first, s_hc);
+      } else {
+        RowTan2Params<R> q{};
+        q.phys_a = pa; q.phys_b = pa + (size_t)2 * P.cnt * PST;   // and k1, or k2
+        row_tan2_body<W, true>(q, b, rank * W, xf, s_ga, s_gb, false, s_hc);
+      }
+      cluster_barrier();                          // row pass -> column pass
+      if (cw < 0) continue;
+      stage_rows<R, M>(row, P.col.rec + (size_t)it * TR_NREC * VEC + at, VEC, 1u << tdj_qrow(st));
+      cplx<R> r[X::E], x[X::E];
+      chain_rhs(P.col.H, id, xf, my_h, r);
+      staged_wait();
+      switch (st) {
+        case 1: chain_tdj_algebra<1>(h, dpar_h, coeff, id, xf, S, row, r, x); break;
+        case 2: chain_tdj_algebra<2>(h, dpar_h, coeff, id, xf, S, row, r, x); break;
+        case 3: chain_tdj_algebra<3>(h, dpar_h, coeff, id, xf, S, row, r, x); break;
+        default: chain_tdj_algebra<4>(h, dpar_h, coeff, id, xf, S, row, r, x); break;
+      }
+      if (!last || P.produce)
+        col_inverse_uv<W>(x, P.col.Ga, b, id.ch, id.ky, true, xf, mu, last ? nullptr : (st & 1) ? s_gb : s_ga);
+    }
+  }
+  __syncwarp();
+  if (cw >= 0)
+    for (int s = xf.l; s < M; s += 32) D[DT_F * VEC + s] = S[DT_F * M + s];
+  cluster_barrier();   // no CTA leaves while a peer may still write its shared memory
+}
+
+// ---------------------------------------------------------------------------
 // Adaptive Lawson-RK4(3) attempts of the primal (timestepping.lawson_rk43,
 // jax_scripts/lib/timestepping.py:151-335) in one launch: cluster b runs state
 // b's attempts until it completes or `amax` attempts were made -- the column

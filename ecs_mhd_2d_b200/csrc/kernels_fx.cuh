@@ -259,30 +259,25 @@ struct RowTan2Params {
 // Linearised products dP of one tangent (du, dv, dbx, dby) about one field set (u, v, bx, by), accumulated.
 template <typename R>
 __device__ __forceinline__ void acc_tan_products(R u, R v, R bx, R by, R du, R dv, R dbx, R dby, cplx<R>& W, R& p3) {
-  W.x += R(2) * ((u * du - v * dv) - (bx * dbx - by * dby));   // dP1
-  W.y += (bx * dby + by * dbx) - (u * dv + v * du);            // dP2
-  p3 += (u * dby + by * du) - (v * dbx + bx * dv);             // dP3
+  // (sums of two products with a fixed order of rounding, whatever code surrounds them)
+  W.x += R(2) * (fpm(u, du, v, dv) - fpm(bx, dbx, by, dby));   // dP1
+  W.y += fpp(bx, dby, by, dbx) - fpp(u, dv, v, du);            // dP2
+  p3 += fpp(u, dby, by, du) - fpp(v, dbx, bx, dv);             // dP3
 }
 
-// The tile of Ga holds the H tile at the end (each group reads and writes its own
-// column of the tiles).
-template <typename R, int N, int XT>
-__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan2(RowTan2Params<R> p) {
-  using X = Xf<R, N>;
-  constexpr int E = X::E, L = X::L, K = X::K, F = K * (XT + 1);
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
-  cplx<R>* s_Ga = s_x + X::smem(XT / X::G);
-  cplx<R>* s_Gb = s_Ga + NG * F;
-  const int tiles = N / XT;
-  const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
+// Rows x0 .. x0 + XT - 1 of tangent b; the tile of Ga holds the H tile at the end (each
+// warp reads and writes its own column of the tiles).  CX: as in row_tan_body.
+template <int XT, bool CX = false, class X>
+__device__ __forceinline__ void row_tan2_body(const RowTan2Params<typename X::R>& p, int b, int x0, const X& xf,
+                                              cplx<typename X::R>* s_Ga, cplx<typename X::R>* s_Gb, bool load_g = true,
+                                              cplx<typename X::R>* hcols = nullptr) {
+  using R = typename X::R;
+  constexpr int E = X::E, L = X::L, K = X::K, N = X::N;
   const int w = threadIdx.x / L;
-  const X xf(s_x, threadIdx.x >> 5);
-  pdl_trigger();
-  load_tables<X>(s_x, p.tw);
-  pdl_wait();
-  load_tile<R, N, XT>(s_Ga, p.Ga + (size_t)b * NG * K * N, NG * K, x0);
-  load_tile<R, N, XT>(s_Gb, p.Gb + (size_t)b * NG * K * N, NG * K, x0);
+  if (!CX || load_g) {
+    load_tile<R, N, XT>(s_Ga, p.Ga + (size_t)b * NG * K * N, NG * K, x0);
+    load_tile<R, N, XT>(s_Gb, p.Gb + (size_t)b * NG * K * N, NG * K, x0);
+  }
   __syncthreads();
   cplx<R> W[E];
   R p3[E];
@@ -304,7 +299,24 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan2(RowTan2Params<R> 
   for (int j = 0; j < E; ++j) Z[j] = mk<R>(p3[j], R(0));
   row_forward<XT>(W, Z, s_Ga, w, xf);
   __syncthreads();
+  if constexpr (CX) {
+    if (hcols) { scatter_h_tile<XT>(s_Ga, hcols, x0, xf); return; }
+  }
   store_tile<R, N, XT>(p.H + (size_t)b * NH * K * N, s_Ga, NH * K, x0);
+}
+
+template <typename R, int N, int XT>
+__global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan2(RowTan2Params<R> p) {
+  using X = Xf<R, N>;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
+  cplx<R>* s_Ga = s_x + X::smem(XT / X::G);
+  const int tiles = N / XT;
+  const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
+  pdl_trigger();
+  load_tables<X>(s_x, p.tw);
+  pdl_wait();
+  row_tan2_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_Ga, s_Ga + NG * X::K * (XT + 1));
 }
 
 enum TdTanSlot { DT_F = 0, DT_K1, DT_A1, DT_FT, DT_K2, DT_NSLOT };
@@ -329,6 +341,38 @@ __host__ __device__ constexpr unsigned tdj_dmask(int stage) {   // slots read (b
        : (1u << DT_F) | (1u << DT_K1) | (1u << DT_A1) | (1u << DT_K2);
 }
 
+// The record row that a stage reads.
+__host__ __device__ constexpr int tdj_qrow(int stage) {
+  return stage == 1 ? (int)TR_K1 : stage == 2 ? (int)TR_A1 : stage == 3 ? (int)TR_K2 : (int)TR_A2;
+}
+// The algebra of a stage at one mode: its output from the derivative r and the record's q.
+template <int STAGE, typename R, class DVf, class DWf>
+__device__ __forceinline__ cplx<R> tdj_algebra(R h, R dpar_h, R L, cplx<R> r, cplx<R> q, DVf&& DV, DWf&& DW) {
+  // d(h X) = (dh/h) (h X) + h dX, with the recorded h X and dX = r + L dx (no forcing)
+  auto dk = [&](cplx<R> dxin) { return lin2_rn(q, dpar_h, cadd(r, cscale(dxin, L)), h); };
+  cplx<R> xin = mk<R>(0, 0);
+  switch (STAGE) {
+    case 0: xin = DV(DT_F); break;
+    case 1: { const cplx<R> dk1 = dk(DV(DT_F)); DW(DT_K1, dk1); xin = dk1; } break;
+    case 2: {
+      const cplx<R> dk1 = DV(DT_K1);
+      const cplx<R> da1 = dk(dk1);
+      DW(DT_A1, da1);
+      const cplx<R> dft = cadd(cadd(DV(DT_F), cdiv_k<2>(dk1)), cdiv_k<8>(da1));
+      DW(DT_FT, dft);
+      xin = dft;
+    } break;
+    case 3: { const cplx<R> dk2 = dk(DV(DT_FT)); DW(DT_K2, dk2); xin = dk2; } break;
+    default: {
+      const cplx<R> da2 = dk(DV(DT_K2));
+      const cplx<R> dfn = cadd(cadd(cadd(DV(DT_F), DV(DT_K1)), cdiv_k<6>(DV(DT_A1))), cdiv_k<3>(da2));
+      DW(DT_F, dfn);
+      xin = dfn;
+    } break;
+  }
+  return xin;
+}
+
 template <typename R, int N, int STAGE>
 __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_tdj(ColTdjParams<R> p) {
   using X = Xf<R, N>;
@@ -346,8 +390,7 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_tdj(ColTdjParams<R> p)
   constexpr unsigned DM = tdj_dmask(STAGE);
   Operands<X, DM> op(rows);
   op.begin(D, VEC);
-  constexpr int QV = STAGE == 1 ? (int)TR_K1 : STAGE == 2 ? (int)TR_A1 : STAGE == 3 ? (int)TR_K2 : (int)TR_A2;
-  const TableRow<X, STAGE != 0> rq(rows + popc_c(DM) * M, Q + QV * VEC);
+  const TableRow<X, STAGE != 0> rq(rows + popc_c(DM) * M, Q + tdj_qrow(STAGE) * VEC);
   const TableRow<X, true> mu(rows + (popc_c(DM) + 1) * M, mu_row<X>(p.tw, ky));
   cplx<R> r[E];
   if (STAGE != 0) col_load_rhs(p.H, b, c, ky, xf, r);
@@ -358,32 +401,9 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_tdj(ColTdjParams<R> p)
       x[i] = mk<R>(0, 0);
       const int slot = xf.slot(i);
       if (slot < 0) continue;
-      const R L = diss_L<R>(xf.kx(i), (R)ky, coeff);
-      auto DV = [&](int d) -> cplx<R> { return op.get(d, i, slot); };
-      auto DW = [&](int d, cplx<R> v) { D[d * VEC + slot] = v; };
-      // d(h X) = (dh/h) (h X) + h dX, with the recorded h X and dX = r + L dx (no forcing)
-      auto dk = [&](cplx<R> dxin) { return cadd(cscale(rq(slot), dpar_h), cscale(cadd(r[i], cscale(dxin, L)), h)); };
-      cplx<R> xin = mk<R>(0, 0);
-      switch (STAGE) {
-        case 0: xin = DV(DT_F); break;
-        case 1: { const cplx<R> dk1 = dk(DV(DT_F)); DW(DT_K1, dk1); xin = dk1; } break;
-        case 2: {
-          const cplx<R> dk1 = DV(DT_K1);
-          const cplx<R> da1 = dk(dk1);
-          DW(DT_A1, da1);
-          const cplx<R> dft = cadd(cadd(DV(DT_F), cdiv_k<2>(dk1)), cdiv_k<8>(da1));
-          DW(DT_FT, dft);
-          xin = dft;
-        } break;
-        case 3: { const cplx<R> dk2 = dk(DV(DT_FT)); DW(DT_K2, dk2); xin = dk2; } break;
-        default: {
-          const cplx<R> da2 = dk(DV(DT_K2));
-          const cplx<R> dfn = cadd(cadd(cadd(DV(DT_F), DV(DT_K1)), cdiv_k<6>(DV(DT_A1))), cdiv_k<3>(da2));
-          DW(DT_F, dfn);
-          xin = dfn;
-        } break;
-      }
-      x[i] = xin;
+      x[i] = tdj_algebra<STAGE, R>(h, dpar_h, diss_L<R>(xf.kx(i), (R)ky, coeff), STAGE != 0 ? r[i] : mk<R>(0, 0),
+                                   STAGE != 0 ? rq(slot) : mk<R>(0, 0), [&](int d) -> cplx<R> { return op.get(d, i, slot); },
+                                   [&](int d, cplx<R> v) { D[d * VEC + slot] = v; });
   }
   if (!p.produce) return;
   // dk1, dk2 go to Gb (paired with the point f / f_temp); df, dft, df' to Ga

@@ -1,6 +1,7 @@
 """Cluster-resident steps of RK4, Lawson-RK6 and TDRK4 (k_fx_chain), and the recording
-Lawson-RK4 steps of linearisations and batched gradients (k_rk4_chain) and their adjoint
-(k_adj_chain), equal the launches per pass bit for bit."""
+Lawson-RK4 steps of linearisations and batched gradients (k_rk4_chain), their adjoint
+(k_adj_chain) and the tangents of TDRK4 steps (k_tdj_chain) equal the launches per pass bit
+for bit."""
 import numpy as np
 import pytest
 import torch
@@ -83,11 +84,12 @@ def test_batched_gradient(cuda, monkeypatch, n, B):
 
 
 # whole record, segments that do not divide the steps, chunks of two regenerated steps; one and several cotangents
+@pytest.mark.parametrize("mode", ["Lawson_RK4", "TDRK4"])
 @pytest.mark.parametrize("n,B,ckpt,items", [(64, 1, 0, 0), (64, 3, 4, 8), (128, 1, 5, 0), (128, 10, 0, 8)])
-def test_transpose_product(cuda, monkeypatch, n, B, ckpt, items):
+def test_products(cuda, monkeypatch, n, B, ckpt, items, mode):
     kw = dict(num_checkpoints=1, ministeps=11, shift_reflect_ny=1, rot=True)
     pd = E.make_param_dict(n, 1 / 40, 1 / 40, forcing="kolmogorov+", **kw)
-    if ckpt:
+    if ckpt and mode == "Lawson_RK4":
         pd["ckpt_every"] = ckpt
     x = {"fields": torch.as_tensor(initial_condition(2, n), device="cuda"), "T": 0.05, "sx": 0.2}
     ct = {"fields": torch.as_tensor(np.stack([initial_condition(40 + b, n) for b in range(B)]), device="cuda"),
@@ -96,7 +98,8 @@ def test_transpose_product(cuda, monkeypatch, n, B, ckpt, items):
     def run():
         if items:
             monkeypatch.setenv("ECS_REGEN_ITEMS", str(items))
-        _, jacT = E.vjp(E.Objective(pd, "Lawson_RK4"), x)
-        return {k: torch.as_tensor(q).cpu() for k, q in jacT(ct)[0].items()}
+        obj = E.Objective(pd, mode)
+        _, jacT = E.vjp(obj, x)
+        return [{k: torch.as_tensor(q).cpu() for k, q in out.items()} for out in (jacT(ct)[0], obj.jvp(x, ct))]
 
     _equal(*_both(monkeypatch, run))
