@@ -1714,7 +1714,7 @@ struct Impl {
     }
     int st = residual(c, &L.cfg, dfields, (const cplx<R>*)c->V, (const cplx<R>*)c->OUT, L.dsx, B, out, s, 1);
     if (st) return st;
-    ++c->launches; k_phase_dot<R><<<B, 256, 0, s>>>((const R*)L.vt, (const R*)L.vx, dfields, odT, odsx, N);
+    ++c->launches; k_phase_dot<R><<<B * SUM_CL, 256, 0, s>>>((const R*)L.vt, (const R*)L.vx, dfields, odT, odsx, N);
     return cuda_err(c, cudaGetLastError(), "jvp");
   }
 
@@ -2144,7 +2144,7 @@ struct Impl {
     ++c->launches; k_box_scale_c<R><<<grid1d((long)B * VEC), 256, 0, s>>>((cplx<R>*)c->V, (long)VEC, N, B, R(-1) / (R(N) * R(N)));
     const int odd = (L.cfg.shift_reflect_ny % 2 + 2) % 2 == 1;
     const double sy = (L.cfg.shift_reflect_ny * 2 * M_PI) / 8;
-    ++c->launches; k_adj_head<R><<<B, 256, 0, s>>>((const cplx<R>*)c->V, (const cplx<R>*)L.phi, L.dsx, 1, sy, odd, L.cfg.rot,
+    ++c->launches; k_adj_head<R><<<B * SUM_CL, 256, 0, s>>>((const cplx<R>*)c->V, (const cplx<R>*)L.phi, L.dsx, 1, sy, odd, L.cfg.rot,
                                      (cplx<R>*)c->D + (size_t)fslot * VEC, (long)nslot * VEC,
                                      gsx, N);
     double tscale = 1.0;
@@ -2538,7 +2538,7 @@ struct Impl {
                     out + (size_t)b * fe, s, 1);
       if (st) return st;
       ++c->launches;
-      k_phase_dot<R><<<1, 256, 0, s>>>((const R*)m.vt + (size_t)b * fe, (const R*)m.vx + (size_t)b * fe,
+      k_phase_dot<R><<<SUM_CL, 256, 0, s>>>((const R*)m.vt + (size_t)b * fe, (const R*)m.vx + (size_t)b * fe,
                                        dfields + (size_t)b * fe, odT + b, odsx + b, N);
     }
     return cuda_err(c, cudaGetLastError(), "jvp_multi");
@@ -2651,7 +2651,7 @@ struct Impl {
       const int odd = (cfgs[b].shift_reflect_ny % 2 + 2) % 2 == 1;
       const double sy = (cfgs[b].shift_reflect_ny * 2 * M_PI) / 8;
       ++c->launches;
-      k_adj_head<R><<<1, 256, 0, s>>>((const cplx<R>*)c->V + (size_t)b * VEC, (const cplx<R>*)F + (size_t)b * VEC,
+      k_adj_head<R><<<SUM_CL, 256, 0, s>>>((const cplx<R>*)c->V + (size_t)b * VEC, (const cplx<R>*)F + (size_t)b * VEC,
                                       sx + b, 1, sy, odd, cfgs[b].rot, (cplx<R>*)c->D + ((size_t)b * nslot + J_OB) * VEC,
                                       (long)nslot * VEC, gsx + b, N);
     }

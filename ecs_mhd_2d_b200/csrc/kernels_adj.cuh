@@ -410,18 +410,19 @@ __global__ void k_adj_reject(cplx<R>* J, int nslot, const cplx<R>* rec, double* 
 
 // Head of the adjoint: from Ybar = cotangent of sym(Phi) (box, already
 // -(c/n^2) rfft2(c_out)), Phibar = sym^T(Ybar) and sxbar = <Phibar, i kx Phi>
-// (symmetry.py:4-25; shift_x uses masked kx).  One block per batch element.
+// (symmetry.py:4-25; shift_x uses masked kx).  One cluster of SUM_CL CTAs per batch
+// element (at n = 128 one CTA took 42 us, a cluster takes 9.5).
 template <typename R>
-__global__ void k_adj_head(const cplx<R>* Ybar, const cplx<R>* phi, const double* sx, int sx_shared, double sy,
+__global__ void __cluster_dims__(SUM_CL, 1, 1) k_adj_head(const cplx<R>* Ybar, const cplx<R>* phi, const double* sx, int sx_shared, double sy,
                            int odd, int rot, cplx<R>* Phibar, long pb_stride, double* sxbar, int n) {
   const Geom g = make_geom(n);
   const size_t VEC = (size_t)2 * g.K * g.M;
-  const int b = blockIdx.x;
+  const int b = blockIdx.x / SUM_CL, r = blockIdx.x % SUM_CL;
   const double s = sx[sx_shared ? 0 : b];
   const cplx<R>* Y = Ybar + (size_t)b * VEC;
   cplx<R>* P = Phibar + (size_t)b * pb_stride;
-  double part = 0.0;
-  for (size_t i = threadIdx.x; i < VEC; i += blockDim.x) {
+  double part = 0.0, none = 0.0;
+  for (size_t i = (size_t)r * blockDim.x + threadIdx.x; i < VEC; i += (size_t)SUM_CL * blockDim.x) {
     // i indexes the SOURCE mode kappa (the mode of Phi); its image is kx_out
     const int slot = i % g.M; const int ky = (i / g.M) % g.K; const int c = (int)(i / ((size_t)g.K * g.M));
     const int kap = slot_to_kx(slot, g.kmax, g.M);
@@ -442,16 +443,8 @@ __global__ void k_adj_head(const cplx<R>* Ybar, const cplx<R>* phi, const double
     // <y, i kap phi> = Re(conj(y) * i kap phi)
     part += (double)y.x * (double)(-km * ph.y) + (double)y.y * (double)(km * ph.x);
   }
-  __shared__ double red[32];
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = part;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0.0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) a += red[w];
-    sxbar[b] = a;
-  }
+  cluster_sum2(part, none);
+  if (r == 0 && threadIdx.x == 0) sxbar[b] = part;
 }
 
 // Ybar = -(c_ky/n^2) * box  (transpose of out = base - irfft2(.))

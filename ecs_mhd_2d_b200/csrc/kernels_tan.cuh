@@ -468,25 +468,46 @@ __global__ void k_tan_shift(const cplx<R>* dphi, long dstride, const cplx<R>* ph
   }
 }
 
+// Sums over the CTAs of a cluster of two partial sums per thread, in a fixed order: valid
+// in thread 0 of its first CTA.
+constexpr int SUM_CL = 8;
+__device__ __forceinline__ void cluster_sum2(double& a, double& b) {
+  cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+  __shared__ double s1[32], s2[32], all[2][SUM_CL];
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) { a += __shfl_xor_sync(0xffffffffu, a, o); b += __shfl_xor_sync(0xffffffffu, b, o); }
+  if ((threadIdx.x & 31) == 0) { s1[threadIdx.x >> 5] = a; s2[threadIdx.x >> 5] = b; }
+  cl.sync();   // (also: every CTA has started before a peer writes its shared memory)
+  if (threadIdx.x == 0) {
+    a = b = 0.0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += s1[w]; b += s2[w]; }
+    const unsigned r = cl.block_rank();
+    *cl.map_shared_rank(&all[0][r], 0) = a;
+    *cl.map_shared_rank(&all[1][r], 0) = b;
+  }
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+    a = b = 0.0;
+    for (int r = 0; r < SUM_CL; ++r) { a += all[0][r]; b += all[1][r]; }
+  }
+}
+
 // Tangents of the phase conditions: dpt = mean(vt * du0), dpx = mean(vx * du0)
-// over 2 n^2 entries (loss_functions.py:124-125); one block per tangent.
+// over 2 n^2 entries (loss_functions.py:124-125); one cluster of SUM_CL CTAs per tangent
+// (at n = 128 one CTA took 55 us, a cluster takes 9.6).
 template <typename R>
-__global__ void k_phase_dot(const R* vt, const R* vx, const R* du, double* dpt, double* dpx, int n) {
-  const int b = blockIdx.x;
+__global__ void __cluster_dims__(SUM_CL, 1, 1) k_phase_dot(const R* vt, const R* vx, const R* du, double* dpt, double* dpx,
+                                                          int n) {
+  const int b = blockIdx.x / SUM_CL, r = blockIdx.x % SUM_CL;
   const long cnt = 2L * n * n;
   const R* d = du + (size_t)b * cnt;
   double st = 0.0, sx = 0.0;
-  for (long i = threadIdx.x; i < cnt; i += blockDim.x) { st += (double)vt[i] * d[i]; sx += (double)vx[i] * d[i]; }
-  __shared__ double s1[32], s2[32];
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) { st += __shfl_xor_sync(0xffffffffu, st, o); sx += __shfl_xor_sync(0xffffffffu, sx, o); }
-  if ((threadIdx.x & 31) == 0) { s1[threadIdx.x >> 5] = st; s2[threadIdx.x >> 5] = sx; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double a = 0, c = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) { a += s1[w]; c += s2[w]; }
-    dpt[b] = a / (double)cnt; dpx[b] = c / (double)cnt;
+  for (long i = r * (long)blockDim.x + threadIdx.x; i < cnt; i += (long)SUM_CL * blockDim.x) {
+    st += (double)vt[i] * d[i];
+    sx += (double)vx[i] * d[i];
   }
+  cluster_sum2(st, sx);
+  if (r == 0 && threadIdx.x == 0) { dpt[b] = st / (double)cnt; dpx[b] = sx / (double)cnt; }
 }
 
 }  // namespace ecs
