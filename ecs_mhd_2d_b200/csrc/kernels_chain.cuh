@@ -252,7 +252,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_tan_chain(ChainParams<R> P) {
         for (int e = xf.l; e < M; e += 32) dsh[d * M + e] = dglob[d * VEC + e];
   }
   const TanCol<R> tc(P.col, b, 0);
-  __syncthreads();
+  if constexpr (DSM) cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  else __syncthreads();
   int prev = -1;   // kind class of the previous pass: 0 column-like, 1 row
   ChainOp next = P.ops[P.op0];
   for (int i = P.op0; i < P.op1; ++i) {
@@ -350,7 +351,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
       my_s[4 * M + s] = P.col.fhat[id.ky * M + s]; my_s[5 * M + s] = mu_row<X>(P.col.tw, id.ky)[s];
     }
   const R h = (R)P.col.ctl[b].h;
-  __syncthreads();
+  if constexpr (DSM) cluster_barrier();   // every CTA has started before a peer writes its shared memory
+  else __syncthreads();
   for (long step = 0; step < P.steps; ++step) {
     ColParams<R> col = P.col;
     if (col.rec) col.rec += step * P.rec_step;
