@@ -1041,13 +1041,10 @@ struct Impl {
 
   // Record `steps` Lawson-RK4 steps of the box state in c->F (batch 1) into rec
   // (Q_NREC vectors per step); ctl/Etab must hold the step size of the call.
-  static void record_rk4_segment(ecs_ctx* c, cplx<R>* rec, long steps, cudaStream_t s) {
+  static int record_rk4_segment(ecs_ctx* c, cplx<R>* rec, long steps, cudaStream_t s) {
     const size_t VEC = 2UL * K * M;
     launch_col_rk4<R, N>(c, 1, COL_START, 1, 0, s);
-    if (step_chain_batch(c, 1)) {
-      rk4_chain(c, 1, steps, s, 0, rec);
-      return;
-    }
+    if (step_chain_batch(c, 1)) return rk4_chain(c, 1, steps, s, 0, rec);
     for (long it = 0; it < steps; ++it) {
       cplx<R>* rs = rec + (size_t)it * Q_NREC * VEC;
       for (int k = 1; k <= 4; ++k) {
@@ -1055,19 +1052,24 @@ struct Impl {
         launch_col_rk4<R, N>(c, 1, k, (k == 4 && it == steps - 1) ? 0 : 1, 0, s, rs, 0);
       }
     }
+    return cuda_err(c, cudaGetLastError(), "record");
   }
 
-  // Lawson-RK4 segment [a0, a0+cnt) of the current linearisation: its record
+  // Lawson-RK4 segment [a0, a0+cnt) of the current linearisation: *rec is its record
   // (recomputed from the checkpoint when the linearisation is segmented).
-  static const cplx<R>* rk4_segment_record(ecs_ctx* c, long a0, long cnt, cudaStream_t s, void* buf = nullptr) {
+  static int rk4_segment_record(ecs_ctx* c, long a0, long cnt, cudaStream_t s, const cplx<R>** rec, void* buf = nullptr) {
     auto& L = c->lin;
     const size_t VEC = 2UL * K * M, vb = VEC * sizeof(cplx<R>);
-    if (!L.seg) return (const cplx<R>*)L.rec + (size_t)a0 * Q_NREC * VEC;
+    if (!L.seg) {
+      *rec = (const cplx<R>*)L.rec + (size_t)a0 * Q_NREC * VEC;
+      return ECS_OK;
+    }
     cplx<R>* dst = (cplx<R>*)(buf ? buf : L.rec);
-    rk4_setup(c, L.dT, L.cfg.num_checkpoints, L.cfg.ministeps, 1, s);
+    *rec = dst;
+    const int st = rk4_setup(c, L.dT, L.cfg.num_checkpoints, L.cfg.ministeps, 1, s);
+    if (st) return st;
     cudaMemcpyAsync(c->F, (cplx<R>*)L.ckpt + (size_t)(a0 / L.seg) * VEC, vb, cudaMemcpyDeviceToDevice, s);
-    record_rk4_segment(c, dst, cnt, s);
-    return dst;
+    return record_rk4_segment(c, dst, cnt, s);
   }
 
   // ---------------------------------------------------------------------
@@ -1407,7 +1409,8 @@ struct Impl {
           if (st) return st;
         }
       } else {
-        record_rk4_segment(c, (cplx<R>*)L.rec, steps, s);
+        st = record_rk4_segment(c, (cplx<R>*)L.rec, steps, s);
+        if (st) return st;
       }
       L.seg = kseg;
       L.nrec = steps;
@@ -1550,7 +1553,9 @@ struct Impl {
       const long kseg = L.seg ? L.seg : L.nrec;
       for (long a0 = 0; a0 < L.nrec; a0 += kseg) {
         const long cnt = std::min(kseg, L.nrec - a0);
-        const cplx<R>* rseg = rk4_segment_record(c, a0, cnt, s);
+        const cplx<R>* rseg;
+        st = rk4_segment_record(c, a0, cnt, s, &rseg);
+        if (st) return st;
         std::vector<long> sitems;
         for (long it = 0; it < cnt; ++it) {
           const long base = it * Q_NREC;
@@ -2202,16 +2207,17 @@ struct Impl {
           if (e != cudaSuccess) return cuda_err(c, e, "pipeline fork");
         }
         void* bufs[2] = {L.rec, L.rec2};
-        auto recompute = [&](long g) -> cudaError_t {   // on the primal stream, into bufs[g & 1]
+        auto recompute = [&](long g) -> int {   // on the primal stream, into bufs[g & 1]
           void* const Gs = c->G; void* const Hs = c->H;
+          const cplx<R>* out;
           c->G = c->Gp; c->H = c->Hp;
-          rk4_segment_record(c, g * kseg, std::min(kseg, L.nrec - g * kseg), c->pstream, bufs[g & 1]);
+          const int st2 = rk4_segment_record(c, g * kseg, std::min(kseg, L.nrec - g * kseg), c->pstream, &out, bufs[g & 1]);
           c->G = Gs; c->H = Hs;
-          return cudaEventRecord(c->pev[g & 1], c->pstream);
+          return st2 ? st2 : cuda_err(c, cudaEventRecord(c->pev[g & 1], c->pstream), "segment recomputation");
         };
         if (pipe) {
-          const cudaError_t e = recompute(nseg - 1);
-          if (e != cudaSuccess) return cuda_err(c, e, "segment recomputation");
+          st = recompute(nseg - 1);
+          if (st) return st;
         }
         for (long g = nseg - 1; g >= 0; --g) {
           const long a0 = g * kseg, cnt = std::min(kseg, L.nrec - a0);
@@ -2220,13 +2226,16 @@ struct Impl {
             cudaError_t e = cudaSuccess;
             if (g > 0) {   // the buffer of segment g-1 was last read by the adjoint of segment g+1
               if (g + 1 < nseg) e = cudaStreamWaitEvent(c->pstream, c->tjoin[0][(g + 1) & 1], 0);
-              if (e == cudaSuccess) e = recompute(g - 1);
+              if (e != cudaSuccess) return cuda_err(c, e, "segment recomputation");
+              st = recompute(g - 1);
+              if (st) return st;
             }
-            if (e == cudaSuccess) e = cudaStreamWaitEvent(s, c->pev[g & 1], 0);
+            e = cudaStreamWaitEvent(s, c->pev[g & 1], 0);
             if (e != cudaSuccess) return cuda_err(c, e, "segment recomputation");
             rseg = (const cplx<R>*)bufs[g & 1];
           } else {
-            rseg = rk4_segment_record(c, a0, cnt, s);
+            st = rk4_segment_record(c, a0, cnt, s, &rseg);
+            if (st) return st;
           }
           std::vector<long> sitems;
           for (long it = 0; it < cnt; ++it) {
