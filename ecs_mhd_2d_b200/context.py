@@ -17,7 +17,9 @@ import torch
 
 from . import _lib
 
-_CACHE = {}
+_CACHE = {}    # contexts by physics, grid, precision and digest of the forcing
+_RECENT = {}   # the last one used of each physics, grid and precision
+_CACHE_LOCK = threading.Lock()
 
 
 def torch_dtype_code(dt):
@@ -188,25 +190,31 @@ def _forcing_view(forcing):
 
 def get_context(param_dict, n, dtype, batch=1):
     """Context for the physics in ``param_dict`` (nu, eta, b0, forcing).  The forcing is
-    read on every call and compared bit by bit with those of the contexts at hand (3 us
-    at n = 64, where a digest of it took 17)."""
+    read on every call and compared bit by bit with that of the last context used of these
+    parameters (3 us at n = 64); another forcing is found by its digest (17 us), however
+    many there are."""
     forcing = _forcing_view(param_dict.get("forcing"))
     if forcing is not None and forcing.size != int(n) * int(n):
         raise ValueError(f"param_dict['forcing'] has shape {forcing.shape}, the fields are {n}x{n}")
     key = (torch.cuda.current_device(), int(n), dtype, float(param_dict["nu"]), float(param_dict["eta"]),
            float(param_dict["b0"][0]), float(param_dict["b0"][1]))
-    held = _CACHE.setdefault(key, [])
-    ctx = next((c for c in held if _same_bits(c._forcing, forcing)), None)
-    if ctx is None:
-        ctx = Context(n, dtype, param_dict["nu"], param_dict["eta"], param_dict["b0"],
-                      None if forcing is None else forcing.copy(), max_batch=batch)
-        held.append(ctx)
+    ctx = _RECENT.get(key)
+    if ctx is None or not _same_bits(ctx._forcing, forcing):
+        digest = None if forcing is None else hashlib.sha1(forcing.tobytes()).hexdigest()
+        with _CACHE_LOCK:   # threads that miss together get one context
+            ctx = _CACHE.get((key, digest))
+            if ctx is None:
+                ctx = Context(n, dtype, param_dict["nu"], param_dict["eta"], param_dict["b0"],
+                              None if forcing is None else forcing.copy(), max_batch=batch)
+                _CACHE[key, digest] = ctx
+            _RECENT[key] = ctx
     ctx.ensure_batch(batch)
     return ctx
 
 
 def clear_cache():
-    for held in list(_CACHE.values()):
-        for c in held:
+    with _CACHE_LOCK:
+        for c in _CACHE.values():
             c.close()
-    _CACHE.clear()
+        _CACHE.clear()
+        _RECENT.clear()
