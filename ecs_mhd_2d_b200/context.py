@@ -10,6 +10,7 @@ from __future__ import annotations
 import ctypes
 import hashlib
 import itertools
+import math
 import threading
 
 import numpy as np
@@ -193,9 +194,12 @@ def get_context(param_dict, n, dtype, batch=1):
     read on every call and compared bit by bit with that of the last context used of these
     parameters (3 us at n = 64); another forcing is found by its digest (17 us), however
     many there are."""
-    forcing = _forcing_view(param_dict.get("forcing"))
-    if forcing is not None and forcing.size != int(n) * int(n):
-        raise ValueError(f"param_dict['forcing'] has shape {forcing.shape}, the fields are {n}x{n}")
+    forcing = param_dict.get("forcing")
+    if forcing is not None:   # before it is staged: the pinned copy is of grid size at most
+        shape = tuple(forcing.shape) if isinstance(forcing, torch.Tensor) else np.shape(forcing)
+        if math.prod(shape) != int(n) * int(n):
+            raise ValueError(f"param_dict['forcing'] has shape {shape}, the fields are {n}x{n}")
+    forcing = _forcing_view(forcing)
     key = (torch.cuda.current_device(), int(n), dtype, float(param_dict["nu"]), float(param_dict["eta"]),
            float(param_dict["b0"][0]), float(param_dict["b0"][1]))
     ctx = _RECENT.get(key)

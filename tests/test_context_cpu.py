@@ -71,3 +71,26 @@ def test_threads_that_miss_together_share(lookup):
     for t in ts:
         t.join()
     assert len(FakeContext.made) == 1 and all(c is got[0] for c in got)
+
+
+class DeviceTensor(torch.Tensor):
+    """A host tensor that says it is on the device."""
+    is_cuda = True
+
+
+def test_forcing_of_another_grid_is_not_staged(lookup, monkeypatch):
+    """The pinned staging copy outlives the call: a forcing that is refused must not size it."""
+    made = []
+    empty = torch.empty
+
+    def host_empty(*a, pin_memory=False, **kw):
+        made.append(a[0])
+        return empty(*a, **kw)
+
+    monkeypatch.setattr(context, "_STAGE", threading.local())
+    monkeypatch.setattr(torch, "empty", host_empty)
+    with pytest.raises(ValueError, match="forcing"):
+        lookup(torch.zeros((64, 64), dtype=torch.float64).as_subclass(DeviceTensor))
+    assert made == []
+    lookup(torch.ones((8, 8), dtype=torch.float64).as_subclass(DeviceTensor))
+    assert made == [64] and np.all(FakeContext.made[-1]._forcing == 1.0)
