@@ -58,9 +58,9 @@ inline int box_grid(int cols) { return (cols + COLWARPS - 1) / COLWARPS; }
 // launches: batch 4 4.1 -> 3.8 ms, 16 4.5 -> 4.0, 32 5.3 -> 4.5, 48 7.2 -> 6.7 (batch 1
 // 2.37 -> 2.48).  Below 16 the cluster-resident sweep runs (chain_batch), in the warp
 // layout; its results are those of the warp layout's passes bit for bit.
-template <typename R, int N, typename F> void with_layout(const ecs_ctx* c, int B, F&& go) {
+template <typename R, int N, typename F> void with_layout(const ecs_ctx* c, int B, bool group_allowed, F&& go) {
   if constexpr (sizeof(R) == 8 && N == 128) {
-    if (B >= c->group_minb) { go((Xf<R, N, true>*)nullptr, std::true_type{}); return; }
+    if (group_allowed && B >= c->group_minb) { go((Xf<R, N, true>*)nullptr, std::true_type{}); return; }
   }
   go((Xf<R, N>*)nullptr, std::false_type{});
 }
@@ -346,7 +346,10 @@ void launch_col_tan(ecs_ctx* c, int B, int stage, int produce, const cplx<R>* re
   p.rec2 = rec2; p.H = (const cplx<R>*)c->H; p.G = (cplx<R>*)c->G; p.D = (cplx<R>*)c->D; p.nslot = nslot;
   p.rec = rec; p.dT = dT; p.t = t; p.h = h; p.dscale = dscale; p.tw = (const cplx<R>*)c->tw;
   p.nu = (R)c->nu; p.eta = (R)c->eta; p.B = B; p.stage = stage; p.produce = produce;
-  with_layout<R, N>(c, B, [&](auto* x, auto grp) {
+  // Several candidates (ctl): the warp layout at every batch, as a call on one of them uses,
+  // so that a candidate's result does not depend on which others share its sweep (from 16
+  // candidates on at n = 128 FP64 the layouts round differently).
+  with_layout<R, N>(c, B, ctl == nullptr, [&](auto* x, auto grp) {
     const Shape sh = col_shape<std::remove_pointer_t<decltype(x)>>(B);
     col_tan_stage(stage, [&](auto st) { launch_step(c, B, k_col_tan<R, N, decltype(st)::value, decltype(grp)::value>, sh, s, p); });
   });
