@@ -122,11 +122,18 @@ template <typename R> __device__ __forceinline__ cplx<R> shfl_c(cplx<R> v, int s
 
 // Programmatic dependent launch.  A stepping kernel is launched with
 // programmatic stream serialization, so it may start while its predecessor in
-// the stream is still running.  It calls pdl_trigger() first (its successor may
-// be scheduled once every CTA of this grid has started) and pdl_wait() before
-// its first access to global memory other than the constant twiddle table:
-// the wait returns when the predecessor grid has completed and its writes are
-// visible.  Every such kernel waits before any early return, so completion of
+// the stream is still running: its launch and the loads of the constant tables
+// overlap the predecessor's tail.  It calls pdl_wait() before its first access to
+// global memory other than those tables: the wait returns when the predecessor
+// grid has completed and its writes are visible.  Then it calls pdl_trigger() (its
+// successor may be scheduled once every CTA of this grid has come to that point).
+// The order matters: with the trigger before the wait, a grid whose CTAs all wait
+// already admits its own successor, and two or three grids of waiting CTAs fill the
+// SMs unevenly.  Measured over 1086 calls (n = 64 to 256, both types, batches 1 to 64),
+// trigger first -> after the wait: 7% faster in the geometric mean, up to 1.9 times
+// (24 Lawson-RK4 steps of 37 FP32 states at n = 64 1.28 -> 0.67 ms, a JVP of 20 steps for
+// 18 tangents there 1.16 -> 0.70), 4% of them slower by more than 3%.
+// Every such kernel waits before any early return, so completion of
 // a grid implies completion of all grids before it.  Both are no-ops for a
 // kernel launched without the attribute.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

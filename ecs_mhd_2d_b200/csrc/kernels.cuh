@@ -194,9 +194,9 @@ template <class X> __host__ __device__ constexpr int col_rows(int n, int extra) 
 // predecessor's results (programmatic launch), the warp's column `id`, its room `rows`.
 #define ECS_COL_PROLOGUE(n, extra)                                                                          \
   __shared__ __align__(16) cplx<typename X::R> s_x[X::smem(COLWARPS) + COLWARPS * col_rows<X>(n, extra) * X::M];\
-  pdl_trigger();                                                                                            \
   load_tables<X>(s_x, p.tw);                                                                                \
   pdl_wait();                                                                                               \
+  pdl_trigger();                                                                                            \
   __syncthreads();                                                                                          \
   const X xf(s_x, threadIdx.x >> 5);                                                                        \
   const ColId<X> id(p.B);                                                                                   \
@@ -520,9 +520,9 @@ __global__ void __launch_bounds__(COLWARPS * 32, 1) k_col_full_vel(ColParams<R> 
   using X = Xf<R, N>;
   constexpr int E = X::E, NK = N / 2 + 1;
   __shared__ __align__(16) cplx<R> s_x[X::smem(COLWARPS)];
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   __syncthreads();
   const X xf(s_x, threadIdx.x >> 5);
   const int u = blockIdx.x * COLWARPS + (int)(threadIdx.x >> 5), b = u / (2 * NK), ch = u & 1, ky = (u >> 1) % NK;
@@ -802,9 +802,9 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_rhs(RowParams<R> p) {
   cplx<R>* s_G = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   if (p.ctl && p.ctl[b].done) return;   // whole block belongs to one batch element
   row_rhs_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_G, s_G);
 }

@@ -91,9 +91,9 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj(RowAdjParams<R> p)
   cplx<R>* s_x = reinterpret_cast<cplx<R>*>(smem_raw);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   if (p.ctl && p.ctl[b].done) return;   // the whole CTA belongs to batch element b
   row_adj_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_x + X::smem(XT / X::G));
 }

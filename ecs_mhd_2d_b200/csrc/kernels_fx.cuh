@@ -313,9 +313,9 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_tan2(RowTan2Params<R> 
   cplx<R>* s_Ga = s_x + X::smem(XT / X::G);
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   row_tan2_body<XT>(p, b, x0, X(s_x, threadIdx.x >> 5), s_Ga, s_Ga + NG * X::K * (XT + 1));
 }
 
@@ -443,9 +443,9 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_adj2(RowAdj2Params<R> 
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
   const int w = threadIdx.x / L;
   const X xf(s_x, threadIdx.x >> 5);
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   load_tile<R, N, XT>(s_G, p.G + (size_t)b * NG * K * N, 3 * K, x0);
   __syncthreads();
   cplx<R> P12[E], P3[E];

@@ -263,9 +263,9 @@ __global__ void __launch_bounds__(XT * Xf<R, N>::L) k_row_err(RowErrParams<R> p)
   __shared__ int s_last;
   const int tiles = N / XT;
   const int b = blockIdx.x / tiles, x0 = (blockIdx.x - b * tiles) * XT;
-  pdl_trigger();
   load_tables<X>(s_x, p.tw);
   pdl_wait();
+  pdl_trigger();
   StepCtl& c = p.ctl[b];
   if (c.done) return;
   const double bm = row_err_max<XT>(p.G, b, x0, X(s_x, threadIdx.x >> 5), s_G, s_max);
