@@ -408,8 +408,14 @@ template <typename R_, int N_, bool GROUP_ = false> struct Xf {
   static constexpr int TW = GROUP ? N : tw_smem(N);
   static constexpr int XB = GROUP ? N : 0;
   static constexpr int KMAX = (N - 1) / 3, K = KMAX + 1, M = 2 * KMAX + 1;
-  // A column pass brings the operands of its algebra through shared memory (see Operands).
-  static constexpr bool STAGED = !GROUP && N <= 128;
+  // A column pass brings the operands of its algebra through shared memory (see Operands) in
+  // FP64 at n = 128, where the rows of a stage would hold up to 128 registers of a lane. At
+  // n = 64 (two values per lane) and in FP32 they fit into registers, and the shared room costs
+  // more than it hides. Measured per call, staged -> in registers: tangents of 20 Lawson-RK4
+  // steps, n = 64 FP64, batch 38 1.23 -> 1.13 ms; 24 steps of 32 states at n = 128 FP32, RK4
+  // 1.77 -> 1.57, Lawson-RK6 3.78 -> 3.17; over both types, batches 1 to 192: tangents 0 to 7%,
+  // cotangents 0 to 4% faster, state_vel at n = 64, batch 1 7.2 -> 7.3 us, batch 16 13.9 -> 9.6.
+  static constexpr bool STAGED = !GROUP && N == 128 && sizeof(R) == 8;
   __device__ static __forceinline__ int pos(int l, int j) {
     if constexpr (GROUP) return l + L * j;
     else return spec_pos<N>(l, j);
