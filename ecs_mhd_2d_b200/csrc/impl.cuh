@@ -562,11 +562,13 @@ struct Impl {
     return B >= minb && B <= hi && (c->chain_res8 > 0 || c->chain_res16 > 0);
   }
 
-  // The batch range of the fixed-step chains: two rounds of 16-warp clusters pay in FP32 at
-  // n = 128 (32 steps, launch per pass / chain: Lawson-RK4 batch 16 1.91 / 1.64 ms, 24
-  // 2.02 / 1.66, Lawson-RK6 24 4.63 / 3.35), not in FP64 (Lawson-RK4 24 2.44 / 2.79).
+  // The batch range of the fixed-step chains: two rounds of 16-warp clusters pay in FP32
+  // (n = 128, 32 steps, launch per pass / chain: Lawson-RK4 batch 16 1.91 / 1.64 ms, 24
+  // 2.02 / 1.66, Lawson-RK6 24 4.63 / 3.35; n = 64, 24 steps, batch 38 0.90 / 0.78, 64
+  // 1.24 / 0.78, Lawson-RK6 1.45 / 1.57, 2.42 / 1.58, TDRK4 0.83 / 0.82, 1.18 / 0.83), not in
+  // FP64 (n = 128, Lawson-RK4 24 2.44 / 2.79).
   static bool step_chain_batch(const ecs_ctx* c, int B) {
-    const int two = sizeof(R) == 4 && N == 128 ? 2 : 1;
+    const int two = sizeof(R) == 4 ? 2 : 1;
     return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb < 0 ? two * c->chain_res16 : c->rk4chain_maxb);
   }
 

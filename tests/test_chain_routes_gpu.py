@@ -75,3 +75,27 @@ def test_default_route(cuda, monkeypatch, call, n, B):
     off = {"ECS_CHAIN_MAXB": "0", "ECS_RK4CHAIN_MAXB": "0", "ECS_RK43CHAIN_MAXB": "0"}
     few, many = (_counted(monkeypatch, n, pd, run, env)[1] for env in ({}, off))
     assert 2 * few < many, (few, many)
+
+
+# FP32: more states than clusters that run at once on a B200, fewer than twice that
+@pytest.mark.parametrize("n,B", [(64, 48), (128, 24)])
+@pytest.mark.parametrize("mode", ["Lawson_RK4", "RK4", "Lawson_RK6", "TDRK4"])
+def test_two_rounds_in_fp32(cuda, monkeypatch, mode, n, B):
+    pd = E.make_param_dict(n, 1 / 40, 1 / 40, forcing="kolmogorov+", data_type=torch.float32)
+    f = np.fft.rfft2(np.stack([initial_condition(i, n) for i in range(B)]))
+    f = torch.as_tensor(f, device="cuda").to(torch.complex64)
+    out = []
+    for env in ({}, {"ECS_RK4CHAIN_MAXB": "0"}):
+        for k, v in env.items():
+            monkeypatch.setenv(k, v)
+        context.clear_cache()
+        try:
+            E.integrate(f, 0.02, 18, pd, mode)
+            ctx = context.get_context(pd, n, torch.float32)
+            before = ctx.lib.ecs_launch_count(ctx.handle)
+            got = E.integrate(f, 0.02, 18, pd, mode).cpu()
+            out.append((got, ctx.lib.ecs_launch_count(ctx.handle) - before))
+        finally:
+            monkeypatch.undo()
+            context.clear_cache()
+    assert torch.equal(out[0][0], out[1][0]) and 2 * out[0][1] < out[1][1], [q[1] for q in out]
