@@ -35,7 +35,6 @@ template <typename C, typename R> __device__ __forceinline__ C cscale(C a, R s) 
 template <typename C, typename R> __device__ __forceinline__ C cimul(C z, R mu) {
   C r; r.x = -mu * z.y; r.y = mu * z.x; return r;
 }
-template <typename C, typename R> __device__ __forceinline__ C cdiv_r(C a, R s) { a.x = a.x / s; a.y = a.y / s; return a; }
 
 // x / D for a positive integer constant D, correctly rounded, without a
 // division instruction.  A power of two is an exact multiplication.  Otherwise
@@ -154,12 +153,6 @@ __host__ __device__ __forceinline__ int pos_to_slot(int p, int n, int kmax, int 
 }
 __host__ __device__ __forceinline__ int slot_to_kx(int s, int kmax, int M) { return s <= kmax ? s : s - M; }
 __host__ __device__ __forceinline__ int pos_to_k(int p, int n) { return p <= n / 2 ? p : p - n; }
-
-template <int N> __device__ __forceinline__ int bitrev(int e) {
-  constexpr int B = (N == 64) ? 6 : (N == 128) ? 7 : (N == 256) ? 8 : (N == 32) ? 5 : 0;
-  static_assert(B > 0, "unsupported N");
-  return (int)(__brev((unsigned)e) >> (32 - B));
-}
 
 // Per-batch-element control block for the fixed-step and adaptive steppers.
 struct StepCtl {

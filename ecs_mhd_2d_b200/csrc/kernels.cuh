@@ -680,52 +680,28 @@ __device__ __forceinline__ void store_one(const cplx<typename X::R> (&W)[X::E], 
 }
 
 // The inverse transforms of a row's packed spectra in tile column w: fields (0, 1) to
-// a, (2, 3) to b (SINGLE: field 2 alone); one copy of the transform in the group layout.
+// a, (2, 3) to b (SINGLE: field 2 alone).
 template <int XT, bool SINGLE = false, class X>
 __device__ __forceinline__ void row_inverse(const cplx<typename X::R>* s_G, int w, const X& xf,
                                             cplx<typename X::R> (&a)[X::E], cplx<typename X::R> (&b)[X::E]) {
   constexpr int F = X::K * (XT + 1);
-  if constexpr (X::GROUP) {
-#pragma unroll 1
-    for (int i = 0; i < 2; ++i) {
-      if (SINGLE && i == 1) load_one<XT>(s_G + 2 * F, w, xf, b);
-      else load_pair<XT>(s_G + 2 * i * F, s_G + (2 * i + 1) * F, w, xf, b);
-      xf.template to_spec<true, true>(b);
-      if (i == 0) {
-#pragma unroll
-        for (int j = 0; j < X::E; ++j) a[j] = b[j];
-      }
-    }
-  } else {
-    load_pair<XT>(s_G, s_G + F, w, xf, a);
-    if (SINGLE) load_one<XT>(s_G + 2 * F, w, xf, b);
-    else load_pair<XT>(s_G + 2 * F, s_G + 3 * F, w, xf, b);
-    xf.template to_spec2<true>(a, b);
-  }
+  load_pair<XT>(s_G, s_G + F, w, xf, a);
+  if (SINGLE) load_one<XT>(s_G + 2 * F, w, xf, b);
+  else load_pair<XT>(s_G + 2 * F, s_G + 3 * F, w, xf, b);
+  xf.template to_spec2<true>(a, b);
   __syncwarp();
 }
 
 // The forward transforms of a row: the packed pair a to fields 0, 1 of tile column w, and
-// b to field 2 (one real field) or, PAIRS, to fields 2, 3.  a is overwritten.
+// b to field 2 (one real field) or, PAIRS, to fields 2, 3.
 template <int XT, bool PAIRS = false, class X>
 __device__ __forceinline__ void row_forward(cplx<typename X::R> (&a)[X::E], cplx<typename X::R> (&b)[X::E],
                                             cplx<typename X::R>* s_H, int w, const X& xf) {
   constexpr int F = X::K * (XT + 1);
-  if constexpr (X::GROUP) {
-#pragma unroll 1
-    for (int i = 0; i < 2; ++i) {
-      xf.template from_spec<false>(a);
-      if (PAIRS || i == 0) split_store<XT>(a, s_H + 2 * i * F, s_H + (2 * i + 1) * F, w, xf);
-      else store_one<XT>(a, s_H + 2 * F, w, xf);
-#pragma unroll
-      for (int j = 0; j < X::E; ++j) a[j] = b[j];
-    }
-  } else {
-    xf.template from_spec2<false>(a, b);
-    split_store<XT>(a, s_H, s_H + F, w, xf);
-    if (PAIRS) split_store<XT>(b, s_H + 2 * F, s_H + 3 * F, w, xf);
-    else store_one<XT>(b, s_H + 2 * F, w, xf);
-  }
+  xf.template from_spec2<false>(a, b);
+  split_store<XT>(a, s_H, s_H + F, w, xf);
+  if (PAIRS) split_store<XT>(b, s_H + 2 * F, s_H + 3 * F, w, xf);
+  else store_one<XT>(b, s_H + 2 * F, w, xf);
 }
 
 // The NH K rows of a row pass's H tile (pitch XT + 1, physical rows x0 ..
@@ -748,9 +724,6 @@ __device__ __forceinline__ void scatter_h_tile(const cplx<typename X::R>* s_H, c
     dst[(((c / CL) * G + ky % G) * 2 + (ADJ ? f & 1 : f == 2 ? 0 : f)) * N + x0 + xt] = s_H[rr * (XT + 1) + xt];
   }
 }
-
-// Threads that work on XT rows of one state.
-template <class X, int XT> __host__ __device__ constexpr int row_threads() { return XT * X::L; }
 
 // The products of one row in physical space.
 template <typename R>

@@ -399,7 +399,6 @@ struct FxChainParams {
   ColFxParams<R> col;
   RowParams<R> row;   // phys, phys_bstride: TDRK4
   long steps;
-  int last_produce;
   long rec_step;      // col.rec: entries from a step's record to the next step's
 };
 
@@ -481,8 +480,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_fx_chain(FxChainParams<R> P) {
       chain_rhs(P.col.H, id, xf, my_h, r);
       chain_fx_stage<SCHEME, X>(st, std::make_integer_sequence<int, fx_stages(SCHEME)>{}, h, coeff, id, xf, S,
                                 (const R*)e, forcing, rec, r, x);
-      if (!last || P.last_produce)
-        col_inverse_uv<W>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, last ? nullptr : s_gt);
+      if (!last) col_inverse_uv<W>(x, P.col.G, b, id.ch, id.ky, true, xf, mu, s_gt);
     }
   }
   __syncwarp();
