@@ -705,13 +705,13 @@ struct Impl {
   }
 
   // Whether a batch of B runs the other fixed-step modes through k_fx_chain: the range of
-  // the Lawson-RK4 chain, or, where only 8-warp clusters have the room, two rounds of them
-  // (Lawson-RK6 in FP64 at n = 128, 32 steps, launch per pass / chain: batch 8 4.31 / 3.83 ms,
-  // 14 4.79 / 3.85, 16 5.32 / 5.68).
+  // the Lawson-RK4 chain, or, where only 8-warp clusters have the room, one round of them
+  // (Lawson-RK6 in FP64 at n = 128, 48 steps, launch per pass / chain: batch 7 4.80 / 2.92 ms,
+  // 8 4.16 / 5.68, 10 4.46 / 5.68, 12 4.68 / 5.68, 14 6.84 / 5.71).
   static bool fx_chain_batch(const ecs_ctx* c, int scheme, int B) {
     if constexpr (N <= 128) {
       if (scheme == FX_RK6 && !fx_chain_fits<R, N, 16, FX_RK6>())
-        return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? 2 * c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
+        return B >= c->rk4chain_minb && B <= (c->rk4chain_maxb < 0 ? c->chain_res8 : c->rk4chain_maxb) && c->chain_res8 > 0;
       return step_chain_batch(c, B);
     }
     return false;
