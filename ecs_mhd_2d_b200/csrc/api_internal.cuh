@@ -14,7 +14,7 @@ struct ecs_ctx {
   ecs::Geom g{};
   double nu = 0, eta = 0, b0x = 0, b0y = 0;
   // tables
-  void* tw = nullptr;      // [N/2] twiddles
+  void* tw = nullptr;      // transform tables and multipliers (XfTable)
   void* fhat = nullptr;    // [K][M] forcing box spectrum (omega)
   // workspace, sized for max_batch
   void* F = nullptr;       // box state / accumulator
@@ -46,15 +46,16 @@ struct ecs_ctx {
   // k_rk4_chain for Lawson-RK4 stepping) run batches up to the number of
   // 16-warp clusters the device holds at once; batches up to the number of
   // 8-warp clusters (16 CTAs each at n = 128) use those.  Measured at n = 128
-  // FP64 (ms per JVP of T = 0.3, per 64 steps; launch per pass -> chain): batch 1
-  // 2.35 -> 2.00 and 2.12 -> 1.82, batch 8 3.89 -> 3.10 and 4.49 -> 2.87, batch 12
-  // 3.43 -> 3.11 and 4.71 -> 2.91; at batch 16 the launch-per-pass path is ahead
-  // (3.98 against 5.37, 3.91 against 5.11).  The adaptive solve has its own range
-  // (rk43_solve).
+  // FP64 (ms per JVP of T = 0.3, per 64 steps; launch per pass / chain): batch 1
+  // 2.92 / 2.97 and 1.69 / 1.78, batch 4 4.66 / 2.98 and 2.10 / 1.78, batch 8 5.20 / 4.72 and
+  // 2.44 / 2.82, batch 12 6.22 / 4.73 and 2.75 / 2.89, batch 14 (48 steps) 2.38 / 2.19; at
+  // batch 16 launches are ahead (5.90 / 8.17, 3.77 / 5.06).  A launch's time depends on how
+  // the waiting CTAs of its successor lie on the SMs and jumps with the batch, a chain's does
+  // not: one line for all lengths and modes.  The adaptive solve has its own range (rk43_solve).
   int chain_res8 = 0, chain_res16 = 0;   // clusters of each shape the device holds at once (set at creation)
   int chain_w = 0;                  // warps per CTA forced for the chains (ECS_CHAIN_WARPS=8 or 16; 0: by batch as above)
   int chain_dsh = 1;                // the 8-warp tangent chain keeps each column's tangent slots in shared memory (ECS_CHAIN_DSLOTS=0: global)
-  int chain_dsm = -1;               // G / H exchange: 1 distributed shared memory, 0 global memory of the tangent and Lawson-RK4 chains (ECS_CHAIN_DSMEM; -1: shared, 9% faster at n = 128: 2.20 -> 2.00 ms per batch-1 JVP of T = 0.3, 2.01 -> 1.82 ms per 64 steps)
+  int chain_dsm = -1;               // G / H exchange: 1 distributed shared memory, 0 global memory of the tangent and Lawson-RK4 chains (ECS_CHAIN_DSMEM; -1: shared, 9% faster at n = 128: 3.25 -> 2.99 ms per batch-1 JVP of T = 0.3, 1.96 -> 1.78 ms per 64 steps)
   int chain_minb = 1, chain_maxb = -1;         // batch range of the tangent chain (ECS_CHAIN_MINB / ECS_CHAIN_MAXB; -1: chain_res16; 0: off)
   int rk4chain_minb = 1, rk4chain_maxb = -1;   // batch range of the Lawson-RK4 chain (ECS_RK4CHAIN_MINB / ECS_RK4CHAIN_MAXB)
   int rk43chain_minb = 1, rk43chain_maxb = -1; // batch range of the adaptive Lawson-RK4(3) solve's chain (ECS_RK43CHAIN_MINB / _MAXB)

@@ -13,7 +13,7 @@
 // Intermediate layouts (per batch element):
 //   G[b][field][ky][x]   column-inverse-transformed fields (complex, x contiguous)
 //   H[b][field][ky][x]   row-forward-transformed fields      (complex, x contiguous)
-//   Phys[x][field][pos]  physical rows in warp-FFT position order (primal record)
+//   Phys[x][pair][e]  physical rows of the pairs (u, v), (B_x, B_y) (primal record; phys_row)
 #pragma once
 
 #include <cuda_runtime.h>

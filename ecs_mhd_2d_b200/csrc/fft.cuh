@@ -1,6 +1,7 @@
-// Transforms of length N in {64, 128, 256}, two layouts.
+// Transforms of length N in {64, 128, 256}, in two layouts (struct Xf below).
 //
-// FP32: one transform per warp.  Lane l holds E = N/32 complex values v[j] at
+// The warp layout, which every pass uses but the column passes of batched FP64 tangents
+// at N = 128: one transform per warp.  Lane l holds E = N/32 complex values v[j] at
 // "positions" e = l + 32*j.
 //
 //  * fft_dif : natural-order input  -> permuted output (lane l, register j holds X[spec_pos<N>(l, j)])
@@ -31,22 +32,15 @@
 // so that the lanes of a stage read consecutive entries, followed by the
 // radix-E pass's table s_tw[N + (k1-1)*32 + l] = W_N^{l k1}, k1 = 1..E-1.
 //
-// FP64 at N = 64 and 128: G = 32 / L transforms per warp, each on a group of L lanes
-// with E = N / L values per lane, natural order in and out (x[l + L j] in register
-// j).  Register passes with one exchange between them: at N = 64 (L = 8, E = 8)
-// radix 8, twiddles, the transposition of the values through the group's N-entry
-// shared buffer, radix 8; at N = 128 radix 16 (4 x 4), twiddles, transposition,
-// radix 8, either on 8 lanes of 16 values (the radix 16 in registers) or on 16 lanes
-// of 8 values (its last butterflies across lanes l, l + 8 after a half swap); the two
-// do the same operations in the same order and agree bit for bit.  The half-swap form above spends
-// most of its issue slots on selects and shuffles (a 128-point transform: 245
-// instructions per warp, 100 of them FP64); this form has few of either, 8 to 16
-// shared-memory accesses per lane and transform, and 83 to 92 FP64 instructions, so
-// that it runs at the FP64 and shared-memory rate of the SM instead of its issue
-// rate.  Measured, cycles per transform and SM at 16 warps: N = 128 93 -> 49 (8 lanes),
-// N = 64 47 -> 25; one warp alone takes 913 cycles for four transforms of 128 (1088
-// for two before).  The buffer is swizzled (entry (k, l) at k L + (l ^ (k mod L))):
-// eight lanes' 16-byte accesses fall on different banks in both directions.
+// The group layout (FP64 at N = 128): two transforms per warp, each on 16 lanes of 8
+// values (x[l + 16 j] in register j), natural order in and out: radix 16 (its last
+// butterflies across lanes l, l + 8 after a half swap), twiddles, the transposition of the
+// values through the group's N-entry shared buffer, radix 8.  The half-swap form above
+// spends most of its issue slots on selects and shuffles (a 128-point transform: 245
+// instructions per warp, 100 of them FP64); this form has few of either and 8 to 16
+// shared-memory accesses per lane and transform.  The buffer is swizzled (entry (k, l) of
+// output digit k at k 8 + (l ^ (k mod 8))): eight lanes' 16-byte accesses fall on different
+// banks in both directions.  What it gives per launch stands at with_layout.
 #pragma once
 
 #include "common.cuh"
@@ -293,12 +287,13 @@ __host__ __device__ inline void twiddle_image(const C* half, C* img) {
 template <typename R, bool INV>
 __device__ __forceinline__ cplx<R> mul_cs(cplx<R> a, R c, R s) { return cmul(a, mk<R>(c, INV ? s : -s)); }
 
-// N = 128 on 16 lanes: lane l holds x[l + 16 j'], that is x[a + 8 j] with a = l mod 8
-// and j = h + 2 j', h = l / 8, so that the butterflies (j, j + 4, j + 8, j + 12) of dft16's
-// first pass lie within a lane (j = h and h + 2), and so do the first sums of its second
-// pass (j = 0, 2 on lanes h = 0; 1, 3 on lanes h = 1); its last sums pair lanes l and l ^ 8,
-// which swap half their values for them.  The operations are dft16's, in its order.
-// Then the transposition hands lane k1 the eight values of its output digit.
+// The radix-16 pass of N = 128 on 16 lanes, as 4 x 4: lane l holds x[l + 16 j'], that is
+// x[a + 8 j] with a = l mod 8 and j = h + 2 j', h = l / 8.  First the radix-4 butterflies
+// over (j, j + 4, j + 8, j + 12), which lie within a lane (j = h and h + 2), then the
+// factors W_16^{j k}, then radix-4 butterflies over j mod 4: their first sums lie within a
+// lane too (j = 0, 2 on lanes h = 0; 1, 3 on lanes h = 1), and the last ones pair lanes l
+// and l ^ 8, which swap half their values for them.  Then the transposition hands lane k1
+// the eight values of its output digit.
 template <typename R, bool INV, bool ZMID>
 __device__ __forceinline__ void dft16_lanes(cplx<R> (&x)[8], int l) {
   const R c1 = R(0.92387953251128675612818318939678829), s1 = R(0.38268343236508977172845998403039887);

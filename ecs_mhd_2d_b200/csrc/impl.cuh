@@ -50,14 +50,17 @@ template <class F> Shape col_shape(int B) {
 inline int box_grid(int cols) { return (cols + COLWARPS - 1) / COLWARPS; }
 
 // Calls go(layout, its GROUP flag as a constant) for a tangent column pass of batch B:
-// the group layout (FP64 at n = 128) from 16 tangents on.  It needs 30% fewer
-// instructions per transform and holds half of a column's operands at a time in registers
-// instead of all in shared memory, but puts half as many warps on the same columns.
-// Measured per launch at batch 64, warp -> group: stage A 18.5 -> 15.1 us, C 32.3 -> 22.9,
-// D 22.5 -> 19.7, E and A 24.2 -> 20.9, B 17.3 -> 17.8; JVPs of T = 0.3, per-pass
-// launches: batch 4 4.1 -> 3.8 ms, 16 4.5 -> 4.0, 32 5.3 -> 4.5, 48 7.2 -> 6.7 (batch 1
-// 2.37 -> 2.48).  Below 16 the cluster-resident sweep runs (chain_batch), in the warp
-// layout; its results are those of the warp layout's passes bit for bit.
+// the group layout (FP64 at n = 128) from 16 tangents of one linearisation on.  It needs 30%
+// fewer instructions per transform and holds half of a column's operands at a time in
+// registers instead of all in shared memory, but puts half as many warps on the same columns.
+// Measured per launch at batch 64, warp -> group: stage A 18.5 -> 15.3 us, C 32.3 -> 22.6,
+// D 22.5 -> 19.7, E and A 24.2 -> 21.1, B 17.3 -> 17.7.  Whole JVPs launched per pass, warp /
+// group (ms; adaptive, T = 0.3; 64 Lawson-RK4 steps): batch 1 2.90 / 3.52, 2.25 / 2.83; 4
+// 4.61 / 3.69, 3.08 / 2.95; 12 6.27 / 4.67, 4.50 / 3.69; 16 6.70 / 5.96, 4.79 / 4.55; 64
+// 13.75 / 12.12, 9.81 / 8.98.  So the group layout is ahead from 4 on.  The line stands at 16
+// all the same: below it adaptive sweeps run as chains (chain_batch), which are in the warp
+// layout, and a tangent's bits then depend on its batch at one place only, above every
+// chain's range and at the smallest group of linearize_jvp's streams.
 template <typename R, int N, typename F> void with_layout(const ecs_ctx* c, int B, bool group_allowed, F&& go) {
   if constexpr (sizeof(R) == 8 && N == 128) {
     if (group_allowed && B >= c->group_minb) { go((Xf<R, N, true>*)nullptr, std::true_type{}); return; }
@@ -562,11 +565,11 @@ struct Impl {
     return B >= minb && B <= hi && (c->chain_res8 > 0 || c->chain_res16 > 0);
   }
 
-  // The batch range of the fixed-step chains: two rounds of 16-warp clusters pay in FP32
-  // (n = 128, 32 steps, launch per pass / chain: Lawson-RK4 batch 16 1.91 / 1.64 ms, 24
-  // 2.02 / 1.66, Lawson-RK6 24 4.63 / 3.35; n = 64, 24 steps, batch 38 0.90 / 0.78, 64
-  // 1.24 / 0.78, Lawson-RK6 1.45 / 1.57, 2.42 / 1.58, TDRK4 0.83 / 0.82, 1.18 / 0.83), not in
-  // FP64 (n = 128, Lawson-RK4 24 2.44 / 2.79).
+  // The batch range of the fixed-step chains: two rounds of 16-warp clusters pay in FP32 over
+  // the range (n = 128, 48 steps, launch per pass / chain: Lawson-RK4 batch 16 1.90 / 2.44 ms,
+  // 18 2.38 / 2.44, 24 2.97 / 2.47, Lawson-RK6 3.86 / 4.92, 5.49 / 4.94, 5.84 / 5.00; n = 64,
+  // 24 steps, batch 38 0.90 / 0.78, 64 1.24 / 0.78, Lawson-RK6 1.45 / 1.57, 2.42 / 1.58, TDRK4
+  // 0.83 / 0.82, 1.18 / 0.83), not in FP64 (n = 128, 32 steps, Lawson-RK4 24 2.49 / 2.86).
   static bool step_chain_batch(const ecs_ctx* c, int B) {
     const int two = sizeof(R) == 4 ? 2 : 1;
     return chain_batch(c, B, c->rk4chain_minb, c->rk4chain_maxb < 0 ? two * c->chain_res16 : c->rk4chain_maxb);
@@ -650,8 +653,8 @@ struct Impl {
 
   // Whether B cotangents of Lawson-RK4 steps run through k_adj_chain: the range of the
   // Lawson-RK4 chain, or, where only 8-warp clusters have the room, one round of them
-  // (FP64 at n = 128, 64 steps, launch per pass / chain: batch 7 4.23 / 2.29 ms, 8
-  // 4.05 / 4.24, 14 4.62 / 4.34).
+  // (FP64 at n = 128, 64 steps, launch per pass / chain: batch 1 2.40 / 2.33 ms, 7 3.47 / 2.35,
+  // 8 3.48 / 4.30, 14 4.40 / 4.38; n = 64, batch 33 3.37 / 1.92).
   static bool adj_chain_batch(const ecs_ctx* c, int B) {
     if constexpr (N <= 128) {
       if (!adj_chain_fits<R, N, 16>())
@@ -684,9 +687,10 @@ struct Impl {
   }
 
   // Whether B tangents of TDRK4 steps run through k_tdj_chain: the Lawson-RK4 chain's range,
-  // or two rounds of 8-warp clusters where only they have the room (FP64 at n = 128, 64 steps,
-  // launch per pass / chain: batch 8 4.51 / 4.31 ms, 14 4.79 / 4.29).  td_chain calls go(warps
-  // per CTA as a constant).
+  // or two rounds of 8-warp clusters where only they have the room (FP64 at n = 128, 48 steps,
+  // launch per pass / chain: batch 7 2.89 / 1.81 ms, 8 2.93 / 3.33, 9 3.22 / 3.31, 10
+  // 3.35 / 3.31, 14 3.67 / 3.32, 15 3.72 / 4.80).  td_chain calls go(warps per CTA as a
+  // constant).
   static bool td_chain_batch(const ecs_ctx* c, int B) {
     if constexpr (N <= 128) {
       if (!td_chain_fits<R, N, 16>())
@@ -879,10 +883,10 @@ struct Impl {
     // Candidates take different numbers of attempts, so a second round of clusters starts
     // as the first ones finish: 8-warp clusters pay up to 1.75 times those that run at
     // once, 16-warp ones up to twice.  Measured, 8 warps / 16 warps / launch per pass
-    // (ms, T = 0.2, atol 1e-8): n = 64, batch 1 1.03 / 1.49 / 1.73, 24 2.34 / 2.74 / 4.51,
-    // 32 3.16 / 2.76 / 4.96, 64 4.80 / 3.81 / 5.40; n = 128, batch 1 1.45 / 2.13 / 1.87,
-    // 12 4.13 / 5.12 / 7.43, 16 5.45 / 5.17 / 7.36, 24 7.30 / 6.10 / 7.77,
-    // 32 9.29 / 8.21 / 7.94.
+    // (ms, T = 0.2, atol 1e-8): n = 64, batch 1 1.37 / 2.03 / 2.66, 24 2.31 / 2.25 / 3.65,
+    // 32 2.65 / 2.26 / 3.93, 64 4.80 / 3.75 / 4.74; n = 128, batch 1 1.94 / 2.96 / 2.50,
+    // 12 4.68 / 4.73 / 5.64, 16 5.37 / 5.41 / 6.44, 24 7.13 / 6.39 / 7.01,
+    // 28 - / 6.54 / 7.15, 32 9.47 / 8.72 / 7.39.
     const int res8 = c->chain_res8 + 3 * c->chain_res8 / 4, res16 = 2 * c->chain_res16;
     if (launch && chain_batch(c, B, c->rk43chain_minb, c->rk43chain_maxb < 0 ? res16 : c->rk43chain_maxb)) {
       // the attempts as one cluster-resident launch, no host round trip (k_rk43_chain)

@@ -19,13 +19,13 @@
 // instead of 10.
 //
 //   column pass (one transform group per (batch, ky, channel), x contiguous; a
-//   group is a warp in FP32 and 8 or 16 lanes in FP64, see fft.cuh):
+//   group is a warp, or 16 lanes in the group layout, see fft.cuh):
 //     [forward FFTs along x of the product rows of the previous RHS: P1, P2
 //      (channel w) or P3 (channel j)]
 //     -> spectral epilogue (multipliers, dealias mask, forcing, stepper stage algebra)
 //     -> stage input -> the two uncurling multipliers i ky/k^2, -i kx/k^2
 //        -> 2 inverse FFTs along x -> G (u, v or B_x, B_y)
-//   row pass (one group per physical row x, CTA = XT rows staged in shared memory):
+//   row pass (one warp per physical row x, CTA = XT rows staged in shared memory):
 //     4 half-spectra rows of G -> 2 complex inverse FFTs (two real fields
 //     packed per transform) -> P1, P2, P3 -> 2 forward FFTs -> split -> H
 //

@@ -390,9 +390,9 @@ __global__ void __launch_bounds__(W * 32, 1) k_rk4_chain(Rk4ChainParams<R> P) {
 // column stay in shared memory.  The passes are k_row_rhs's (k_row_tan's for TDRK4's
 // Jacobian-vector products, on the physical fields that the row's own warp left in
 // row.phys the pass before) and k_col_fx's.  The stage input of the first stage is in G.
-// Measured, 32 steps, launch per pass -> this: n = 128, batch 1 Lawson-RK6 2.75 -> 1.97 ms,
-// RK4 1.35 -> 0.93, TDRK4 1.36 -> 0.98; batch 12 5.27 -> 3.83, 2.38 -> 1.44, 2.22 -> 1.56;
-// n = 64, batch 8 2.41 -> 1.10, 1.09 -> 0.54, 1.09 -> 0.57.
+// Measured, 32 steps, launch per pass -> this: n = 128, batch 1 Lawson-RK6 2.85 -> 1.98 ms,
+// RK4 1.38 -> 0.95, TDRK4 1.38 -> 1.00; batch 7 Lawson-RK6 3.36 -> 1.99; n = 64, batch 8
+// 1.78 -> 1.11, 0.87 -> 0.56, 0.86 -> 0.58, batch 24 2.69 -> 1.67, 1.26 -> 0.80, 1.20 -> 0.84.
 // ---------------------------------------------------------------------------
 template <typename R>
 struct FxChainParams {
@@ -498,7 +498,7 @@ __global__ void __launch_bounds__(W * 32, 1) k_fx_chain(FxChainParams<R> P) {
 // global G (an AJ_PRE pass, or the launch before), and the last column pass writes it if
 // a step precedes.
 // Measured, transpose products of 64 steps, launch per pass -> this: n = 64, batch 1
-// 1.81 -> 1.30 ms, batch 8 2.72 -> 1.30; n = 128, batch 1 2.94 -> 2.27, batch 7 4.23 -> 2.29.
+// 1.75 -> 1.37 ms, batch 8 1.94 -> 1.37; n = 128, batch 1 2.40 -> 2.33, batch 7 3.47 -> 2.35.
 // ---------------------------------------------------------------------------
 template <typename R>
 struct AdjChainParams {
@@ -613,8 +613,8 @@ __global__ void __launch_bounds__(W * 32, 1) k_adj_chain(AdjChainParams<R> P) {
 // launch, with the layout of k_rk4_chain.  The tiles of df and of dk1 / dk2 lie beside each
 // other; the H tile of a single row pass takes the second's place, that of a dual one the
 // first's.  The first row pass reads global Ga and the last column pass writes it.
-// Measured, tangents of 64 steps, launch per pass -> this: n = 64, batch 1 1.91 -> 1.33 ms,
-// batch 12 3.23 -> 1.32; n = 128, batch 1 3.13 -> 2.32, batch 7 4.68 -> 2.30.
+// Measured, tangents of 64 steps, launch per pass -> this: n = 64, batch 1 1.96 -> 1.40 ms,
+// batch 12 2.22 -> 1.39; n = 128, batch 1 2.74 -> 2.36, batch 7 3.77 -> 2.33.
 // ---------------------------------------------------------------------------
 template <typename R>
 struct TdChainParams {
