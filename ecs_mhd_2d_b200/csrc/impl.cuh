@@ -71,9 +71,9 @@ template <typename R, int N, typename F> void with_layout(const ecs_ctx* c, int 
 // Launch a stepping kernel of batch B; with c->pdl set, with programmatic
 // stream serialization (the kernel waits on its predecessor itself, see
 // pdl_wait), so that a kernel's launch and prologue overlap its predecessor's
-// tail.  Measured at n=128 FP64: the batch-64 tangent kernels gain 5-7%, and
-// single-state chains inside CUDA graphs gain 10-24% (gradient, plain JVP,
-// Lawson-RK4), except the pipelined linearisation's primal (see below).
+// tail.  Measured at n = 128 FP64, plain order -> this: an adaptive JVP of 64 tangents
+// (T = 0.3) 14.1 -> 12.1 ms, 48 steps of one state launched per pass in Lawson-RK6
+// 3.84 -> 2.80, RK4 1.85 -> 1.30.
 template <typename... P, typename... A>
 inline void launch_step(ecs_ctx* c, int B, void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                         A... args) {
@@ -111,15 +111,20 @@ inline void launch_cluster(ecs_ctx* c, int B, int cl, void (*k)(P...), dim3 grid
   cudaLaunchKernelEx(&cfg, k, args...);
 }
 
-// Scope in which batches below 8 launch without programmatic dependent launch:
-// the adaptive Lawson-RK4(3) solve and the fixed-step integrations measured
-// 5-10% slower with it at batch 1, and the batch-1 primal that runs beside the
-// tangent batch (pipelined linearisation) would park early-launched CTAs on
-// SMs that the tangents need.  Graphs captured inside the scope keep it.
+// Scope in which batches below 8 launch without programmatic dependent launch if `on`. The
+// adaptive Lawson-RK4(3) solve, the fixed-step integrations and the batch-1 primal that runs
+// beside a tangent batch (pipelined linearisation) take it at n = 256, where a state's launches
+// fill the SMs and waiting CTAs of the next take room from them.  Measured in FP64, plain order /
+// programmatic (ms; adaptive solve T = 0.1, 48 steps of Lawson-RK6, of RK4): n = 256, batch 1
+// 2.61 / 2.78, 5.73 / 5.97, 2.74 / 2.84, batch 4 3.20 / 3.61, 7.75 / 8.82, 3.53 / 4.12; n = 128,
+// batch 1 1.35 / 1.15, 3.84 / 2.80, 1.85 / 1.30, batch 4 1.43 / 1.40, 4.05 / 3.41, 1.93 / 1.60;
+// linearisation with 16 and 64 tangents (adaptive, T = 0.5) at n = 128 13.3 / 11.9 and
+// 19.8 / 19.4, at n = 64 8.3 / 7.7 and 12.0 / 11.1.  Graphs captured inside the scope keep it.
 struct PlainOrder {
   ecs_ctx* c;
-  explicit PlainOrder(ecs_ctx* c_) : c(c_) { ++c->plain_order; }
-  ~PlainOrder() { --c->plain_order; }
+  int on;
+  PlainOrder(ecs_ctx* c_, bool on_) : c(c_), on(on_) { c->plain_order += on; }
+  ~PlainOrder() { c->plain_order -= on; }
   PlainOrder(const PlainOrder&) = delete;
   PlainOrder& operator=(const PlainOrder&) = delete;
 };
@@ -754,7 +759,7 @@ struct Impl {
   // Fixed-step RK4 / Lawson-RK6 / TDRK4 over `steps` steps from slot X_F of S43
   // (h and e from fx_setup): one cluster-resident launch, or 16-step CUDA graphs per scheme.
   static int integrate_fx(ecs_ctx* c, int scheme, int B, long steps, cudaStream_t s) {
-    PlainOrder plain_order(c);
+    PlainOrder plain_order(c, N > 128);
     if (steps <= 0) return ECS_OK;
     constexpr int GS = 16;
     R* phys = nullptr;
@@ -873,7 +878,7 @@ struct Impl {
   static int rk43_solve(ecs_ctx* c, const ecs_shoot_cfg* cfg, const double* T, int B, cudaStream_t s,
                         cplx<R>* rec = nullptr, double* rec_h = nullptr, int* rec_acc = nullptr, int cap = 0,
                         bool launch = true) {
-    PlainOrder plain_order(c);
+    PlainOrder plain_order(c, N > 128);
     const long amax = (long)cfg->checkpoints * cfg->max_steps_per_checkpoint;
     if (amax <= 0) return set_err(c, ECS_ERR_INVALID, "checkpoints * max_steps_per_checkpoint must be > 0");
     ++c->launches; k_rk43_setup<<<(B + 127) / 128, 128, 0, s>>>(T, cfg->h0, c->ctl, B);
@@ -889,7 +894,10 @@ struct Impl {
     // 28 - / 6.54 / 7.15, 32 9.47 / 8.72 / 7.39.
     const int res8 = c->chain_res8 + 3 * c->chain_res8 / 4, res16 = 2 * c->chain_res16;
     if (launch && chain_batch(c, B, c->rk43chain_minb, c->rk43chain_maxb < 0 ? res16 : c->rk43chain_maxb)) {
-      // the attempts as one cluster-resident launch, no host round trip (k_rk43_chain)
+      // the attempts as one cluster-resident launch, no host round trip (k_rk43_chain); below
+      // batch 8 in plain order, as a cluster that is placed while the passes before it still
+      // run takes 2% longer (n = 128, T = 0.5: 4.85 ms against 4.76)
+      PlainOrder plain_chain(c, true);
       if constexpr (N <= 128) {
         Rk43ChainParams<R> P{};
         Col43Params<R>& q = P.col;
@@ -1277,7 +1285,7 @@ struct Impl {
     int st = lin_prologue(c, cfg, fields, T, sx, s);
     if (!st) st = grow(c, &L.rec, &L.rec_bytes, (size_t)steps * NR * vb);
     if (st) return st;
-    PlainOrder plain_order(c);
+    PlainOrder plain_order(c, N > 128);
     cudaMemcpyAsync((cplx<R>*)c->S43 + X_F * VEC, L.f0box, vb, cudaMemcpyDeviceToDevice, s);
     ++c->launches;
     k_fx_setup<R><<<grid1d((long)VEC), 256, 0, s>>>(T, cfg->num_checkpoints, cfg->ministeps, 6, c->ctl, (R*)c->Etab, N,
@@ -1818,7 +1826,7 @@ struct Impl {
     auto primal_chunk = [&](long k) -> cudaError_t {
       void* const Gs = c->G; void* const Hs = c->H;
       c->G = c->Gp; c->H = c->Hp;
-      PlainOrder plain_order(c);
+      PlainOrder plain_order(c, N > 128);
       if (k == 0) launch_col_rk4<R, N>(c, 1, COL_START, 1, 0, ps);
       for (long it = k * CS; it < std::min(steps, (k + 1) * CS); ++it) {
         cplx<R>* rs = rec + (size_t)it * Q_NREC * VEC;
